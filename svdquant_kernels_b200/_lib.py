@@ -53,6 +53,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
 
 
 class SvdqLibraryError(RuntimeError):
@@ -79,6 +80,22 @@ def load() -> ctypes.CDLL:
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+def host():
+    """Load (once) the native host path of the operators; raise if it is not there."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise SvdqLibraryError(f"{_PKG_DIR}/_host.so is missing or does not fit this torch ({e}). Build it with "
+                                   "`python -m svdquant_kernels_b200.build`.") from e
+        from . import ops
+        module.bind(ops._SPLIT_WS, ops._quantize_checked, ops._gemm_checked)
+        _host = module
+    return _host
 
 
 def status_string(code: int) -> str:

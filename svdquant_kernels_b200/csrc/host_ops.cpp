@@ -1,0 +1,463 @@
+// Host path of the operators: contract checks, output allocation, lookup of the layout twins and the
+// launch, in one native call per operator, for the Python operators (ops.py) and for the dispatcher
+// (torch.ops.svdq_b200.*).
+//
+// A layer of a few hundred rows keeps the GPU busy for some 15-20 us, so the host's part decides how fast
+// such layers can follow each other.  In Python it took 20 us per operator (about 60 interpreter-level
+// calls: assertions, tensor attributes, five torch.empty, ctypes conversions) and the registered ops
+// another 20 us in torch.library's Python wrappers; here an operator takes a few microseconds.
+//
+// Only calls that need nothing but a launch are taken: plain contiguous CUDA tensors on the current
+// device that meet every condition of the contract and whose twins exist.  For anything else (first use
+// of a weight, strided inputs, a shape that breaks the contract, tensor subclasses) the functions return
+// None and the Python operator, which owns the checks and their messages, does the call.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/Storage.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/library.h>
+
+#include "../../include/svdq_b200.h"
+
+namespace {
+
+using at::ScalarType;
+using at::Tensor;
+
+PyObject* g_twins_name = nullptr;     // interned "_svdq_twins": attribute of a storage object, see ops._attach
+PyObject* g_split_ws = nullptr;       // ops._SPLIT_WS: {(device, stream): workspace}
+PyObject* g_py_quantize = nullptr;    // the Python operators behind the dispatcher, for calls not taken here
+PyObject* g_py_gemm = nullptr;
+
+int dtype_code(ScalarType t) {
+  return t == at::kHalf ? SVDQ_DTYPE_F16 : t == at::kBFloat16 ? SVDQ_DTYPE_BF16 : t == at::kFloat ? SVDQ_DTYPE_F32 : -1;
+}
+
+struct GilAcquire {
+  PyGILState_STATE st = PyGILState_Ensure();
+  ~GilAcquire() { PyGILState_Release(st); }
+};
+struct GilRelease {
+  PyThreadState* st = PyEval_SaveThread();
+  ~GilRelease() { PyEval_RestoreThread(st); }
+};
+struct Ref {                            // owned reference
+  PyObject* p;
+  explicit Ref(PyObject* o) : p(o) {}
+  Ref(const Ref&) = delete;
+  ~Ref() { Py_XDECREF(p); }
+};
+
+// The twin recorded for `owner` on its storage object (the records ops._attach keeps: {(offset, numel):
+// (twin, version)}); an undefined tensor if there is none or it is out of date.  GIL held.
+Tensor attached(const Tensor& owner, bool any_version = false) {
+  Ref st(THPStorage_Wrap(owner.storage()));
+  if (st.p == nullptr) { PyErr_Clear(); return Tensor(); }
+  Ref recs(PyObject_GetAttr(st.p, g_twins_name));
+  if (recs.p == nullptr) { PyErr_Clear(); return Tensor(); }
+  if (!PyDict_Check(recs.p)) return Tensor();
+  Ref key(Py_BuildValue("(LL)", static_cast<long long>(owner.storage_offset()), static_cast<long long>(owner.numel())));
+  PyObject* rec = key.p != nullptr ? PyDict_GetItemWithError(recs.p, key.p) : nullptr;     // borrowed
+  if (rec == nullptr || !PyTuple_Check(rec) || PyTuple_GET_SIZE(rec) != 2) { PyErr_Clear(); return Tensor(); }
+  if (!any_version && PyLong_AsLong(PyTuple_GET_ITEM(rec, 1)) != static_cast<long>(owner._version())) return Tensor();
+  PyObject* twin = PyTuple_GET_ITEM(rec, 0);
+  return THPVariable_Check(twin) ? THPVariable_Unpack(twin) : Tensor();
+}
+
+// Record `twin` as the derived form of `owner`'s current contents.  GIL held; false with a Python error set.
+bool attach(const Tensor& owner, const Tensor& twin) {
+  Ref st(THPStorage_Wrap(owner.storage()));
+  if (st.p == nullptr) return false;
+  PyObject* recs = PyObject_GetAttr(st.p, g_twins_name);
+  if (recs == nullptr) {
+    PyErr_Clear();
+    recs = PyDict_New();
+    if (recs == nullptr || PyObject_SetAttr(st.p, g_twins_name, recs) != 0) { Py_XDECREF(recs); return false; }
+  }
+  Ref hold(recs);
+  Ref key(Py_BuildValue("(LL)", static_cast<long long>(owner.storage_offset()), static_cast<long long>(owner.numel())));
+  Ref wrapped(THPVariable_Wrap(twin));
+  if (key.p == nullptr || wrapped.p == nullptr) return false;
+  Ref rec(Py_BuildValue("(Ol)", wrapped.p, static_cast<long>(owner._version())));
+  return rec.p != nullptr && PyDict_SetItem(recs, key.p, rec.p) == 0;
+}
+
+// A tensor the kernels can take as it is: on the current device, contiguous, no subclass behaviour, and
+// with a version counter (inference tensors have none, so no twin can be tied to their contents).
+bool plain(const Tensor& t, c10::DeviceIndex dev) {
+  return t.defined() && t.is_cuda() && t.device().index() == dev && t.is_contiguous() && !t.is_inference() &&
+         t.layout() == at::kStrided && !t.is_conj() && !t.is_neg();
+}
+
+Tensor empty(at::IntArrayRef sizes, ScalarType t, c10::DeviceIndex dev) {
+  return Tensor(at::detail::empty_cuda(sizes, t, c10::Device(c10::kCUDA, dev), std::nullopt));
+}
+
+void throw_status(const char* what, int rc) {
+  throw std::runtime_error(std::string(what) + ": svdq status " + std::to_string(rc) + " (" + svdq_status_string(rc) + ")");
+}
+
+bool int_sized(int64_t v) { return v >= 0 && v <= INT32_MAX; }
+
+struct Quantized {
+  Tensor act, ascales, lora_act;
+};
+
+// GIL held.  False: not taken.
+bool quantize(const Tensor& x, const Tensor& ld, const Tensor& smooth, int64_t pad, const Quantized* into, Quantized& out) {
+  if (!x.is_cuda()) return false;
+  const c10::DeviceIndex dev = c10::cuda::current_device();
+  if (!plain(x, dev) || !plain(ld, dev) || x.dim() != 2 || ld.dim() != 2) return false;
+  const ScalarType t = x.scalar_type();
+  if ((t != at::kHalf && t != at::kBFloat16) || ld.scalar_type() != t) return false;
+  const int64_t M = x.size(0), K = x.size(1), R = ld.size(1);
+  if (ld.size(0) != K || K % 16 != 0 || K == 0 || M == 0 || pad < 1) return false;
+  const int64_t Mp = (M + pad - 1) / pad * pad;
+  if (!int_sized(Mp) || !int_sized(K) || !int_sized(R)) return false;
+  Tensor table;
+  if (smooth.defined()) {
+    if (!plain(smooth, dev) || smooth.dim() != 1 || smooth.size(0) != K || smooth.scalar_type() != t) return false;
+    table = attached(smooth);
+    if (!table.defined()) return false;
+  }
+  const bool want_swz = Mp % 128 == 0 && K % 64 == 0;
+  Tensor swz, la16;
+  if (into != nullptr) {
+    out = *into;
+    if (!plain(out.act, dev) || !plain(out.ascales, dev) || !plain(out.lora_act, dev)) return false;
+    if (out.act.scalar_type() != at::kByte || out.act.dim() != 2 || out.act.size(0) != Mp || out.act.size(1) != K / 2) return false;
+    if (out.ascales.scalar_type() != at::kFloat8_e4m3fn || out.ascales.dim() != 2 || out.ascales.size(0) != K / 16 ||
+        out.ascales.size(1) != Mp)
+      return false;
+    if (out.lora_act.scalar_type() != at::kFloat || out.lora_act.dim() != 2 || out.lora_act.size(0) != Mp || out.lora_act.size(1) != R)
+      return false;
+    swz = attached(out.ascales, true);
+    la16 = attached(out.lora_act, true);
+    if (la16.defined() && la16.scalar_type() != t) la16 = Tensor();
+  } else {
+    out.act = empty({Mp, K / 2}, at::kByte, dev);
+    out.ascales = empty({K / 16, Mp}, at::kFloat8_e4m3fn, dev);
+    out.lora_act = empty({Mp, R}, at::kFloat, dev);
+  }
+  if (want_swz && !swz.defined()) swz = empty({Mp * (K / 16)}, at::kByte, dev);
+  if (R > 0 && !la16.defined())
+    la16 = empty({svdq_lora_act16_elems(static_cast<int>(Mp), static_cast<int>(R), dtype_code(t))}, t, dev);
+  void* const stream = c10::cuda::getCurrentCUDAStream(dev).stream();
+  auto ptr = [](const Tensor& v) -> void* { return v.defined() && v.numel() > 0 ? v.data_ptr() : nullptr; };
+  int rc;
+  {
+    GilRelease nogil;
+    rc = svdq_quantize_w4a4_act_fuse_lora(ptr(x), ptr(ld), ptr(smooth), ptr(table), ptr(out.act), ptr(out.ascales),
+                                          static_cast<float*>(ptr(out.lora_act)), ptr(swz), ptr(la16), static_cast<int>(M),
+                                          static_cast<int>(K), static_cast<int>(R), static_cast<int>(Mp), dtype_code(t), 0, stream);
+  }
+  if (rc != SVDQ_OK) throw_status("quantize_w4a4_act_fuse_lora", rc);
+  if (swz.defined() && !attach(out.ascales, swz)) throw python_error();
+  if (la16.defined() && !attach(out.lora_act, la16)) throw python_error();
+  return true;
+}
+
+struct GemmArgs {
+  Tensor act, wgt, ascales, wscales, lora_act, lora_up, wcscales, bias, smooth_next, out;   // the last six may be undefined
+};
+struct GemmResult {
+  Tensor y, qout, oscales;                                                                  // the last two with smooth_next
+};
+
+// GIL held.  False: not taken.
+bool gemm(const GemmArgs& a, ScalarType out_t, GemmResult& r) {
+  if (!a.act.is_cuda()) return false;
+  const c10::DeviceIndex dev = c10::cuda::current_device();
+  if (out_t != at::kHalf && out_t != at::kBFloat16) return false;
+  if (!plain(a.act, dev) || !plain(a.wgt, dev) || !plain(a.ascales, dev) || !plain(a.wscales, dev)) return false;
+  if (a.act.scalar_type() != at::kByte || a.wgt.scalar_type() != at::kByte || a.act.dim() != 2 || a.wgt.dim() != 2) return false;
+  if (a.ascales.scalar_type() != at::kFloat8_e4m3fn || a.wscales.scalar_type() != at::kFloat8_e4m3fn) return false;
+  const int64_t M = a.act.size(0), K = a.act.size(1) * 2, N = a.wgt.size(0), G = K / 16;
+  if (a.wgt.size(1) * 2 != K || M == 0 || N == 0 || K == 0 || M % 128 != 0 || N % 128 != 0 || K % 64 != 0) return false;
+  if (!int_sized(M) || !int_sized(N) || !int_sized(K)) return false;
+  if (a.ascales.dim() != 2 || a.ascales.size(0) != G || a.ascales.size(1) != M) return false;
+  if (a.wscales.dim() != 2 || a.wscales.size(0) != G || a.wscales.size(1) != N) return false;
+  if (a.lora_act.defined() != a.lora_up.defined()) return false;
+  int64_t R = 0;
+  Tensor la, lu, lu16;
+  if (a.lora_act.defined()) {
+    if (!plain(a.lora_act, dev) || !plain(a.lora_up, dev) || a.lora_act.dim() != 2 || a.lora_up.dim() != 2) return false;
+    R = a.lora_up.size(1);
+    if (a.lora_act.size(0) != M || a.lora_up.size(0) != N || a.lora_act.size(1) != R || R % 16 != 0 || !int_sized(R)) return false;
+    if (a.lora_up.scalar_type() != out_t) return false;
+    if (R > 0) {
+      la = attached(a.lora_act);
+      if (!la.defined() || la.scalar_type() != out_t) return false;
+      lu = a.lora_up;
+      if (out_t == at::kBFloat16) {
+        lu16 = attached(a.lora_up);
+        if (!lu16.defined()) return false;                   // recorded empty if a value does not fit fp16
+      }
+    }
+  }
+  for (const Tensor* v : {&a.wcscales, &a.bias, &a.smooth_next})
+    if (v->defined() && (!plain(*v, dev) || v->dim() != 1 || v->size(0) != N || v->scalar_type() != out_t)) return false;
+  const Tensor sa = attached(a.ascales), sw = attached(a.wscales);
+  if (!sa.defined() || !sw.defined()) return false;
+  if (a.out.defined()) {
+    if (!plain(a.out, dev) || a.out.dim() != 2 || a.out.size(0) != M || a.out.size(1) != N || a.out.scalar_type() != out_t) return false;
+    r.y = a.out;
+  }
+  void* const stream = c10::cuda::getCurrentCUDAStream(dev).stream();
+  const int m = static_cast<int>(M), n = static_cast<int>(N), k = static_cast<int>(K), rr = static_cast<int>(R), dt = dtype_code(out_t);
+  auto ptr = [](const Tensor& v) -> void* { return v.defined() && v.numel() > 0 ? v.data_ptr() : nullptr; };
+  if (a.smooth_next.defined()) {
+    if (!r.y.defined()) r.y = empty({M, N}, out_t, dev);
+    r.qout = empty({M, N / 2}, at::kByte, dev);
+    r.oscales = empty({N / 16, M}, at::kFloat8_e4m3fn, dev);
+    const Tensor oswz = empty({M * (N / 16)}, at::kByte, dev);
+    int rc;
+    {
+      GilRelease nogil;
+      rc = svdq_gemm_w4a4_next(ptr(a.act), ptr(a.wgt), ptr(sa), ptr(sw), ptr(la), ptr(lu), ptr(lu16), ptr(a.wcscales), ptr(a.bias),
+                               ptr(r.y), ptr(a.smooth_next), ptr(r.qout), ptr(r.oscales), ptr(oswz), m, n, k, rr, dt, 0, stream);
+    }
+    if (rc != SVDQ_OK) throw_status("gemm_w4a4_next", rc);
+    if (!attach(r.oscales, oswz)) throw python_error();
+    return true;
+  }
+  Tensor ws;                                                  // split-K: the workspace of this device and stream
+  const unsigned long long need = svdq_gemm_w4a4_workspace_bytes(m, n, k, rr);
+  if (need > 0) {
+    Ref key(Py_BuildValue("(iK)", static_cast<int>(dev), static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(stream))));
+    PyObject* w = key.p != nullptr ? PyDict_GetItemWithError(g_split_ws, key.p) : nullptr;
+    if (w == nullptr || !THPVariable_Check(w)) { PyErr_Clear(); return false; }            // made on the first call
+    ws = THPVariable_Unpack(w);
+    if (static_cast<unsigned long long>(ws.numel()) < need) return false;
+  }
+  if (!r.y.defined()) r.y = empty({M, N}, out_t, dev);
+  int rc;
+  {
+    GilRelease nogil;
+    rc = svdq_gemm_w4a4_ws(ptr(a.act), ptr(a.wgt), ptr(sa), ptr(sw), ptr(la), ptr(lu), ptr(lu16), ptr(a.wcscales), ptr(a.bias),
+                           ptr(r.y), m, n, k, rr, dt, 0, ptr(ws), ws.defined() ? static_cast<unsigned long long>(ws.numel()) : 0, stream);
+  }
+  if (rc != SVDQ_OK) throw_status("gemm_w4a4", rc);
+  return true;
+}
+
+// ---------------------------------------------------------------------------
+// Python entry points
+// ---------------------------------------------------------------------------
+// None -> undefined tensor; a tensor subclass or anything else -> false
+bool unpack(PyObject* o, Tensor& t, bool optional) {
+  if (o == Py_None) { t = Tensor(); return optional; }
+  if (!THPVariable_CheckExact(o)) return false;
+  t = THPVariable_Unpack(o);
+  return true;
+}
+
+PyObject* py_quantize(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 5) { PyErr_SetString(PyExc_TypeError, "quantize(input, lora_down, smooth, pad_size, out)"); return nullptr; }
+  Tensor x, ld, smooth;
+  if (!unpack(args[0], x, false) || !unpack(args[1], ld, false) || !unpack(args[2], smooth, true) || !PyLong_CheckExact(args[3]))
+    Py_RETURN_NONE;
+  int overflow = 0;
+  const long long pad = PyLong_AsLongLongAndOverflow(args[3], &overflow);
+  if (overflow != 0) Py_RETURN_NONE;
+  Quantized into, out;
+  const bool reuse = args[4] != Py_None;
+  if (reuse) {
+    if (!PyTuple_Check(args[4]) || PyTuple_GET_SIZE(args[4]) != 3 || !unpack(PyTuple_GET_ITEM(args[4], 0), into.act, false) ||
+        !unpack(PyTuple_GET_ITEM(args[4], 1), into.ascales, false) || !unpack(PyTuple_GET_ITEM(args[4], 2), into.lora_act, false))
+      Py_RETURN_NONE;
+  }
+  if (!quantize(x, ld, smooth, pad, reuse ? &into : nullptr, out)) Py_RETURN_NONE;
+  if (reuse) return Py_NewRef(args[4]);
+  Ref a(THPVariable_Wrap(std::move(out.act))), s(THPVariable_Wrap(std::move(out.ascales))), l(THPVariable_Wrap(std::move(out.lora_act)));
+  if (a.p == nullptr || s.p == nullptr || l.p == nullptr) return nullptr;
+  return PyTuple_Pack(3, a.p, s.p, l.p);
+  END_HANDLE_TH_ERRORS
+}
+
+PyObject* py_gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 11) {
+    PyErr_SetString(PyExc_TypeError, "gemm(act, wgt, ascales, wscales, lora_act, lora_up, wcscales, bias, out_dtype, smooth_next, out)");
+    return nullptr;
+  }
+  GemmArgs a;
+  if (!unpack(args[0], a.act, false) || !unpack(args[1], a.wgt, false) || !unpack(args[2], a.ascales, false) ||
+      !unpack(args[3], a.wscales, false) || !unpack(args[4], a.lora_act, true) || !unpack(args[5], a.lora_up, true) ||
+      !unpack(args[6], a.wcscales, true) || !unpack(args[7], a.bias, true) || !unpack(args[9], a.smooth_next, true) ||
+      !unpack(args[10], a.out, true))
+    Py_RETURN_NONE;
+  ScalarType t = a.lora_up.defined() ? a.lora_up.scalar_type() : at::kHalf;
+  if (args[8] != Py_None) {
+    if (!THPDtype_Check(args[8])) Py_RETURN_NONE;
+    t = reinterpret_cast<THPDtype*>(args[8])->scalar_type;
+  }
+  GemmResult r;
+  if (!gemm(a, t, r)) Py_RETURN_NONE;
+  PyObject* y = args[10] != Py_None ? Py_NewRef(args[10]) : THPVariable_Wrap(std::move(r.y));
+  if (!a.smooth_next.defined() || y == nullptr) return y;
+  Ref hold(y), q(THPVariable_Wrap(std::move(r.qout))), s(THPVariable_Wrap(std::move(r.oscales)));
+  if (q.p == nullptr || s.p == nullptr) return nullptr;
+  return PyTuple_Pack(3, y, q.p, s.p);
+  END_HANDLE_TH_ERRORS
+}
+
+PyObject* py_pack(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 2) { PyErr_SetString(PyExc_TypeError, "pack(x, pad_size)"); return nullptr; }
+  Tensor x;
+  if (!unpack(args[0], x, false) || !PyLong_CheckExact(args[1])) Py_RETURN_NONE;
+  int overflow = 0;
+  const long long pad = PyLong_AsLongLongAndOverflow(args[1], &overflow);
+  if (!x.is_cuda()) Py_RETURN_NONE;
+  const c10::DeviceIndex dev = c10::cuda::current_device();
+  if (overflow != 0 || pad < 1 || !plain(x, dev) || x.dim() != 2 || dtype_code(x.scalar_type()) < 0) Py_RETURN_NONE;
+  const int64_t rows = x.size(0), K = x.size(1);
+  if (rows == 0 || K == 0 || K % 16 != 0) Py_RETURN_NONE;
+  const int64_t rp = (rows + pad - 1) / pad * pad;
+  if (!int_sized(rp) || !int_sized(K)) Py_RETURN_NONE;
+  Tensor packed = empty({rp, K / 2}, at::kByte, dev), scales = empty({K / 16, rp}, at::kFloat8_e4m3fn, dev), swz;
+  if (rp % 128 == 0 && K % 64 == 0) swz = empty({rp * (K / 16)}, at::kByte, dev);
+  void* const stream = c10::cuda::getCurrentCUDAStream(dev).stream();
+  int rc;
+  {
+    GilRelease nogil;
+    rc = svdq_quantize_nvfp4_rows(x.data_ptr(), packed.data_ptr(), scales.data_ptr(), swz.defined() ? swz.data_ptr() : nullptr,
+                                  static_cast<int>(rows), static_cast<int>(rp), static_cast<int>(K), dtype_code(x.scalar_type()), stream);
+  }
+  if (rc != SVDQ_OK) throw_status("quantize_nvfp4_rows", rc);
+  if (swz.defined() && !attach(scales, swz)) throw python_error();
+  Ref p(THPVariable_Wrap(std::move(packed))), s(THPVariable_Wrap(std::move(scales)));
+  if (p.p == nullptr || s.p == nullptr) return nullptr;
+  return PyTuple_Pack(2, p.p, s.p);
+  END_HANDLE_TH_ERRORS
+}
+
+// bind(split_workspaces, quantize, gemm): the workspace table and the Python operators of ops.py
+PyObject* py_bind(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  if (nargs != 3 || !PyDict_Check(args[0])) { PyErr_SetString(PyExc_TypeError, "bind(split_workspaces, quantize, gemm)"); return nullptr; }
+  Py_XSETREF(g_split_ws, Py_NewRef(args[0]));
+  Py_XSETREF(g_py_quantize, Py_NewRef(args[1]));
+  Py_XSETREF(g_py_gemm, Py_NewRef(args[2]));
+  Py_RETURN_NONE;
+}
+
+// ---------------------------------------------------------------------------
+// dispatcher (torch.ops.svdq_b200.*)
+// ---------------------------------------------------------------------------
+using OptTensor = std::optional<Tensor>;
+
+Tensor value(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
+PyObject* wrap(const Tensor& t) { return t.defined() ? THPVariable_Wrap(t) : Py_NewRef(Py_None); }
+Tensor take(PyObject* o) {
+  TORCH_CHECK(o != nullptr && THPVariable_Check(o), "svdq_b200: the Python operator returned something else than tensors");
+  return THPVariable_Unpack(o);
+}
+
+std::tuple<Tensor, Tensor, Tensor> op_quantize(const Tensor& x, const Tensor& ld, const OptTensor& smooth, int64_t pad) {
+  GilAcquire gil;
+  TORCH_CHECK(g_py_quantize != nullptr, "svdq_b200: import svdquant_kernels_b200.torch_ops first");
+  Quantized q;
+  if (quantize(x, ld, value(smooth), pad, nullptr, q)) return {q.act, q.ascales, q.lora_act};
+  Ref args(Py_BuildValue("(NNN)", wrap(x), wrap(ld), wrap(value(smooth))));
+  Ref kw(Py_BuildValue("{s:L}", "pad_size", static_cast<long long>(pad)));
+  if (args.p == nullptr || kw.p == nullptr) throw python_error();
+  Ref res(PyObject_Call(g_py_quantize, args.p, kw.p));
+  if (res.p == nullptr) throw python_error();
+  TORCH_CHECK(PyTuple_Check(res.p) && PyTuple_GET_SIZE(res.p) == 3);
+  return {take(PyTuple_GET_ITEM(res.p, 0)), take(PyTuple_GET_ITEM(res.p, 1)), take(PyTuple_GET_ITEM(res.p, 2))};
+}
+
+Tensor op_gemm(const Tensor& act, const Tensor& wgt, const Tensor& ascales, const Tensor& wscales, const OptTensor& lora_act,
+               const OptTensor& lora_up, const OptTensor& wcscales, const OptTensor& bias, std::optional<ScalarType> out_dtype) {
+  GilAcquire gil;
+  TORCH_CHECK(g_py_gemm != nullptr, "svdq_b200: import svdquant_kernels_b200.torch_ops first");
+  GemmArgs a{act, wgt, ascales, wscales, value(lora_act), value(lora_up), value(wcscales), value(bias), Tensor(), Tensor()};
+  const ScalarType t = out_dtype.has_value() ? *out_dtype : a.lora_up.defined() ? a.lora_up.scalar_type() : at::kHalf;
+  GemmResult r;
+  if (gemm(a, t, r)) return r.y;
+  PyObject* dt = Py_None;
+  if (out_dtype.has_value()) dt = reinterpret_cast<PyObject*>(torch::getTHPDtype(*out_dtype));
+  Ref args(Py_BuildValue("(NNNNNNNNO)", wrap(act), wrap(wgt), wrap(ascales), wrap(wscales), wrap(a.lora_act), wrap(a.lora_up),
+                         wrap(a.wcscales), wrap(a.bias), dt));
+  if (args.p == nullptr) throw python_error();
+  Ref res(PyObject_Call(g_py_gemm, args.p, nullptr));
+  if (res.p == nullptr) throw python_error();
+  return take(res.p);
+}
+
+// The operators have no backward pass: results of inputs that require a gradient carry a node that says so
+// when it is reached.
+template <typename... In>
+std::shared_ptr<torch::autograd::Node> no_backward(const char* name, const In&... in) {
+  if (!torch::autograd::compute_requires_grad(in...)) return nullptr;
+  auto node = std::make_shared<torch::autograd::NotImplemented>(name);
+  node->set_next_edges(torch::autograd::collect_next_edges(in...));
+  return node;
+}
+
+// (Called through the dispatcher again, so that tracing and fake tensors, which sit below autograd, are seen.)
+using QuantizeSig = std::tuple<Tensor, Tensor, Tensor>(const Tensor&, const Tensor&, const OptTensor&, c10::SymInt);
+using GemmSig = Tensor(const Tensor&, const Tensor&, const Tensor&, const Tensor&, const OptTensor&, const OptTensor&,
+                       const OptTensor&, const OptTensor&, std::optional<ScalarType>);
+
+std::tuple<Tensor, Tensor, Tensor> op_quantize_autograd(const Tensor& x, const Tensor& ld, const OptTensor& smooth, c10::SymInt pad) {
+  static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("svdq_b200::quantize_w4a4_act_fuse_lora", "").typed<QuantizeSig>();
+  const auto node = no_backward("svdq_b200::quantize_w4a4_act_fuse_lora", x, ld, value(smooth));
+  at::AutoDispatchBelowADInplaceOrView below;
+  auto r = op.call(x, ld, smooth, std::move(pad));
+  if (node) {                                                 // the integer codes are not differentiable
+    torch::autograd::set_history(std::get<1>(r), node);
+    torch::autograd::set_history(std::get<2>(r), node);
+  }
+  return r;
+}
+
+Tensor op_gemm_autograd(const Tensor& act, const Tensor& wgt, const Tensor& ascales, const Tensor& wscales, const OptTensor& lora_act,
+                        const OptTensor& lora_up, const OptTensor& wcscales, const OptTensor& bias, std::optional<ScalarType> out_dtype) {
+  static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("svdq_b200::gemm_w4a4", "").typed<GemmSig>();
+  const auto node = no_backward("svdq_b200::gemm_w4a4", act, wgt, ascales, wscales, value(lora_act), value(lora_up), value(wcscales), value(bias));
+  at::AutoDispatchBelowADInplaceOrView below;
+  Tensor y = op.call(act, wgt, ascales, wscales, lora_act, lora_up, wcscales, bias, out_dtype);
+  if (node) torch::autograd::set_history(y, node);
+  return y;
+}
+
+TORCH_LIBRARY(svdq_b200, m) {
+  m.def("quantize_w4a4_act_fuse_lora(Tensor input, Tensor lora_down, Tensor? smooth=None, SymInt pad_size=256) -> (Tensor, Tensor, Tensor)");
+  m.def("gemm_w4a4(Tensor act, Tensor wgt, Tensor ascales, Tensor wscales, Tensor? lora_act_in=None, Tensor? lora_up=None, "
+        "Tensor? wcscales=None, Tensor? bias=None, ScalarType? out_dtype=None) -> Tensor");
+}
+TORCH_LIBRARY_IMPL(svdq_b200, CUDA, m) {
+  m.impl("quantize_w4a4_act_fuse_lora", op_quantize);
+  m.impl("gemm_w4a4", op_gemm);
+}
+TORCH_LIBRARY_IMPL(svdq_b200, AutogradCUDA, m) {
+  m.impl("quantize_w4a4_act_fuse_lora", op_quantize_autograd);
+  m.impl("gemm_w4a4", op_gemm_autograd);
+}
+
+PyMethodDef g_methods[] = {
+    {"quantize", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_quantize)), METH_FASTCALL, nullptr},
+    {"gemm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_gemm)), METH_FASTCALL, nullptr},
+    {"pack", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_pack)), METH_FASTCALL, nullptr},
+    {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_bind)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_host", "Native host path of the operators.", -1, g_methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host() {
+  g_twins_name = PyUnicode_InternFromString("_svdq_twins");
+  return g_twins_name != nullptr ? PyModule_Create(&g_module) : nullptr;
+}

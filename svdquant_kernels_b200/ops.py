@@ -25,6 +25,10 @@ MMA needs lora_act in lora_up's format and a single bf16 copy is too coarse);
 arrive unmodified, and otherwise (tensors from elsewhere, e.g. weight scales)
 derives them once with two small kernels of the same library and caches them
 on the tensor object.
+
+The ordinary call - contiguous CUDA tensors, twins at hand - is checked, allocated and launched by the
+native host path (csrc/host_ops.cpp); the Python bodies here take every other call and raise on broken
+contracts.
 """
 from __future__ import annotations
 
@@ -122,6 +126,16 @@ def quantize_w4a4_act_fuse_lora(
 ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """`out = (act, ascales, lora_act)` writes into tensors of a previous call (same shapes) instead
     of allocating; their layout twins are reused as well, so a steady-state call allocates nothing."""
+    if fp4 and _force == _lib.QUANT_AUTO:
+        res = (_lib._host or _lib.host()).quantize(input, lora_down, smooth, pad_size, out)
+        if res is not None:
+            return res
+    return _quantize_checked(input, lora_down, smooth, fp4=fp4, pad_size=pad_size, out=out, _force=_force)
+
+
+def _quantize_checked(input, lora_down, smooth, *, fp4=True, pad_size=256, out=None, _force=_lib.QUANT_AUTO):
+    """The operator with its contract checks, for calls the native host path does not take: first uses of a
+    smooth tensor, inputs that are not contiguous or on another device, forced forms, broken contracts."""
     assert input.dim() == 2 and lora_down.dim() == 2
     assert input.is_cuda and lora_down.is_cuda
     assert input.dtype == lora_down.dtype
@@ -201,6 +215,9 @@ def _la16_elems(rows: int, R: int, dtype: torch.dtype) -> int:
 
 def quantize_nvfp4_rows(x: torch.Tensor, *, pad_size: int = 1) -> Tuple[torch.Tensor, torch.Tensor]:
     """GPU row packer: `[rows, K]` f16/bf16/f32 -> (`[rows_pad, K/2]` u8, `[K/16, rows_pad]` e4m3)."""
+    res = (_lib._host or _lib.host()).pack(x, pad_size)
+    if res is not None:
+        return res
     assert x.dim() == 2 and x.is_cuda
     assert x.dtype in _DT
     rows, K = x.shape
@@ -305,6 +322,19 @@ def gemm_w4a4(
     the `[M, N]` result of this call goes into columns `[col0, col0 + N)` of the local `[M, N_total]`
     tensor `y_full` and of the peers' copies at the raw device pointers `peer_ptrs`; `y_full` is
     returned.  See `sharding.linear_columns_fused` for the ordering the caller owes."""
+    if tiler_mn is None and _columns is None and _splits is None and lora_schedule == "interleave":
+        res = (_lib._host or _lib.host()).gemm(act, wgt, ascales, wscales, lora_act_in, lora_up, wcscales, bias, out_dtype,
+                                               smooth_next, out)
+        if res is not None:
+            return res
+    return _gemm_checked(act, wgt, ascales, wscales, lora_act_in, lora_up, wcscales, bias, out_dtype, tiler_mn=tiler_mn,
+                         lora_schedule=lora_schedule, smooth_next=smooth_next, out=out, _columns=_columns, _splits=_splits)
+
+
+def _gemm_checked(act, wgt, ascales, wscales, lora_act_in=None, lora_up=None, wcscales=None, bias=None, out_dtype=None, *,
+                  tiler_mn=None, lora_schedule="interleave", smooth_next=None, out=None, _columns=None, _splits=None):
+    """The operator with its contract checks, for calls the native host path does not take: first uses of
+    weights whose twins are not made yet, tensors in other layouts or types, forced forms, broken contracts."""
     if out_dtype is None:
         out_dtype = lora_up.dtype if lora_up is not None else torch.float16
     assert act.is_cuda and wgt.is_cuda and ascales.is_cuda and wscales.is_cuda, "all inputs must live on CUDA"

@@ -1,0 +1,67 @@
+"""The native host path of the operators (csrc/host_ops.cpp) against the checked Python bodies it stands in for: the same
+outputs where it takes a call, the same errors where it does not."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _layer(dtype, M=300, K=512, N=384, R=32):
+    from svdquant_kernels_b200 import ops
+    g = torch.Generator().manual_seed(6)
+    x = torch.randn(M, K, generator=g).to(dtype).cuda()
+    sm = (torch.rand(K, generator=g) + 0.5).to(dtype).cuda()
+    ld = (torch.randn(K, R, generator=g) / K ** 0.5).to(dtype).cuda()
+    lu = (torch.randn(N, R, generator=g) * 0.01).to(dtype).cuda()
+    wc = (torch.rand(N, generator=g) + 0.5).to(dtype).cuda()
+    wgt, wsc = ops.quantize_nvfp4_rows((torch.randn(N, K, generator=g) * 0.02).cuda())
+    return x, sm, ld, lu, wc, wgt, wsc
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_native_calls_equal_the_checked_ones(dtype):
+    from svdquant_kernels_b200 import _lib, ops
+    x, sm, ld, lu, wc, wgt, wsc = _layer(dtype)
+    host = _lib.host()
+    q0 = ops._quantize_checked(x, ld, sm)                      # makes the smooth table
+    y0 = ops._gemm_checked(q0[0], wgt, q0[1], wsc, q0[2], lu, wc, None, dtype, smooth_next=wc)
+    q1 = host.quantize(x, ld, sm, 256, None)
+    y1 = host.gemm(q1[0], wgt, q1[1], wsc, q1[2], lu, wc, None, dtype, wc, None)
+    assert q1 is not None and y1 is not None
+    q2 = host.quantize(x, ld, sm, 256, q1)                     # into the tensors of the last call
+    assert q2 is q1
+    into = torch.empty_like(y0[0])
+    y2 = host.gemm(q2[0], wgt, q2[1], wsc, q2[2], lu, wc, None, dtype, None, into)
+    assert y2 is into
+    torch.cuda.synchronize()
+    for a, b in zip((*q0, *y0, y0[0]), (*q1, *y1, y2)):
+        assert a.dtype == b.dtype and torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+
+
+def test_other_calls_are_left_to_the_checked_body():
+    from svdquant_kernels_b200 import _lib, ops
+    x, sm, ld, lu, wc, wgt, wsc = _layer(torch.float16)
+    host = _lib.host()
+    assert host.quantize(x, ld, sm, 256, None) is None         # no smooth table yet
+    act, asc, la = ops.quantize_w4a4_act_fuse_lora(x, ld, sm)
+    assert host.quantize(x, ld, sm, 256, None) is not None
+    sm.mul_(1.0)                                               # edited in place: the table is out of date
+    assert host.quantize(x, ld, sm, 256, None) is None
+    strided = x.repeat(1, 2)[:, :512]
+    assert host.quantize(strided, ld, None, 256, None) is None
+    assert torch.equal(ops.quantize_w4a4_act_fuse_lora(strided, ld, sm)[0], act)
+    asc.view(torch.uint8).add_(0)                              # so is the twin of the scales
+    assert host.gemm(act, wgt, asc, wsc, la, lu, wc, None, torch.float16, None, None) is None
+    with pytest.raises(AssertionError):
+        ops.gemm_w4a4(act, wgt[:, :-32], asc, wsc, la, lu)
+    with pytest.raises(AssertionError):
+        torch.ops.svdq_b200.quantize_w4a4_act_fuse_lora(x, ld.float(), sm)
+
+
+def test_registered_ops_have_no_backward():
+    from svdquant_kernels_b200 import torch_ops  # noqa: F401
+    x, sm, ld, lu, wc, wgt, wsc = _layer(torch.float16)
+    act, asc, la = torch.ops.svdq_b200.quantize_w4a4_act_fuse_lora(x.requires_grad_(), ld, sm)
+    assert la.requires_grad and not act.requires_grad
+    with pytest.raises(RuntimeError):
+        la.sum().backward()
