@@ -149,18 +149,39 @@ __device__ __forceinline__ uint32_t cvt_e2m1x8(float2 a, float2 b, float2 c, flo
   return r;
 }
 
-// amax of a 16-element group -> scale byte: e4m3(clamp(amax / 6, 1e-12, 448)), the divide correctly rounded
-__device__ __forceinline__ uint32_t group_scale_byte(const float2 (&f)[8]) {
-  const float m0 = max3abs(f[0].x, f[0].y, f[1].x), m1 = max3abs(f[1].y, f[2].x, f[2].y);
-  const float m2 = max3abs(f[3].x, f[3].y, f[4].x), m3 = max3abs(f[4].y, f[5].x, f[5].y);
-  const float m4 = max3abs(f[6].x, f[6].y, f[7].x);
-  const float amax = fmaxf(max3abs(m0, m1, m2), max3abs(m3, m4, f[7].y));
-  // amax / 6, correctly rounded (amax is finite and >= 0; tiny quotients are clamped away below)
+// Four or eight floats -> their codes, element i in bits 4 i .. 4 i + 3
+template <int N> __device__ __forceinline__ uint32_t cvt_e2m1(const float (&w)[N]);
+template <> __device__ __forceinline__ uint32_t cvt_e2m1<8>(const float (&w)[8]) {
+  return cvt_e2m1x8(make_float2(w[0], w[1]), make_float2(w[2], w[3]), make_float2(w[4], w[5]), make_float2(w[6], w[7]));
+}
+template <> __device__ __forceinline__ uint32_t cvt_e2m1<4>(const float (&w)[4]) {
+  uint32_t r;
+  asm("{\n\t.reg .b8 q0, q1, z;\n\tmov.b16 {z, _}, 0;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 q0, %2, %1;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 q1, %4, %3;\n\t"
+      "mov.b32 %0, {q0, q1, z, z};\n\t}"
+      : "=r"(r)
+      : "f"(w[0]), "f"(w[1]), "f"(w[2]), "f"(w[3]));
+  return r;
+}
+
+// amax -> scale byte: e4m3(clamp(amax / 6, 1e-12, 448)), the divide correctly rounded (amax is finite and >= 0;
+// tiny quotients are clamped away)
+__device__ __forceinline__ uint32_t scale_byte(float amax) {
   const float r6 = 0.16666667163372039794921875f;   // RN(1/6)
   const float s0 = amax * r6;
   float s = fmaf(fmaf(-6.0f, s0, amax), r6, s0);
   s = fminf(fmaxf(s, 1e-12f), 448.0f);
   return static_cast<uint32_t>(__nv_cvt_float_to_fp8(s, __NV_SATFINITE, __NV_E4M3));
+}
+
+// amax of a 16-element group -> scale byte
+__device__ __forceinline__ uint32_t group_scale_byte(const float2 (&f)[8]) {
+  const float m0 = max3abs(f[0].x, f[0].y, f[1].x), m1 = max3abs(f[1].y, f[2].x, f[2].y);
+  const float m2 = max3abs(f[3].x, f[3].y, f[4].x), m3 = max3abs(f[4].y, f[5].x, f[5].y);
+  const float m4 = max3abs(f[6].x, f[6].y, f[7].x);
+  const float amax = fmaxf(max3abs(m0, m1, m2), max3abs(m3, m4, f[7].y));
+  return scale_byte(amax);
 }
 
 // Main path of the codes: k = {2^(2-E), ~1/(4J)} of the group's scale byte.
