@@ -321,7 +321,8 @@ int svdq_linear_plan_forward_host(svdq_linear_plan* plan, const void* x_host, vo
  * every submitted batch has its y on the host.  x_host / y_host of a batch must stay valid (and y
  * unread) until a wait, or the second-next submit, has returned.  Page-locked buffers are copied
  * from and to directly; pageable ones pass through staging buffers of the plan.
- * svdq_linear_plan_forward_host(...) is submit followed by wait.
+ * svdq_linear_plan_forward_host(...) gives the same result as submit followed by wait; it walks the rows of
+ * its one batch in chunks, so that the copies in, the kernels and the copies out overlap within the call.
  */
 int svdq_linear_plan_submit(svdq_linear_plan* plan, const void* x_host, void* y_host, int M);
 int svdq_linear_plan_wait(svdq_linear_plan* plan);

@@ -60,7 +60,8 @@ int svdq_prepare_smooth(const void* smooth, void* smooth_table, int K, int dtype
 
 static int quantize_entry(const void* x, const void* lora_down, const void* smooth, const void* smooth_table, void* act,
                           void* ascales, float* lora_act, void* ascales_swz, void* lora_act16, int M, int K, int R,
-                          int M_pad, int dtype, int flags, void* workspace, size_t workspace_bytes, void* stream) {
+                          int M_pad, int dtype, int flags, void* workspace, size_t workspace_bytes, void* stream,
+                          int split_rows = 0) {
   if (dtype != SVDQ_DTYPE_F16 && dtype != SVDQ_DTYPE_BF16) return SVDQ_ERR_DTYPE;
   if (M < 0 || K <= 0 || R < 0 || M_pad < M || K % 16 != 0) return SVDQ_ERR_SHAPE;
   if (M_pad == 0) return SVDQ_OK;
@@ -87,7 +88,7 @@ static int quantize_entry(const void* x, const void* lora_down, const void* smoo
   }
   if (fused_ok && flags != SVDQ_QUANT_FORCE_GENERIC)
     return launch_quantize_fused(x, lora_down, smooth_table, act, ascales, lora_act, ascales_swz, lora_act16, M, K, R,
-                                 M_pad, dtype, st);
+                                 M_pad, dtype, st, split_rows);
   int rc = launch_quantize_rows(x, smooth, act, ascales, ascales_swz, M, M_pad, K, dtype, st);
   if (rc != SVDQ_OK) return rc;
   return launch_lora_down(x, lora_down, lora_act, lora_act16, M, M_pad, K, R, dtype, st);
@@ -384,15 +385,26 @@ int svdq_selftest_divide(unsigned long long* mismatches_device, void* stream) {
 // copies of neighbouring calls overlap the kernels and each other (PCIe is full duplex).  A slot's
 // life: x copy -> quantizer + GEMM -> y copy; events hand it from stream to stream and keep a slot's
 // next use behind its previous one.
+//
+// A single call (forward_host) has no neighbour to overlap with, so it walks its rows in chunks through the
+// same three streams: while chunk i is multiplied, chunk i + 1 comes in and chunk i - 1 goes out.  The copies
+// bound it (33.4 MB in and 26.7 MB out at 4352 x 3840 -> 3072: 0.61 and 0.48 ms alone, 0.65 ms side by side), and
+// one after the other with the kernels between they took 1.15 ms; in chunks 0.86 ms.
 constexpr int kPlanSlots = 2;
+// Chunks of forward_host: at least 6 MB of the wider side, at most kPlanChunks of them.  A shorter chunk leaves less
+// of the call uncovered at its ends, but every pair of copies that runs side by side costs about 15 us more than
+// its bytes (1 / 2 / 4 / 6 / 8 / 12 / 16 MB: 1.10 / 0.94 / 0.88 / 0.86 / 0.86 / 0.89 / 0.94 ms).
+constexpr int kPlanChunks = 32;
+constexpr size_t kPlanChunkBytes = 6u << 20;
 
 struct PlanSlot {
   void *x, *act, *ascales, *ascales_swz, *lora_act16, *y;
   float* lora_act;
   void *x_pin, *y_pin;                                           // pinned staging for pageable caller buffers
   cudaEvent_t x_ready, computed, y_done;
+  cudaEvent_t y_part[kPlanChunks];                               // pageable y: its chunks' copies (made when first needed)
   void* y_user;                                                  // pageable destination still to be filled from y_pin
-  size_t y_bytes;
+  size_t y_bytes, y_chunk_bytes;
   bool busy;
 };
 
@@ -499,58 +511,95 @@ int svdq_linear_plan_create(svdq_linear_plan** out, int max_M, int K, int N, int
 }
 
 // Finish the call that last used slot `i`: wait for its y copy and, for a pageable y, move the rows
-// out of the staging buffer.
+// out of the staging buffer, chunk by chunk as they arrive.
 static int plan_retire(svdq_linear_plan* p, int i) {
   PlanSlot& q = p->slot[i];
   if (!q.busy) return SVDQ_OK;
   q.busy = false;
-  if (cudaEventSynchronize(q.y_done) != cudaSuccess) return SVDQ_ERR_CUDA;
-  if (q.y_user != nullptr) { memcpy(q.y_user, q.y_pin, q.y_bytes); q.y_user = nullptr; }
+  if (q.y_user != nullptr) {
+    char* const to = static_cast<char*>(q.y_user);
+    const char* const from = static_cast<const char*>(q.y_pin);
+    q.y_user = nullptr;
+    int c = 0;
+    for (size_t at = 0; at < q.y_bytes; at += q.y_chunk_bytes, ++c) {
+      if (cudaEventSynchronize(q.y_part[c]) != cudaSuccess) return SVDQ_ERR_CUDA;
+      memcpy(to + at, from + at, q.y_bytes - at < q.y_chunk_bytes ? q.y_bytes - at : q.y_chunk_bytes);
+    }
+  }
+  return cudaEventSynchronize(q.y_done) == cudaSuccess ? SVDQ_OK : SVDQ_ERR_CUDA;
+}
+
+// Queue one call in chunks of `chunk` rows (a multiple of 256).  A chunk has its own piece of every per-call
+// buffer; the K splits of quantizer and GEMM are those of the whole call, so that the chunking does not show
+// in the result (every row's sums are formed in the same order).
+static int plan_queue(svdq_linear_plan* p, const void* x_host, void* y_host, int M, int chunk) {
+  const int i = static_cast<int>(p->submitted % kPlanSlots);
+  int rc = plan_retire(p, i);                      // at most kPlanSlots calls are in flight
+  if (rc != SVDQ_OK) return rc;
+  PlanSlot& q = p->slot[i];
+  const int K = p->K, N = p->N, R = p->R;
+  const size_t x_row = static_cast<size_t>(K) * 2, y_row = static_cast<size_t>(N) * 2;
+  const int M_pad = (M + 255) / 256 * 256;
+  const int splits = gemm_split_plan(M_pad, N, K, R);
+  const int variant = splits >= 2 ? 10000 * splits + 128 : 0;
+  // page-locked caller buffers are copied from and to directly; pageable ones go through the slot's staging
+  const bool x_pinned = is_pinned_host(x_host), y_pinned = is_pinned_host(y_host);
+  char* const y_dst = static_cast<char*>(y_pinned ? y_host : q.y_pin);
+  const bool bf16 = p->dtype == SVDQ_DTYPE_BF16;
+  // x copies: after the kernels of the slot's previous call have read the old x (`computed` of a never-used
+  // slot is complete by definition); kernels: after the slot's previous y has left the device
+  bool bad = cudaStreamWaitEvent(p->s_in, q.computed, 0) != cudaSuccess;
+  bad = bad || cudaStreamWaitEvent(p->s_run, q.y_done, 0) != cudaSuccess;
+  int c = 0;
+  for (int m0 = 0; m0 < M && !bad; m0 += chunk, ++c) {
+    const int rows = M - m0 < chunk ? M - m0 : chunk;
+    const int rows_pad = (rows + 255) / 256 * 256;
+    const size_t pad0 = static_cast<size_t>(m0);                   // chunks before this one are whole: padded rows = rows
+    const char* x_src = static_cast<const char*>(x_host) + m0 * x_row;
+    if (!x_pinned) {
+      memcpy(static_cast<char*>(q.x_pin) + m0 * x_row, x_src, rows * x_row);
+      x_src = static_cast<const char*>(q.x_pin) + m0 * x_row;
+    }
+    char* const x = static_cast<char*>(q.x) + m0 * x_row;
+    char* const act = static_cast<char*>(q.act) + pad0 * (K / 2);
+    char* const sc = static_cast<char*>(q.ascales) + pad0 * (K / 16);
+    char* const swz = static_cast<char*>(q.ascales_swz) + pad0 * (K / 16);
+    float* const la = q.lora_act + pad0 * R;
+    char* const la16 = static_cast<char*>(q.lora_act16) + 2 * lora16_elems(pad0, R, bf16);
+    char* const y = static_cast<char*>(q.y) + pad0 * y_row;
+    bad = bad || cudaMemcpyAsync(x, x_src, rows * x_row, cudaMemcpyHostToDevice, p->s_in) != cudaSuccess;
+    bad = bad || cudaEventRecord(q.x_ready, p->s_in) != cudaSuccess;
+    bad = bad || cudaStreamWaitEvent(p->s_run, q.x_ready, 0) != cudaSuccess;
+    if (bad) break;
+    rc = quantize_entry(x, p->lora_down, p->smooth, p->smooth_table, act, sc, la, swz, la16, rows, K, R, rows_pad, p->dtype,
+                        SVDQ_QUANT_AUTO, p->quant_ws, p->quant_ws_bytes, p->s_run, M_pad);
+    if (rc != SVDQ_OK) return rc;
+    rc = svdq_gemm_w4a4_ws(act, p->wgt, swz, p->wscales_swz, R > 0 ? la16 : nullptr, R > 0 ? p->lora_up : nullptr,
+                           R > 0 ? p->lora_up_f16 : nullptr, p->wc, p->bias, y, rows_pad, N, K, R, p->dtype, variant,
+                           splits >= 2 ? p->split_ws : nullptr, splits >= 2 ? p->split_ws_bytes : 0, p->s_run);
+    if (rc != SVDQ_OK) return rc;
+    bad = bad || cudaEventRecord(q.computed, p->s_run) != cudaSuccess;
+    bad = bad || cudaStreamWaitEvent(p->s_out, q.computed, 0) != cudaSuccess;
+    bad = bad || cudaMemcpyAsync(y_dst + m0 * y_row, y, rows * y_row, cudaMemcpyDeviceToHost, p->s_out) != cudaSuccess;
+    if (!y_pinned) {
+      if (q.y_part[c] == nullptr) bad = bad || cudaEventCreateWithFlags(&q.y_part[c], cudaEventDisableTiming) != cudaSuccess;
+      bad = bad || cudaEventRecord(q.y_part[c], p->s_out) != cudaSuccess;
+    }
+  }
+  bad = bad || cudaEventRecord(q.y_done, p->s_out) != cudaSuccess;
+  if (bad) return SVDQ_ERR_CUDA;
+  q.y_user = y_pinned ? nullptr : y_host;
+  q.y_bytes = M * y_row;
+  q.y_chunk_bytes = chunk * y_row;
+  q.busy = true;
+  ++p->submitted;
   return SVDQ_OK;
 }
 
 int svdq_linear_plan_submit(svdq_linear_plan* p, const void* x_host, void* y_host, int M) {
   if (p == nullptr || x_host == nullptr || y_host == nullptr) return SVDQ_ERR_NULL;
   if (M <= 0 || M > p->max_M) return SVDQ_ERR_SHAPE;
-  const int i = static_cast<int>(p->submitted % kPlanSlots);
-  int rc = plan_retire(p, i);                      // at most kPlanSlots calls are in flight
-  if (rc != SVDQ_OK) return rc;
-  PlanSlot& q = p->slot[i];
-  const int M_pad = (M + 255) / 256 * 256;
-  const size_t xbytes = static_cast<size_t>(M) * p->K * 2, ybytes = static_cast<size_t>(M) * p->N * 2;
-  // page-locked caller buffers are copied from and to directly; pageable ones go through the slot's staging
-  const void* x_src = x_host;
-  if (!is_pinned_host(x_host)) { memcpy(q.x_pin, x_host, xbytes); x_src = q.x_pin; }
-  const bool y_pinned = is_pinned_host(y_host);
-  bool bad = false;
-  // x copy: after the kernels of the slot's previous call have read the old x (stream order on s_run
-  // plus this wait; `computed` of a never-used slot is complete by definition)
-  bad = bad || cudaStreamWaitEvent(p->s_in, q.computed, 0) != cudaSuccess;
-  bad = bad || cudaMemcpyAsync(q.x, x_src, xbytes, cudaMemcpyHostToDevice, p->s_in) != cudaSuccess;
-  bad = bad || cudaEventRecord(q.x_ready, p->s_in) != cudaSuccess;
-  // kernels: after x has landed and the slot's previous y has left the device
-  bad = bad || cudaStreamWaitEvent(p->s_run, q.x_ready, 0) != cudaSuccess;
-  bad = bad || cudaStreamWaitEvent(p->s_run, q.y_done, 0) != cudaSuccess;
-  if (bad) return SVDQ_ERR_CUDA;
-  rc = svdq_quantize_w4a4_act_fuse_lora_ws(q.x, p->lora_down, p->smooth, p->smooth_table, q.act, q.ascales, q.lora_act,
-                                           q.ascales_swz, q.lora_act16, M, p->K, p->R, M_pad, p->dtype, SVDQ_QUANT_AUTO,
-                                           p->quant_ws, p->quant_ws_bytes, p->s_run);
-  if (rc != SVDQ_OK) return rc;
-  rc = svdq_gemm_w4a4_ws(q.act, p->wgt, q.ascales_swz, p->wscales_swz, p->R > 0 ? q.lora_act16 : nullptr,
-                         p->R > 0 ? p->lora_up : nullptr, p->R > 0 ? p->lora_up_f16 : nullptr, p->wc, p->bias, q.y, M_pad,
-                         p->N, p->K, p->R, p->dtype, 0, p->split_ws, p->split_ws_bytes, p->s_run);
-  if (rc != SVDQ_OK) return rc;
-  bad = bad || cudaEventRecord(q.computed, p->s_run) != cudaSuccess;
-  // y copy
-  bad = bad || cudaStreamWaitEvent(p->s_out, q.computed, 0) != cudaSuccess;
-  bad = bad || cudaMemcpyAsync(y_pinned ? y_host : q.y_pin, q.y, ybytes, cudaMemcpyDeviceToHost, p->s_out) != cudaSuccess;
-  bad = bad || cudaEventRecord(q.y_done, p->s_out) != cudaSuccess;
-  if (bad) return SVDQ_ERR_CUDA;
-  q.y_user = y_pinned ? nullptr : y_host;
-  q.y_bytes = ybytes;
-  q.busy = true;
-  ++p->submitted;
-  return SVDQ_OK;
+  return plan_queue(p, x_host, y_host, M, (M + 255) / 256 * 256);
 }
 
 int svdq_linear_plan_wait(svdq_linear_plan* p) {
@@ -564,7 +613,13 @@ int svdq_linear_plan_wait(svdq_linear_plan* p) {
 }
 
 int svdq_linear_plan_forward_host(svdq_linear_plan* p, const void* x_host, void* y_host, int M) {
-  const int rc = svdq_linear_plan_submit(p, x_host, y_host, M);
+  if (p == nullptr || x_host == nullptr || y_host == nullptr) return SVDQ_ERR_NULL;
+  if (M <= 0 || M > p->max_M) return SVDQ_ERR_SHAPE;
+  const size_t row = static_cast<size_t>(p->K > p->N ? p->K : p->N) * 2;
+  const int M_pad = (M + 255) / 256 * 256;
+  int chunk = static_cast<int>((kPlanChunkBytes + row * 256 - 1) / (row * 256)) * 256;
+  while ((M_pad + chunk - 1) / chunk > kPlanChunks) chunk += 256;
+  const int rc = plan_queue(p, x_host, y_host, M, chunk);
   return rc != SVDQ_OK ? rc : svdq_linear_plan_wait(p);
 }
 
@@ -582,6 +637,8 @@ void svdq_linear_plan_destroy(svdq_linear_plan* p) {
     if (q.x_ready != nullptr) cudaEventDestroy(q.x_ready);
     if (q.computed != nullptr) cudaEventDestroy(q.computed);
     if (q.y_done != nullptr) cudaEventDestroy(q.y_done);
+    for (cudaEvent_t e : q.y_part)
+      if (e != nullptr) cudaEventDestroy(e);
   }
   void* dev[] = {p->wgt, p->wscales_swz, p->lora_down, p->lora_up, p->lora_up_f16, p->smooth, p->smooth_table, p->wc, p->bias,
                  p->split_ws, p->quant_ws};

@@ -597,7 +597,7 @@ int launch_smooth_table(const void* smooth, void* table, int K, int dtype, cudaS
 }
 
 template <typename T, int RP>
-static int launch_qf(const void* x, const void* w, const qf::Params& p, cudaStream_t stream) {
+static int launch_qf(const void* x, const void* w, const qf::Params& p, cudaStream_t stream, int split_rows) {
   using C = qf::Cfg<RP>;
   CUtensorMap tmX, tmW;
   int rc;
@@ -624,7 +624,7 @@ static int launch_qf(const void* x, const void* w, const qf::Params& p, cudaStre
     capped[dev] = true;
   }
   const bool known = dev >= 0 && dev < 64;
-  int ks = pick_k_split(p.M_pad, p.K, known ? cap4[dev] : 0, known ? cap8[dev] : 0);
+  int ks = pick_k_split(split_rows > p.M_pad ? split_rows : p.M_pad, p.K, known ? cap4[dev] : 0, known ? cap8[dev] : 0);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(p.M_pad / qf::TILE_M, ks, 1);
   cfg.blockDim = dim3(qf::NUM_THREADS, 1, 1);
@@ -669,7 +669,7 @@ int quantize_fused_max_clusters(int R, int ks, int dtype) {
 
 int launch_quantize_fused(const void* x, const void* lora_down, const void* smooth_table, void* act, void* ascales,
                           float* lora_act, void* ascales_swz, void* lora_act16, int M, int K, int R, int M_pad,
-                          int dtype, cudaStream_t stream) {
+                          int dtype, cudaStream_t stream, int split_rows) {
   if (!quantize_fused_supported(M, K, R, M_pad)) return SVDQ_ERR_UNSUPPORTED;
   if (reinterpret_cast<uintptr_t>(smooth_table) % 16 != 0) return SVDQ_ERR_ALIGN;   // bulk copies start on 16-byte boundaries
   qf::Params p;
@@ -682,13 +682,13 @@ int launch_quantize_fused(const void* x, const void* lora_down, const void* smoo
   p.M = M; p.K = K; p.R = R; p.M_pad = M_pad;
   const int rp = R <= 64 ? 64 : (R <= 128 ? 128 : 256);
   if (dtype == SVDQ_DTYPE_F16) {
-    if (rp == 64) return launch_qf<__half, 64>(x, lora_down, p, stream);
-    if (rp == 128) return launch_qf<__half, 128>(x, lora_down, p, stream);
-    return launch_qf<__half, 256>(x, lora_down, p, stream);
+    if (rp == 64) return launch_qf<__half, 64>(x, lora_down, p, stream, split_rows);
+    if (rp == 128) return launch_qf<__half, 128>(x, lora_down, p, stream, split_rows);
+    return launch_qf<__half, 256>(x, lora_down, p, stream, split_rows);
   } else if (dtype == SVDQ_DTYPE_BF16) {
-    if (rp == 64) return launch_qf<__nv_bfloat16, 64>(x, lora_down, p, stream);
-    if (rp == 128) return launch_qf<__nv_bfloat16, 128>(x, lora_down, p, stream);
-    return launch_qf<__nv_bfloat16, 256>(x, lora_down, p, stream);
+    if (rp == 64) return launch_qf<__nv_bfloat16, 64>(x, lora_down, p, stream, split_rows);
+    if (rp == 128) return launch_qf<__nv_bfloat16, 128>(x, lora_down, p, stream, split_rows);
+    return launch_qf<__nv_bfloat16, 256>(x, lora_down, p, stream, split_rows);
   }
   return SVDQ_ERR_DTYPE;
 }

@@ -22,7 +22,7 @@ bool quantize_fused_supported(int M, int K, int R, int M_pad);
 int launch_smooth_table(const void* smooth, void* table, int K, int dtype, cudaStream_t stream);
 int launch_quantize_fused(const void* x, const void* lora_down, const void* smooth_table, void* act, void* ascales,
                           float* lora_act, void* ascales_swz, void* lora_act16, int M, int K, int R, int M_pad,
-                          int dtype, cudaStream_t stream);
+                          int dtype, cudaStream_t stream, int split_rows = 0);   // split K as for this many padded rows (0: M_pad)
 
 int quantize_fused_max_clusters(int R, int ks, int dtype);
 
