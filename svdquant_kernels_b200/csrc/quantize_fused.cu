@@ -86,6 +86,10 @@ struct Cfg {
   static constexpr int X_STAGE_BYTES = X_BYTES + 1024;            // tile + table slab, padded to the 1 KB swizzled tiles need
   static constexpr int W_BYTES = SLAB_K * RP * 2;                 // lora_down slab
   static constexpr int W_STAGES = RP > 128 ? 3 : 4;
+  // MMA-issuing warps.  Two take the slabs by turns; then both rings must be even, so that an issuer meets only slabs
+  // of its own in a stage: one that went on to slab i could otherwise look at the stage while slab i - W_STAGES,
+  // the other issuer's, is still on its way into it, and a one-bit parity would tell it that slab i is there.
+  static constexpr int ISSUERS = W_STAGES % 2 == 0 ? 2 : 1;
   static constexpr int W_RING_BYTES = W_STAGES * W_BYTES;
   static constexpr int RECV_BYTES = (TILE_M / 2) * RP * 4;        // two K ranks: the peer's partial sums of this CTA's 32 rows
   static constexpr int STAGES_RAW = (232448 - 1024 - 512 - 1024 - RECV_BYTES - W_RING_BYTES) / X_STAGE_BYTES;
@@ -96,11 +100,10 @@ struct Cfg {
   static constexpr int RING_BYTES = STAGES * X_STAGE_BYTES;
   static constexpr int BARS_OFF = RING_BYTES + W_RING_BYTES;
   static constexpr int SMEM_BYTES = 1024 + BARS_OFF + 512 + 1024 + RECV_BYTES;   // rings, barriers, scale-constant table, receive buffer
-  // Two accumulators: slabs alternate between two issuing warps (see the MMA issuers), each with its own.
-  static constexpr int TMEM_COLS = 2 * (RP < 32 ? 32 : RP);       // power of two >= 64
+  static constexpr int TMEM_COLS = ISSUERS * RP;                  // an accumulator per issuer; a power of two >= 64
   static constexpr int EPI_COLS = RP / 4 < 32 ? 32 : RP / 4;      // accumulator columns per epilogue warp
   static_assert(TILE_M * RP * 4 <= RING_BYTES, "partial accumulator must fit in the x ring");
-  static_assert(STAGES >= QUANT_GROUPS && STAGES % QUANT_GROUPS == 0, "ring depth");
+  static_assert(STAGES >= QUANT_GROUPS && STAGES % QUANT_GROUPS == 0 && (ISSUERS == 1 || STAGES % 2 == 0), "ring depth");
   static_assert((2 * STAGES + 2 * W_STAGES + 3) * 8 + 64 <= 512, "barrier block");
   static_assert(2 * RECV_BYTES <= W_RING_BYTES, "the exchange stages both halves of the accumulator in the lora_down ring");
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
@@ -175,7 +178,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     *lora_unfit = 0u;
     for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1 + QUANT_WARPS / QUANT_GROUPS); }
     for (int s = 0; s < C::W_STAGES; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], 1); }
-    mbar_init(acc_done, my_slabs > 1 ? 2 : 1);     // one arrival per MMA issuer that has slabs
+    mbar_init(acc_done, C::ISSUERS == 2 && my_slabs > 1 ? 2 : 1);     // one arrival per MMA issuer that has slabs
     mbar_init(recv_bar, 1);                    // armed below with the bytes of the peer's two copies
     mbar_init(ack_bar, 1);
     if (kDirectExchange && ks == 2 && has_lora) mbar_arrive_expect_tx(recv_bar, C::RECV_BYTES);
@@ -195,7 +198,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   // start together; this costs a fraction of a microsecond, before the wait for the kernel ahead.)
   if (kDirectExchange && ks == 2 && has_lora) cluster_sync_all();
   tc_fence_after_sync();
-  const uint32_t tmem_acc = *tmem_slot;
+  const uint32_t tmem_acc = __shfl_sync(0xffffffffu, *tmem_slot, 0);   // warp-uniform, like the warp index
   // set-up done; what follows reads and writes global memory
   pdl_trigger();
   pdl_wait();
@@ -239,38 +242,39 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
         __syncwarp();
       }
     }
-  } else if (warp == 1 || warp == 3) {
+  } else if (warp == 1 || (warp == 3 && C::ISSUERS == 2)) {
     // ------------------------------ MMA issuers ------------------------------
     // Two warps, even and odd slabs, each into an accumulator of its own (added up in the epilogue, always in
-    // the same order).  One thread's loop - two barrier waits, four MMAs, three commits - takes about 0.3 us
-    // per slab whatever the tensor pipe has to do (it is busy a quarter of the time), which made a single
-    // issuer the slowest agent of the kernel: the x ring ran full behind it and the epilogue started late.
+    // the same order).  One thread's loop - two barrier waits, four MMAs, three commits - takes longer than the tensor
+    // pipe has to do for a slab, which made a single issuer the slowest agent of the kernel: the x ring ran full
+    // behind it and the epilogue started late.  Operands are constants added to warp-uniform values.
     constexpr uint64_t kDescA = smem_desc_base(0, 1024, kSwizzle128B);               // x tile, K-major
     constexpr uint64_t kDescB = smem_desc_base(SLAB_K * 128, 1024, kSwizzle128B);    // lora_down slab, R-major (its own ring)
     constexpr uint32_t kIdesc = idesc_f16(kBf16, kBf16, TILE_M, RP, false, true);
     const int issuer = warp >> 1;                                  // 0 or 1
     const uint32_t acc = tmem_acc + issuer * RP;
-    const int last = ((my_slabs - 1 - issuer) & ~1) + issuer;      // this issuer's last slab (negative: none)
-    bool ok = true;
-    for (int i = issuer; i < my_slabs && ok; i += 2) {
-      const uint32_t s = i % C::STAGES, ph = (i / C::STAGES) & 1;
-      if (!uwait(&full[s], ph, kDevWaitFull, i)) { ok = false; break; }
-      const uint32_t sw = i % C::W_STAGES;
-      if (has_lora && !uwait(&wfull[sw], (i / C::W_STAGES) & 1, kDevWaitFull, 0x50000 + i)) { ok = false; break; }
+    const int last = C::ISSUERS == 1 ? my_slabs - 1 : ((my_slabs - 1 - issuer) & ~1) + issuer;   // this issuer's last slab (negative: none)
+    const uint32_t x16 = smem_desc_addr(smem), w16 = smem_desc_addr(wring);
+    uint32_t s = issuer, ph = 0, sw = issuer, phw = 0;
+    for (int i = issuer; i < my_slabs; i += C::ISSUERS) {
+      if (!uwait(&full[s], ph, kDevWaitFull, i)) break;
+      if (has_lora && !uwait(&wfull[sw], phw, kDevWaitFull, 0x50000 + i)) break;
       tc_fence_after_sync();
-      const uint32_t a_addr = smem_u32(smem + s * C::X_STAGE_BYTES);
-      const uint32_t b_addr = smem_u32(wring + sw * C::W_BYTES);
+      const uint64_t da = kDescA + (x16 + s * (C::X_STAGE_BYTES / 16)), db = kDescB + (w16 + sw * (C::W_BYTES / 16));
       if (elect_one()) {
         if (has_lora) {
 #pragma unroll
-          for (int j = 0; j < SLAB_K / 16; ++j)
-            mma_f16<1>(acc, smem_desc(kDescA, a_addr + j * 32), smem_desc(kDescB, b_addr + j * 2048), kIdesc,
-                       (i != issuer || j != 0) ? 1u : 0u);
+          for (int j = 0; j < SLAB_K / 16; ++j) mma_f16<1>(acc, da + j * 2, db + j * 128, kIdesc, j != 0 || i != issuer ? 1u : 0u);
+          tc_commit(&empty[s]);
+          tc_commit(&wempty[sw]);
+          if (i == last) tc_commit(acc_done);
+        } else {
+          mbar_arrive(&empty[s]);
         }
-        if (has_lora) { tc_commit(&empty[s]); tc_commit(&wempty[sw]); if (i == last) tc_commit(acc_done); }
-        else mbar_arrive(&empty[s]);
       }
       __syncwarp();
+      s += C::ISSUERS; if (s >= C::STAGES) { s -= C::STAGES; ph ^= 1; }
+      sw += C::ISSUERS; if (sw >= C::W_STAGES) { sw -= C::W_STAGES; phw ^= 1; }
     }
   } else if (warp >= AUX_WARPS) {
     // ------------------------------ quantize warps ------------------------------
@@ -340,7 +344,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   // slab, the odd slabs' (always in this order)
   auto acc_ld = [&](uint32_t taddr, uint32_t (&v)[32]) {
     tmem_ld_32x32(taddr, v);
-    if (my_slabs > 1) {
+    if (C::ISSUERS == 2 && my_slabs > 1) {
       uint32_t w[32];
       tmem_ld_32x32(taddr + RP, w);
       tmem_ld_wait();

@@ -364,6 +364,9 @@ __host__ __device__ constexpr uint64_t smem_desc_base(uint32_t lbo_bytes, uint32
   return (uint64_t((lbo_bytes >> 4) & 0x3FFF) << 16) | (uint64_t((sbo_bytes >> 4) & 0x3FFF) << 32) |
          (uint64_t(1) << 46) | (uint64_t(swizzle_code & 7) << 61);
 }
+// The address field of a descriptor as an addend, for descriptors built by adding offsets (in 16-byte units) to it.
+// The mask matters: in a cluster the shared addresses of other ranks than 0 have bits above the 18 of the field.
+__device__ __forceinline__ uint32_t smem_desc_addr(const void* p) { return (smem_u32(p) >> 4) & 0x3FFF; }
 __device__ __forceinline__ uint64_t smem_desc(uint64_t base, uint32_t smem_addr) {
   return base | uint64_t((smem_addr >> 4) & 0x3FFF);
 }
