@@ -9,23 +9,33 @@
 // The reference's own kernel for this op is
 // cute_kernels/gemm_w4a4/kernel_v2_fa4.py:841-1589.
 //
-// Work decomposition (384 threads per CTA, one CTA per SM):
+// Work decomposition (320 threads per CTA, one CTA per SM):
 //   warps 0-7  epilogue: tensor memory -> registers -> affine -> 16 bit ->
-//              swizzled shared memory -> TMA store (a 32-row x BN/2 strip per warp)
+//              swizzled shared memory -> TMA store (a 32-row x 64-column strip per warp at a time)
 //   warp  8    producer: TMA loads into a ring of shared-memory stages
-//   warp  9    MMA issuer: tcgen05.mma + commits
-//   warps 10-11 scale copiers: tcgen05.cp of the stage's scale atoms into a
-//              multi-buffered scale area of tensor memory, a few slabs ahead;
-//              each warp takes two of the slab's four k-blocks
-// Issuing one tcgen05.cp costs its thread about 30 cycles (measured), and a
-// 256-wide slab needs 12 scale copies next to its 4 MMAs, which together with
-// the waits is more than the 512 cycles the slab's MMAs run for; so the two
-// kinds are issued by different warps and handshake through mbarriers: each
-// copier's commit is one of the arrivals the stage's "full" barrier waits for
-// (beside the producer's, which carries the operand bytes), so the MMA issuer
-// waits once per slab and finds operands in shared memory and scales in tensor
-// memory.  All single-lane roles stay converged and elect one lane per
-// instruction, so descriptors and addresses live in uniform registers.
+//   warp  9    issuer: tcgen05.cp of a slab's scale atoms into tensor memory, its
+//              tcgen05.mma's, and the commits
+// Copies and MMAs of one thread run in its order, so the issuer waits for one
+// barrier per slab and never for the copies; two scale buffers let a slab's
+// copies run beside the MMAs of the slab before.  A 256 x 256 x 256 slab keeps the
+// tensor pipe busy for 512 cycles, and its 12 copies, 4 MMAs and commits go out
+// in about 270 (8 cycles a copy, 40 an MMA) plus 160 for the wait and the loop, as
+// long as descriptors and addresses live in uniform registers: the issuing code
+// stays converged, elects one lane per slab and builds every operand by adding
+// constants to warp-uniform values.  (With address arithmetic and predicates per
+// k-block the same slab took 640 cycles to issue, more than it takes to run;
+// copies in warps of their own cost a barrier handshake per slab and left the
+// issuer at about 600.)
+//
+// Accumulators.  Tensor memory (512 columns) does not hold two 256-column
+// accumulators beside the scales, but it holds three halves: tile t of a CTA uses
+// columns [0, 256) or [128, 384) by turns.  The epilogue drains the half that the
+// next tile needs too first, which takes about 300 cycles, hands it back, and has
+// the whole of the next tile for the rest.  The hand-back is a relaxed remote
+// arrival: as a releasing one it waited for everything the thread had under way,
+// 1500 cycles per strip, and held up both the next tile and the epilogue.
+// 4352 x 3840 -> 3072 / -> 15360, x 15360 -> 3840, x 10240 -> 3072 with all this:
+// 30.4 / 118.9 / 102.8 / 56.3 -> 28.2 / 109.7 / 95.9 / 52.4 us.
 //
 // CG = 1: a CTA computes a 128 x BN tile.
 // CG = 2: two CTAs of a cluster compute a 256 x BN tile with cta_group::2
@@ -37,9 +47,6 @@
 //
 // A stage holds one 256-element K slab: A 128 x 128 B, B rows x 128 B (both
 // 128-byte swizzled, K-major, two E2M1 codes per byte) and their scale atoms.
-// The scale atoms are requested first and complete on a barrier of their own,
-// which is all the scale copiers wait for: a stage's scales are in tensor
-// memory by the time its operand tiles land.
 // The LoRA-up product reuses the very same ring: a slab of 64 rank elements of
 // lora_act (128 rows x 128 B) and lora_up (B rows x 128 B) has exactly the byte
 // footprint of a main slab, so it is ceil(R/64) more ring passes per output
@@ -85,23 +92,19 @@ constexpr int BK = 256;          // K elements per stage (128 bytes of codes per
 constexpr int A_BYTES = BM * 128;
 constexpr int SFA_BYTES = BM * (BK / 16);  // 2048
 constexpr int EPI_WARPS = 8;
-constexpr int SF_WARPS = 2;       // scale copiers: each takes two of a slab's four k-blocks
-constexpr int NUM_THREADS = (EPI_WARPS + 2 + SF_WARPS) * 32;
+constexpr int NUM_THREADS = (EPI_WARPS + 2) * 32;
 constexpr int STORE_BUF_BYTES = 32 * 128;  // one 32-row x 64-column strip of y
-
 template <int CG, int BN, bool NEXT = false>
 struct Cfg {
   static constexpr int B_ROWS = BN / CG;                           // rows of B this CTA loads
   static constexpr int B_BYTES = B_ROWS * 128;
   static constexpr int SFB_BYTES = BN * (BK / 16);
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES + SFA_BYTES + SFB_BYTES;
-  static constexpr int ACC_STAGES = (BN <= 128) ? 2 : 1;
-  // One 32-row x 64-column staging strip per epilogue warp.  The accumulator is drained into
-  // registers in one burst and released before any staging happens, so a second strip would only
-  // take shared memory away from the load ring.
-  static constexpr int GROUPS_PER_WARP = BN / 128;                 // 64-column strips each epilogue warp handles per tile
-  static constexpr int STORE_BUFS = 1;
-  static constexpr int STORE_BYTES = EPI_WARPS * STORE_BUFS * STORE_BUF_BYTES;
+  // Accumulators: tile t of a CTA starts at column 128 (t % 2).  128-column tiles simply alternate; 256-column
+  // tiles share the middle 128 columns with their neighbours.
+  static constexpr bool SHARED_ACC = BN == 256;
+  static constexpr int ACC_COLS = 128 + BN;
+  static constexpr int STORE_BYTES = EPI_WARPS * STORE_BUF_BYTES;
   // per-column rows of the current tile: wcscales, bias and, for the next layer's quantisation, -smooth_next and
   // 1 / smooth_next (that fourth kilobyte would cost the plain 256 x 256 form its fifth ring stage)
   static constexpr int AFFINE_BYTES = NEXT ? 4096 : 3072;
@@ -111,16 +114,15 @@ struct Cfg {
   static constexpr int SFA_COLS = 16;                 // 4 k-blocks x 4 columns
   static constexpr int SFB_COLS = 4 * (BN / 32);      // 4 k-blocks x BN/32 columns
   static constexpr int SF_COLS = SFA_COLS + SFB_COLS; // one scale buffer
-  // Scale buffers in tensor memory.  Copies and MMAs execute in issue order on one pipe, and an MMA
-  // may only be issued once its scales have landed, so the copier has to run several slabs ahead of
-  // the MMA issuer or every slab pays a copy + wake-up bubble.
-  static constexpr int SF_BUFS_FIT = (512 - ACC_STAGES * BN) / SF_COLS;
-  static constexpr int SF_BUFS = SF_BUFS_FIT > 6 ? 6 : SF_BUFS_FIT;
+  // Scale buffers in tensor memory.  Copies into them and the MMAs that read them are issued by one thread and run
+  // in its order; a second buffer lets a slab's copies run beside the MMAs of the slab before.
+  static constexpr int SF_BUFS_FIT = (512 - ACC_COLS) / SF_COLS;
+  static constexpr int SF_BUFS = SF_BUFS_FIT > 4 ? 4 : SF_BUFS_FIT;
   static constexpr int TMEM_COLS = 512;
   static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + STORE_BYTES + TAIL_BYTES;
-  static_assert(ACC_STAGES * BN + SF_BUFS * SF_COLS <= TMEM_COLS, "tensor memory budget");
+  static_assert(ACC_COLS + SF_BUFS * SF_COLS <= TMEM_COLS && SF_BUFS >= 2, "tensor memory budget");
   static_assert(STAGES >= 3, "ring too shallow");
-  static_assert((3 * STAGES + 2 * ACC_STAGES + 2 * SF_BUFS) * 8 + 16 <= 512, "barrier block");
+  static_assert((2 * STAGES + 5) * 8 + 16 <= 512, "barrier block");
 };
 
 // Column-sharded form: one tensor map per peer's copy of the result (same geometry as this GPU's).
@@ -245,13 +247,12 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint8_t* tail = store_bufs + C::STORE_BYTES;
   float* affine = reinterpret_cast<float*>(tail);                 // [3 or 4][BN] : wcscales, bias, -smooth_next, 1/smooth_next of the current tile
   uint64_t* bars = reinterpret_cast<uint64_t*>(tail + C::AFFINE_BYTES);
-  uint64_t* full = bars;                                          // [STAGES]     A / B (or LoRA) operands landed and scales copied (leader CTA's copy is used)
-  uint64_t* empty = bars + C::STAGES;                             // [STAGES]     stage consumed by the MMAs (per CTA)
-  uint64_t* full_sf = bars + 2 * C::STAGES;                       // [STAGES]     the stage's scale atoms landed (leader's copy)
-  uint64_t* acc_full = bars + 3 * C::STAGES;                      // [ACC_STAGES] accumulator complete (per CTA)
-  uint64_t* acc_empty = acc_full + C::ACC_STAGES;                 // [ACC_STAGES] accumulator drained (leader's copy is used)
-  uint64_t* sf_empty = acc_empty + C::ACC_STAGES;                 // [SF_BUFS] scale buffer consumed by the MMAs (leader CTA)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sf_empty + C::SF_BUFS);
+  uint64_t* full = bars;                                          // [STAGES] operands and scales landed (leader CTA's copy is used)
+  uint64_t* empty = bars + C::STAGES;                             // [STAGES] stage consumed by the MMAs (per CTA)
+  uint64_t* acc_full = bars + 2 * C::STAGES;                      // [2]      accumulator complete (per CTA)
+  uint64_t* acc_empty = acc_full + 2;                             // [2]      accumulator drained (leader's copy is used)
+  uint64_t* acc_shared = acc_empty + 2;                           // its columns that the next tile uses too are drained (leader's copy)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_shared + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile uint32_t* sk_ticket = tmem_slot + 2;                   // split-K: the ticket this CTA drew for its tile
   const WaitCtx ctx{abort_flag};
@@ -271,11 +272,9 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    // full[s]: the producer's arrival (with the operand bytes) and one arrival per scale copier, made when the
-    // stage's scales are in tensor memory (at once for a LoRA slab): the MMA issuer waits once per slab
-    for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], 1 + SF_WARPS); mbar_init(&empty[s], 1); mbar_init(&full_sf[s], 1); }
-    for (int a = 0; a < C::ACC_STAGES; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], EPI_WARPS * CG); }
-    for (int b = 0; b < C::SF_BUFS; ++b) mbar_init(&sf_empty[b], 1);
+    for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], EPI_WARPS * CG); }
+    mbar_init(acc_shared, EPI_WARPS * CG);
     fence_barrier_init();
   }
   if (warp == EPI_WARPS && lane == 0) {
@@ -296,8 +295,8 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   // the kernel before this one in the stream; from here on its outputs are read.
   pdl_trigger();
   pdl_wait();
-  const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_sf = tmem_base + C::ACC_STAGES * BN;       // SF_BUFS buffers of [SFA 16 | SFB] columns
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);   // warp-uniform, for the same reason as the warp index
+  const uint32_t tmem_sf = tmem_base + C::ACC_COLS;              // SF_BUFS buffers of [SFA 16 | SFB] columns
 
   const int kt_main = (p.K + BK - 1) / BK;   // the last slab may hold fewer than four 64-element k-blocks
   const int lora_slabs = (p.R + 63) / 64;
@@ -305,12 +304,13 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   // as an fp16 plane; a tile whose 32-row blocks all carry a zero "does not fit fp16" word takes
   // the fp16 plane and the fp16 copy of lora_up in a single pass.  Every role of both CTAs
   // evaluates this per tile from the same words, so they agree on the number of slabs.
-  auto lora_fp16 = [&](int mb) -> bool {
-    if (!kBf16 || p.R == 0 || p.la_flags == nullptr) return false;
+  // The words come from L2, so a role asks for the next tile's while it works on this one's.
+  auto lora_words = [&](int work) -> uint32_t {
+    if (!kBf16 || p.R == 0 || p.la_flags == nullptr || work >= p.tiles_m * p.tiles_n * (SK ? p.splits : 1)) return 1u;
     constexpr int kWords = CG * BM / 32;
-    const uint32_t w = lane < kWords ? __ldg(p.la_flags + mb * kWords + lane) : 0u;
-    return __all_sync(0xffffffffu, w == 0u) != 0;
+    return lane < kWords ? __ldg(p.la_flags + (SK ? work / p.splits : work) % p.tiles_m * kWords + lane) : 0u;
   };
+  auto lora_fp16 = [&](uint32_t words) -> bool { return kBf16 && __all_sync(0xffffffffu, words == 0u) != 0; };
   auto lora_parts = [&](bool fp16_pass) -> int { return (kBf16 && !fp16_pass) ? 2 : 1; };
   const int total_tiles = p.tiles_m * p.tiles_n;
   const int k_groups4 = p.K / 64;            // scale atoms along K
@@ -347,15 +347,16 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   auto lora_stride = [&](bool fp16_pass) -> int { return (kBf16 && !fp16_pass) ? p.stride2 : p.stride1; };
   if (warp == EPI_WARPS) {
     // ------------------------------ producer (both CTAs) ------------------------------
-    uint32_t it = 0;
+    uint32_t s = 0, ph = 1, it = 0;
     bool ok = true;
+    uint32_t words = lora_words(pair);
     for (int w = pair; w < total_work && ok; w += num_pairs) {
       const int tile = SK ? w / S : w, split = SK ? w - tile * S : 0;
       const int mb = tile % p.tiles_m, nb = tile / p.tiles_m;
       const int m0 = (mb * CG + rank) * BM;
-      const int n0 = nb * BN;
-      const int nrow0 = n0 + rank * C::B_ROWS;
-      const bool la_fp16 = lora_fp16(mb);
+      const int nrow0 = nb * BN + static_cast<int>(rank) * C::B_ROWS;
+      const bool la_fp16 = lora_fp16(words);
+      words = lora_words(w + num_pairs);
       const int kt_all = kt_main + lora_parts(la_fp16) * lora_slabs;
       int kt_lo, kt_hi;
       slab_range(split, kt_all, kt_lo, kt_hi);
@@ -363,34 +364,27 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       walk.start(kt_main, kt_all, p.interleave, lora_stride(la_fp16), kt_lo);
       for (int pos = kt_lo; pos < kt_hi; ++pos, ++it) {
         const int kt = walk.at(pos);
-        const uint32_t s = it % C::STAGES, ph = (it / C::STAGES) & 1;
-        if (!uwait(&empty[s], ph ^ 1, ctx, kDevWaitEmpty, it)) { ok = false; break; }
+        if (!uwait(&empty[s], ph, ctx, kDevWaitEmpty, it)) { ok = false; break; }
         uint8_t* st = smem + s * C::STAGE_BYTES;
         // Codes past K are zero-filled by TMA.  The scale atoms of a (128-row block, slab) are four
         // consecutive 512-byte rows of the swizzled scale buffer seen as a [blocks * K/64, 512 B] matrix;
         // a short last slab just fetches (and never uses) the rows that follow.  Every byte of a box
         // counts toward the barrier whether it was in bounds or not.
-        // Two barriers per stage: the scale atoms (6 KB, requested first) complete on full_sf, the
-        // operand tiles on full.  The scale copiers work off full_sf, so a stage's scales are already in
-        // tensor memory when its operands land and the MMAs can start at once.  A LoRA slab has no
-        // scales; its full_sf is completed by a plain arrival so that both barriers flip once per slab.
         constexpr uint32_t kSfBytes = SFA_BYTES + C::SFB_BYTES, kAbBytes = A_BYTES + C::B_BYTES;
-        // the barriers that count this CTA's bytes: its own for CG = 1, the leader's for a pair
+        // the barrier that counts this CTA's bytes: its own for CG = 1, the leader's for a pair
         const uint32_t bar = (CG == 2) ? map_to_cta(smem_u32(&full[s]), 0) : smem_u32(&full[s]);
-        const uint32_t bar_sf = (CG == 2) ? map_to_cta(smem_u32(&full_sf[s]), 0) : smem_u32(&full_sf[s]);
         if (elect_one()) {
           if (kt < kt_main) {
-            if (rank == 0) mbar_arrive_expect_tx(&full_sf[s], kSfBytes * CG);
-            tma_load_2d_bar<CG>(st + A_BYTES + C::B_BYTES, &tmSFA, 0, (mb * CG + rank) * k_groups4 + kt * 4, bar_sf);
+            if (rank == 0) mbar_arrive_expect_tx(&full[s], (kSfBytes + kAbBytes) * CG);
+            tma_load_2d_bar<CG>(st + A_BYTES + C::B_BYTES, &tmSFA, 0, (mb * CG + rank) * k_groups4 + kt * 4, bar);
 #pragma unroll
             for (int h = 0; h < BN / 128; ++h)
               tma_load_2d_bar<CG>(st + A_BYTES + C::B_BYTES + SFA_BYTES + h * 2048, &tmSFB, 0,
-                                  (nb * (BN / 128) + h) * k_groups4 + kt * 4, bar_sf);
-            if (rank == 0) mbar_arrive_expect_tx(&full[s], kAbBytes * CG);
+                                  (nb * (BN / 128) + h) * k_groups4 + kt * 4, bar);
             tma_load_2d_bar<CG>(st, &tmA, kt * 128, m0, bar);
             tma_load_2d_bar<CG>(st + A_BYTES, &tmB, kt * 128, nrow0, bar);
           } else {
-            if (rank == 0) { mbar_arrive(&full_sf[s]); mbar_arrive_expect_tx(&full[s], kAbBytes * CG); }
+            if (rank == 0) mbar_arrive_expect_tx(&full[s], kAbBytes * CG);
             const int lt = kt - kt_main;
             const int part = lt / lora_slabs, r0 = (lt % lora_slabs) * 64;
             if (la_fp16) {
@@ -403,133 +397,98 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
         }
         __syncwarp();
+        if (++s == C::STAGES) { s = 0; ph ^= 1; }
       }
     }
   } else if (warp == EPI_WARPS + 1) {
     // ------------------------------ MMA issuer (leader CTA only) ------------------------------
     if (rank == 0) {
       constexpr uint64_t kDescAB = smem_desc_base(0, 1024, kSwizzle128B);   // K-major, 8-row groups 1024 B apart
+      constexpr uint64_t kDescSF = smem_desc_base(0, 128, kSwizzleNone);    // 8 x 16 B core matrices, 128 B apart
       constexpr uint32_t kIdescMain = idesc_nvfp4(BM * CG, BN);
       constexpr uint32_t kIdescLora = idesc_f16(kBf16, kBf16, BM * CG, BN, false, false);
       constexpr uint32_t kIdescLoraF16 = idesc_f16(false, false, BM * CG, BN, false, false);
       constexpr uint16_t kMask = (CG == 2) ? 3 : 1;
-      uint32_t it = 0, tcount = 0, sf_it = 0;
+      const uint32_t smem16 = smem_desc_addr(smem);
+      uint32_t s = 0, ph = 0, tcount = 0, sb = 0, it = 0;
       bool ok = true;
+      uint32_t words = lora_words(pair);
       for (int w = pair; w < total_work && ok; w += num_pairs, ++tcount) {
         const int tile = SK ? w / S : w, split = SK ? w - tile * S : 0;
-        const uint32_t as = tcount % C::ACC_STAGES, aph = (tcount / C::ACC_STAGES) & 1;
-        if (!uwait(&acc_empty[as], aph ^ 1, ctx, kDevWaitAccFree, tcount)) { ok = false; break; }
-        tc_fence_after_sync();
-        const uint32_t tmem_acc = tmem_base + as * BN;
-        const bool la_fp16 = lora_fp16(tile % p.tiles_m);
+        const uint32_t as = tcount & 1;
+        const bool la_fp16 = lora_fp16(words);
+        words = lora_words(w + num_pairs);
         const int kt_all = kt_main + lora_parts(la_fp16) * lora_slabs;
-        const uint32_t idesc_lora = la_fp16 ? kIdescLoraF16 : kIdescLora;
         int kt_lo, kt_hi;
         slab_range(split, kt_all, kt_lo, kt_hi);
         SlabWalk walk;
         walk.start(kt_main, kt_all, p.interleave, lora_stride(la_fp16), kt_lo);
+        if (!uwait(&acc_empty[as], ((tcount >> 1) & 1) ^ 1, ctx, kDevWaitAccFree, tcount)) break;
+        tc_fence_after_sync();
+        const uint32_t acc = tmem_base + as * 128;
+        // 256-column tiles: the half shared with the tile before (in 128-column tiles acc_empty covers everything)
+        if (C::SHARED_ACC && tcount > 0) {
+          if (!uwait(acc_shared, (tcount - 1) & 1, ctx, kDevWaitAccFree, 0x20000 + tcount)) break;
+          tc_fence_after_sync();
+        }
         for (int pos = kt_lo; pos < kt_hi; ++pos, ++it) {
           const int kt = walk.at(pos);
-          const uint32_t s = it % C::STAGES, ph = (it / C::STAGES) & 1;
           if (!uwait(&full[s], ph, ctx, kDevWaitFull, it)) { ok = false; break; }
-          const bool main_slab = kt < kt_main;
-          const uint32_t sb = sf_it % C::SF_BUFS;            // its scales are in tensor memory: the copiers arrived on full[s]
           tc_fence_after_sync();
-          const uint32_t a_addr = smem_u32(smem + s * C::STAGE_BYTES);
-          const uint32_t b_addr = a_addr + A_BYTES;
-          const uint32_t tsfa = tmem_sf + sb * C::SF_COLS, tsfb = tsfa + C::SFA_COLS;
-          const int nkb = main_slab ? min(4, k_groups4 - kt * 4) : min(4, (p.R - ((kt - kt_main) % lora_slabs) * 64) / 16);
+          const uint32_t stage16 = smem16 + s * (C::STAGE_BYTES / 16);
+          const uint64_t da = kDescAB + stage16, db = da + A_BYTES / 16;
+          const uint32_t accumulate = pos == kt_lo ? 0u : 1u;
           if (elect_one()) {
-            if (main_slab) {
+            if (kt < kt_main) {
+              const uint64_t dsa = kDescSF + stage16 + (A_BYTES + C::B_BYTES) / 16, dsb = dsa + SFA_BYTES / 16;
+              const uint32_t tsfa = tmem_sf + sb * C::SF_COLS, tsfb = tsfa + C::SFA_COLS;
+              // the slab's k-blocks: all their scales, then their MMAs
+              auto k_blocks = [&](int nkb) {
 #pragma unroll
-              for (int j = 0; j < 4; ++j)
-                if (j < nkb)
-                  mma_nvfp4<CG>(tmem_acc, smem_desc(kDescAB, a_addr + j * 32), smem_desc(kDescAB, b_addr + j * 32),
-                                kIdescMain, tsfa + j * 4, tsfb + j * (BN / 32), ((pos - kt_lo) | j) != 0 ? 1u : 0u);
-              tc_commit_local<CG>(&sf_empty[sb]);   // scale buffer reusable once these MMAs are done
+                for (int j = 0; j < 4; ++j)
+                  if (j < nkb) {
+                    tmem_cp_scales<CG>(tsfa + j * 4, dsa + j * 32);
+#pragma unroll
+                    for (int h = 0; h < BN / 128; ++h) tmem_cp_scales<CG>(tsfb + j * (BN / 32) + h * 4, dsb + h * 128 + j * 32);
+                  }
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                  if (j < nkb)
+                    mma_nvfp4<CG>(acc, da + j * 2, db + j * 2, kIdescMain, tsfa + j * 4, tsfb + j * (BN / 32), j != 0 ? 1u : accumulate);
+              };
+              const int nkb = k_groups4 - kt * 4;
+              if (nkb >= 4) k_blocks(4); else k_blocks(nkb);      // the last slab may be short
             } else {
+              const uint32_t idesc = la_fp16 ? kIdescLoraF16 : kIdescLora;
+              const int nkb = (p.R - ((kt - kt_main) % lora_slabs) * 64) / 16;
 #pragma unroll
               for (int j = 0; j < 4; ++j)
-                if (j < nkb)
-                  mma_f16<CG>(tmem_acc, smem_desc(kDescAB, a_addr + j * 32), smem_desc(kDescAB, b_addr + j * 32),
-                              idesc_lora, ((pos - kt_lo) | j) != 0 ? 1u : 0u);
+                if (j < nkb) mma_f16<CG>(acc, da + j * 2, db + j * 2, idesc, j != 0 ? 1u : accumulate);
             }
             tc_commit_mask<CG>(&empty[s], kMask);          // stage reusable (in both CTAs) once these MMAs have read it
             if (pos == kt_hi - 1) tc_commit_mask<CG>(&acc_full[as], kMask);    // accumulator complete
           }
           __syncwarp();
-          if (main_slab) ++sf_it;
-        }
-      }
-    }
-  } else if (warp >= EPI_WARPS + 2) {
-    // ------------------------------ scale copiers (leader CTA only) ------------------------------
-    // Copies the scale atoms of main slab n into scale buffer n % SF_BUFS, up to SF_BUFS - 1 slabs ahead of the MMAs.
-    if (rank == 0) {
-      constexpr uint64_t kDescSF = smem_desc_base(0, 128, kSwizzleNone);    // 8 x 16 B core matrices, 128 B apart
-      const int jlo = (warp - (EPI_WARPS + 2)) * (4 / SF_WARPS);            // this warp's k-blocks: jlo, jlo + 1
-      uint32_t it = 0, sf_it = 0;
-      bool ok = true;
-      for (int w = pair; w < total_work && ok; w += num_pairs) {
-        const int tile = SK ? w / S : w, split = SK ? w - tile * S : 0;
-        const bool la_fp16 = lora_fp16(tile % p.tiles_m);
-        const int kt_all = kt_main + lora_parts(la_fp16) * lora_slabs;
-        int kt_lo, kt_hi;
-        slab_range(split, kt_all, kt_lo, kt_hi);
-        SlabWalk walk;
-        walk.start(kt_main, kt_all, p.interleave, lora_stride(la_fp16), kt_lo);
-        for (int pos = kt_lo; pos < kt_hi; ++pos, ++it) {
-          const int kt = walk.at(pos);
-          // Every slab's barrier is waited on in order, LoRA slabs (which carry no scales) included: a
-          // waiter that skipped ahead could get two ring revolutions in front of the producer, where the
-          // parity of a barrier no longer tells the revolutions apart.
-          const uint32_t s = it % C::STAGES, ph = (it / C::STAGES) & 1;
-          if (!uwait(&full_sf[s], ph, ctx, kDevWaitFull, 0x20000 + it)) { ok = false; break; }
-          if (kt >= kt_main) {                               // no scales: this copier's arrival on the stage's barrier at once
-            if (elect_one()) mbar_arrive(&full[s]);
-            __syncwarp();
-            continue;
-          }
-          const uint32_t sb = sf_it % C::SF_BUFS;
-          if (!uwait(&sf_empty[sb], ((sf_it / C::SF_BUFS) & 1) ^ 1, ctx, kDevWaitMisc, 0x20000 + it)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t sfa_addr = smem_u32(smem + s * C::STAGE_BYTES) + A_BYTES + C::B_BYTES;
-          const uint32_t sfb_addr = sfa_addr + SFA_BYTES;
-          const uint32_t tsfa = tmem_sf + sb * C::SF_COLS, tsfb = tsfa + C::SFA_COLS;
-          const int nkb = min(4, k_groups4 - kt * 4);
-          if (elect_one()) {
-#pragma unroll
-            for (int jj = 0; jj < 4 / SF_WARPS; ++jj) {
-              const int j = jlo + jj;
-              if (j < nkb) {
-                tmem_cp_scales<CG>(tsfa + j * 4, smem_desc(kDescSF, sfa_addr + j * 512));
-#pragma unroll
-                for (int h = 0; h < BN / 128; ++h)
-                  tmem_cp_scales<CG>(tsfb + j * (BN / 32) + h * 4, smem_desc(kDescSF, sfb_addr + h * 2048 + j * 512));
-              }
-            }
-            tc_commit_local<CG>(&full[s]);                   // arrives once these copies are done
-          }
-          __syncwarp();
-          ++sf_it;
+          if (++sb == C::SF_BUFS) sb = 0;
+          if (++s == C::STAGES) { s = 0; ph ^= 1; }
         }
       }
     }
   } else {
     // ------------------------------ epilogue (warps 0-7, both CTAs) ------------------------------
-    // Warp w drains the 32 accumulator rows of lane quarter w % 4 and the column half w / 4.
+    // Warp w drains the 32 accumulator rows of lane quarter w % 4, in strips of 64 columns: half w / 4 of each 128.
     const OutT* wc = static_cast<const OutT*>(p.wc);
     const OutT* bias = static_cast<const OutT*>(p.bias);
     const int quarter = warp & 3, chalf = warp >> 2;
-    uint8_t* my_bufs = store_bufs + warp * (C::STORE_BUFS * STORE_BUF_BYTES);
+    uint8_t* buf = store_bufs + warp * STORE_BUF_BYTES;
     const uint32_t swz = static_cast<uint32_t>(lane & 7);
-    uint32_t tcount = 0, nstore = 0;
+    uint32_t tcount = 0;
     bool ok = true;
     for (int w = pair; w < total_work && ok; w += num_pairs, ++tcount) {
       const int tile = SK ? w / S : w, split = SK ? w - tile * S : 0;
       const int mb = tile % p.tiles_m, nb = tile / p.tiles_m;
       const int m0 = (mb * CG + rank) * BM, n0 = nb * BN;
-      const uint32_t as = tcount % C::ACC_STAGES, aph = (tcount / C::ACC_STAGES) & 1;
+      const uint32_t as = tcount & 1, aph = (tcount >> 1) & 1;
       // stage this tile's per-column affine terms (the previous tile's readers are past the barrier below)
       [[maybe_unused]] bool odd_smooth = false;     // NEXT: some smooth_next of this tile is outside [2^-20, 2^20]
       for (int c = threadIdx.x; c < BN; c += EPI_WARPS * 32) {
@@ -556,29 +515,35 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       if (!mbar_wait(&acc_full[as], aph, ctx, kDevWaitAcc, tcount)) ok = false;
       tc_fence_after_sync();
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + as * BN + chalf * (BN / 2);
-      // Drain: every column this warp owns goes to registers in one burst, the accumulator is handed
-      // back at once, and only then do the affine, the packing and the stores happen.
-      uint32_t v[C::GROUPS_PER_WARP][2][32];
-      if constexpr (C::GROUPS_PER_WARP == 2) tmem_ld_32x32_x128(taddr, &v[0][0][0]);
-      else tmem_ld_32x32_x64(taddr, &v[0][0][0]);
+#pragma unroll 1
+      for (int q = 0; q < BN / 128; ++q) {
+      // A 256-column tile's shared half first: the next tile is waiting for those columns.
+      const int half = C::SHARED_ACC ? (q == 0 ? 1 - static_cast<int>(as) : static_cast<int>(as)) : 0;
+      const int cbase = half * 128 + chalf * 64;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + as * 128 + cbase;
+      // Drain: the strip goes to registers in one burst, its columns are handed back at once, and only then do the
+      // affine, the packing and the store happen.
+      uint32_t v[2][32];
+      tmem_ld_32x32_x64(taddr, &v[0][0]);
       tmem_ld_wait();
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {
-        if constexpr (CG == 2) mbar_arrive_cluster(&acc_empty[as], 0); else mbar_arrive(&acc_empty[as]);
+        uint64_t* bar = (C::SHARED_ACC && q == 0) ? acc_shared : &acc_empty[as];
+        if constexpr (CG == 2) mbar_arrive_cluster_relaxed(bar, 0); else mbar_arrive(bar);
       }
       bool finish = true;                       // this CTA writes the tile's rows of y
       if constexpr (SK) {
         if (S > 1) {
-          // Each thread parks its 16 x GROUPS_PER_WARP float4s at [j][thread] of the CTA's partial tile
+          // Each thread parks its 16 float4s at [j][thread] of the CTA's partial tile
           // (consecutive threads, consecutive 16 bytes) and later reads the same places of the other
           // partials, so no thread ever needs another thread's accumulator values.
-          constexpr int kVec = C::GROUPS_PER_WARP * 16;
+          static_assert(!SK || BN == 128, "a thread parks one strip");
+          constexpr int kVec = 16;
           constexpr int kTileVec = BM * BN / 4;
           const int tid = threadIdx.x;
           float4* mine = p.ws_partials + static_cast<size_t>(tile * S + split) * kTileVec;
-          const uint32_t* vf = &v[0][0][0];
+          const uint32_t* vf = &v[0][0];
 #pragma unroll
           for (int j = 0; j < kVec; ++j)
             __stcg(mine + j * (EPI_WARPS * 32) + tid,
@@ -595,7 +560,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             // per partial with all of a thread's loads in flight together, and the same order of
             // additions whatever order the CTAs finished in.
             const float4* first = p.ws_partials + static_cast<size_t>(tile * S) * kTileVec + tid;
-            uint32_t* vw = &v[0][0][0];
+            uint32_t* vw = &v[0][0];
 #pragma unroll
             for (int j = 0; j < kVec; ++j) {
               const float4 t = __ldcg(first + j * (EPI_WARPS * 32));
@@ -624,13 +589,9 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
       }
       if (finish) {
-#pragma unroll
-      for (int g = 0; g < C::GROUPS_PER_WARP; ++g, ++nstore) {
-        uint8_t* buf = my_bufs + (nstore % C::STORE_BUFS) * STORE_BUF_BYTES;
-        // the TMA store that last read this buffer must be done with it
-        if (lane == 0) tma_store_wait_read<C::STORE_BUFS - 1>();
+        // the TMA store that last read this warp's buffer must be done with it
+        if (lane == 0) tma_store_wait_read<0>();
         __syncwarp();
-        const int cbase = chalf * (BN / 2) + g * 64;
 #pragma unroll
         for (int hc = 0; hc < 2; ++hc) {
           const float4* wc4 = reinterpret_cast<const float4*>(affine + cbase + hc * 32);
@@ -640,8 +601,8 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           [[maybe_unused]] uint32_t qcodes[4], qscales[2];
           // the four fp32 results of columns 4 i .. 4 i + 3 of this half strip
           auto affine_at = [&](int i, float& a0, float& a1, float& a2, float& a3) {
-            a0 = __uint_as_float(v[g][hc][4 * i]); a1 = __uint_as_float(v[g][hc][4 * i + 1]);
-            a2 = __uint_as_float(v[g][hc][4 * i + 2]); a3 = __uint_as_float(v[g][hc][4 * i + 3]);
+            a0 = __uint_as_float(v[hc][4 * i]); a1 = __uint_as_float(v[hc][4 * i + 1]);
+            a2 = __uint_as_float(v[hc][4 * i + 2]); a3 = __uint_as_float(v[hc][4 * i + 3]);
             if (wc != nullptr) {
               const float4 w4 = wc4[i];
               a0 = __fmul_rn(a0, w4.x); a1 = __fmul_rn(a1, w4.y); a2 = __fmul_rn(a2, w4.z); a3 = __fmul_rn(a3, w4.w);
