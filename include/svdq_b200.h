@@ -57,8 +57,9 @@ const char* svdq_status_string(int status);
 int svdq_version(void);
 
 /*
- * One-time preparation of a smoothing vector: writes {smooth[k], 1/smooth[k]} as K float pairs
- * followed by one 8-byte flag word (so smooth_table holds 8*K + 8 bytes, 16-byte aligned).
+ * One-time preparation of a smoothing vector: writes the reciprocals and the factors the kernels
+ * multiply and divide by, two floats per column in an order of the kernels' own, followed by one
+ * 8-byte flag word (so smooth_table holds 8*K + 8 bytes, 16-byte aligned).
  * smooth is a per-layer constant, so callers build the table once and pass it with every
  * quantizer call.  No counterpart in the reference, which divides inside its kernel
  * (triton_kernels/quantize_w4a4_act_fuse_lora/kernel.py:153-158).

@@ -10,7 +10,7 @@
 // Decomposition.  A cluster of KS (1, 2, 4 or 8) CTAs owns one tile of 64 rows; CTA k
 // owns a contiguous range of 64-column slabs of K.  Per slab one producer warp
 // TMA-loads the x tile (64 x 64, 128-byte swizzle) with the slab's 64 entries of
-// the smoothing table (four 128-byte bulk copies) into a stage of the x ring, a
+// the smoothing table (one bulk copy) into a stage of the x ring, a
 // second one the matching lora_down slab (64 x R) into a ring of its own.
 // Two kinds of consumers read an x stage: two MMA-issuing warps (even and odd
 // slabs) accumulate x_tile @ lora_down_slab into [64 x R] fp32 accumulators in
@@ -33,21 +33,8 @@
 // scale bytes are adjacent in the atom layout; with a lane per row and a warp
 // per group the same stores touched 32 sectors each and cost 4 us more.
 //
-// Codes.  The scale byte is J * 2^E (J = 1..15), so floor(4 |v| / 2^E) is an
-// integer m and the E2M1 code is the number of n in {1,3,5,7,10,14,20} with
-// n J <= m.  m / (4 J) times (1 + 2^-20) is never on the wrong side of a
-// rounding bound of E2M1, so the hardware float -> E2M1 conversion of it
-// (cvt.rn.satfinite.e2m1x2.f32) yields exactly that count, with the sign, two
-// codes per instruction; see quantize_group.
-//
-// Exact arithmetic.  x / smooth must equal the IEEE quotient.  It is computed
-// as fma(x, r_hi, RN(x * r_lo)) with r_hi + r_lo = 1/s to 2^-47 from the table
-// (quantize_math.cuh); for operands with at most 11 significant bits this is the
-// correctly rounded quotient (checked exhaustively over mantissas), provided
-// nothing over- or underflows: the table builder raises a flag when a smooth
-// value lies outside [2^-60, 2^60] (2^16 for bf16) and the kernel then divides
-// with __fdiv_rn.  amax / 6 uses a three-step form q0 = a*r, q = fma(fma(-6, q0, a), r, q0)
-// (checked exhaustively as well).
+// Arithmetic: one multiplication per element in the place of each division, exact in every decision; see
+// quantize_math.cuh.
 #include "nvfp4_math.cuh"
 #include "quantize_math.cuh"
 #include "sm100.cuh"
@@ -72,34 +59,35 @@ constexpr int QUANT_WARPS = 4 * QUANT_GROUPS;
 constexpr bool kDirectExchange = SVDQ_DIRECT_EXCHANGE != 0;
 constexpr int AUX_WARPS = 4;                // x producer, MMA issuer (even slabs), lora_down producer, MMA issuer (odd slabs); with two K ranks they exchange the LoRA sums
 constexpr int NUM_THREADS = (AUX_WARPS + QUANT_WARPS) * 32;
-constexpr int TB_BYTES = SLAB_K * 8;       // {smooth, 1/smooth} of a slab's columns
-constexpr int TB_GROUP_STRIDE = 144;       // spacing of the four 128-byte group pieces in a stage
-
+constexpr int TB_BYTES = SLAB_K * 4;       // smoothing-table entries of a slab's columns
 
 template <int RP>
 struct Cfg {
-  // Two rings.  An x stage holds a 64 x 64 tile of x (8 KB) and the slab's 64 table entries; it is read by
-  // the MMA and by one quantize group and released by both.  A lora_down slab (64 x RP, 16 KB at rank
-  // 128) would make that stage three times as large and the ring a third as deep, and the stage would stay
+  // Two rings.  An x stage holds a 64 x 64 tile of x (8 KB) and, in an area of their own, the slab's 64 table
+  // entries; it is read by the MMA and by one quantize group and released by both.  A lora_down slab (64 x RP, 16 KB at
+  // rank 128) would make that stage three times as large and the ring a third as deep, and the stage would stay
   // held for the slab's four MMAs; in a ring of its own, which only the MMA reads, a few stages are enough
   // (the slabs come out of L2) and the x ring gets the rest of the shared memory.
-  static constexpr int X_STAGE_BYTES = X_BYTES + 1024;            // tile + table slab, padded to the 1 KB swizzled tiles need
   static constexpr int W_BYTES = SLAB_K * RP * 2;                 // lora_down slab
-  static constexpr int W_STAGES = RP > 128 ? 3 : 4;
+  // Six lora_down stages: a slab comes out of L2 in about 1.7 us while x streams in beside it, and slabs pass at
+  // 0.3 us (2 / 4 / 6 / 8 stages, 4352 rows: K = 3840 22.0 / 16.2 / 14.9 / 15.6 us, K = 10240 42.5 / 30.3 / 29.0 / 29.5);
+  // at rank 256 three are what fits.
+  static constexpr int W_STAGES = RP > 128 ? 3 : 6;
   // MMA-issuing warps.  Two take the slabs by turns; then both rings must be even, so that an issuer meets only slabs
   // of its own in a stage: one that went on to slab i could otherwise look at the stage while slab i - W_STAGES,
   // the other issuer's, is still on its way into it, and a one-bit parity would tell it that slab i is there.
   static constexpr int ISSUERS = W_STAGES % 2 == 0 ? 2 : 1;
   static constexpr int W_RING_BYTES = W_STAGES * W_BYTES;
   static constexpr int RECV_BYTES = (TILE_M / 2) * RP * 4;        // two K ranks: the peer's partial sums of this CTA's 32 rows
-  static constexpr int STAGES_RAW = (232448 - 1024 - 512 - 1024 - RECV_BYTES - W_RING_BYTES) / X_STAGE_BYTES;
+  static constexpr int STAGES_RAW = (232448 - 1024 - 512 - RECV_BYTES - W_RING_BYTES) / (X_BYTES + TB_BYTES);
   // A multiple of the group count: a group then always meets the same stages, and the slab it waits
   // for is the direct successor (in that stage) of one it consumed itself.  A one-bit phase parity
   // cannot tell "one revolution behind" from "one ahead"; this rule makes the second impossible.
   static constexpr int STAGES = ((STAGES_RAW > 16 ? 16 : STAGES_RAW) / QUANT_GROUPS) * QUANT_GROUPS;
-  static constexpr int RING_BYTES = STAGES * X_STAGE_BYTES;
-  static constexpr int BARS_OFF = RING_BYTES + W_RING_BYTES;
-  static constexpr int SMEM_BYTES = 1024 + BARS_OFF + 512 + 1024 + RECV_BYTES;   // rings, barriers, scale-constant table, receive buffer
+  static constexpr int RING_BYTES = STAGES * X_BYTES;
+  static constexpr int TB_OFF = RING_BYTES + W_RING_BYTES;
+  static constexpr int BARS_OFF = TB_OFF + STAGES * TB_BYTES;
+  static constexpr int SMEM_BYTES = 1024 + BARS_OFF + 512 + RECV_BYTES;          // rings, table entries, barriers, receive buffer
   static constexpr int TMEM_COLS = ISSUERS * RP;                  // an accumulator per issuer; a power of two >= 64
   static constexpr int EPI_COLS = RP / 4 < 32 ? 32 : RP / 4;      // accumulator columns per epilogue warp
   static_assert(TILE_M * RP * 4 <= RING_BYTES, "partial accumulator must fit in the x ring");
@@ -110,7 +98,7 @@ struct Cfg {
 };
 
 struct Params {
-  const float2* table;    // [K/2] entries of qmath::smooth_table_entry followed by one flag word, or null (no smoothing)
+  const float* table;     // smoothing table (layout in quantize_math.cuh), or null (no smoothing)
   uint8_t* act;           // [M_pad, K/2]
   uint8_t* scales;        // [K/16, M_pad]
   uint8_t* scales_swz;    // atom order or null
@@ -125,8 +113,6 @@ __device__ __forceinline__ uint32_t partial_slot(uint32_t row, uint32_t c4, uint
   return row * rp4 + (c4 ^ (row & 7u));
 }
 
-using qmath::quantize_group;
-using qmath::smooth_divide;
 using qmath::unpack_group;
 
 template <typename T, int RP>
@@ -151,8 +137,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ack_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   uint32_t* lora_unfit = tmem_slot + 2;        // bf16 form: some LoRA value this CTA wrote does not fit fp16
-  float2* scale_lut = reinterpret_cast<float2*>(smem + C::BARS_OFF + 512);   // per scale byte: {2^(2-E), ~1/(4J)}
-  float4* recv = reinterpret_cast<float4*>(smem + C::BARS_OFF + 512 + 1024);  // [32 rows][RP / 4], slots as partial_slot
+  float4* recv = reinterpret_cast<float4*>(smem + C::BARS_OFF + 512);        // [32 rows][RP / 4], slots as partial_slot
   const WaitCtx ctx{abort_flag};
 
   // warp index through a shuffle: provably warp-uniform, so the role branches are convergent code
@@ -190,7 +175,6 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     tmem_alloc(tmem_slot, C::TMEM_COLS);
     tmem_relinquish();
   }
-  qmath::fill_scale_lut(scale_lut, threadIdx.x, NUM_THREADS);
   tc_fence_before_sync();
   __syncthreads();
   // Two K ranks hand their partial sums to each other through the copy engine, counted on the partner's
@@ -203,7 +187,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   pdl_trigger();
   pdl_wait();
   // out-of-range smooth anywhere in K (flag word behind the table) selects the IEEE divide
-  const bool use_fdiv = has_table && reinterpret_cast<const uint32_t*>(p.table + p.K)[0] != 0u;
+  const bool use_fdiv = has_table && reinterpret_cast<const uint32_t*>(p.table + 2 * p.K)[0] != 0u;
 
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
@@ -211,18 +195,11 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     for (int i = 0; i < my_slabs; ++i) {
       const uint32_t s = i % C::STAGES, ph = (i / C::STAGES) & 1;
       if (!uwait(&empty[s], ph ^ 1, kDevWaitEmpty, i)) break;
-      uint8_t* st = smem + s * C::X_STAGE_BYTES;
       const int k0 = k_begin + i * SLAB_K;
       if (elect_one()) {
         mbar_arrive_expect_tx(&full[s], stage_bytes);
-        tma_load_2d(st, &tmX, k0, m0, &full[s]);
-        if (has_table) {
-          // one 128-byte piece per 16-column group, 144 bytes apart: the four groups a quad of lanes
-          // reads at once then sit in different banks
-#pragma unroll
-          for (int gq = 0; gq < 4; ++gq)
-            bulk_load_1d(st + X_BYTES + gq * TB_GROUP_STRIDE, p.table + k0 + gq * 16, 128, &full[s]);
-        }
+        tma_load_2d(smem + s * X_BYTES, &tmX, k0, m0, &full[s]);
+        if (has_table) bulk_load_1d(smem + C::TB_OFF + s * TB_BYTES, p.table + (use_fdiv ? p.K : 0) + k0, TB_BYTES, &full[s]);
       }
       __syncwarp();
     }
@@ -260,7 +237,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       if (!uwait(&full[s], ph, kDevWaitFull, i)) break;
       if (has_lora && !uwait(&wfull[sw], phw, kDevWaitFull, 0x50000 + i)) break;
       tc_fence_after_sync();
-      const uint64_t da = kDescA + (x16 + s * (C::X_STAGE_BYTES / 16)), db = kDescB + (w16 + sw * (C::W_BYTES / 16));
+      const uint64_t da = kDescA + (x16 + s * (X_BYTES / 16)), db = kDescB + (w16 + sw * (C::W_BYTES / 16));
       if (elect_one()) {
         if (has_lora) {
 #pragma unroll
@@ -292,7 +269,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     for (int i = grp; i < my_slabs; i += QUANT_GROUPS) {
       const uint32_t s = i % C::STAGES, ph = (i / C::STAGES) & 1;
       if (!mbar_wait(&full[s], ph, ctx, kDevWaitFull, 0x10000 + i)) break;
-      const uint8_t* st = smem + s * C::X_STAGE_BYTES;
+      const uint8_t* st = smem + s * X_BYTES;
       uint4 raw[2][2];
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
@@ -302,17 +279,14 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
         raw[rr][1] = *reinterpret_cast<const uint4*>(xrow + (((2 * g + 1) ^ (row & 7)) << 4));
       }
       float2 f[2][8];
-      if (has_table && !use_fdiv) {
+      if (has_table) {
         unpack_group<T, false>(raw[0][0], raw[0][1], f[0]);
         unpack_group<T, false>(raw[1][0], raw[1][1], f[1]);
+        // this lane's 16 columns' entries landed with the slab
+        qmath::smooth_divide2(f[0], f[1], reinterpret_cast<const float4*>(smem + C::TB_OFF + s * TB_BYTES) + g, use_fdiv);
       } else {
         unpack_group<T, true>(raw[0][0], raw[0][1], f[0]);
         unpack_group<T, true>(raw[1][0], raw[1][1], f[1]);
-      }
-      if (has_table) {
-        // {smooth, 1/smooth} of this lane's 16 columns landed with the slab
-        const float4* tb = reinterpret_cast<const float4*>(st + X_BYTES + g * TB_GROUP_STRIDE);
-        qmath::smooth_divide2(f[0], f[1], tb, use_fdiv);
       }
       // Hand the stage back.  The ring was read through the generic proxy and will be overwritten
       // through the async proxy (TMA); mbarrier arrivals are performed by a separate unit and do not
@@ -330,7 +304,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
         // one group after the other, each stored as soon as it is done: running both groups' scale chains
         // side by side and keeping their results in registers until the end measured 5-8 % slower
         uint32_t c_lo, c_hi, s_b;
-        qmath::quantize_group(f[rr], scale_lut, c_lo, c_hi, s_b);
+        qmath::quantize_group_near(f[rr], c_lo, c_hi, s_b);
         *reinterpret_cast<uint2*>(act_base + static_cast<size_t>(row) * (p.K >> 1) + (k0 >> 1)) = make_uint2(c_lo, c_hi);
         p.scales[static_cast<size_t>(gi) * p.M_pad + m0 + row] = static_cast<uint8_t>(s_b);
         if (p.scales_swz != nullptr) p.scales_swz[sf_swizzled_offset(m0 + row, gi, groups)] = static_cast<uint8_t>(s_b);
@@ -533,12 +507,12 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   }
 }
 
-// Per column pair one table entry (qmath::smooth_table_entry), then one flag word: 1 if any smooth value
-// lies outside [2^-60, 2^60] (2^16 for bf16; negative, zero and NaN count as outside), where the two-step
-// divide could over- or underflow or leave a zero with the wrong sign; the entries then hold the smooth
-// values themselves and the kernels divide with __fdiv_rn.
+// The smoothing table: K reciprocals, K factors, one flag word: 1 if any smooth value lies outside [2^-60, 2^60]
+// (2^16 for bf16; negative, zero and NaN count as outside), where the multiplications could over- or underflow or
+// leave a zero with the wrong sign; the kernels then divide by the factors with __fdiv_rn.  (K not a multiple of 64
+// is outside the fused kernels' contract: no slabs, no permutation.)
 template <typename T>
-__global__ void smooth_table_kernel(const T* __restrict__ smooth, float2* __restrict__ table, int K) {
+__global__ void smooth_table_kernel(const T* __restrict__ smooth, float* __restrict__ table, int K) {
   // upper bound: 2^60 for fp16 inputs; 2^16 for bf16 inputs, whose smallest subnormal (2^-133)
   // divided by anything larger would underflow to a signed zero
   constexpr float kMaxSmooth = std::is_same<T, __nv_bfloat16>::value ? 65536.0f : 1.1529215e18f;
@@ -548,13 +522,12 @@ __global__ void smooth_table_kernel(const T* __restrict__ smooth, float2* __rest
   for (int i = threadIdx.x; i < K; i += blockDim.x) {
     const float s = to_f32(smooth[i]);
     if (!(s >= 8.6736174e-19f && s <= kMaxSmooth)) bad = 1;      // also: negative, zero or NaN
+    const int slot = K % 64 == 0 ? qmath::smooth_table_slot(i) : i;
+    table[slot] = qmath::smooth_reciprocal(s);
+    table[K + slot] = s;
   }
   __syncthreads();
-  const bool exact_divide = bad != 0;
-  float4* pairs = reinterpret_cast<float4*>(table);
-  for (int i = threadIdx.x; i < K / 2; i += blockDim.x)
-    pairs[i] = qmath::smooth_table_entry(to_f32(smooth[2 * i]), to_f32(smooth[2 * i + 1]), exact_divide);
-  if (threadIdx.x == 0) *reinterpret_cast<uint2*>(table + K) = make_uint2(exact_divide ? 1u : 0u, 0u);
+  if (threadIdx.x == 0) *reinterpret_cast<uint2*>(table + 2 * K) = make_uint2(bad != 0 ? 1u : 0u, 0u);
 }
 
 }  // namespace qf
@@ -592,9 +565,9 @@ bool quantize_fused_supported(int M, int K, int R, int M_pad) {
 
 int launch_smooth_table(const void* smooth, void* table, int K, int dtype, cudaStream_t stream) {
   if (dtype == SVDQ_DTYPE_F16)
-    qf::smooth_table_kernel<__half><<<1, 1024, 0, stream>>>(static_cast<const __half*>(smooth), static_cast<float2*>(table), K);
+    qf::smooth_table_kernel<__half><<<1, 1024, 0, stream>>>(static_cast<const __half*>(smooth), static_cast<float*>(table), K);
   else if (dtype == SVDQ_DTYPE_BF16)
-    qf::smooth_table_kernel<__nv_bfloat16><<<1, 1024, 0, stream>>>(static_cast<const __nv_bfloat16*>(smooth), static_cast<float2*>(table), K);
+    qf::smooth_table_kernel<__nv_bfloat16><<<1, 1024, 0, stream>>>(static_cast<const __nv_bfloat16*>(smooth), static_cast<float*>(table), K);
   else
     return SVDQ_ERR_DTYPE;
   return cudaGetLastError() == cudaSuccess ? SVDQ_OK : SVDQ_ERR_LAUNCH;
@@ -677,7 +650,7 @@ int launch_quantize_fused(const void* x, const void* lora_down, const void* smoo
   if (!quantize_fused_supported(M, K, R, M_pad)) return SVDQ_ERR_UNSUPPORTED;
   if (reinterpret_cast<uintptr_t>(smooth_table) % 16 != 0) return SVDQ_ERR_ALIGN;   // bulk copies start on 16-byte boundaries
   qf::Params p;
-  p.table = static_cast<const float2*>(smooth_table);
+  p.table = static_cast<const float*>(smooth_table);
   p.act = static_cast<uint8_t*>(act);
   p.scales = static_cast<uint8_t*>(ascales);
   p.scales_swz = static_cast<uint8_t*>(ascales_swz);

@@ -1,32 +1,38 @@
-// Per-group arithmetic of the activation quantizer, shared by both fused kernels.
+// Per-group arithmetic of the quantizers.
 //
 // Results follow baseline/kernels/quantize_w4a4_act_fuse_lora/ref.py:40-48 and
 // baseline/kernels/_nvfp4.py:27-41, :82-91 of the reference bit for bit; none of it
-// runs a per-element IEEE divide.  Two fp32 lanes at a time where the hardware has
-// a packed instruction (mul / fma on f32x2), three-input |max| for the group amax,
-// and a 128-entry table in shared memory for the two constants that depend on the
-// scale byte.
+// runs a per-element IEEE divide.
 //
-// Smoothing divide.  x / s must equal the IEEE quotient.  With r_hi = RU(1/s) (rounded up) and
-// r_lo = RN(1/s - r_hi) <= 0, r_hi + r_lo equals 1/s to 2^-47, and q = fma(x, r_hi, RN(x * r_lo)) is
-// the correctly rounded quotient for operands of at most 11 significant bits: such a quotient is
-// never closer than 2^-36 (relative) to a midpoint between two fp32 numbers, unless it is exactly
-// representable (checked exhaustively over mantissa pairs on the CPU).  Rounding r_hi UP makes r_lo
-// non-positive (-0 when 1/s is exact), which is what turns a -0 input into a +0 quotient:
-// (-0) * r_lo = +0 and (-0) * r_hi + (+0) = +0, as the reference's sign rule needs.  Nothing may
-// over- or underflow: the table builder sets a flag when a smooth value lies outside the safe range,
-// and then stores {s0, s1, -, -} for the kernels to divide with __fdiv_rn.  Per column pair the table
-// holds {r_hi0, r_hi1, r_lo0, r_lo1}.
+// Activations (the fused kernels).  Only decisions leave the kernel - a scale byte per group, a code per
+// element - so nothing needs the quotients themselves, only the side of each bound they are on.  Inputs
+// and smoothing factors have at most 11 significant bits, scales 4 and bounds of codes 3, so a quotient
+// x / s that is not exactly on a bound is off it by more than 2^-19.2 of it (a scale's rounding
+// bound: 2^-18.5).  One fp32 multiplication by a reciprocal is good to 2^-23, and errs on a known side if
+// the reciprocal is nudged: f = x r with r = RN((1 / s)(1 + 2^-22)) is above the exact quotient by
+// 2^-24 to 2^-21.4 of it.
+//   codes   the E2M1 conversion (nearest, two elements an instruction) of f c, c = rcp(scale)(1 + 2^-21):
+//           a quotient on a bound comes out above it, as the definition wants, one below it stays below
+//   scales  RN(f RN((1/6)(1 - 2^-22))), rounded to 20 significant bits: a quotient on a rounding bound of
+//           E4M3, which has at most 5, is put back on it exactly (so that its tie rule decides), any
+//           other stays on its side
+// (checked exhaustively over significand pairs on the CPU).  A group costs some 60 instructions, a third of
+// the two-step IEEE quotient with a truncation that this replaced, and a smoothing factor's table entry
+// is 4 bytes instead of 8; with the same kernel around it 4352 rows of 3840 / 10240 / 15360 columns
+// went from 16.4 / 33.5 / 54.9 to 16.2 / 30.4 / 49.8 us.  f = fma(x, r, +0) turns a -0 input into +0, which the reference's sign rule wants.
+// Nothing may over- or underflow: the table builder sets a flag when a smooth value lies outside the safe
+// range, and the kernels then divide with __fdiv_rn, after which the same steps hold (f exact).
+// Groups whose scale byte is 0 (everything non-zero saturates) or the 448 clamp (ratios are unbounded)
+// compare against the seven exact products instead.
 //
-// Codes.  The scale byte is J * 2^E (J = 1..15), so m = trunc(4 v / 2^E) is an integer
-// with v's sign and the E2M1 code is the number of n in {1,3,5,7,10,14,20} with
-// n J <= |m|.  m / (4 J) lies on a rounding bound of E2M1 exactly when |m| = n J and at
+// fp32 values (weights, the next layer's activations in the GEMM's epilogue) have 24 significant bits, so
+// their quotient by the scale needs an exact floor.  The scale byte is J * 2^E (J = 1..15), so
+// m = trunc(4 v / 2^E) is an integer with v's sign and the E2M1 code is the number of n in
+// {1,3,5,7,10,14,20} with n J <= |m|.  m / (4 J) lies on a rounding bound of E2M1 exactly when |m| = n J and at
 // least 1/(4 J) away from every bound otherwise, so RN(m * RN(1/(4 J)) * (1 + 2^-20))
 // is strictly above the bound in the first case and on the right side of it in the
 // second, and the hardware conversion cvt.rn.satfinite.e2m1x2.f32 of it returns the
 // reference's code, sign included (checked exhaustively over J and m on the CPU).
-// Groups whose scale byte is 0 (everything non-zero saturates) or the 448 clamp
-// (ratios are unbounded) compare against the seven exact products instead.
 #pragma once
 
 #include "nvfp4_math.cuh"
@@ -37,7 +43,7 @@ namespace qmath {
 
 // Widen a pair of 16-bit values.  CANON adds +0 first, which turns -0 into +0 and changes nothing
 // else (the reference gives a zero the sign bit only when the value tests < 0).  The smoothing
-// divide of the fast path does the same by itself (see above), so only the other paths ask for it.
+// does the same by itself (see above), so only calls without it ask for it.
 template <typename T, bool CANON> __device__ __forceinline__ float2 unpack2(uint32_t v);
 template <> __device__ __forceinline__ float2 unpack2<__half, true>(uint32_t v) {
   return __half22float2(__hadd2(*reinterpret_cast<__half2*>(&v), __float2half2_rn(0.0f)));
@@ -61,57 +67,38 @@ __device__ __forceinline__ void unpack_group(const uint4& lo16, const uint4& hi1
   for (int j = 0; j < 8; ++j) f[j] = unpack2<T, CANON>(w[j]);
 }
 
-// Smoothing divide of one 16-element group; tb points at the group's eight table entries in shared
-// memory (the same address in every lane of a quad column): {r_hi0, r_hi1, r_lo0, r_lo1}, or
-// {s0, s1, -, -} when the launch divides with __fdiv_rn.
-__device__ __forceinline__ void smooth_divide(float2 (&f)[8], const float4* tb, bool use_fdiv) {
-  if (!use_fdiv) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float4 t = tb[j];
-      f[j] = __ffma2_rn(f[j], make_float2(t.x, t.y), __fmul2_rn(f[j], make_float2(t.z, t.w)));
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float4 t = tb[j];
-      f[j].x = __fadd_rn(__fdiv_rn(f[j].x, t.x), 0.0f);           // an underflow to -0 counts as +0
-      f[j].y = __fadd_rn(__fdiv_rn(f[j].y, t.y), 0.0f);
-    }
-  }
+// The smoothing table (svdq_prepare_smooth): K reciprocals, then K smoothing factors, as floats, then the flag
+// word.  Inside each 64-column slab the entries lie so that the four lanes of a quad, which work on the slab's
+// four 16-column groups, read 64 consecutive bytes at once: chunk j (four columns) of group g at float4 4 j + g.
+__host__ __device__ __forceinline__ int smooth_table_slot(int k) {
+  return (k & ~63) | ((k & 12) << 2) | ((k & 48) >> 2) | (k & 3);
+}
+// table entry of one column; float64 keeps the nudged reciprocal to a single rounding
+__device__ __forceinline__ float smooth_reciprocal(float s) {
+  return static_cast<float>((1.0 / static_cast<double>(s)) * (1.0 + 2.384185791015625e-07));
 }
 
-// Two rows of the same 16 columns: every table entry is loaded once.  A 16-byte shared-memory load costs
-// four wavefronts of the load/store unit however many lanes share its address, and that unit (x loads, table
-// loads, the stores, the MMA's operand reads and the TMA's writes all pass through it) is what the fused
-// quantizer saturates.
+// Near quotients of two rows of the same 16 columns; tb points at the group's chunk 0 of the slab's 64 entries in
+// shared memory (the smoothing factors themselves when the launch divides with __fdiv_rn).  Every entry is loaded
+// once for both rows: a 16-byte shared-memory load costs its wavefronts however many lanes share its address,
+// and the load/store unit is what the fused quantizer keeps busiest.
 __device__ __forceinline__ void smooth_divide2(float2 (&f0)[8], float2 (&f1)[8], const float4* tb, bool use_fdiv) {
-  if (!use_fdiv) {
+  const float2 zero = make_float2(0.0f, 0.0f);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float4 t = tb[j];
-      const float2 hi = make_float2(t.x, t.y), lo = make_float2(t.z, t.w);
-      f0[j] = __ffma2_rn(f0[j], hi, __fmul2_rn(f0[j], lo));
-      f1[j] = __ffma2_rn(f1[j], hi, __fmul2_rn(f1[j], lo));
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float4 t = tb[j];
-      f0[j].x = __fadd_rn(__fdiv_rn(f0[j].x, t.x), 0.0f);          // an underflow to -0 counts as +0
-      f0[j].y = __fadd_rn(__fdiv_rn(f0[j].y, t.y), 0.0f);
-      f1[j].x = __fadd_rn(__fdiv_rn(f1[j].x, t.x), 0.0f);
-      f1[j].y = __fadd_rn(__fdiv_rn(f1[j].y, t.y), 0.0f);
+  for (int j = 0; j < 4; ++j) {
+    const float4 t = tb[4 * j];
+    const float2 a = make_float2(t.x, t.y), b = make_float2(t.z, t.w);
+    if (!use_fdiv) {
+      f0[2 * j] = __ffma2_rn(f0[2 * j], a, zero); f0[2 * j + 1] = __ffma2_rn(f0[2 * j + 1], b, zero);
+      f1[2 * j] = __ffma2_rn(f1[2 * j], a, zero); f1[2 * j + 1] = __ffma2_rn(f1[2 * j + 1], b, zero);
+    } else {
+      auto div = [](float2 v, float2 d) {                          // an underflow to -0 counts as +0
+        return make_float2(__fadd_rn(__fdiv_rn(v.x, d.x), 0.0f), __fadd_rn(__fdiv_rn(v.y, d.y), 0.0f));
+      };
+      f0[2 * j] = div(f0[2 * j], a); f0[2 * j + 1] = div(f0[2 * j + 1], b);
+      f1[2 * j] = div(f1[2 * j], a); f1[2 * j + 1] = div(f1[2 * j + 1], b);
     }
   }
-}
-
-// Table entry of one column pair (see above); `exact_divide` selects the {s0, s1} form.
-__device__ __forceinline__ float4 smooth_table_entry(float s0, float s1, bool exact_divide) {
-  if (exact_divide) return make_float4(s0, s1, 0.0f, 0.0f);
-  const float h0 = __frcp_ru(s0), h1 = __frcp_ru(s1);
-  const float e0 = fmaf(-s0, h0, 1.0f), e1 = fmaf(-s1, h1, 1.0f);   // exact: 1 - s * r_hi, <= 0
-  return make_float4(h0, h1, e0 == 0.0f ? -0.0f : __fmul_rn(e0, h0), e1 == 0.0f ? -0.0f : __fmul_rn(e1, h1));
 }
 
 // {2^(2-E), RN(1/(4 J)) (1 + 2^-20)} of scale byte sb = J 2^E; {0, 0} for the two bytes that take the compare path
@@ -175,14 +162,15 @@ __device__ __forceinline__ uint32_t scale_byte(float amax) {
   return static_cast<uint32_t>(__nv_cvt_float_to_fp8(s, __NV_SATFINITE, __NV_E4M3));
 }
 
-// amax of a 16-element group -> scale byte
-__device__ __forceinline__ uint32_t group_scale_byte(const float2 (&f)[8]) {
+// max |f| of a 16-element group
+__device__ __forceinline__ float group_amax(const float2 (&f)[8]) {
   const float m0 = max3abs(f[0].x, f[0].y, f[1].x), m1 = max3abs(f[1].y, f[2].x, f[2].y);
   const float m2 = max3abs(f[3].x, f[3].y, f[4].x), m3 = max3abs(f[4].y, f[5].x, f[5].y);
   const float m4 = max3abs(f[6].x, f[6].y, f[7].x);
-  const float amax = fmaxf(max3abs(m0, m1, m2), max3abs(m3, m4, f[7].y));
-  return scale_byte(amax);
+  return fmaxf(max3abs(m0, m1, m2), max3abs(m3, m4, f[7].y));
 }
+// amax of a 16-element group -> scale byte
+__device__ __forceinline__ uint32_t group_scale_byte(const float2 (&f)[8]) { return scale_byte(group_amax(f)); }
 
 // Main path of the codes: k = {2^(2-E), ~1/(4J)} of the group's scale byte.
 // m = trunc(4 v / 2^E) keeps the sign of v (also as -0 for a small negative v, whose code is
@@ -234,15 +222,35 @@ __device__ __forceinline__ void quantize_group_with(float2 (&f)[8], uint32_t sb,
   else group_codes_compare(f, sb, code_lo, code_hi);
 }
 
-// One 16-element group (smoothed, fp32): amax, scale byte, eight code bytes.  scale_lut: the table
-// fill_scale_lut made in shared memory, or null to work the two constants out on the spot.
-__device__ __forceinline__ void quantize_group(float2 (&f)[8], const float2* scale_lut,
-                                               uint32_t& code_lo, uint32_t& code_hi, uint32_t& sbyte) {
-  const uint32_t sb = group_scale_byte(f);
+// Scale byte from the largest near quotient of a group (see the head of this file).  Values above 448 saturate in
+// the conversion, values below the smallest scale's rounding bound give byte 0: no clamps.
+__device__ __forceinline__ uint32_t scale_byte_near(float amax) {
+  const float v = amax * 0.16666662693023681640625f;                   // RN((1/6)(1 - 2^-22))
+  const float snapped = __uint_as_float((__float_as_uint(v) + 8u) & 0xFFFFFFF0u);
+  return static_cast<uint32_t>(__nv_cvt_float_to_fp8(snapped, __NV_SATFINITE, __NV_E4M3));
+}
+__device__ __forceinline__ float rcp_approx(float v) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+// One 16-element group of near quotients: scale byte and eight code bytes
+__device__ __forceinline__ void quantize_group_near(const float2 (&f)[8], uint32_t& code_lo, uint32_t& code_hi, uint32_t& sbyte) {
+  const uint32_t sb = scale_byte_near(group_amax(f));
   sbyte = sb;
-  const float2 k = scale_lut != nullptr ? scale_lut[sb] : scale_constants(sb);
-  if (k.x != 0.0f) group_codes_fast(f, k, code_lo, code_hi);
-  else group_codes_compare(f, sb, code_lo, code_hi);
+  if (sb - 1u < 0x7Du) {
+    const __half_raw h = __nv_cvt_fp8_to_halfraw(static_cast<__nv_fp8_storage_t>(sb), __NV_E4M3);
+    const float c = rcp_approx(__half2float(__half(h))) * 1.000000476837158203125f;     // 1 + 2^-21
+    const float2 cc = make_float2(c, c);
+    float2 w[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = __fmul2_rn(f[j], cc);
+    code_lo = cvt_e2m1x8(w[0], w[1], w[2], w[3]);
+    code_hi = cvt_e2m1x8(w[4], w[5], w[6], w[7]);
+  } else {
+    group_codes_compare(f, sb, code_lo, code_hi);
+  }
 }
 
 }  // namespace qmath

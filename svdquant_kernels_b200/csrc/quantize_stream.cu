@@ -42,8 +42,7 @@ constexpr int W_BYTES = SLAB_K * RP * 2;   // lora_down slab: 16 KB
 constexpr int QUANT_WARPS = 16;
 constexpr int AUX_WARPS = 4;               // producer, MMA issuer, two helpers; together they drain the accumulator
 constexpr int NUM_THREADS = (AUX_WARPS + QUANT_WARPS) * 32;
-constexpr int TB_BYTES = SLAB_K * 8;       // table entries of a slab's columns
-constexpr int TB_GROUP_STRIDE = 144;       // spacing of the four 128-byte group pieces in a stage
+constexpr int TB_BYTES = SLAB_K * 4;       // table entries of a slab's columns
 constexpr int kTicketBytes = 2048;         // arrival counters [256], then completion counters [256]
 
 template <int TM>
@@ -56,7 +55,7 @@ struct Cfg {
   // a multiple of the group count, so that a group always meets the same stages (see quantize_fused.cu)
   static constexpr int STAGES = STAGES_RAW > 8 ? 8 : (STAGES_RAW / QUANT_GROUPS) * QUANT_GROUPS;
   static constexpr int RING_BYTES = STAGES * STAGE_BYTES;
-  static constexpr int SMEM_BYTES = 1024 + RING_BYTES + 512 + 1024;   // ring, barriers, scale-constant table
+  static constexpr int SMEM_BYTES = 1024 + RING_BYTES + 512;          // ring, barriers
   static constexpr int TMEM_COLS = TM;
   static_assert(TM == 128 || TM == 256, "tile height");
   static_assert(GROUP_WARPS * 16 == TM, "16 rows per quantize warp");
@@ -64,7 +63,7 @@ struct Cfg {
 };
 
 struct Params {
-  const float2* table;    // [K/2] entries of qmath::smooth_table_entry followed by one flag word, or null (no smoothing)
+  const float* table;     // smoothing table (layout in quantize_math.cuh), or null (no smoothing)
   uint8_t* act;           // [M_pad, K/2]
   uint8_t* scales;        // [K/16, M_pad]
   uint8_t* scales_swz;    // atom order or null
@@ -137,7 +136,6 @@ quantize_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   uint32_t* lora_unfit = tmem_slot + 2;        // [8] bf16 form: per 32 rows of the tile, some value does not fit fp16
-  float2* scale_lut = reinterpret_cast<float2*>(smem + C::RING_BYTES + 512);
   const WaitCtx ctx{abort_flag};
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -170,7 +168,6 @@ quantize_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     tmem_alloc(tmem_slot, C::TMEM_COLS);
     tmem_relinquish();
   }
-  qmath::fill_scale_lut(scale_lut, threadIdx.x, NUM_THREADS);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -178,7 +175,7 @@ quantize_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
   // set-up done; what follows reads and writes global memory
   pdl_trigger();
   pdl_wait();
-  const bool use_fdiv = has_table && reinterpret_cast<const uint32_t*>(p.table + p.K)[0] != 0u;
+  const bool use_fdiv = has_table && reinterpret_cast<const uint32_t*>(p.table + 2 * p.K)[0] != 0u;
 
   bool aux_ok = true;
   if (warp == 0) {
@@ -197,11 +194,7 @@ quantize_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
           tma_load_2d(st + C::X_BYTES, &tmW, 0, k0, &full[s]);
           tma_load_2d(st + C::X_BYTES + SLAB_K * 128, &tmW, 64, k0, &full[s]);
         }
-        if (has_table) {
-#pragma unroll
-          for (int gq = 0; gq < 4; ++gq)
-            bulk_load_1d(st + C::X_BYTES + W_BYTES + gq * TB_GROUP_STRIDE, p.table + k0 + gq * 16, 128, &full[s]);
-        }
+        if (has_table) bulk_load_1d(st + C::X_BYTES + W_BYTES, p.table + (use_fdiv ? p.K : 0) + k0, TB_BYTES, &full[s]);
       }
       __syncwarp();
     }
@@ -258,17 +251,13 @@ quantize_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
         raw[rr][1] = *reinterpret_cast<const uint4*>(xrow + (((2 * g + 1) ^ (row & 7)) << 4));
       }
       float2 f[2][8];
-      if (has_table && !use_fdiv) {
+      if (has_table) {
         qmath::unpack_group<T, false>(raw[0][0], raw[0][1], f[0]);
         qmath::unpack_group<T, false>(raw[1][0], raw[1][1], f[1]);
+        qmath::smooth_divide2(f[0], f[1], reinterpret_cast<const float4*>(st + C::X_BYTES + W_BYTES) + g, use_fdiv);
       } else {
         qmath::unpack_group<T, true>(raw[0][0], raw[0][1], f[0]);
         qmath::unpack_group<T, true>(raw[1][0], raw[1][1], f[1]);
-      }
-      if (has_table) {
-        const float4* tb = reinterpret_cast<const float4*>(st + C::X_BYTES + W_BYTES + g * TB_GROUP_STRIDE);
-        qmath::smooth_divide(f[0], tb, use_fdiv);
-        qmath::smooth_divide(f[1], tb, use_fdiv);
       }
       // Hand the stage back: the ring was read through the generic proxy and will be overwritten through
       // the async proxy (TMA); an mbarrier arrival does not wait for earlier shared-memory loads.
@@ -285,7 +274,7 @@ quantize_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
         // one group after the other, each stored as soon as it is done: running both groups' scale chains
         // side by side and keeping their results in registers until the end measured 5-8 % slower
         uint32_t c_lo, c_hi, s_b;
-        qmath::quantize_group(f[rr], scale_lut, c_lo, c_hi, s_b);
+        qmath::quantize_group_near(f[rr], c_lo, c_hi, s_b);
         *reinterpret_cast<uint2*>(act_base + static_cast<size_t>(row) * (p.K >> 1) + (k0 >> 1)) = make_uint2(c_lo, c_hi);
         p.scales[static_cast<size_t>(gi) * p.M_pad + m0 + row] = static_cast<uint8_t>(s_b);
         if (p.scales_swz != nullptr) p.scales_swz[sf_swizzled_offset(m0 + row, gi, groups)] = static_cast<uint8_t>(s_b);
@@ -475,7 +464,7 @@ int launch_quantize_stream(const void* x, const void* lora_down, const void* smo
   }
   if (reinterpret_cast<uintptr_t>(smooth_table) % 16 != 0) return SVDQ_ERR_ALIGN;
   qs::Params p;
-  p.table = static_cast<const float2*>(smooth_table);
+  p.table = static_cast<const float*>(smooth_table);
   p.act = static_cast<uint8_t*>(act);
   p.scales = static_cast<uint8_t*>(ascales);
   p.scales_swz = static_cast<uint8_t*>(ascales_swz);
