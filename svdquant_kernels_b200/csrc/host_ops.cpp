@@ -26,6 +26,8 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/library.h>
 
+#include <unordered_map>
+
 #include "../../include/svdq_b200.h"
 
 namespace {
@@ -57,20 +59,65 @@ struct Ref {                            // owned reference
   ~Ref() { Py_XDECREF(p); }
 };
 
-// The twin recorded for `owner` on its storage object (the records ops._attach keeps: {(offset, numel):
-// (twin, version)}); an undefined tensor if there is none or it is out of date.  GIL held.
-Tensor attached(const Tensor& owner, bool any_version = false) {
+// A twin as the launches need it; `hold` keeps a twin with a storage of its own alive.
+struct Twin {
+  void* ptr = nullptr;
+  ScalarType type = at::kByte;
+  int64_t numel = 0;
+  Tensor hold;
+  bool found() const { return ptr != nullptr || hold.defined(); }
+  void* data() const { return numel > 0 ? ptr : nullptr; }
+};
+
+// Twins that live in their owner's own storage (see `allocate_together`): storage -> where they are and for
+// which version of which tensor of that storage they hold.  A weak reference keeps the StorageImpl's address from
+// being used again while an entry exists, not its memory; entries of storages that are gone are swept out every
+// kSweep insertions.  All access with the GIL held.
+struct InnerTwin {
+  int64_t offset, numel;                // the owner: storage offset in its own elements, element count
+  uint32_t version;
+  int64_t byte_offset, twin_numel;      // the twin
+  ScalarType type;
+};
+struct InnerTwins {
+  c10::weak_intrusive_ptr<c10::StorageImpl> storage;
+  InnerTwin rec[2];
+};
+constexpr size_t kSweep = 256;
+std::unordered_map<const c10::StorageImpl*, InnerTwins>& inner_twins() {
+  static auto* table = new std::unordered_map<const c10::StorageImpl*, InnerTwins>();     // outlives every tensor
+  return *table;
+}
+InnerTwin* inner_twin(const Tensor& owner) {
+  auto& table = inner_twins();
+  if (table.empty()) return nullptr;
+  const auto it = table.find(owner.storage().unsafeGetStorageImpl());
+  if (it == table.end()) return nullptr;
+  for (InnerTwin& r : it->second.rec)
+    if (r.offset == owner.storage_offset() && r.numel == owner.numel()) return &r;
+  return nullptr;
+}
+
+// The twin recorded for `owner`: in its own storage, or on its storage object (the records ops._attach keeps:
+// {(offset, numel): (twin, version)}); not found if there is none or it is out of date.  GIL held.
+Twin attached(const Tensor& owner, bool any_version = false) {
+  if (const InnerTwin* r = inner_twin(owner)) {
+    if (any_version || r->version == owner._version())
+      return Twin{static_cast<char*>(owner.storage().mutable_data()) + r->byte_offset, r->type, r->twin_numel, Tensor()};
+  }
   Ref st(THPStorage_Wrap(owner.storage()));
-  if (st.p == nullptr) { PyErr_Clear(); return Tensor(); }
+  if (st.p == nullptr) { PyErr_Clear(); return Twin(); }
   Ref recs(PyObject_GetAttr(st.p, g_twins_name));
-  if (recs.p == nullptr) { PyErr_Clear(); return Tensor(); }
-  if (!PyDict_Check(recs.p)) return Tensor();
+  if (recs.p == nullptr) { PyErr_Clear(); return Twin(); }
+  if (!PyDict_Check(recs.p)) return Twin();
   Ref key(Py_BuildValue("(LL)", static_cast<long long>(owner.storage_offset()), static_cast<long long>(owner.numel())));
   PyObject* rec = key.p != nullptr ? PyDict_GetItemWithError(recs.p, key.p) : nullptr;     // borrowed
-  if (rec == nullptr || !PyTuple_Check(rec) || PyTuple_GET_SIZE(rec) != 2) { PyErr_Clear(); return Tensor(); }
-  if (!any_version && PyLong_AsLong(PyTuple_GET_ITEM(rec, 1)) != static_cast<long>(owner._version())) return Tensor();
+  if (rec == nullptr || !PyTuple_Check(rec) || PyTuple_GET_SIZE(rec) != 2) { PyErr_Clear(); return Twin(); }
+  if (!any_version && PyLong_AsLong(PyTuple_GET_ITEM(rec, 1)) != static_cast<long>(owner._version())) return Twin();
   PyObject* twin = PyTuple_GET_ITEM(rec, 0);
-  return THPVariable_Check(twin) ? THPVariable_Unpack(twin) : Tensor();
+  if (!THPVariable_Check(twin)) return Twin();
+  const Tensor& t = THPVariable_Unpack(twin);
+  return Twin{t.numel() > 0 ? t.data_ptr() : nullptr, t.scalar_type(), t.numel(), t};
 }
 
 // Record `twin` as the derived form of `owner`'s current contents.  GIL held; false with a Python error set.
@@ -91,6 +138,13 @@ bool attach(const Tensor& owner, const Tensor& twin) {
   return rec.p != nullptr && PyDict_SetItem(recs, key.p, rec.p) == 0;
 }
 
+// Record a twin found or made by this file: an inner one only needs its version brought up to date.
+bool record(const Tensor& owner, const Twin& twin) {
+  if (twin.hold.defined()) return attach(owner, twin.hold);
+  if (InnerTwin* r = inner_twin(owner)) r->version = owner._version();
+  return true;
+}
+
 // A tensor the kernels can take as it is: on the current device, contiguous, no subclass behaviour, and
 // with a version counter (inference tensors have none, so no twin can be tied to their contents).
 bool plain(const Tensor& t, c10::DeviceIndex dev) {
@@ -100,6 +154,14 @@ bool plain(const Tensor& t, c10::DeviceIndex dev) {
 
 Tensor empty(at::IntArrayRef sizes, ScalarType t, c10::DeviceIndex dev) {
   return Tensor(at::detail::empty_cuda(sizes, t, c10::Device(c10::kCUDA, dev), std::nullopt));
+}
+
+// A tensor on part of `base`'s storage, with a version counter of its own (no view of anything).
+Tensor on_storage(const Tensor& base, int64_t byte_offset, at::IntArrayRef sizes, ScalarType t) {
+  Tensor r = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(base.storage()), base.key_set(), c10::scalarTypeToTypeMeta(t));
+  r.unsafeGetTensorImpl()->set_storage_offset(byte_offset / static_cast<int64_t>(c10::elementSize(t)));
+  r.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+  return r;
 }
 
 void throw_status(const char* what, int rc) {
@@ -112,6 +174,42 @@ struct Quantized {
   Tensor act, ascales, lora_act;
 };
 
+// The quantizer's three outputs and their twins on one storage.  Calls of a few hundred rows are bound by the host, and
+// there five allocations, two records on storage objects and five releases were half of a call's 8.4 us.  They
+// live and die together in practice; above kTogetherBytes, where the GPU sets the pace, each gets a storage of its own.
+constexpr int64_t kTogetherBytes = 4 << 20;
+bool allocate_together(int64_t Mp, int64_t K, int64_t R, ScalarType t, bool want_swz, c10::DeviceIndex dev, Quantized& out,
+                       Twin& swz, Twin& la16) {
+  auto up = [](int64_t n) { return (n + 511) & ~int64_t{511}; };
+  const int64_t n_act = Mp * (K / 2), n_sc = Mp * (K / 16), n_la = Mp * R * 4;
+  const int64_t n_16 = R > 0 ? svdq_lora_act16_elems(static_cast<int>(Mp), static_cast<int>(R), dtype_code(t)) : 0;
+  const int64_t o_sc = up(n_act), o_swz = o_sc + up(n_sc), o_la = o_swz + (want_swz ? up(n_sc) : 0), o_16 = o_la + up(n_la);
+  const int64_t total = o_16 + n_16 * 2;
+  if (total > kTogetherBytes) return false;
+  const Tensor base = empty({total}, at::kByte, dev);
+  out.act = on_storage(base, 0, {Mp, K / 2}, at::kByte);
+  out.ascales = on_storage(base, o_sc, {K / 16, Mp}, at::kFloat8_e4m3fn);
+  out.lora_act = on_storage(base, o_la, {Mp, R}, at::kFloat);
+  char* const p = static_cast<char*>(base.storage().mutable_data());
+  auto& table = inner_twins();
+  static size_t inserted = 0;
+  if (++inserted % kSweep == 0)
+    for (auto it = table.begin(); it != table.end();) it = it->second.storage.expired() ? table.erase(it) : std::next(it);
+  InnerTwins e{c10::weak_intrusive_ptr<c10::StorageImpl>(c10::intrusive_ptr<c10::StorageImpl>::unsafe_reclaim_from_nonowning(
+                   base.storage().unsafeGetStorageImpl())),
+               {{-1, -1, 0, 0, 0, at::kByte}, {-1, -1, 0, 0, 0, at::kByte}}};
+  if (want_swz) {
+    swz = Twin{p + o_swz, at::kByte, n_sc, Tensor()};
+    e.rec[0] = InnerTwin{o_sc, n_sc, out.ascales._version(), o_swz, n_sc, at::kByte};
+  }
+  if (R > 0) {
+    la16 = Twin{p + o_16, t, n_16, Tensor()};
+    e.rec[1] = InnerTwin{o_la / 4, Mp * R, out.lora_act._version(), o_16, n_16, t};
+  }
+  if (want_swz || R > 0) table.insert_or_assign(base.storage().unsafeGetStorageImpl(), std::move(e));
+  return true;
+}
+
 // GIL held.  False: not taken.
 bool quantize(const Tensor& x, const Tensor& ld, const Tensor& smooth, int64_t pad, const Quantized* into, Quantized& out) {
   if (!x.is_cuda()) return false;
@@ -123,14 +221,15 @@ bool quantize(const Tensor& x, const Tensor& ld, const Tensor& smooth, int64_t p
   if (ld.size(0) != K || K % 16 != 0 || K == 0 || M == 0 || pad < 1) return false;
   const int64_t Mp = (M + pad - 1) / pad * pad;
   if (!int_sized(Mp) || !int_sized(K) || !int_sized(R)) return false;
-  Tensor table;
+  Twin table;
   if (smooth.defined()) {
     if (!plain(smooth, dev) || smooth.dim() != 1 || smooth.size(0) != K || smooth.scalar_type() != t) return false;
     table = attached(smooth);
-    if (!table.defined()) return false;
+    if (!table.found()) return false;
   }
   const bool want_swz = Mp % 128 == 0 && K % 64 == 0;
-  Tensor swz, la16;
+  Twin swz, la16;
+  bool recorded = false;
   if (into != nullptr) {
     out = *into;
     if (!plain(out.act, dev) || !plain(out.ascales, dev) || !plain(out.lora_act, dev)) return false;
@@ -142,27 +241,36 @@ bool quantize(const Tensor& x, const Tensor& ld, const Tensor& smooth, int64_t p
       return false;
     swz = attached(out.ascales, true);
     la16 = attached(out.lora_act, true);
-    if (la16.defined() && la16.scalar_type() != t) la16 = Tensor();
+    if (la16.found() && la16.type != t) la16 = Twin();
   } else {
-    out.act = empty({Mp, K / 2}, at::kByte, dev);
-    out.ascales = empty({K / 16, Mp}, at::kFloat8_e4m3fn, dev);
-    out.lora_act = empty({Mp, R}, at::kFloat, dev);
+    recorded = allocate_together(Mp, K, R, t, want_swz, dev, out, swz, la16);
+    if (!recorded) {
+      out.act = empty({Mp, K / 2}, at::kByte, dev);
+      out.ascales = empty({K / 16, Mp}, at::kFloat8_e4m3fn, dev);
+      out.lora_act = empty({Mp, R}, at::kFloat, dev);
+    }
   }
-  if (want_swz && !swz.defined()) swz = empty({Mp * (K / 16)}, at::kByte, dev);
-  if (R > 0 && !la16.defined())
-    la16 = empty({svdq_lora_act16_elems(static_cast<int>(Mp), static_cast<int>(R), dtype_code(t))}, t, dev);
+  auto fresh = [&](int64_t n, ScalarType type) {
+    Tensor h = empty({n}, type, dev);
+    void* const ptr = h.data_ptr();
+    return Twin{ptr, type, n, std::move(h)};
+  };
+  if (want_swz && !swz.found()) swz = fresh(Mp * (K / 16), at::kByte);
+  if (R > 0 && !la16.found()) la16 = fresh(svdq_lora_act16_elems(static_cast<int>(Mp), static_cast<int>(R), dtype_code(t)), t);
   void* const stream = c10::cuda::getCurrentCUDAStream(dev).stream();
   auto ptr = [](const Tensor& v) -> void* { return v.defined() && v.numel() > 0 ? v.data_ptr() : nullptr; };
   int rc;
   {
     GilRelease nogil;
-    rc = svdq_quantize_w4a4_act_fuse_lora(ptr(x), ptr(ld), ptr(smooth), ptr(table), ptr(out.act), ptr(out.ascales),
-                                          static_cast<float*>(ptr(out.lora_act)), ptr(swz), ptr(la16), static_cast<int>(M),
+    rc = svdq_quantize_w4a4_act_fuse_lora(ptr(x), ptr(ld), ptr(smooth), table.data(), ptr(out.act), ptr(out.ascales),
+                                          static_cast<float*>(ptr(out.lora_act)), swz.data(), la16.data(), static_cast<int>(M),
                                           static_cast<int>(K), static_cast<int>(R), static_cast<int>(Mp), dtype_code(t), 0, stream);
   }
   if (rc != SVDQ_OK) throw_status("quantize_w4a4_act_fuse_lora", rc);
-  if (swz.defined() && !attach(out.ascales, swz)) throw python_error();
-  if (la16.defined() && !attach(out.lora_act, la16)) throw python_error();
+  if (!recorded) {
+    if (swz.found() && !record(out.ascales, swz)) throw python_error();
+    if (la16.found() && !record(out.lora_act, la16)) throw python_error();
+  }
   return true;
 }
 
@@ -188,7 +296,8 @@ bool gemm(const GemmArgs& a, ScalarType out_t, GemmResult& r) {
   if (a.wscales.dim() != 2 || a.wscales.size(0) != G || a.wscales.size(1) != N) return false;
   if (a.lora_act.defined() != a.lora_up.defined()) return false;
   int64_t R = 0;
-  Tensor la, lu, lu16;
+  Twin la, lu16;
+  Tensor lu;
   if (a.lora_act.defined()) {
     if (!plain(a.lora_act, dev) || !plain(a.lora_up, dev) || a.lora_act.dim() != 2 || a.lora_up.dim() != 2) return false;
     R = a.lora_up.size(1);
@@ -196,18 +305,18 @@ bool gemm(const GemmArgs& a, ScalarType out_t, GemmResult& r) {
     if (a.lora_up.scalar_type() != out_t) return false;
     if (R > 0) {
       la = attached(a.lora_act);
-      if (!la.defined() || la.scalar_type() != out_t) return false;
+      if (!la.found() || la.type != out_t) return false;
       lu = a.lora_up;
       if (out_t == at::kBFloat16) {
         lu16 = attached(a.lora_up);
-        if (!lu16.defined()) return false;                   // recorded empty if a value does not fit fp16
+        if (!lu16.found()) return false;                     // recorded empty if a value does not fit fp16
       }
     }
   }
   for (const Tensor* v : {&a.wcscales, &a.bias, &a.smooth_next})
     if (v->defined() && (!plain(*v, dev) || v->dim() != 1 || v->size(0) != N || v->scalar_type() != out_t)) return false;
-  const Tensor sa = attached(a.ascales), sw = attached(a.wscales);
-  if (!sa.defined() || !sw.defined()) return false;
+  const Twin sa = attached(a.ascales), sw = attached(a.wscales);
+  if (!sa.found() || !sw.found()) return false;
   if (a.out.defined()) {
     if (!plain(a.out, dev) || a.out.dim() != 2 || a.out.size(0) != M || a.out.size(1) != N || a.out.scalar_type() != out_t) return false;
     r.y = a.out;
@@ -223,7 +332,7 @@ bool gemm(const GemmArgs& a, ScalarType out_t, GemmResult& r) {
     int rc;
     {
       GilRelease nogil;
-      rc = svdq_gemm_w4a4_next(ptr(a.act), ptr(a.wgt), ptr(sa), ptr(sw), ptr(la), ptr(lu), ptr(lu16), ptr(a.wcscales), ptr(a.bias),
+      rc = svdq_gemm_w4a4_next(ptr(a.act), ptr(a.wgt), sa.data(), sw.data(), la.data(), ptr(lu), lu16.data(), ptr(a.wcscales), ptr(a.bias),
                                ptr(r.y), ptr(a.smooth_next), ptr(r.qout), ptr(r.oscales), ptr(oswz), m, n, k, rr, dt, 0, stream);
     }
     if (rc != SVDQ_OK) throw_status("gemm_w4a4_next", rc);
@@ -243,7 +352,7 @@ bool gemm(const GemmArgs& a, ScalarType out_t, GemmResult& r) {
   int rc;
   {
     GilRelease nogil;
-    rc = svdq_gemm_w4a4_ws(ptr(a.act), ptr(a.wgt), ptr(sa), ptr(sw), ptr(la), ptr(lu), ptr(lu16), ptr(a.wcscales), ptr(a.bias),
+    rc = svdq_gemm_w4a4_ws(ptr(a.act), ptr(a.wgt), sa.data(), sw.data(), la.data(), ptr(lu), lu16.data(), ptr(a.wcscales), ptr(a.bias),
                            ptr(r.y), m, n, k, rr, dt, 0, ptr(ws), ws.defined() ? static_cast<unsigned long long>(ws.numel()) : 0, stream);
   }
   if (rc != SVDQ_OK) throw_status("gemm_w4a4", rc);
@@ -340,6 +449,17 @@ PyObject* py_pack(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   Ref p(THPVariable_Wrap(std::move(packed))), s(THPVariable_Wrap(std::move(scales)));
   if (p.p == nullptr || s.p == nullptr) return nullptr;
   return PyTuple_Pack(2, p.p, s.p);
+  END_HANDLE_TH_ERRORS
+}
+
+// inner_twin(owner, any_version): the twin in owner's own storage as a tensor, or None
+PyObject* py_inner_twin(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 2 || !THPVariable_Check(args[0])) { PyErr_SetString(PyExc_TypeError, "inner_twin(owner, any_version)"); return nullptr; }
+  const Tensor& owner = THPVariable_Unpack(args[0]);
+  const InnerTwin* r = inner_twin(owner);
+  if (r == nullptr || (r->version != owner._version() && PyObject_IsTrue(args[1]) != 1)) Py_RETURN_NONE;
+  return THPVariable_Wrap(on_storage(owner, r->byte_offset, {r->twin_numel}, r->type));
   END_HANDLE_TH_ERRORS
 }
 
@@ -451,6 +571,7 @@ PyMethodDef g_methods[] = {
     {"quantize", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_quantize)), METH_FASTCALL, nullptr},
     {"gemm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_gemm)), METH_FASTCALL, nullptr},
     {"pack", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_pack)), METH_FASTCALL, nullptr},
+    {"inner_twin", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_inner_twin)), METH_FASTCALL, nullptr},
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_bind)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_host", "Native host path of the operators.", -1, g_methods, nullptr, nullptr, nullptr, nullptr};

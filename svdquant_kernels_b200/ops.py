@@ -68,13 +68,13 @@ def _attach(owner: torch.Tensor, twin: torch.Tensor) -> None:
 
 
 def _attached(owner: torch.Tensor, any_version: bool = False) -> Optional[torch.Tensor]:
+    """The recorded twin of `owner`, or None.  Outputs of a small quantizer call share one storage with their
+    twins, and the native host path keeps the record."""
     recs = getattr(owner.untyped_storage(), _TWIN, None)
-    if recs is None:
-        return None
-    rec = recs.get((owner.storage_offset(), owner.numel()))
-    if rec is None or (rec[1] != owner._version and not any_version):
-        return None
-    return rec[0]
+    rec = None if recs is None else recs.get((owner.storage_offset(), owner.numel()))
+    if rec is not None and (rec[1] == owner._version or any_version):
+        return rec[0]
+    return None if _lib._host is None else _lib._host.inner_twin(owner, any_version)
 
 
 class _on_device:
@@ -97,7 +97,7 @@ class _on_device:
 
 
 def _smooth_table(smooth: torch.Tensor) -> torch.Tensor:
-    """{smooth, 1/smooth} pairs + flag word for the fused kernel; built once per smooth tensor."""
+    """Smoothing table of the fused kernel (svdq_prepare_smooth); built once per smooth tensor."""
     twin = _attached(smooth)
     if twin is not None:
         return twin
