@@ -10,8 +10,8 @@
 // cute_kernels/gemm_w4a4/kernel_v2_fa4.py:841-1589.
 //
 // Work decomposition (320 threads per CTA, one CTA per SM):
-//   warps 0-7  epilogue: tensor memory -> registers -> affine -> 16 bit ->
-//              swizzled shared memory -> TMA store (a 32-row x 64-column strip per warp at a time)
+//   warps 0-7  epilogue: tensor memory -> registers -> affine -> 16 bit -> y, a
+//              32-row x 64-column strip per warp at a time
 //   warp  8    producer: TMA loads into a ring of shared-memory stages
 //   warp  9    issuer: tcgen05.cp of a slab's scale atoms into tensor memory, its
 //              tcgen05.mma's, and the commits
@@ -61,10 +61,11 @@
 // whose rows all fit takes a single fp16 pass instead (decided per tile by every
 // role from the same words, so all agree on the tile's slab count).
 //
-// Column-sharded form (n_peers > 0): the launch fills N columns of a wider result
-// that every GPU holds in full; each finished strip also leaves the staging buffer
-// as one TMA store per peer, into the peers' copies over NVLink (lane stores of 16
-// bytes measured the same: the link, not the store path, sets the pace).
+// Column-sharded form (TP): the launch fills N columns of a wider result that every
+// GPU holds in full; each finished strip goes through a staging buffer in shared
+// memory and leaves it as one TMA store into the local copy and one per peer, into
+// the peers' copies over NVLink (lane stores of 16 bytes measured the same there: the
+// link, not the store path, sets the pace).
 //
 // Split-K form (SK = true, one CTA per 128 x 128 tile part): for problems with few tiles and a
 // long K, S CTAs share a tile's slabs.  Each parks its fp32 partial tile in a caller-owned
@@ -94,7 +95,7 @@ constexpr int SFA_BYTES = BM * (BK / 16);  // 2048
 constexpr int EPI_WARPS = 8;
 constexpr int NUM_THREADS = (EPI_WARPS + 2) * 32;
 constexpr int STORE_BUF_BYTES = 32 * 128;  // one 32-row x 64-column strip of y
-template <int CG, int BN, bool NEXT = false>
+template <int CG, int BN, bool NEXT = false, bool TP = false>
 struct Cfg {
   static constexpr int B_ROWS = BN / CG;                           // rows of B this CTA loads
   static constexpr int B_BYTES = B_ROWS * 128;
@@ -104,10 +105,10 @@ struct Cfg {
   // tiles share the middle 128 columns with their neighbours.
   static constexpr bool SHARED_ACC = BN == 256;
   static constexpr int ACC_COLS = 128 + BN;
-  static constexpr int STORE_BYTES = EPI_WARPS * STORE_BUF_BYTES;
+  static constexpr int STORE_BYTES = TP ? EPI_WARPS * STORE_BUF_BYTES : 0;
   // per-column rows of the current tile: wcscales, bias and, for the next layer's quantisation, -smooth_next and
-  // 1 / smooth_next (that fourth kilobyte would cost the plain 256 x 256 form its fifth ring stage)
-  static constexpr int AFFINE_BYTES = NEXT ? 4096 : 3072;
+  // 1 / smooth_next
+  static constexpr int AFFINE_BYTES = (NEXT ? 4 : 2) * BN * 4;
   static constexpr int TAIL_BYTES = AFFINE_BYTES + 512 /*barriers*/;
   static constexpr int STAGES_RAW = (232448 - 1024 - STORE_BYTES - TAIL_BYTES) / STAGE_BYTES;
   static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
@@ -125,22 +126,25 @@ struct Cfg {
   static_assert((2 * STAGES + 5) * 8 + 16 <= 512, "barrier block");
 };
 
-// Column-sharded form: one tensor map per peer's copy of the result (same geometry as this GPU's).
+// Column-sharded form: tensor maps of this GPU's copy of the result and of the peers' (same geometry).
 struct PeerMaps {
-  CUtensorMap m[7];
+  CUtensorMap y, m[7];
 };
+struct NoMaps {};
 
 struct Params {
+  void* y;              // [M, N] (column-sharded form: through the tensor maps instead)
+  int y_wide;           // y is 32-byte aligned: one store instruction per 16 columns instead of two
   const void* wc;       // [N] or null
   const void* bias;     // [N] or null
   const uint32_t* la_flags;   // bf16 only: per 32 rows of lora_act, non-zero = does not fit fp16; null = always two-pass
   int M, N, K, R;
   int tiles_m, tiles_n; // in units of (CG*128) x BN
   // Column-sharded (tensor-parallel) form: this launch computes columns [col0, col0 + N) of a
-  // [M, y_ld] result that every rank holds in full.  The local copy is written through tmY (built over
+  // [M, y_ld] result that every rank holds in full.  The local copy is written through a tensor map (built over
   // the local full matrix); each finished strip is also stored, by TMA from the same staging buffer,
   // into the same place of every peer's matrix (peer-mapped memory, one tensor map per peer).
-  int col0, y_ld, n_peers;
+  int col0, n_peers;
   // Split-K form (SK kernels only): a tile's slabs are shared by `splits` CTAs; each writes its fp32
   // partial tile to ws_partials[(tile * splits + split) * BM * BN], takes a ticket from
   // ws_tickets[tile], and the CTA that draws the last ticket adds the partials in split order, runs
@@ -229,23 +233,23 @@ __device__ __noinline__ uint4 next_group_codes(float2 a0, float2 a1, float2 a2, 
   return make_uint4(lo, hi, sb, 0u);
 }
 
-template <int CG, int BN, typename OutT, bool SK = false, bool NEXT = false>
+template <int CG, int BN, typename OutT, bool SK = false, bool NEXT = false, bool TP = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmLA, const __grid_constant__ CUtensorMap tmLU,
-                 const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmSFA,
-                 const __grid_constant__ CUtensorMap tmSFB, const __grid_constant__ CUtensorMap tmLAf,
-                 const __grid_constant__ CUtensorMap tmLUf, const __grid_constant__ PeerMaps peers, const Params p) {
-  using C = Cfg<CG, BN, NEXT>;
+                 const __grid_constant__ CUtensorMap tmSFA, const __grid_constant__ CUtensorMap tmSFB,
+                 const __grid_constant__ CUtensorMap tmLAf, const __grid_constant__ CUtensorMap tmLUf,
+                 const __grid_constant__ typename std::conditional<TP, PeerMaps, NoMaps>::type maps, const Params p) {
+  using C = Cfg<CG, BN, NEXT, TP>;
   constexpr bool kBf16 = std::is_same<OutT, __nv_bfloat16>::value;
 
   extern __shared__ uint8_t smem_raw[];
   // 1 KB alignment by pointer arithmetic (not an integer round trip) so that the compiler keeps
   // the shared address space and emits shared-memory loads and stores
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  uint8_t* store_bufs = smem + C::STAGES * C::STAGE_BYTES;        // 1024-aligned: every stage is a multiple of 1 KB
-  uint8_t* tail = store_bufs + C::STORE_BYTES;
-  float* affine = reinterpret_cast<float*>(tail);                 // [3 or 4][BN] : wcscales, bias, -smooth_next, 1/smooth_next of the current tile
+  [[maybe_unused]] uint8_t* store_bufs = smem + C::STAGES * C::STAGE_BYTES;   // TP; 1024-aligned: every stage is a multiple of 1 KB
+  uint8_t* tail = smem + C::STAGES * C::STAGE_BYTES + C::STORE_BYTES;
+  float* affine = reinterpret_cast<float*>(tail);                 // [2 or 4][BN] : wcscales, bias, -smooth_next, 1/smooth_next of the current tile
   uint64_t* bars = reinterpret_cast<uint64_t*>(tail + C::AFFINE_BYTES);
   uint64_t* full = bars;                                          // [STAGES] operands and scales landed (leader CTA's copy is used)
   uint64_t* empty = bars + C::STAGES;                             // [STAGES] stage consumed by the MMAs (per CTA)
@@ -278,7 +282,8 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     fence_barrier_init();
   }
   if (warp == EPI_WARPS && lane == 0) {
-    tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); tma_prefetch_desc(&tmY);
+    tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB);
+    if constexpr (TP) tma_prefetch_desc(&maps.y);
     tma_prefetch_desc(&tmSFA); tma_prefetch_desc(&tmSFB);
     if (p.R > 0) { tma_prefetch_desc(&tmLA); tma_prefetch_desc(&tmLU); }
     if (p.R > 0 && p.la_flags != nullptr) { tma_prefetch_desc(&tmLAf); tma_prefetch_desc(&tmLUf); }
@@ -480,8 +485,6 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const OutT* wc = static_cast<const OutT*>(p.wc);
     const OutT* bias = static_cast<const OutT*>(p.bias);
     const int quarter = warp & 3, chalf = warp >> 2;
-    uint8_t* buf = store_bufs + warp * STORE_BUF_BYTES;
-    const uint32_t swz = static_cast<uint32_t>(lane & 7);
     uint32_t tcount = 0;
     bool ok = true;
     for (int w = pair; w < total_work && ok; w += num_pairs, ++tcount) {
@@ -513,85 +516,14 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       } else {
         asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
       }
-      if (!mbar_wait(&acc_full[as], aph, ctx, kDevWaitAcc, tcount)) ok = false;
-      tc_fence_after_sync();
-#pragma unroll 1
-      for (int q = 0; q < BN / 128; ++q) {
-      // A 256-column tile's shared half first: the next tile is waiting for those columns.
-      const int half = C::SHARED_ACC ? (q == 0 ? 1 - static_cast<int>(as) : static_cast<int>(as)) : 0;
-      const int cbase = half * 128 + chalf * 64;
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + as * 128 + cbase;
-      // Drain: the strip goes to registers in one burst, its columns are handed back at once, and only then do the
-      // affine, the packing and the store happen.
-      uint32_t v[2][32];
-      tmem_ld_32x32_x64(taddr, &v[0][0]);
-      tmem_ld_wait();
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) {
-        uint64_t* bar = (C::SHARED_ACC && q == 0) ? acc_shared : &acc_empty[as];
-        if constexpr (CG == 2) mbar_arrive_cluster_relaxed(bar, 0); else mbar_arrive(bar);
-      }
-      bool finish = true;                       // this CTA writes the tile's rows of y
-      if constexpr (SK) {
-        if (S > 1) {
-          // Each thread parks its 16 float4s at [j][thread] of the CTA's partial tile
-          // (consecutive threads, consecutive 16 bytes) and later reads the same places of the other
-          // partials, so no thread ever needs another thread's accumulator values.
-          static_assert(!SK || BN == 128, "a thread parks one strip");
-          constexpr int kVec = 16;
-          constexpr int kTileVec = BM * BN / 4;
-          const int tid = threadIdx.x;
-          float4* mine = p.ws_partials + static_cast<size_t>(tile * S + split) * kTileVec;
-          const uint32_t* vf = &v[0][0];
-#pragma unroll
-          for (int j = 0; j < kVec; ++j)
-            __stcg(mine + j * (EPI_WARPS * 32) + tid,
-                   make_float4(__uint_as_float(vf[4 * j]), __uint_as_float(vf[4 * j + 1]), __uint_as_float(vf[4 * j + 2]),
-                               __uint_as_float(vf[4 * j + 3])));
-          __threadfence();
-          asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
-          if (tid == 0) *sk_ticket = atomicAdd(p.ws_tickets + tile, 1u);
-          asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
-          finish = *sk_ticket == static_cast<uint32_t>(S - 1);
-          if (finish) {
-            __threadfence();
-            // Partial sp is added as a whole before partial sp + 1 is looked at: one round trip to L2
-            // per partial with all of a thread's loads in flight together, and the same order of
-            // additions whatever order the CTAs finished in.
-            const float4* first = p.ws_partials + static_cast<size_t>(tile * S) * kTileVec + tid;
-            uint32_t* vw = &v[0][0];
-#pragma unroll
-            for (int j = 0; j < kVec; ++j) {
-              const float4 t = __ldcg(first + j * (EPI_WARPS * 32));
-              vw[4 * j] = __float_as_uint(t.x); vw[4 * j + 1] = __float_as_uint(t.y);
-              vw[4 * j + 2] = __float_as_uint(t.z); vw[4 * j + 3] = __float_as_uint(t.w);
-            }
-#pragma unroll 1
-            for (int sp = 1; sp < S; ++sp) {
-              const float4* part = first + static_cast<size_t>(sp) * kTileVec;
-#pragma unroll
-              for (int h = 0; h < kVec; h += 8) {
-                float4 t[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) t[j] = __ldcg(part + (h + j) * (EPI_WARPS * 32));
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                  vw[4 * (h + j)] = __float_as_uint(__uint_as_float(vw[4 * (h + j)]) + t[j].x);
-                  vw[4 * (h + j) + 1] = __float_as_uint(__uint_as_float(vw[4 * (h + j) + 1]) + t[j].y);
-                  vw[4 * (h + j) + 2] = __float_as_uint(__uint_as_float(vw[4 * (h + j) + 2]) + t[j].z);
-                  vw[4 * (h + j) + 3] = __float_as_uint(__uint_as_float(vw[4 * (h + j) + 3]) + t[j].w);
-                }
-              }
-            }
-            if (tid == 0) p.ws_tickets[tile] = 0u;      // every split has drawn its ticket: ready for the next launch
-          }
+      // One strip: 64 columns from column cbase of the tile, the 64 accumulator values of this lane's row in v.
+      auto strip = [&](uint32_t (&v)[64], int cbase) {
+        [[maybe_unused]] uint8_t* buf = store_bufs + warp * STORE_BUF_BYTES;     // TP: this warp's staging strip
+        if constexpr (TP) {
+          // the TMA store that last read this warp's buffer must be done with it
+          if (lane == 0) tma_store_wait_read<0>();
+          __syncwarp();
         }
-      }
-      if (finish) {
-        // the TMA store that last read this warp's buffer must be done with it
-        if (lane == 0) tma_store_wait_read<0>();
-        __syncwarp();
 #pragma unroll
         for (int hc = 0; hc < 2; ++hc) {
           const float4* wc4 = reinterpret_cast<const float4*>(affine + cbase + hc * 32);
@@ -601,8 +533,8 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           [[maybe_unused]] uint32_t qcodes[4], qscales[2];
           // the four fp32 results of columns 4 i .. 4 i + 3 of this half strip
           auto affine_at = [&](int i, float& a0, float& a1, float& a2, float& a3) {
-            a0 = __uint_as_float(v[hc][4 * i]); a1 = __uint_as_float(v[hc][4 * i + 1]);
-            a2 = __uint_as_float(v[hc][4 * i + 2]); a3 = __uint_as_float(v[hc][4 * i + 3]);
+            a0 = __uint_as_float(v[hc * 32 + 4 * i]); a1 = __uint_as_float(v[hc * 32 + 4 * i + 1]);
+            a2 = __uint_as_float(v[hc * 32 + 4 * i + 2]); a3 = __uint_as_float(v[hc * 32 + 4 * i + 3]);
             if (wc != nullptr) {
               const float4 w4 = wc4[i];
               a0 = __fmul_rn(a0, w4.x); a1 = __fmul_rn(a1, w4.y); a2 = __fmul_rn(a2, w4.z); a3 = __fmul_rn(a3, w4.w);
@@ -645,22 +577,116 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               }
             }
           }
-          // row `lane` of the strip: 16-byte chunks hc*4 .. hc*4+3, XOR-swizzled like the TMA box
+          if constexpr (TP) {
+            // row `lane` of the strip: 16-byte chunks hc*4 .. hc*4+3, XOR-swizzled like the TMA box
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const uint32_t chunk = static_cast<uint32_t>(hc * 4 + i) ^ swz;
-            *reinterpret_cast<uint4*>(buf + lane * 128 + chunk * 16) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t chunk = static_cast<uint32_t>(hc * 4 + i) ^ static_cast<uint32_t>(lane & 7);
+              *reinterpret_cast<uint4*>(buf + lane * 128 + chunk * 16) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+            }
+          } else {
+            // Straight from the registers, whole 32-byte sectors: by TMA from shared memory the strips of the eight
+            // warps, all ready at once, held up the operand loads behind them in the same engine for some 500 cycles,
+            // twice a tile (4352 x 3840 -> 3072 28.2 -> 26.6 us, -> 15360 110.9 -> 108.1, x 15360 96.6 -> 95.5).
+            OutT* dst = static_cast<OutT*>(p.y) + static_cast<size_t>(m0 + quarter * 32 + lane) * p.N + n0 + cbase + hc * 32;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              if (p.y_wide) {
+                st_global_v8(dst + 16 * i, o + 8 * i);
+              } else {
+                *reinterpret_cast<uint4*>(dst + 16 * i) = make_uint4(o[8 * i], o[8 * i + 1], o[8 * i + 2], o[8 * i + 3]);
+                *reinterpret_cast<uint4*>(dst + 16 * i + 8) = make_uint4(o[8 * i + 4], o[8 * i + 5], o[8 * i + 6], o[8 * i + 7]);
+              }
+            }
           }
         }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          tma_store_2d(&tmY, buf, p.col0 + n0 + cbase, m0 + quarter * 32);
-          // the same strip into every peer's matrix: the copy engine sends it over NVLink while the warp goes on
-          for (int d = 0; d < p.n_peers; ++d) tma_store_2d(&peers.m[d], buf, p.col0 + n0 + cbase, m0 + quarter * 32);
-          tma_store_commit();
+        if constexpr (TP) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_2d(&maps.y, buf, p.col0 + n0 + cbase, m0 + quarter * 32);
+            // the same strip into every peer's matrix: the copy engine sends it over NVLink while the warp goes on
+            for (int d = 0; d < p.n_peers; ++d) tma_store_2d(&maps.m[d], buf, p.col0 + n0 + cbase, m0 + quarter * 32);
+            tma_store_commit();
+          }
+        }
+      };
+      if (!mbar_wait(&acc_full[as], aph, ctx, kDevWaitAcc, tcount)) ok = false;
+      tc_fence_after_sync();
+#pragma unroll 1
+      for (int q = 0; q < BN / 128; ++q) {
+      // A 256-column tile's shared half first: the next tile is waiting for those columns.
+      const int half = C::SHARED_ACC ? (q == 0 ? 1 - static_cast<int>(as) : static_cast<int>(as)) : 0;
+      const int cbase = half * 128 + chalf * 64;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + as * 128 + cbase;
+      // Drain: the strip goes to registers in one burst, its columns are handed back at once, and only then do the
+      // affine, the packing and the store happen.
+      uint32_t v[64];
+      tmem_ld_32x32_x64(taddr, v);
+      tmem_ld_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        uint64_t* bar = (C::SHARED_ACC && q == 0) ? acc_shared : &acc_empty[as];
+        if constexpr (CG == 2) mbar_arrive_cluster_relaxed(bar, 0); else mbar_arrive(bar);
+      }
+      bool finish = true;                       // this CTA writes the tile's rows of y
+      if constexpr (SK) {
+        if (S > 1) {
+          // Each thread parks its 16 float4s at [j][thread] of the CTA's partial tile
+          // (consecutive threads, consecutive 16 bytes) and later reads the same places of the other
+          // partials, so no thread ever needs another thread's accumulator values.
+          static_assert(!SK || BN == 128, "a thread parks one strip");
+          constexpr int kVec = 16;
+          constexpr int kTileVec = BM * BN / 4;
+          const int tid = threadIdx.x;
+          float4* mine = p.ws_partials + static_cast<size_t>(tile * S + split) * kTileVec;
+          const uint32_t* vf = v;
+#pragma unroll
+          for (int j = 0; j < kVec; ++j)
+            __stcg(mine + j * (EPI_WARPS * 32) + tid,
+                   make_float4(__uint_as_float(vf[4 * j]), __uint_as_float(vf[4 * j + 1]), __uint_as_float(vf[4 * j + 2]),
+                               __uint_as_float(vf[4 * j + 3])));
+          __threadfence();
+          asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
+          if (tid == 0) *sk_ticket = atomicAdd(p.ws_tickets + tile, 1u);
+          asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
+          finish = *sk_ticket == static_cast<uint32_t>(S - 1);
+          if (finish) {
+            __threadfence();
+            // Partial sp is added as a whole before partial sp + 1 is looked at: one round trip to L2
+            // per partial with all of a thread's loads in flight together, and the same order of
+            // additions whatever order the CTAs finished in.
+            const float4* first = p.ws_partials + static_cast<size_t>(tile * S) * kTileVec + tid;
+            uint32_t* vw = v;
+#pragma unroll
+            for (int j = 0; j < kVec; ++j) {
+              const float4 t = __ldcg(first + j * (EPI_WARPS * 32));
+              vw[4 * j] = __float_as_uint(t.x); vw[4 * j + 1] = __float_as_uint(t.y);
+              vw[4 * j + 2] = __float_as_uint(t.z); vw[4 * j + 3] = __float_as_uint(t.w);
+            }
+#pragma unroll 1
+            for (int sp = 1; sp < S; ++sp) {
+              const float4* part = first + static_cast<size_t>(sp) * kTileVec;
+#pragma unroll
+              for (int h = 0; h < kVec; h += 8) {
+                float4 t[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) t[j] = __ldcg(part + (h + j) * (EPI_WARPS * 32));
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                  vw[4 * (h + j)] = __float_as_uint(__uint_as_float(vw[4 * (h + j)]) + t[j].x);
+                  vw[4 * (h + j) + 1] = __float_as_uint(__uint_as_float(vw[4 * (h + j) + 1]) + t[j].y);
+                  vw[4 * (h + j) + 2] = __float_as_uint(__uint_as_float(vw[4 * (h + j) + 2]) + t[j].z);
+                  vw[4 * (h + j) + 3] = __float_as_uint(__uint_as_float(vw[4 * (h + j) + 3]) + t[j].w);
+                }
+              }
+            }
+            if (tid == 0) p.ws_tickets[tile] = 0u;      // every split has drawn its ticket: ready for the next launch
+          }
         }
       }
+      if (finish) strip(v, cbase);
       }
       // affine[] may be overwritten after this barrier; it also makes the eight warps agree on whether to go on
       uint32_t any_failed;
@@ -670,8 +696,10 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           : "=r"(any_failed) : "r"(ok ? 1u : 0u), "n"(EPI_WARPS * 32) : "memory");
       ok = any_failed == 0;
     }
-    if (lane == 0) tma_store_wait_all<0>();   // global writes of this warp are complete before the CTA ends
-    __syncwarp();
+    if constexpr (TP) {
+      if (lane == 0) tma_store_wait_all<0>();   // global writes of this warp are complete before the CTA ends
+      __syncwarp();
+    }
   }
 
   // ------------------------------ teardown ------------------------------
@@ -696,21 +724,19 @@ bool gemm_supported(int M, int N, int K, int R) {
   return M > 0 && N > 0 && K > 0 && M % 128 == 0 && N % 128 == 0 && K % 64 == 0 && R >= 0 && R % 16 == 0;
 }
 
-template <int CG, int BN, typename OutT, bool SK = false, bool NEXT = false>
+template <int CG, int BN, typename OutT, bool SK = false, bool NEXT = false, bool TP = false>
 static int launch_gemm_t(const void* act, const void* wgt, const void* sfa, const void* sfb, const void* la,
                          const void* lu, const void* lu_f16, const void* wc, const void* bias, void* y, int M, int N,
                          int K, int R, const GemmTp& tp, cudaStream_t stream, int splits = 1) {
-  using C = gemm::Cfg<CG, BN, NEXT>;
+  using C = gemm::Cfg<CG, BN, NEXT, TP>;
   constexpr bool kBf16 = std::is_same<OutT, __nv_bfloat16>::value;
-  CUtensorMap tmA, tmB, tmLA, tmLU, tmY, tmSFA, tmSFB, tmLAf, tmLUf;
+  CUtensorMap tmA, tmB, tmLA, tmLU, tmSFA, tmSFB, tmLAf, tmLUf;
   int rc;
   const uint64_t atoms_k = K / 64;
   if ((rc = make_tmap_2d(&tmSFA, sfa, 4, (M / 128) * atoms_k, 128, 512, 4, 128, kTmapSwizzleNone)) != SVDQ_OK) return rc;
   if ((rc = make_tmap_2d(&tmSFB, sfb, 4, (N / 128) * atoms_k, 128, 512, 4, 128, kTmapSwizzleNone)) != SVDQ_OK) return rc;
   if ((rc = make_tmap_2d(&tmA, act, 1, M, K / 2, K / 2, gemm::BM, 128, kTmapSwizzle128)) != SVDQ_OK) return rc;
   if ((rc = make_tmap_2d(&tmB, wgt, 1, N, K / 2, K / 2, C::B_ROWS, 128, kTmapSwizzle128)) != SVDQ_OK) return rc;
-  const int y_ld = tp.y_ld > 0 ? tp.y_ld : N;      // y may be the [M, y_ld] matrix this launch fills N columns of
-  if ((rc = make_tmap_2d(&tmY, y, 2, M, y_ld, static_cast<uint64_t>(y_ld) * 2, 32, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
   if (R > 0) {
     const uint64_t la_rows = static_cast<uint64_t>(M) * (std::is_same<OutT, __nv_bfloat16>::value ? 2 : 1);
     if ((rc = make_tmap_2d(&tmLA, la, 2, la_rows, R, static_cast<uint64_t>(R) * 2, gemm::BM, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
@@ -732,11 +758,18 @@ static int launch_gemm_t(const void* act, const void* wgt, const void* sfa, cons
   p.wc = wc; p.bias = bias;
   p.M = M; p.N = N; p.K = K; p.R = R;
   p.tiles_m = M / (gemm::BM * CG); p.tiles_n = N / BN;
-  p.col0 = tp.y_ld > 0 ? tp.col0 : 0; p.y_ld = y_ld; p.n_peers = tp.n_peers;
-  gemm::PeerMaps peers;
-  for (int d = 0; d < 7; ++d) peers.m[d] = tmY;
-  for (int d = 0; d < tp.n_peers; ++d)
-    if ((rc = make_tmap_2d(&peers.m[d], tp.y_peer[d], 2, M, y_ld, static_cast<uint64_t>(y_ld) * 2, 32, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
+  p.y = y;
+  p.y_wide = reinterpret_cast<uintptr_t>(y) % 32 == 0 ? 1 : 0;
+  p.col0 = tp.col0; p.n_peers = tp.n_peers;
+  typename std::conditional<TP, gemm::PeerMaps, gemm::NoMaps>::type maps;
+  if constexpr (TP) {
+    // the [M, y_ld] matrix this launch fills N columns of, here and on the peers
+    const uint64_t pitch = static_cast<uint64_t>(tp.y_ld) * 2;
+    if ((rc = make_tmap_2d(&maps.y, y, 2, M, tp.y_ld, pitch, 32, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
+    for (int d = 0; d < 7; ++d) maps.m[d] = maps.y;
+    for (int d = 0; d < tp.n_peers; ++d)
+      if ((rc = make_tmap_2d(&maps.m[d], tp.y_peer[d], 2, M, tp.y_ld, pitch, 32, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
+  }
   p.splits = SK ? splits : 1;
   p.interleave = tp.interleave;
   {
@@ -750,7 +783,7 @@ static int launch_gemm_t(const void* act, const void* wgt, const void* sfa, cons
   p.qout = static_cast<uint8_t*>(tp.qout);
   p.oscales = static_cast<uint8_t*>(tp.oscales);
   p.oscales_swz = static_cast<uint8_t*>(tp.oscales_swz);
-  auto kern = gemm::gemm_w4a4_kernel<CG, BN, OutT, SK, NEXT>;
+  auto kern = gemm::gemm_w4a4_kernel<CG, BN, OutT, SK, NEXT, TP>;
   // the attribute is per device: remember which devices of this process have it
   static bool configured[64] = {};
   int dev = 0;
@@ -774,18 +807,18 @@ static int launch_gemm_t(const void* act, const void* wgt, const void* sfa, cons
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  if (cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmLA, tmLU, tmY, tmSFA, tmSFB, tmLAf, tmLUf, peers, p) != cudaSuccess) return SVDQ_ERR_LAUNCH;
+  if (cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmLA, tmLU, tmSFA, tmSFB, tmLAf, tmLUf, maps, p) != cudaSuccess) return SVDQ_ERR_LAUNCH;
   return SVDQ_OK;
 }
 
-template <typename OutT, bool NEXT>
+template <typename OutT, bool NEXT, bool TP>
 static int launch_gemm_dt(int cg, int bn, const void* act, const void* wgt, const void* sfa, const void* sfb,
                           const void* la, const void* lu, const void* lu_f16, const void* wc, const void* bias, void* y,
                           int M, int N, int K, int R, const GemmTp& tp, cudaStream_t stream) {
-  if (cg == 2 && bn == 256) return launch_gemm_t<2, 256, OutT, false, NEXT>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
-  if (cg == 2 && bn == 128) return launch_gemm_t<2, 128, OutT, false, NEXT>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
-  if (cg == 1 && bn == 256) return launch_gemm_t<1, 256, OutT, false, NEXT>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
-  return launch_gemm_t<1, 128, OutT, false, NEXT>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
+  if (cg == 2 && bn == 256) return launch_gemm_t<2, 256, OutT, false, NEXT, TP>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
+  if (cg == 2 && bn == 128) return launch_gemm_t<2, 128, OutT, false, NEXT, TP>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
+  if (cg == 1 && bn == 256) return launch_gemm_t<1, 256, OutT, false, NEXT, TP>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
+  return launch_gemm_t<1, 128, OutT, false, NEXT, TP>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
 }
 
 // Split-K plan for a problem with few tiles: 128 x 128 tiles, each tile's slabs shared by S CTAs that
@@ -883,12 +916,19 @@ int launch_gemm_w4a4(const void* act, const void* wgt, const void* ascales_swz, 
   }
   if ((cg != 1 && cg != 2) || (bn != 128 && bn != 256)) return SVDQ_ERR_UNSUPPORTED;
   if (M % (128 * cg) != 0 || N % bn != 0) return SVDQ_ERR_SHAPE;
-  if (dtype == SVDQ_DTYPE_F16)
-    return next ? launch_gemm_dt<__half, true>(cg, bn, act, wgt, ascales_swz, wscales_swz, lora_act16, lora_up, nullptr, wcscales, bias, y, M, N, K, R, tp, stream)
-                : launch_gemm_dt<__half, false>(cg, bn, act, wgt, ascales_swz, wscales_swz, lora_act16, lora_up, nullptr, wcscales, bias, y, M, N, K, R, tp, stream);
-  if (dtype == SVDQ_DTYPE_BF16)
-    return next ? launch_gemm_dt<__nv_bfloat16, true>(cg, bn, act, wgt, ascales_swz, wscales_swz, lora_act16, lora_up, lora_up_f16, wcscales, bias, y, M, N, K, R, tp, stream)
-                : launch_gemm_dt<__nv_bfloat16, false>(cg, bn, act, wgt, ascales_swz, wscales_swz, lora_act16, lora_up, lora_up_f16, wcscales, bias, y, M, N, K, R, tp, stream);
+  const bool sharded = tp.y_ld > 0;
+  auto launch = [&](auto dt) {
+    using T = decltype(dt);
+    const void* lu16 = std::is_same<T, __half>::value ? nullptr : lora_up_f16;
+    auto go = [&](auto next_c, auto tp_c) {
+      return launch_gemm_dt<T, decltype(next_c)::value, decltype(tp_c)::value>(cg, bn, act, wgt, ascales_swz, wscales_swz, lora_act16, lora_up, lu16,
+                                                                              wcscales, bias, y, M, N, K, R, tp, stream);
+    };
+    if (next) return go(std::true_type{}, std::false_type{});
+    return sharded ? go(std::false_type{}, std::true_type{}) : go(std::false_type{}, std::false_type{});
+  };
+  if (dtype == SVDQ_DTYPE_F16) return launch(__half{});
+  if (dtype == SVDQ_DTYPE_BF16) return launch(__nv_bfloat16{});
   return SVDQ_ERR_DTYPE;
 }
 
