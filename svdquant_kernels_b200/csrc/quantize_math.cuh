@@ -237,8 +237,10 @@ __device__ __forceinline__ float rcp_approx(float v) {
 
 // One 16-element group of near quotients: scale byte and eight code bytes
 __device__ __forceinline__ void quantize_group_near(const float2 (&f)[8], uint32_t& code_lo, uint32_t& code_hi, uint32_t& sbyte) {
-  const uint32_t sb = scale_byte_near(group_amax(f));
+  const float amax = group_amax(f);
+  const uint32_t sb = scale_byte_near(amax);
   sbyte = sb;
+  code_lo = code_hi = 0u;
   if (sb - 1u < 0x7Du) {
     const __half_raw h = __nv_cvt_fp8_to_halfraw(static_cast<__nv_fp8_storage_t>(sb), __NV_E4M3);
     const float c = rcp_approx(__half2float(__half(h))) * 1.000000476837158203125f;     // 1 + 2^-21
@@ -248,7 +250,10 @@ __device__ __forceinline__ void quantize_group_near(const float2 (&f)[8], uint32
     for (int j = 0; j < 8; ++j) w[j] = __fmul2_rn(f[j], cc);
     code_lo = cvt_e2m1x8(w[0], w[1], w[2], w[3]);
     code_hi = cvt_e2m1x8(w[4], w[5], w[6], w[7]);
-  } else {
+  } else if (amax != 0.0f) {
+    // Not for groups of zeros: rows of the padding are nothing else, and with them in this path the warps that hold
+    // them took twice the time of the others (any row count that is not a multiple of the padding: 3840 columns,
+    // 500 rows 20.4 us against 9.6 us for 512, two K ranks each).
     group_codes_compare(f, sb, code_lo, code_hi);
   }
 }
