@@ -7,7 +7,7 @@
 // (triton_kernels/quantize_w4a4_act_fuse_lora/kernel.py:115-286); results
 // follow baseline/kernels/quantize_w4a4_act_fuse_lora/ref.py:19-50.
 //
-// Decomposition.  A cluster of KS (1, 2, 4 or 8) CTAs owns one tile of 64 rows; CTA k
+// Decomposition.  A cluster of KS (1 to 16) CTAs owns one tile of 64 rows; CTA k
 // owns a contiguous range of 64-column slabs of K.  Per slab one producer warp
 // TMA-loads the x tile (64 x 64, 128-byte swizzle) with the slab's 64 entries of
 // the smoothing table (one bulk copy) into a stage of the x ring, a
@@ -19,9 +19,10 @@
 // accumulators are summed in a fixed order (two ranks: through the copy engine
 // into the partner's shared memory; more: through distributed shared memory
 // loads): no atomics, no zero-fill, no scratch in global
-// memory.  Large inputs run with KS = 2; clusters of 4 and 8 are for inputs of
-// a few hundred rows, where pairs would leave most SMs idle (256 x 10240:
-// 36.0 -> 12.9 us), and are taken only if all of them are resident at once.  (64-row tiles with pairs, not 128-row tiles with quads: a B200 keeps
+// memory.  Large inputs run with KS = 2; larger clusters are for inputs of
+// a few hundred to two thousand rows, where pairs would leave most SMs idle (256 x 10240:
+// 36.0 -> 6.3 us), and are taken only if all of them are resident at once.
+// (64-row tiles with pairs, not 128-row tiles with quads: a B200 keeps
 // at most 33 four-CTA clusters of this size resident, one short of the 34 row
 // tiles of a 4352-row activation, while 68 pairs fit in one wave.  128-row tiles
 // whose K ranks meet through global memory were measured too: what they save in
@@ -136,7 +137,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   uint64_t* ack_bar = recv_bar + 1;            // two K ranks: the peer has received what this CTA sent
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ack_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint32_t* lora_unfit = tmem_slot + 2;        // bf16 form: some LoRA value this CTA wrote does not fit fp16
+  uint32_t* lora_unfit = tmem_slot + 2;        // bf16 form: some LoRA value this CTA wrote does not fit fp16 (other than two K ranks: a bit per 32 rows)
   float4* recv = reinterpret_cast<float4*>(smem + C::BARS_OFF + 512);        // [32 rows][RP / 4], slots as partial_slot
   const WaitCtx ctx{abort_flag};
 
@@ -436,7 +437,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
                     const float4 o = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
                                                  __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
                     store_lora16x4<T>(p.lora16, gm * p.R + c, static_cast<size_t>(p.M_pad) * p.R, o);
-                    if (kBf16 && !fits_f16(o)) atomicOr(lora_unfit, 1u);
+                    if (kBf16 && !fits_f16(o)) atomicOr(lora_unfit, 1u << (row / 32));
                   }
                 }
               }
@@ -449,18 +450,26 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       tc_fence_before_sync();
       __syncwarp();
       cluster_sync_all();                                     // every CTA's partial is in its shared memory
-      // CTA k sums rows [k*64/KS, (k+1)*64/KS) over the cluster, in rank order
-      const uint32_t rows_per = TILE_M / ks;
-      const uint32_t row_lo = krank * rows_per;
-      const uint32_t items = rows_per * RP4;
+      // CTA k sums float4s [k T / KS, (k + 1) T / KS) of the tile's T over the cluster
+      const uint32_t item_lo = krank * (TILE_M * RP4) / ks, item_hi = (krank + 1) * (TILE_M * RP4) / ks;
       const uint32_t base_addr = smem_u32(partial);
-      for (uint32_t it = threadIdx.x; it < items; it += NUM_THREADS) {
-        const uint32_t row = row_lo + it / RP4, c4 = it % RP4;
+      for (uint32_t it = item_lo + threadIdx.x; it < item_hi; it += NUM_THREADS) {
+        const uint32_t row = it / RP4, c4 = it % RP4;
         const uint32_t off = base_addr + partial_slot(row, c4, RP4) * 16u;
-        float4 acc = ld_cluster_f4(map_to_cta(off, 0));
-        for (uint32_t j = 1; j < ks; ++j) {
-          const float4 t = ld_cluster_f4(map_to_cta(off, j));
-          acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
+        // Its own part first, then the next ranks in turn (a fixed order for every element): with all CTAs asking rank 0
+        // first, then rank 1, one SM at a time would serve them all.  In batches, so that remote loads travel together.
+        float4 acc = partial[partial_slot(row, c4, RP4)];
+#pragma unroll 1
+        for (uint32_t j0 = 1; j0 < ks; j0 += 5) {
+          float4 t[5];
+#pragma unroll
+          for (uint32_t i = 0; i < 5; ++i) {
+            const uint32_t r = krank + j0 + i;
+            if (j0 + i < ks) t[i] = ld_cluster_f4(map_to_cta(off, r < ks ? r : r - ks));
+          }
+#pragma unroll
+          for (uint32_t i = 0; i < 5; ++i)
+            if (j0 + i < ks) { acc.x += t[i].x; acc.y += t[i].y; acc.z += t[i].z; acc.w += t[i].w; }
         }
         const int c = c4 * 4;
         if (c < p.R) {
@@ -468,23 +477,20 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
           *reinterpret_cast<float4*>(p.lora + gm * p.R + c) = acc;
           if (p.lora16 != nullptr) {
             store_lora16x4<T>(p.lora16, gm * p.R + c, static_cast<size_t>(p.M_pad) * p.R, acc);
-            if (kBf16 && !fits_f16(acc)) atomicOr(lora_unfit, 1u);
+            // one "does not fit fp16" word per 32 rows, kept as bits of the first CTA's word until all have had their say
+            if (kBf16 && !fits_f16(acc)) {
+              red_or_cluster(map_to_cta(smem_u32(lora_unfit), 0), 1u << (row / 32));
+              fence_acq_rel_cluster();
+            }
           }
         }
       }
-      cluster_sync_all();                                     // nobody leaves while its memory is being read
-      if (kBf16 && p.lora16 != nullptr) {
-        // One "does not fit fp16" word per 32 rows, and KS / 2 CTAs wrote rows of the same block: the
-        // first of them gathers the others' verdicts (all final since the barrier above) and stores
-        // the exact word; nobody leaves before that read is over.
-        const uint32_t share = ks / 2;
-        if (threadIdx.x == 0 && krank % share == 0) {
-          uint32_t unfit = 0u;
-          for (uint32_t j = 0; j < share; ++j) unfit |= ld_cluster_u32(map_to_cta(smem_u32(lora_unfit), krank + j));
-          lora16_flags(p.lora16, static_cast<size_t>(p.M_pad) * p.R)[m0 / 32 + krank / share] = unfit;
-        }
-        cluster_sync_all();
-      }
+      // Nobody leaves while its memory is being read.  What was read is in use above, and the rare verdict is fenced: the
+      // arrival itself has nothing to wait for (as a releasing one it waited for all the stores above).
+      cluster_arrive_relaxed();
+      cluster_wait();
+      if (kBf16 && p.lora16 != nullptr && krank == 0 && threadIdx.x < 2)
+        lora16_flags(p.lora16, static_cast<size_t>(p.M_pad) * p.R)[m0 / 32 + threadIdx.x] = (*lora_unfit >> threadIdx.x) & 1u;
     }
   }
 
@@ -494,7 +500,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     // one word per 32 rows: this CTA wrote rows [m0, m0 + 64) alone
     uint32_t* flags = lora16_flags(p.lora16, static_cast<size_t>(p.M_pad) * p.R);
     const uint32_t unfit = *lora_unfit;
-    flags[m0 / 32] = unfit; flags[m0 / 32 + 1] = unfit;
+    flags[m0 / 32] = unfit & 1u; flags[m0 / 32 + 1] = (unfit >> 1) & 1u;
   }
   if (*abort_flag) {
     const unsigned long long t0 = globaltimer_ns();
@@ -533,26 +539,30 @@ __global__ void smooth_table_kernel(const T* __restrict__ smooth, float* __restr
 }  // namespace qf
 
 // How many CTAs share one row tile along K (0 = no admissible split).
-// Clusters of 4 and 8 serve inputs of a few hundred to a couple of thousand rows, where two CTAs per
-// row tile would leave most SMs idle; they are taken only if all of them can be resident at once
-// (max4 / max8: clusters of that size the device can hold).  Cost in slabs; the constant is the
-// cluster reduction of the LoRA partial sums.
-static int pick_k_split(int M_pad, int K, int max4, int max8) {
+// Clusters of more than two serve inputs of a few hundred to a couple of thousand rows, where two CTAs per row
+// tile would leave most SMs idle; they are taken only if all of them can be resident at once (max_clusters(ks):
+// clusters of that size the device can hold; 33 of four CTAs, 22 of six, 15 of eight, 11 of ten, 7 of sixteen).
+// Cost in slabs (0.24 us); the constants are the ways of bringing the LoRA partial sums together, which hardly depend
+// on the cluster size (256 x 3840: 4 / 6 / 8 / 10 / 16 CTAs 8.3 / 7.2 / 6.5 / 6.3 / 5.9 us; 256 x 15360: 8 / 16 CTAs
+// 13.0 / 9.5 us; 1003 x 3840: 2 / 4 / 6 CTAs 10.0 / 7.3 / 6.5 us).
+template <typename MaxClusters>
+static int pick_k_split(int M_pad, int K, MaxClusters max_clusters) {
   const int tiles = M_pad / qf::TILE_M;
   const int slabs = K / qf::SLAB_K;
   const int sms = sm_count();
   int best = 0;
   double best_cost = 1e30;
-  for (int ks : {1, 2, 4, 8}) {
+  for (int ks : {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16}) {
     if (ks > slabs) continue;
     const int ctas = tiles * ks;
-    if (ks > 2 && (ctas > sms || tiles > (ks == 4 ? max4 : max8))) continue;
+    if (ks > 2 && ctas > sms) continue;
     const int waves = (ctas + sms - 1) / sms;
-    const double cost = static_cast<double>(waves) * ((slabs + ks - 1) / ks) + (ks == 1 ? 0.0 : ks == 2 ? 2.0 : 1.0 + 0.5 * ks);
-    if (cost < best_cost) { best_cost = cost; best = ks; }
+    const double cost = static_cast<double>(waves) * ((slabs + ks - 1) / ks) + (ks == 1 ? 0.0 : ks == 2 ? 2.0 : 3.0 + 0.05 * ks);
+    if (cost < best_cost && (ks <= 2 || tiles <= max_clusters(ks))) { best_cost = cost; best = ks; }
   }
   return best;
 }
+constexpr int kMaxKSplit = 16;
 
 template <typename T, int RP> static int max_clusters_t(int ks);
 
@@ -560,7 +570,7 @@ bool quantize_fused_supported(int M, int K, int R, int M_pad) {
   if (M <= 0 || K <= 0 || M_pad < M) return false;
   if (M_pad % qf::TILE_M != 0 || K % qf::SLAB_K != 0) return false;
   if (R < 0 || R > 256 || R % 8 != 0) return false;
-  return pick_k_split(M_pad, K, 0, 0) != 0;
+  return K >= qf::SLAB_K;
 }
 
 int launch_smooth_table(const void* smooth, void* table, int K, int dtype, cudaStream_t stream) {
@@ -591,17 +601,18 @@ static int launch_qf(const void* x, const void* w, const qf::Params& p, cudaStre
   if (cudaGetDevice(&dev) != cudaSuccess) return SVDQ_ERR_CUDA;
   if (dev < 0 || dev >= 64 || !configured[dev]) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) != cudaSuccess) return SVDQ_ERR_LAUNCH;
+    // clusters of more than eight
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return SVDQ_ERR_LAUNCH;
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  static int cap4[64], cap8[64];
-  static bool capped[64] = {};
-  if (dev >= 0 && dev < 64 && !capped[dev]) {
-    cap4[dev] = max_clusters_t<T, RP>(4);
-    cap8[dev] = max_clusters_t<T, RP>(8);
-    capped[dev] = true;
-  }
-  const bool known = dev >= 0 && dev < 64;
-  int ks = pick_k_split(split_rows > p.M_pad ? split_rows : p.M_pad, p.K, known ? cap4[dev] : 0, known ? cap8[dev] : 0);
+  // clusters the device can hold, by size and device, asked for when first needed (value + 2; 0: not asked yet)
+  static int caps[64][kMaxKSplit + 1];
+  auto max_clusters = [&](int k) -> int {
+    if (dev < 0 || dev >= 64) return 0;
+    if (caps[dev][k] == 0) caps[dev][k] = max_clusters_t<T, RP>(k) + 2;
+    return caps[dev][k] - 2;
+  };
+  const int ks = pick_k_split(split_rows > p.M_pad ? split_rows : p.M_pad, p.K, max_clusters);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(p.M_pad / qf::TILE_M, ks, 1);
   cfg.blockDim = dim3(qf::NUM_THREADS, 1, 1);
@@ -624,7 +635,9 @@ template <typename T, int RP>
 static int max_clusters_t(int ks) {
   using C = qf::Cfg<RP>;
   auto kern = qf::quantize_fused_kernel<T, RP>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) != cudaSuccess) return -1;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) != cudaSuccess ||
+      cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+    return -1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(64, ks, 1);
   cfg.blockDim = dim3(qf::NUM_THREADS, 1, 1);
