@@ -50,7 +50,8 @@ enum {
 /* bits that may be OR-ed into the `variant` argument of the GEMM entry points */
 enum {
   SVDQ_GEMM_LORA_INTERLEAVE = 1 << 24,  /* a tile's LoRA-up slabs spread evenly among its main K slabs */
-  SVDQ_GEMM_LORA_AT_END = 1 << 25       /* ... after them */
+  SVDQ_GEMM_LORA_AT_END = 1 << 25,      /* ... after them */
+  SVDQ_GEMM_NO_SPLIT = 1 << 26          /* no split-K of the library's own choice */
 };
 
 const char* svdq_status_string(int status);
@@ -175,6 +176,7 @@ int svdq_lora_up_to_f16(const void* lora_up_bf16_host, void* out_f16_host, long 
  * Contract: M % 128 == 0, N % 128 == 0, K % 64 == 0, R % 16 == 0 (svdq_gemm_w4a4_supported).
  * variant: 0 = let the library pick; 128 / 256 = one CTA per 128 x variant tile;
  *          2128 / 2256 = CTA pairs on 256 x 128 / 256 x 256 tiles (needs M % 256 == 0).
+ *          OR-ed with SVDQ_GEMM_NO_SPLIT the library does not split K by itself (see svdq_gemm_w4a4_ws).
  *          OR-ed with SVDQ_GEMM_LORA_INTERLEAVE or SVDQ_GEMM_LORA_AT_END it also fixes where a tile's
  *          LoRA-up slabs run: spread evenly among its main K slabs (launch_v2's lora_schedule =
  *          "interleave", cute_kernels/gemm_w4a4/kernel_v2_fa4.py:126, :299-303) or after them; with
@@ -210,10 +212,12 @@ int svdq_gemm_w4a4_next(const void* act, const void* wgt, const void* ascales_sw
  * svdq_gemm_w4a4 with a caller-owned workspace in device memory, for problems with few output tiles
  * (a few hundred rows: the small-M shapes of GEMM_SHAPES in
  * cute_kernels/gemm_w4a4/harness.py:17-24, where the reference's kernels leave most SMs idle).
- * With variant 0 and a workspace of at least svdq_gemm_w4a4_workspace_bytes(M, N, K, R) bytes the
- * library shares each 128 x 128 tile's K loop among several CTAs (split-K): each adds its part in
+ * With variant 0, M an odd multiple of 128 and a workspace of at least
+ * svdq_gemm_w4a4_workspace_bytes(M, N, K, R) bytes (room for forced splits otherwise) the library shares each 128 x 128 tile's K loop among several CTAs (split-K): each adds its part in
  * fp32, parks it in the workspace, and the CTA that arrives last sums the parts in a fixed order
  * and writes y, so results do not depend on timing.  variant 10000 * S + 128 forces S CTAs per tile.
+ * M a multiple of 256: svdq_gemm_w4a4 itself, with or without a workspace, shares 256 x 128 tiles among
+ * the CTA pairs of a cluster, equally deterministic; variant 10000 * S + 2128 forces S pairs per tile.
  * svdq_gemm_w4a4_workspace_bytes returns 0 where splitting does not apply; then (or with a NULL or
  * smaller workspace) the call is svdq_gemm_w4a4.
  * The first 1024 bytes of the workspace are ticket counters: zero them once before the first call;

@@ -414,8 +414,6 @@ struct svdq_linear_plan {
   PlanSlot slot[kPlanSlots];
   unsigned long long submitted;
   void *wgt, *wscales_swz, *lora_down, *lora_up, *lora_up_f16, *smooth, *smooth_table, *wc, *bias;  // resident weights
-  void* split_ws;                                                // split-K workspace of the GEMM (few-row calls, long K), or null
-  size_t split_ws_bytes;
   void* quant_ws;                                                // workspace of the quantizer's streaming form, or null
   size_t quant_ws_bytes;
 };
@@ -488,12 +486,6 @@ int svdq_linear_plan_create(svdq_linear_plan** out, int max_M, int K, int N, int
   }
   if (rc == SVDQ_OK) rc = dev_upload(&p->wc, wcscales_host, static_cast<size_t>(N) * 2, st);
   if (rc == SVDQ_OK) rc = dev_upload(&p->bias, bias_host, static_cast<size_t>(N) * 2, st);
-  if (rc == SVDQ_OK && gemm_split_plan(256, N, K, R) > 1) {
-    // a call with few rows may take the split-K form: tiles x splits never exceeds the SM count
-    p->split_ws_bytes = kSplitTicketBytes + static_cast<size_t>(sm_count()) * (128 * 128 * 4);
-    if (cudaMalloc(&p->split_ws, p->split_ws_bytes) != cudaSuccess ||
-        cudaMemsetAsync(p->split_ws, 0, kSplitTicketBytes, st) != cudaSuccess) rc = SVDQ_ERR_CUDA;
-  }
   if (rc == SVDQ_OK && R > 0) {
     // calls of any height up to max_M: room for eight K ranks of the tallest one
     p->quant_ws_bytes = 2048 + static_cast<size_t>(8) * max_M_pad * 128 * 4;
@@ -540,8 +532,8 @@ static int plan_queue(svdq_linear_plan* p, const void* x_host, void* y_host, int
   const int K = p->K, N = p->N, R = p->R;
   const size_t x_row = static_cast<size_t>(K) * 2, y_row = static_cast<size_t>(N) * 2;
   const int M_pad = (M + 255) / 256 * 256;
-  const int splits = gemm_split_plan(M_pad, N, K, R);
-  const int variant = splits >= 2 ? 10000 * splits + 128 : 0;
+  const int splits = gemm_cluster_split(M_pad, N, K, R);
+  const int variant = splits >= 2 ? 10000 * splits + 2128 : kGemmNoSplit;
   // page-locked caller buffers are copied from and to directly; pageable ones go through the slot's staging
   const bool x_pinned = is_pinned_host(x_host), y_pinned = is_pinned_host(y_host);
   char* const y_dst = static_cast<char*>(y_pinned ? y_host : q.y_pin);
@@ -574,9 +566,8 @@ static int plan_queue(svdq_linear_plan* p, const void* x_host, void* y_host, int
     rc = quantize_entry(x, p->lora_down, p->smooth, p->smooth_table, act, sc, la, swz, la16, rows, K, R, rows_pad, p->dtype,
                         SVDQ_QUANT_AUTO, p->quant_ws, p->quant_ws_bytes, p->s_run, M_pad);
     if (rc != SVDQ_OK) return rc;
-    rc = svdq_gemm_w4a4_ws(act, p->wgt, swz, p->wscales_swz, R > 0 ? la16 : nullptr, R > 0 ? p->lora_up : nullptr,
-                           R > 0 ? p->lora_up_f16 : nullptr, p->wc, p->bias, y, rows_pad, N, K, R, p->dtype, variant,
-                           splits >= 2 ? p->split_ws : nullptr, splits >= 2 ? p->split_ws_bytes : 0, p->s_run);
+    rc = svdq_gemm_w4a4(act, p->wgt, swz, p->wscales_swz, R > 0 ? la16 : nullptr, R > 0 ? p->lora_up : nullptr,
+                           R > 0 ? p->lora_up_f16 : nullptr, p->wc, p->bias, y, rows_pad, N, K, R, p->dtype, variant, p->s_run);
     if (rc != SVDQ_OK) return rc;
     bad = bad || cudaEventRecord(q.computed, p->s_run) != cudaSuccess;
     bad = bad || cudaStreamWaitEvent(p->s_out, q.computed, 0) != cudaSuccess;
@@ -640,8 +631,7 @@ void svdq_linear_plan_destroy(svdq_linear_plan* p) {
     for (cudaEvent_t e : q.y_part)
       if (e != nullptr) cudaEventDestroy(e);
   }
-  void* dev[] = {p->wgt, p->wscales_swz, p->lora_down, p->lora_up, p->lora_up_f16, p->smooth, p->smooth_table, p->wc, p->bias,
-                 p->split_ws, p->quant_ws};
+  void* dev[] = {p->wgt, p->wscales_swz, p->lora_down, p->lora_up, p->lora_up_f16, p->smooth, p->smooth_table, p->wc, p->bias, p->quant_ws};
   for (void* d : dev)
     if (d != nullptr) cudaFree(d);
   if (p->s_in != nullptr) cudaStreamDestroy(p->s_in);

@@ -67,8 +67,11 @@
 // the peers' copies over NVLink (lane stores of 16 bytes measured the same there: the
 // link, not the store path, sets the pace).
 //
-// Split-K form (SK = true, one CTA per 128 x 128 tile part): for problems with few tiles and a
-// long K, S CTAs share a tile's slabs.  Each parks its fp32 partial tile in a caller-owned
+// Split-K within clusters (SK = kClusterSplit): for problems with few tiles and a long K, the S pairs
+// of a cluster share a 256 x 128 tile's slabs and add their partial tiles up through distributed shared memory.
+//
+// Split-K through a workspace (SK = kWorkspaceSplit, one CTA per 128 x 128 tile part; row counts that are an odd multiple
+// of 128, or on request): S CTAs share a tile's slabs.  Each parks its fp32 partial tile in a caller-owned
 // workspace (thread t writes float4 j at [j][t], so every access is a whole line per warp and a
 // thread later reads back exactly the places its namesakes wrote), fences, and draws a ticket
 // from the tile's counter; the CTA that draws ticket S - 1 adds the S partials in split order -
@@ -145,7 +148,7 @@ struct Params {
   // the local full matrix); each finished strip is also stored, by TMA from the same staging buffer,
   // into the same place of every peer's matrix (peer-mapped memory, one tensor map per peer).
   int col0, n_peers;
-  // Split-K form (SK kernels only): a tile's slabs are shared by `splits` CTAs; each writes its fp32
+  // Split-K forms (SK kernels only): a tile's slabs are shared by `splits` CTAs or pairs.  Workspace form: each writes its fp32
   // partial tile to ws_partials[(tile * splits + split) * BM * BN], takes a ticket from
   // ws_tickets[tile], and the CTA that draws the last ticket adds the partials in split order, runs
   // the epilogue and puts the ticket counter back to zero.
@@ -233,7 +236,10 @@ __device__ __noinline__ uint4 next_group_codes(float2 a0, float2 a1, float2 a2, 
   return make_uint4(lo, hi, sb, 0u);
 }
 
-template <int CG, int BN, typename OutT, bool SK = false, bool NEXT = false, bool TP = false>
+// How a tile's K loop is split over CTAs (see the header comment): not at all, through a workspace, within a cluster
+enum SplitForm : int { kNoSplit = 0, kWorkspaceSplit = 1, kClusterSplit = 2 };
+
+template <int CG, int BN, typename OutT, int SK = kNoSplit, bool NEXT = false, bool TP = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmLA, const __grid_constant__ CUtensorMap tmLU,
@@ -270,7 +276,11 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   // in uniform registers.  Single-lane roles also vote on every wait result for the same reason.
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = (CG == 2) ? cluster_ctarank() : 0u;      // 0 = leader of the pair
+  // rank 0 = leader of the pair; where in the cluster the leader is: a constant wherever the cluster is the pair, else a
+  // warp-uniform value (the issuing loop must not lose its uniform registers to it: 0.2 instead of 0.17 us per slab)
+  const uint32_t cta = (CG == 1) ? 0u : SK == kClusterSplit ? __shfl_sync(0xffffffffu, cluster_ctarank(), 0) : cluster_ctarank();
+  const uint32_t rank = SK == kClusterSplit ? (cta & 1u) : cta;
+  const uint32_t leader = SK == kClusterSplit ? (cta & ~1u) : 0u;
   const int pair = blockIdx.x / CG;
   const int num_pairs = gridDim.x / CG;
 
@@ -377,7 +387,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         // counts toward the barrier whether it was in bounds or not.
         constexpr uint32_t kSfBytes = SFA_BYTES + C::SFB_BYTES, kAbBytes = A_BYTES + C::B_BYTES;
         // the barrier that counts this CTA's bytes: its own for CG = 1, the leader's for a pair
-        const uint32_t bar = (CG == 2) ? map_to_cta(smem_u32(&full[s]), 0) : smem_u32(&full[s]);
+        const uint32_t bar = (CG == 2) ? map_to_cta(smem_u32(&full[s]), leader) : smem_u32(&full[s]);
         if (elect_one()) {
           if (kt < kt_main) {
             if (rank == 0) mbar_arrive_expect_tx(&full[s], (kSfBytes + kAbBytes) * CG);
@@ -413,7 +423,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       constexpr uint32_t kIdescMain = idesc_nvfp4(BM * CG, BN);
       constexpr uint32_t kIdescLora = idesc_f16(kBf16, kBf16, BM * CG, BN, false, false);
       constexpr uint32_t kIdescLoraF16 = idesc_f16(false, false, BM * CG, BN, false, false);
-      constexpr uint16_t kMask = (CG == 2) ? 3 : 1;
+      const uint16_t mask = static_cast<uint16_t>((CG == 2 ? 3u : 1u) << leader);     // both CTAs of the pair
       const uint32_t smem16 = smem_desc_addr(smem);
       uint32_t s = 0, ph = 0, tcount = 0, sb = 0, it = 0;
       bool ok = true;
@@ -470,8 +480,8 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               for (int j = 0; j < 4; ++j)
                 if (j < nkb) mma_f16<CG>(acc, da + j * 2, db + j * 2, idesc, j != 0 ? 1u : accumulate);
             }
-            tc_commit_mask<CG>(&empty[s], kMask);          // stage reusable (in both CTAs) once these MMAs have read it
-            if (pos == kt_hi - 1) tc_commit_mask<CG>(&acc_full[as], kMask);    // accumulator complete
+            tc_commit_mask<CG>(&empty[s], mask);          // stage reusable (in both CTAs) once these MMAs have read it
+            if (pos == kt_hi - 1) tc_commit_mask<CG>(&acc_full[as], mask);    // accumulator complete
           }
           __syncwarp();
           if (++sb == C::SF_BUFS) sb = 0;
@@ -628,15 +638,15 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       __syncwarp();
       if (lane == 0) {
         uint64_t* bar = (C::SHARED_ACC && q == 0) ? acc_shared : &acc_empty[as];
-        if constexpr (CG == 2) mbar_arrive_cluster_relaxed(bar, 0); else mbar_arrive(bar);
+        if constexpr (CG == 2) mbar_arrive_cluster_relaxed(bar, leader); else mbar_arrive(bar);
       }
       bool finish = true;                       // this CTA writes the tile's rows of y
-      if constexpr (SK) {
+      if constexpr (SK == kWorkspaceSplit) {
         if (S > 1) {
           // Each thread parks its 16 float4s at [j][thread] of the CTA's partial tile
           // (consecutive threads, consecutive 16 bytes) and later reads the same places of the other
           // partials, so no thread ever needs another thread's accumulator values.
-          static_assert(!SK || BN == 128, "a thread parks one strip");
+          static_assert(BN == 128, "a thread parks one strip");
           constexpr int kVec = 16;
           constexpr int kTileVec = BM * BN / 4;
           const int tid = threadIdx.x;
@@ -686,6 +696,17 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
         }
       }
+      if constexpr (SK == kClusterSplit) {
+        // The CTA's partial tile, 128 rows of 128 fp32, into the ring (all its loads have been consumed); 16-byte slots
+        // XOR-swizzled by the row, so that neither these stores nor the sums below meet a bank conflict.
+        float4* part = reinterpret_cast<float4*>(smem);
+        const int row = quarter * 32 + lane;
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          part[row * 32 + ((chalf * 16 + j) ^ (row & 7))] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                                                     __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+        finish = false;
+      }
       if (finish) strip(v, cbase);
       }
       // affine[] may be overwritten after this barrier; it also makes the eight warps agree on whether to go on
@@ -699,6 +720,60 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if constexpr (TP) {
       if (lane == 0) tma_store_wait_all<0>();   // global writes of this warp are complete before the CTA ends
       __syncwarp();
+    }
+  }
+
+  if constexpr (SK == kClusterSplit) {
+    // ------------------------------ split-K sums (every thread of the cluster) ------------------------------
+    // The cluster's S pairs hold partial tiles; of the 128 rows of either side, pair i sums and writes out rows
+    // [128 i / S, 128 (i + 1) / S), its own part first and then the other pairs' in turn: a fixed order for every element,
+    // and no two pairs ask the same one at the same time.  A warp takes a row at a time, a lane four of its columns: with
+    // 512 consecutive bytes per load 2 / 4 pairs take 3400 / 4200 cycles for it (lanes 32 bytes apart 4900 / 6800; the
+    // copy engine pushing the same bytes into the owners' rings measured 0.1 us more).
+    static_assert(CG == 2 && BN == 128 && !NEXT && !TP && C::STAGES * C::STAGE_BYTES >= BM * BN * 4, "cluster split");
+    __syncwarp();
+    cluster_sync_all();
+    if (warp < EPI_WARPS && *abort_flag == 0) {
+      const int tile = pair / S, me = static_cast<int>(cta >> 1);
+      const int m0 = ((tile % p.tiles_m) * CG + rank) * BM, n0 = tile / p.tiles_m * BN;
+      const int row_lo = me * BM / S, row_hi = (me + 1) * BM / S;
+      const float4 w4 = reinterpret_cast<const float4*>(affine)[lane], b4 = reinterpret_cast<const float4*>(affine + BN)[lane];
+      const bool has_wc = p.wc != nullptr, has_bias = p.bias != nullptr;
+      const float4* part = reinterpret_cast<const float4*>(smem);
+      constexpr int RB = 8;                                         // rows of a warp in flight
+      for (int row0 = row_lo + warp; row0 < row_hi; row0 += EPI_WARPS * RB) {
+        float4 acc[RB];
+#pragma unroll
+        for (int k = 0; k < RB; ++k) {
+          const int row = row0 + k * EPI_WARPS;
+          if (row < row_hi) acc[k] = part[row * 32 + (lane ^ (row & 7))];
+        }
+#pragma unroll 1
+        for (int j = 1; j < S; ++j) {
+          const int r = me + j;
+          const uint32_t from = map_to_cta(smem_u32(part), 2u * static_cast<uint32_t>(r < S ? r : r - S) + rank);
+          float4 t[RB];
+#pragma unroll
+          for (int k = 0; k < RB; ++k) {
+            const int row = row0 + k * EPI_WARPS;
+            if (row < row_hi) t[k] = ld_cluster_f4(from + (row * 32 + (lane ^ (row & 7))) * 16);
+          }
+#pragma unroll
+          for (int k = 0; k < RB; ++k)
+            if (row0 + k * EPI_WARPS < row_hi) { acc[k].x += t[k].x; acc[k].y += t[k].y; acc[k].z += t[k].z; acc[k].w += t[k].w; }
+        }
+#pragma unroll
+        for (int k = 0; k < RB; ++k) {
+          const int row = row0 + k * EPI_WARPS;
+          if (row < row_hi) {
+            float4 f = acc[k];
+            if (has_wc) f = make_float4(__fmul_rn(f.x, w4.x), __fmul_rn(f.y, w4.y), __fmul_rn(f.z, w4.z), __fmul_rn(f.w, w4.w));
+            if (has_bias) f = make_float4(__fadd_rn(f.x, b4.x), __fadd_rn(f.y, b4.y), __fadd_rn(f.z, b4.z), __fadd_rn(f.w, b4.w));
+            *reinterpret_cast<uint2*>(static_cast<OutT*>(p.y) + static_cast<size_t>(m0 + row) * p.N + n0 + 4 * lane) =
+                make_uint2(pack2f<OutT>(f.x, f.y), pack2f<OutT>(f.z, f.w));
+          }
+        }
+      }
     }
   }
 
@@ -724,7 +799,7 @@ bool gemm_supported(int M, int N, int K, int R) {
   return M > 0 && N > 0 && K > 0 && M % 128 == 0 && N % 128 == 0 && K % 64 == 0 && R >= 0 && R % 16 == 0;
 }
 
-template <int CG, int BN, typename OutT, bool SK = false, bool NEXT = false, bool TP = false>
+template <int CG, int BN, typename OutT, int SK = gemm::kNoSplit, bool NEXT = false, bool TP = false>
 static int launch_gemm_t(const void* act, const void* wgt, const void* sfa, const void* sfb, const void* la,
                          const void* lu, const void* lu_f16, const void* wc, const void* bias, void* y, int M, int N,
                          int K, int R, const GemmTp& tp, cudaStream_t stream, int splits = 1) {
@@ -770,7 +845,7 @@ static int launch_gemm_t(const void* act, const void* wgt, const void* sfa, cons
     for (int d = 0; d < tp.n_peers; ++d)
       if ((rc = make_tmap_2d(&maps.m[d], tp.y_peer[d], 2, M, tp.y_ld, pitch, 32, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
   }
-  p.splits = SK ? splits : 1;
+  p.splits = SK != gemm::kNoSplit ? splits : 1;
   p.interleave = tp.interleave;
   {
     const int kt_main = (K + gemm::BK - 1) / gemm::BK, ls = (R + 63) / 64;
@@ -790,6 +865,7 @@ static int launch_gemm_t(const void* act, const void* wgt, const void* sfa, cons
   if (cudaGetDevice(&dev) != cudaSuccess) return SVDQ_ERR_CUDA;
   if (dev < 0 || dev >= 64 || !configured[dev]) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) != cudaSuccess) return SVDQ_ERR_LAUNCH;
+    if (SK == gemm::kClusterSplit && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return SVDQ_ERR_LAUNCH;
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
   const int tiles = p.tiles_m * p.tiles_n * p.splits;
@@ -802,7 +878,7 @@ static int launch_gemm_t(const void* act, const void* wgt, const void* sfa, cons
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CG; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[0].val.clusterDim.x = SK == gemm::kClusterSplit ? CG * splits : CG; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
@@ -815,12 +891,56 @@ template <typename OutT, bool NEXT, bool TP>
 static int launch_gemm_dt(int cg, int bn, const void* act, const void* wgt, const void* sfa, const void* sfb,
                           const void* la, const void* lu, const void* lu_f16, const void* wc, const void* bias, void* y,
                           int M, int N, int K, int R, const GemmTp& tp, cudaStream_t stream) {
-  if (cg == 2 && bn == 256) return launch_gemm_t<2, 256, OutT, false, NEXT, TP>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
-  if (cg == 2 && bn == 128) return launch_gemm_t<2, 128, OutT, false, NEXT, TP>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
-  if (cg == 1 && bn == 256) return launch_gemm_t<1, 256, OutT, false, NEXT, TP>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
-  return launch_gemm_t<1, 128, OutT, false, NEXT, TP>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
+  if (cg == 2 && bn == 256) return launch_gemm_t<2, 256, OutT, gemm::kNoSplit, NEXT, TP>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
+  if (cg == 2 && bn == 128) return launch_gemm_t<2, 128, OutT, gemm::kNoSplit, NEXT, TP>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
+  if (cg == 1 && bn == 256) return launch_gemm_t<1, 256, OutT, gemm::kNoSplit, NEXT, TP>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
+  return launch_gemm_t<1, 128, OutT, gemm::kNoSplit, NEXT, TP>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
 }
 
+// Clusters of `ctas` CTAs of the cluster-split kernel that the current device can hold at once, asked for when first
+// needed (all instantiations have the same block and shared-memory size).
+static int gemm_max_clusters(int ctas) {
+  static int caps[64][17];                          // value + 2; 0: not asked yet
+  int dev = 0;
+  if (ctas < 1 || ctas > 16 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (caps[dev][ctas] == 0) {
+    using C = gemm::Cfg<2, 128>;
+    auto kern = gemm::gemm_w4a4_kernel<2, 128, __half, gemm::kClusterSplit>;
+    int n = -1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(64 * ctas, 1, 1);
+    cfg.blockDim = dim3(gemm::NUM_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = C::SMEM_BYTES;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ctas; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = -1;
+    }
+    caps[dev][ctas] = n + 2;
+  }
+  return caps[dev][ctas] - 2;
+}
+
+// Pairs that share each 256 x 128 tile's K loop within a cluster (1: no split).  A pair streams a slab in about 0.17 us;
+// the cluster's sums and its barriers cost about 2.7 us, which n slabs repay from n (1 - 1 / S) = 18 on (256 rows, sustained:
+// 3072 columns, K = 3840 / 10240 with S = 2 6.6 -> 7.6 / 10.5 -> 10.0 us; 3840 columns, K = 15360, S = 2 16.1 -> 14.1;
+// 1792 columns, K = 9408, S = 4 12.1 -> 8.8; 1280 columns, K = 11520, S = 4 11.2 -> 8.4; 1024 columns, K = 5120, S = 4
+// 7.1 -> 7.0).  At least six slabs per pair; all clusters resident at once.
+int gemm_cluster_split(int M, int N, int K, int R) {
+  if (!gemm_supported(M, N, K, R) || M % 256 != 0) return 1;
+  const long long tiles = static_cast<long long>(M / 256) * (N / 128);
+  const int n = (K + gemm::BK - 1) / gemm::BK + (R + 63) / 64;
+  for (int s = 8; s >= 2; --s)
+    if (n >= 6 * s && n * (s - 1) >= 18 * s && tiles * 2 * s <= sm_count() && tiles <= gemm_max_clusters(2 * s)) return s;
+  return 1;
+}
+
+// Workspace form, for row counts that are an odd multiple of 128.
 // Split-K plan for a problem with few tiles: 128 x 128 tiles, each tile's slabs shared by S CTAs that
 // all run at once (tiles * S <= SMs).  One CTA streams a tile's slabs at about 0.3 us each however
 // few tiles there are (32 KB per slab through one SM's load path), so with a few dozen tiles most
@@ -852,7 +972,8 @@ size_t gemm_split_workspace_bytes(int M, int N, int K, int R) {
 constexpr int kLoraInterleaveDefault = 0;
 
 // variant: 0 = choose; 128 / 256 = one CTA per tile with that N tile; 2128 / 2256 = CTA pairs (256-row tiles);
-// 10000 * S + 128 = split-K with S CTAs per 128 x 128 tile (needs the workspace)
+// 10000 * S + 128 = split-K with S CTAs per 128 x 128 tile (needs the workspace); 10000 * S + 2128 = split-K with the S
+// pairs of a cluster per 256 x 128 tile
 int launch_gemm_w4a4(const void* act, const void* wgt, const void* ascales_swz, const void* wscales_swz,
                      const void* lora_act16, const void* lora_up, const void* lora_up_f16, const void* wcscales,
                      const void* bias, void* y, int M, int N, int K, int R, int dtype, int variant,
@@ -863,17 +984,33 @@ int launch_gemm_w4a4(const void* act, const void* wgt, const void* ascales_swz, 
   if (variant & SVDQ_GEMM_LORA_INTERLEAVE) tp.interleave = 1;
   else if (variant & SVDQ_GEMM_LORA_AT_END) tp.interleave = 0;
   else tp.interleave = kLoraInterleaveDefault;
-  variant &= ~(SVDQ_GEMM_LORA_INTERLEAVE | SVDQ_GEMM_LORA_AT_END);
+  const bool may_split = (variant & kGemmNoSplit) == 0;
+  variant &= ~(SVDQ_GEMM_LORA_INTERLEAVE | SVDQ_GEMM_LORA_AT_END | kGemmNoSplit);
   if (tp.n_peers < 0 || tp.n_peers > 7) return SVDQ_ERR_SHAPE;
   if (tp.y_ld > 0 && (tp.col0 < 0 || tp.col0 % 64 != 0 || tp.col0 + N > tp.y_ld || tp.y_ld % 8 != 0)) return SVDQ_ERR_SHAPE;
   if (tp.y_ld <= 0 && tp.n_peers > 0) return SVDQ_ERR_SHAPE;
   const bool next = tp.smooth_next != nullptr;
   if (next && (tp.qout == nullptr || tp.oscales == nullptr || tp.y_ld > 0 || variant >= 10000)) return SVDQ_ERR_UNSUPPORTED;
   int cg, bn;
-  if (!next && (variant == 0 || variant >= 10000)) {
+  if (!next && tp.y_ld <= 0 && ((variant == 0 && may_split) || (variant >= 10000 && variant % 10000 == 2128))) {
+    // split-K within clusters: planned, or forced by the caller
+    const int s = variant == 0 ? gemm_cluster_split(M, N, K, R) : variant / 10000;
+    if (variant >= 10000) {
+      const long long tiles = static_cast<long long>(M / 256) * (N / 128);
+      if (M % 256 != 0 || s < 2 || s > 8 || s > (K + gemm::BK - 1) / gemm::BK || tiles > gemm_max_clusters(2 * s)) return SVDQ_ERR_UNSUPPORTED;
+    }
+    if (s >= 2) {
+      if (dtype == SVDQ_DTYPE_F16)
+        return launch_gemm_t<2, 128, __half, gemm::kClusterSplit>(act, wgt, ascales_swz, wscales_swz, lora_act16, lora_up, nullptr, wcscales, bias, y, M, N, K, R, tp, stream, s);
+      if (dtype == SVDQ_DTYPE_BF16)
+        return launch_gemm_t<2, 128, __nv_bfloat16, gemm::kClusterSplit>(act, wgt, ascales_swz, wscales_swz, lora_act16, lora_up, lora_up_f16, wcscales, bias, y, M, N, K, R, tp, stream, s);
+      return SVDQ_ERR_DTYPE;
+    }
+  }
+  if (!next && (variant == 0 || (variant >= 10000 && variant % 10000 == 128))) {
     // split-K: planned (variant 0, plain form, workspace large enough) or forced by the caller
     int s = 1;
-    if (variant == 0 && tp.y_ld <= 0 && tp.ws != nullptr) {
+    if (variant == 0 && may_split && M % 256 != 0 && tp.y_ld <= 0 && tp.ws != nullptr) {
       s = gemm_split_plan(M, N, K, R);
       if (s >= 2 && tp.ws_bytes < gemm_split_workspace_bytes(M, N, K, R)) s = 1;
     } else if (variant >= 10000) {
@@ -886,9 +1023,9 @@ int launch_gemm_w4a4(const void* act, const void* wgt, const void* ascales_swz, 
     }
     if (s >= 2) {
       if (dtype == SVDQ_DTYPE_F16)
-        return launch_gemm_t<1, 128, __half, true>(act, wgt, ascales_swz, wscales_swz, lora_act16, lora_up, nullptr, wcscales, bias, y, M, N, K, R, tp, stream, s);
+        return launch_gemm_t<1, 128, __half, gemm::kWorkspaceSplit>(act, wgt, ascales_swz, wscales_swz, lora_act16, lora_up, nullptr, wcscales, bias, y, M, N, K, R, tp, stream, s);
       if (dtype == SVDQ_DTYPE_BF16)
-        return launch_gemm_t<1, 128, __nv_bfloat16, true>(act, wgt, ascales_swz, wscales_swz, lora_act16, lora_up, lora_up_f16, wcscales, bias, y, M, N, K, R, tp, stream, s);
+        return launch_gemm_t<1, 128, __nv_bfloat16, gemm::kWorkspaceSplit>(act, wgt, ascales_swz, wscales_swz, lora_act16, lora_up, lora_up_f16, wcscales, bias, y, M, N, K, R, tp, stream, s);
       return SVDQ_ERR_DTYPE;
     }
   }

@@ -340,7 +340,7 @@ bool gemm(const GemmArgs& a, ScalarType out_t, GemmResult& r) {
     return true;
   }
   Tensor ws;                                                  // split-K: the workspace of this device and stream
-  const unsigned long long need = svdq_gemm_w4a4_workspace_bytes(m, n, k, rr);
+  const unsigned long long need = m % 256 != 0 ? svdq_gemm_w4a4_workspace_bytes(m, n, k, rr) : 0;
   if (need > 0) {
     Ref key(Py_BuildValue("(iK)", static_cast<int>(dev), static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(stream))));
     PyObject* w = key.p != nullptr ? PyDict_GetItemWithError(g_split_ws, key.p) : nullptr;

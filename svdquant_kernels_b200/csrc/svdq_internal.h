@@ -54,6 +54,8 @@ struct GemmTp {
 constexpr size_t kSplitTicketBytes = 1024;     // 256 ticket counters
 constexpr int kSplitMaxTiles = 74;             // split-K is for problems with at most this many 128 x 128 tiles
 constexpr int kSplitMax = 6;                   // CTAs per tile at most
+constexpr int kGemmNoSplit = SVDQ_GEMM_NO_SPLIT;
+int gemm_cluster_split(int M, int N, int K, int R);
 int gemm_split_plan(int M, int N, int K, int R);
 size_t gemm_split_workspace_bytes(int M, int N, int K, int R);
 int launch_gemm_w4a4(const void* act, const void* wgt, const void* ascales_swz, const void* wscales_swz,

@@ -314,9 +314,9 @@ def gemm_w4a4(
     cast) divided by smooth_next - the `act` / `ascales` of a following W4A4 linear, made in this
     GEMM's epilogue instead of by a quantizer pass over y.
 
-    Problems with few output tiles (a few hundred rows) take the split-K form (svdq_gemm_w4a4_ws) with
-    a workspace cached per device and stream; `_splits = S` forces S CTAs per 128 x 128 tile, `_splits = 1`
-    forbids splitting.
+    Problems with few output tiles (a few hundred rows) and a long K split it: within clusters of CTAs, or, for an odd
+    multiple of 128 rows, through a workspace cached per device and stream (svdq_gemm_w4a4_ws).  `_splits = S` forces
+    the workspace form with S CTAs per 128 x 128 tile, `_splits = 1` forbids splitting.
 
     `_columns = (y_full, peer_ptrs, col0)` selects the column-sharded form (svdq_gemm_w4a4_columns):
     the `[M, N]` result of this call goes into columns `[col0, col0 + N)` of the local `[M, N_total]`
@@ -427,10 +427,12 @@ def _gemm_checked(act, wgt, ascales, wscales, lora_act_in=None, lora_up=None, wc
             _attach(oscales, oswz)
         return y, qout, oscales
     ws = None
+    if _splits == 1 and variant == 0:
+        variant = _lib.GEMM_NO_SPLIT
     if _splits is not None and _splits > 1:
         variant = 10000 * _splits + 128
         ws = _split_workspace(dev, 1024 + (M // 128) * (N // 128) * _splits * 65536)
-    elif variant == 0 and _splits is None:
+    elif variant == 0 and _splits is None and M % 256 != 0:    # whole 256-row tiles split within clusters
         need = int(lib.svdq_gemm_w4a4_workspace_bytes(M, N, K, R))
         if need > 0:
             ws = _split_workspace(dev, need)
