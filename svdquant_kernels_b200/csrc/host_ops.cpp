@@ -65,6 +65,7 @@ struct Twin {
   ScalarType type = at::kByte;
   int64_t numel = 0;
   Tensor hold;
+  c10::intrusive_ptr<c10::StorageImpl> hold_storage = {};
   bool found() const { return ptr != nullptr || hold.defined(); }
   void* data() const { return numel > 0 ? ptr : nullptr; }
 };
@@ -98,12 +99,42 @@ InnerTwin* inner_twin(const Tensor& owner) {
   return nullptr;
 }
 
+// What `attached` last found on the storage objects of weights and smoothing factors, which a layer looks up on every
+// call: a hash lookup instead of half a dozen Python calls (0.25 us each, three a layer).  An entry holds nothing alive,
+// is good for one version of one tensor, and is swept like those above.
+struct KnownTwin {
+  c10::weak_intrusive_ptr<c10::StorageImpl> owner, twin;
+  int64_t offset, numel;
+  uint32_t version;
+  void* ptr;
+  ScalarType type;
+  int64_t twin_numel;
+};
+std::unordered_map<const c10::StorageImpl*, KnownTwin>& known_twins() {
+  static auto* table = new std::unordered_map<const c10::StorageImpl*, KnownTwin>();
+  return *table;
+}
+c10::weak_intrusive_ptr<c10::StorageImpl> weak(const Tensor& t) {
+  return c10::weak_intrusive_ptr<c10::StorageImpl>(
+      c10::intrusive_ptr<c10::StorageImpl>::unsafe_reclaim_from_nonowning(t.storage().unsafeGetStorageImpl()));
+}
+
 // The twin recorded for `owner`: in its own storage, or on its storage object (the records ops._attach keeps:
 // {(offset, numel): (twin, version)}); not found if there is none or it is out of date.  GIL held.
 Twin attached(const Tensor& owner, bool any_version = false) {
   if (const InnerTwin* r = inner_twin(owner)) {
     if (any_version || r->version == owner._version())
-      return Twin{static_cast<char*>(owner.storage().mutable_data()) + r->byte_offset, r->type, r->twin_numel, Tensor()};
+      return Twin{static_cast<char*>(owner.storage().mutable_data()) + r->byte_offset, r->type, r->twin_numel, Tensor(), {}};
+  }
+  auto& known = known_twins();
+  const c10::StorageImpl* const impl = owner.storage().unsafeGetStorageImpl();
+  if (!any_version) {
+    const auto it = known.find(impl);
+    if (it != known.end() && it->second.offset == owner.storage_offset() && it->second.numel == owner.numel() &&
+        it->second.version == owner._version()) {
+      auto alive = it->second.twin.lock();
+      if (alive) return Twin{it->second.ptr, it->second.type, it->second.twin_numel, Tensor(), std::move(alive)};
+    }
   }
   Ref st(THPStorage_Wrap(owner.storage()));
   if (st.p == nullptr) { PyErr_Clear(); return Twin(); }
@@ -117,7 +148,15 @@ Twin attached(const Tensor& owner, bool any_version = false) {
   PyObject* twin = PyTuple_GET_ITEM(rec, 0);
   if (!THPVariable_Check(twin)) return Twin();
   const Tensor& t = THPVariable_Unpack(twin);
-  return Twin{t.numel() > 0 ? t.data_ptr() : nullptr, t.scalar_type(), t.numel(), t};
+  void* const ptr = t.numel() > 0 ? t.data_ptr() : nullptr;
+  if (!any_version && ptr != nullptr) {
+    static size_t inserted = 0;
+    if (++inserted % kSweep == 0)
+      for (auto it = known.begin(); it != known.end();) it = it->second.owner.expired() ? known.erase(it) : std::next(it);
+    known.insert_or_assign(impl, KnownTwin{weak(owner), weak(t), owner.storage_offset(), owner.numel(), static_cast<uint32_t>(owner._version()),
+                                           ptr, t.scalar_type(), t.numel()});
+  }
+  return Twin{ptr, t.scalar_type(), t.numel(), t, {}};
 }
 
 // Record `twin` as the derived form of `owner`'s current contents.  GIL held; false with a Python error set.
@@ -195,15 +234,14 @@ bool allocate_together(int64_t Mp, int64_t K, int64_t R, ScalarType t, bool want
   static size_t inserted = 0;
   if (++inserted % kSweep == 0)
     for (auto it = table.begin(); it != table.end();) it = it->second.storage.expired() ? table.erase(it) : std::next(it);
-  InnerTwins e{c10::weak_intrusive_ptr<c10::StorageImpl>(c10::intrusive_ptr<c10::StorageImpl>::unsafe_reclaim_from_nonowning(
-                   base.storage().unsafeGetStorageImpl())),
+  InnerTwins e{weak(base),
                {{-1, -1, 0, 0, 0, at::kByte}, {-1, -1, 0, 0, 0, at::kByte}}};
   if (want_swz) {
-    swz = Twin{p + o_swz, at::kByte, n_sc, Tensor()};
+    swz = Twin{p + o_swz, at::kByte, n_sc, Tensor(), {}};
     e.rec[0] = InnerTwin{o_sc, n_sc, out.ascales._version(), o_swz, n_sc, at::kByte};
   }
   if (R > 0) {
-    la16 = Twin{p + o_16, t, n_16, Tensor()};
+    la16 = Twin{p + o_16, t, n_16, Tensor(), {}};
     e.rec[1] = InnerTwin{o_la / 4, Mp * R, out.lora_act._version(), o_16, n_16, t};
   }
   if (want_swz || R > 0) table.insert_or_assign(base.storage().unsafeGetStorageImpl(), std::move(e));
@@ -253,7 +291,7 @@ bool quantize(const Tensor& x, const Tensor& ld, const Tensor& smooth, int64_t p
   auto fresh = [&](int64_t n, ScalarType type) {
     Tensor h = empty({n}, type, dev);
     void* const ptr = h.data_ptr();
-    return Twin{ptr, type, n, std::move(h)};
+    return Twin{ptr, type, n, std::move(h), {}};
   };
   if (want_swz && !swz.found()) swz = fresh(Mp * (K / 16), at::kByte);
   if (R > 0 && !la16.found()) la16 = fresh(svdq_lora_act16_elems(static_cast<int>(Mp), static_cast<int>(R), dtype_code(t)), t);
