@@ -8,6 +8,7 @@
 // smooth divide only on the quantised branch, zero rows up to the padded height).
 #include "nvfp4_math.cuh"
 #include "quantize_math.cuh"
+#include "sm100.cuh"
 #include "svdq_internal.h"
 
 #include <type_traits>
@@ -36,6 +37,9 @@ quantize_rows_kernel(const T* __restrict__ x, const T* __restrict__ smooth, uint
   __shared__ float2 lut[qmath::kScaleLutEntries];
   qmath::fill_scale_lut(lut, threadIdx.x, kPackThreads);
   __syncthreads();
+  // launched with programmatic serialization: nothing below may run before the kernel ahead has finished
+  pdl_trigger();
+  pdl_wait();
   const int groups = K >> 4;
   const int gtiles = (groups + kPackGroups - 1) / kPackGroups;      // neighbouring blocks: the same rows, the next columns
   const int m0 = static_cast<int>(blockIdx.x / gtiles) * kPackRows, g0 = static_cast<int>(blockIdx.x % gtiles) * kPackGroups;
@@ -198,20 +202,24 @@ int launch_quantize_rows(const void* x, const void* smooth, void* codes, void* s
   uint8_t* c = static_cast<uint8_t*>(codes);
   uint8_t* s = static_cast<uint8_t*>(scales);
   uint8_t* sw = static_cast<uint8_t*>(scales_swz);
+  auto launch = [&](auto kern, auto* xp, auto* sp) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(kPackThreads, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, xp, sp, c, s, sw, rows, rows_pad, K) == cudaSuccess ? SVDQ_OK : SVDQ_ERR_LAUNCH;
+  };
   switch (dtype) {
-    case SVDQ_DTYPE_F16:
-      quantize_rows_kernel<__half><<<grid, kPackThreads, 0, stream>>>(static_cast<const __half*>(x), static_cast<const __half*>(smooth), c, s, sw, rows, rows_pad, K);
-      break;
-    case SVDQ_DTYPE_BF16:
-      quantize_rows_kernel<__nv_bfloat16><<<grid, kPackThreads, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(smooth), c, s, sw, rows, rows_pad, K);
-      break;
-    case SVDQ_DTYPE_F32:
-      quantize_rows_kernel<float><<<grid, kPackThreads, 0, stream>>>(static_cast<const float*>(x), static_cast<const float*>(smooth), c, s, sw, rows, rows_pad, K);
-      break;
-    default:
-      return SVDQ_ERR_DTYPE;
+    case SVDQ_DTYPE_F16: return launch(quantize_rows_kernel<__half>, static_cast<const __half*>(x), static_cast<const __half*>(smooth));
+    case SVDQ_DTYPE_BF16: return launch(quantize_rows_kernel<__nv_bfloat16>, static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(smooth));
+    case SVDQ_DTYPE_F32: return launch(quantize_rows_kernel<float>, static_cast<const float*>(x), static_cast<const float*>(smooth));
+    default: return SVDQ_ERR_DTYPE;
   }
-  return cudaGetLastError() == cudaSuccess ? SVDQ_OK : SVDQ_ERR_LAUNCH;
 }
 
 // The CUDA-core paths do not look at magnitudes: they mark every row block of a bf16 form as
