@@ -786,7 +786,9 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     while (globaltimer_ns() - t0 < 50000ull) { __nanosleep(1000); }
     __syncthreads();
   }
-  if constexpr (CG == 2) cluster_sync_all();   // the partner may still read this CTA's shared memory / signal its barriers
+  // The partner may still read this CTA's shared memory / signal its barriers.  Nothing that was written has to be visible to
+  // it: as a releasing arrival this one waited for the stores of y.
+  if constexpr (CG == 2) { cluster_arrive_relaxed(); cluster_wait(); }
   if (warp == EPI_WARPS + 1) {
     tc_fence_after_sync();
     if constexpr (CG == 1) tmem_dealloc(tmem_base, C::TMEM_COLS); else tmem_dealloc_pair(tmem_base, C::TMEM_COLS);
