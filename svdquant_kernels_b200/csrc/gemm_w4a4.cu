@@ -112,7 +112,8 @@ struct Cfg {
   // per-column rows of the current tile: wcscales, bias and, for the next layer's quantisation, -smooth_next and
   // 1 / smooth_next
   static constexpr int AFFINE_BYTES = (NEXT ? 4 : 2) * BN * 4;
-  static constexpr int TAIL_BYTES = AFFINE_BYTES + 512 /*barriers*/;
+  static constexpr int LUT_BYTES = NEXT ? qmath::kScaleLutEntries * 8 : 0;    // the constants of each scale byte
+  static constexpr int TAIL_BYTES = AFFINE_BYTES + LUT_BYTES + 512 /*barriers*/;
   static constexpr int STAGES_RAW = (232448 - 1024 - STORE_BYTES - TAIL_BYTES) / STAGE_BYTES;
   static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
   static constexpr int SFA_COLS = 16;                 // 4 k-blocks x 4 columns
@@ -197,7 +198,8 @@ template <> __device__ __forceinline__ float as_f32<__nv_bfloat16>(__nv_bfloat16
 // division, the scale and both code paths made the epilogue too large for the instruction cache (the top
 // stall reason was "no instruction", at 17 % issue utilisation).
 __device__ __noinline__ uint4 next_group_codes(float2 a0, float2 a1, float2 a2, float2 a3, float2 a4, float2 a5,
-                                               float2 a6, float2 a7, const float4* ns4, const float4* r4, int tile_fdiv) {
+                                               float2 a6, float2 a7, const float4* ns4, const float4* r4, const float2* lut,
+                                               int tile_fdiv) {
   const float2 a[8] = {a0, a1, a2, a3, a4, a5, a6, a7};
   float2 q[8];
   // IEEE divide of the uncast fp32 values, as the reference does; + 0 turns a -0 quotient into +0 (the
@@ -232,7 +234,9 @@ __device__ __noinline__ uint4 next_group_codes(float2 a0, float2 a1, float2 a2, 
     sb = qmath::group_scale_byte(q);
   }
   uint32_t lo, hi;
-  qmath::quantize_group_with(q, sb, lo, hi);
+  const float2 k = lut[sb];
+  if (k.x != 0.0f) qmath::group_codes_fast(q, k, lo, hi);
+  else qmath::group_codes_compare(q, sb, lo, hi);
   return make_uint4(lo, hi, sb, 0u);
 }
 
@@ -256,7 +260,8 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   [[maybe_unused]] uint8_t* store_bufs = smem + C::STAGES * C::STAGE_BYTES;   // TP; 1024-aligned: every stage is a multiple of 1 KB
   uint8_t* tail = smem + C::STAGES * C::STAGE_BYTES + C::STORE_BYTES;
   float* affine = reinterpret_cast<float*>(tail);                 // [2 or 4][BN] : wcscales, bias, -smooth_next, 1/smooth_next of the current tile
-  uint64_t* bars = reinterpret_cast<uint64_t*>(tail + C::AFFINE_BYTES);
+  [[maybe_unused]] float2* scale_lut = reinterpret_cast<float2*>(tail + C::AFFINE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(tail + C::AFFINE_BYTES + C::LUT_BYTES);
   uint64_t* full = bars;                                          // [STAGES] operands and scales landed (leader CTA's copy is used)
   uint64_t* empty = bars + C::STAGES;                             // [STAGES] stage consumed by the MMAs (per CTA)
   uint64_t* acc_full = bars + 2 * C::STAGES;                      // [2]      accumulator complete (per CTA)
@@ -302,6 +307,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if constexpr (CG == 1) { tmem_alloc(tmem_slot, C::TMEM_COLS); tmem_relinquish(); }
     else { tmem_alloc_pair(tmem_slot, C::TMEM_COLS); tmem_relinquish_pair(); }
   }
+  if constexpr (NEXT) qmath::fill_scale_lut(scale_lut, threadIdx.x, NUM_THREADS);
   tc_fence_before_sync();
   __syncthreads();
   if constexpr (CG == 2) cluster_sync_all();   // both CTAs' barriers exist before anything remote touches them
@@ -567,7 +573,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 const int e4 = (cbase + hc * 32) / 4 + (i - 3);      // float4 index of the group's first column
                 const uint4 r = next_group_codes(qf[0], qf[1], qf[2], qf[3], qf[4], qf[5], qf[6], qf[7],
                                                  reinterpret_cast<const float4*>(affine + 2 * BN) + e4,
-                                                 reinterpret_cast<const float4*>(affine + 3 * BN) + e4, tile_fdiv ? 1 : 0);
+                                                 reinterpret_cast<const float4*>(affine + 3 * BN) + e4, scale_lut, tile_fdiv ? 1 : 0);
                 qcodes[2 * (i >> 2)] = r.x; qcodes[2 * (i >> 2) + 1] = r.y; qscales[i >> 2] = r.z;
               }
             }

@@ -215,13 +215,6 @@ __device__ __forceinline__ float2 divide_by_constant2(float2 a, float2 neg_s, fl
   return __ffma2_rn(e, r, q0);
 }
 
-// quantize_group with the scale byte already worked out
-__device__ __forceinline__ void quantize_group_with(float2 (&f)[8], uint32_t sb, uint32_t& code_lo, uint32_t& code_hi) {
-  const float2 k = scale_constants(sb);
-  if (k.x != 0.0f) group_codes_fast(f, k, code_lo, code_hi);
-  else group_codes_compare(f, sb, code_lo, code_hi);
-}
-
 // Scale byte from the largest near quotient of a group (see the head of this file).  Values above 448 saturate in
 // the conversion, values below the smallest scale's rounding bound give byte 0: no clamps.
 __device__ __forceinline__ uint32_t scale_byte_near(float amax) {
