@@ -15,23 +15,26 @@
 
 namespace svdq {
 
-// A block packs a tile of 128 rows x 8 groups.  It is bound by memory (15360 x 3840 fp32: 236 MB in, 37 MB out), so every
-// access is laid out for it: consecutive lanes load consecutive 16 bytes of a row (four lanes per group for fp32, two
-// for 16-bit types; the group's amax meets through shuffles) with four loads of a thread in flight, codes leave as
-// whole sectors, and the scale bytes, which belong to one column of the tile each, are turned in shared memory so
-// that both layouts are written in runs of 128 bytes and more.  That matrix takes 50 us, 5.4 TB/s (a thread per
-// group, whose loads lie 64 bytes apart and whose scale bytes each touch a sector of their own: 75 us).  Six blocks
-// per SM (40 registers) and four loads a thread: 5 / 7 / 8 blocks 51.5 / 54 / 58 us, 2 / 8 / 16 loads 56 / 56 / 88 us.
-constexpr int kPackRows = 128, kPackGroups = 8, kPackThreads = 256;
+// A block packs a tile of 128 rows x 4 groups, one 512-byte atom of the tensor core's scale layout.  It is bound by
+// memory (15360 x 3840 fp32: 236 MB in, 33 MB out), so every access is laid out for it: consecutive lanes load
+// consecutive 16 bytes of a row (four lanes per group for fp32, two for 16-bit types; the group's amax meets through
+// shuffles) with several loads of a thread in flight, codes leave as whole sectors, and the scale bytes, which belong
+// to one column of the tile each, are turned in shared memory so that both layouts are written in runs of 128 bytes
+// and more.  That matrix takes 48 us, 5.6 TB/s (a thread per group, whose loads lie 64 bytes apart and whose scale
+// bytes each touch a sector of their own: 75 us).  Small blocks, ten per SM (48 registers), because a block loads
+// nothing while it turns its scales: 3072 x 3840 fp32 takes 12.5 us (8 groups, 256 threads, six blocks per SM: 14.4;
+// nine of the small blocks: 15.6, a second wave; twelve: 14.7).  A 16-byte piece of a 16-bit type is twice the
+// arithmetic of one of fp32 and needs half as many loads ahead: 15360 x 3840 bf16 takes 38 us with two, 44 with four.
+constexpr int kPackRows = 128, kPackGroups = 4, kPackThreads = 128;
 
 template <typename T>
-__global__ void __launch_bounds__(kPackThreads, 6)
+__global__ void __launch_bounds__(kPackThreads, 10)
 quantize_rows_kernel(const T* __restrict__ x, const T* __restrict__ smooth, uint8_t* __restrict__ codes,
                      uint8_t* __restrict__ scales, uint8_t* __restrict__ scales_swz, int rows, int rows_pad, int K) {
   constexpr int EPL = 16 / sizeof(T);                     // elements per lane
   constexpr int LPG = 16 / EPL;                           // lanes per group
   constexpr int ITEMS = kPackRows * kPackGroups * LPG;    // 16-byte pieces of a tile
-  constexpr int BATCH = 4;
+  constexpr int BATCH = sizeof(T) == 4 ? 4 : 2;
   using Code = typename std::conditional<EPL == 4, uint16_t, uint32_t>::type;
   __shared__ __align__(16) uint8_t sc[kPackGroups][kPackRows];
   __shared__ float2 lut[qmath::kScaleLutEntries];
