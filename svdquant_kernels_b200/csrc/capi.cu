@@ -1,6 +1,7 @@
 // extern "C" surface of libsvdq_b200.so (declared in include/svdq_b200.h):
 // argument validation, dispatch between the fused and the generic quantizer,
 // the device status word, and the host-buffer "plan" used for end-to-end runs.
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -26,6 +27,22 @@ int read_and_clear_status(unsigned int out[4]) {
 }
 
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+// Copies `n` 16-byte pieces between device memory and page-locked host memory (either way), a block 1024 of them
+// with four loads of a thread in flight.  Used for the copies of a short host call, which a copy engine starts and
+// hands over too slowly (see kPlanKernelCopyBytes).
+__global__ void __launch_bounds__(256) plan_copy_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, unsigned int n) {
+  pdl_trigger();
+  pdl_wait();
+  const unsigned int i0 = blockIdx.x * 1024u + threadIdx.x;
+  uint4 v[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (i0 + j * 256u < n) v[j] = __ldcv(src + i0 + j * 256u);
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (i0 + j * 256u < n) dst[i0 + j * 256u] = v[j];
+}
 
 }  // namespace svdq
 
@@ -383,19 +400,27 @@ int svdq_selftest_divide(unsigned long long* mismatches_device, void* stream) {
 // ---------------------------------------------------------------------------
 // Two slots of per-call buffers and three streams (host->device, compute, device->host), so that the
 // copies of neighbouring calls overlap the kernels and each other (PCIe is full duplex).  A slot's
-// life: x copy -> quantizer + GEMM -> y copy; events hand it from stream to stream and keep a slot's
-// next use behind its previous one.
+// life: x copy -> quantizer + GEMM -> y copy; events hand it from stream to stream, and a slot's next use
+// begins when the host has seen its previous y arrive.
 //
 // A single call (forward_host) has no neighbour to overlap with, so it walks its rows in chunks through the
 // same three streams: while chunk i is multiplied, chunk i + 1 comes in and chunk i - 1 goes out.  The copies
 // bound it (33.4 MB in and 26.7 MB out at 4352 x 3840 -> 3072: 0.61 and 0.48 ms alone, 0.65 ms side by side), and
 // one after the other with the kernels between they took 1.15 ms; in chunks 0.86 ms.
 constexpr int kPlanSlots = 2;
-// Chunks of forward_host: at least 6 MB of the wider side, at most kPlanChunks of them.  A shorter chunk leaves less
-// of the call uncovered at its ends, but every pair of copies that runs side by side costs about 15 us more than
-// its bytes (1 / 2 / 4 / 6 / 8 / 12 / 16 MB: 1.10 / 0.94 / 0.88 / 0.86 / 0.86 / 0.89 / 0.94 ms).
-constexpr int kPlanChunks = 32;
-constexpr size_t kPlanChunkBytes = 6u << 20;
+// A short chunk leaves less of the call uncovered at its ends, but every pair of copies that runs side by side costs
+// some 15-25 us more than its bytes.  With T bytes on the wider side in chunks of c bytes the ends cost c and the
+// T / c pairs a constant each, so the best c goes with the square root of T: c = sqrt(1.5 MB x T) (0.4 / 0.8 / 1.5 MB
+// in its place: 2048 x 1280 -> 1280 0.208 / 0.203 / 0.207 ms, 0.228 as one chunk; 1600 x 3840 -> 3072 0.413 / 0.376 /
+// 0.375, 0.386 in chunks of 6 MB and up; 4352 x 3840 -> 3072 0.94 / 0.87 / 0.86), up to 8 MB (at 4352 x 3840 -> 15360
+// chunks of 16 MB take 1 % longer than of 8).
+constexpr int kPlanChunks = 32;                                // at most
+constexpr size_t kPlanChunkBytes = 8u << 20, kPlanChunkCost = 3u << 19;
+// A call of one chunk stays in one stream, where nothing waits for an event of another, and copies of up to 2 MB are
+// kernels in it: a copy engine takes some 5 us to start and to hand over, a kernel is chained to its neighbours by
+// programmatic serialization.  3 x 960 -> 256 35.1 -> 25.8 us, 64 x 3840 -> 3072 57.4 -> 51.5, 256 x 3840 -> 3072
+// (1.9 MB) 103 -> 98; at 2.3 MB the engine is 2 % faster again.
+constexpr size_t kPlanKernelCopyBytes = 2u << 20;
 
 struct PlanSlot {
   void *x, *act, *ascales, *ascales_swz, *lora_act16, *y;
@@ -418,10 +443,33 @@ struct svdq_linear_plan {
   size_t quant_ws_bytes;
 };
 
-static bool is_pinned_host(const void* ptr) {
+// Whether `ptr` is page-locked host memory, and the address under which kernels reach it (null: they cannot).
+static bool is_pinned_host(const void* ptr, void** device_alias) {
   cudaPointerAttributes a;
+  *device_alias = nullptr;
   if (cudaPointerGetAttributes(&a, ptr) != cudaSuccess) { cudaGetLastError(); return false; }
-  return a.type == cudaMemoryTypeHost;
+  if (a.type != cudaMemoryTypeHost) return false;
+  *device_alias = a.devicePointer;
+  return true;
+}
+
+// One copy of a call between the host and the device.  `alias` is the device's address of the host side if a kernel
+// is to do it, else null.
+static bool plan_copy(void* dst, const void* src, size_t bytes, void* alias, bool to_device, cudaStream_t st) {
+  if (alias == nullptr)
+    return cudaMemcpyAsync(dst, src, bytes, to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, st) == cudaSuccess;
+  const unsigned int n = static_cast<unsigned int>(bytes / 16);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((n + 1023u) / 1024u, 1, 1);
+  cfg.blockDim = dim3(256, 1, 1);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, plan_copy_kernel, static_cast<uint4*>(to_device ? dst : alias),
+                            static_cast<const uint4*>(to_device ? alias : src), n) == cudaSuccess;
 }
 
 static int dev_upload(void** dst, const void* src, size_t bytes, cudaStream_t st) {
@@ -521,10 +569,18 @@ static int plan_retire(svdq_linear_plan* p, int i) {
   return cudaEventSynchronize(q.y_done) == cudaSuccess ? SVDQ_OK : SVDQ_ERR_CUDA;
 }
 
+// A call that could not be queued whole: nothing of it may still run when the slot is used again.
+static int plan_give_up(svdq_linear_plan* p, int rc) {
+  cudaStreamSynchronize(p->s_in);
+  cudaStreamSynchronize(p->s_run);
+  cudaStreamSynchronize(p->s_out);
+  return rc;
+}
+
 // Queue one call in chunks of `chunk` rows (a multiple of 256).  A chunk has its own piece of every per-call
 // buffer; the K splits of quantizer and GEMM are those of the whole call, so that the chunking does not show
 // in the result (every row's sums are formed in the same order).
-static int plan_queue(svdq_linear_plan* p, const void* x_host, void* y_host, int M, int chunk) {
+static int plan_queue(svdq_linear_plan* p, const void* x_host, void* y_host, int M, int chunk, bool alone) {
   const int i = static_cast<int>(p->submitted % kPlanSlots);
   int rc = plan_retire(p, i);                      // at most kPlanSlots calls are in flight
   if (rc != SVDQ_OK) return rc;
@@ -535,13 +591,18 @@ static int plan_queue(svdq_linear_plan* p, const void* x_host, void* y_host, int
   const int splits = gemm_cluster_split(M_pad, N, K, R);
   const int variant = splits >= 2 ? 10000 * splits + 2128 : kGemmNoSplit;
   // page-locked caller buffers are copied from and to directly; pageable ones go through the slot's staging
-  const bool x_pinned = is_pinned_host(x_host), y_pinned = is_pinned_host(y_host);
+  void *x_alias, *y_alias;
+  const bool x_pinned = is_pinned_host(x_host, &x_alias), y_pinned = is_pinned_host(y_host, &y_alias);
   char* const y_dst = static_cast<char*>(y_pinned ? y_host : q.y_pin);
+  // a call that nothing overlaps with stays in one stream, and its short copies are kernels
+  const bool one_stream = alone && chunk >= M;
+  if (!x_pinned) is_pinned_host(q.x_pin, &x_alias);
+  if (!y_pinned) is_pinned_host(q.y_pin, &y_alias);
+  if (!one_stream || M * x_row > kPlanKernelCopyBytes || !aligned16(x_alias)) x_alias = nullptr;
+  if (!one_stream || M * y_row > kPlanKernelCopyBytes || !aligned16(y_alias)) y_alias = nullptr;
+  cudaStream_t const s_in = one_stream ? p->s_run : p->s_in, s_out = one_stream ? p->s_run : p->s_out;
   const bool bf16 = p->dtype == SVDQ_DTYPE_BF16;
-  // x copies: after the kernels of the slot's previous call have read the old x (`computed` of a never-used
-  // slot is complete by definition); kernels: after the slot's previous y has left the device
-  bool bad = cudaStreamWaitEvent(p->s_in, q.computed, 0) != cudaSuccess;
-  bad = bad || cudaStreamWaitEvent(p->s_run, q.y_done, 0) != cudaSuccess;
+  bool bad = false;
   int c = 0;
   for (int m0 = 0; m0 < M && !bad; m0 += chunk, ++c) {
     const int rows = M - m0 < chunk ? M - m0 : chunk;
@@ -559,26 +620,30 @@ static int plan_queue(svdq_linear_plan* p, const void* x_host, void* y_host, int
     float* const la = q.lora_act + pad0 * R;
     char* const la16 = static_cast<char*>(q.lora_act16) + 2 * lora16_elems(pad0, R, bf16);
     char* const y = static_cast<char*>(q.y) + pad0 * y_row;
-    bad = bad || cudaMemcpyAsync(x, x_src, rows * x_row, cudaMemcpyHostToDevice, p->s_in) != cudaSuccess;
-    bad = bad || cudaEventRecord(q.x_ready, p->s_in) != cudaSuccess;
-    bad = bad || cudaStreamWaitEvent(p->s_run, q.x_ready, 0) != cudaSuccess;
+    bad = bad || !plan_copy(x, x_src, rows * x_row, x_alias, true, s_in);
+    if (!one_stream) {
+      bad = bad || cudaEventRecord(q.x_ready, s_in) != cudaSuccess;
+      bad = bad || cudaStreamWaitEvent(p->s_run, q.x_ready, 0) != cudaSuccess;
+    }
     if (bad) break;
     rc = quantize_entry(x, p->lora_down, p->smooth, p->smooth_table, act, sc, la, swz, la16, rows, K, R, rows_pad, p->dtype,
                         SVDQ_QUANT_AUTO, p->quant_ws, p->quant_ws_bytes, p->s_run, M_pad);
-    if (rc != SVDQ_OK) return rc;
+    if (rc != SVDQ_OK) return plan_give_up(p, rc);
     rc = svdq_gemm_w4a4(act, p->wgt, swz, p->wscales_swz, R > 0 ? la16 : nullptr, R > 0 ? p->lora_up : nullptr,
                            R > 0 ? p->lora_up_f16 : nullptr, p->wc, p->bias, y, rows_pad, N, K, R, p->dtype, variant, p->s_run);
-    if (rc != SVDQ_OK) return rc;
-    bad = bad || cudaEventRecord(q.computed, p->s_run) != cudaSuccess;
-    bad = bad || cudaStreamWaitEvent(p->s_out, q.computed, 0) != cudaSuccess;
-    bad = bad || cudaMemcpyAsync(y_dst + m0 * y_row, y, rows * y_row, cudaMemcpyDeviceToHost, p->s_out) != cudaSuccess;
+    if (rc != SVDQ_OK) return plan_give_up(p, rc);
+    if (!one_stream) {
+      bad = bad || cudaEventRecord(q.computed, p->s_run) != cudaSuccess;
+      bad = bad || cudaStreamWaitEvent(s_out, q.computed, 0) != cudaSuccess;
+    }
+    bad = bad || !plan_copy(y_dst + m0 * y_row, y, rows * y_row, y_alias, false, s_out);
     if (!y_pinned) {
       if (q.y_part[c] == nullptr) bad = bad || cudaEventCreateWithFlags(&q.y_part[c], cudaEventDisableTiming) != cudaSuccess;
-      bad = bad || cudaEventRecord(q.y_part[c], p->s_out) != cudaSuccess;
+      bad = bad || cudaEventRecord(q.y_part[c], s_out) != cudaSuccess;
     }
   }
-  bad = bad || cudaEventRecord(q.y_done, p->s_out) != cudaSuccess;
-  if (bad) return SVDQ_ERR_CUDA;
+  bad = bad || cudaEventRecord(q.y_done, s_out) != cudaSuccess;
+  if (bad) return plan_give_up(p, SVDQ_ERR_CUDA);
   q.y_user = y_pinned ? nullptr : y_host;
   q.y_bytes = M * y_row;
   q.y_chunk_bytes = chunk * y_row;
@@ -590,7 +655,7 @@ static int plan_queue(svdq_linear_plan* p, const void* x_host, void* y_host, int
 int svdq_linear_plan_submit(svdq_linear_plan* p, const void* x_host, void* y_host, int M) {
   if (p == nullptr || x_host == nullptr || y_host == nullptr) return SVDQ_ERR_NULL;
   if (M <= 0 || M > p->max_M) return SVDQ_ERR_SHAPE;
-  return plan_queue(p, x_host, y_host, M, (M + 255) / 256 * 256);
+  return plan_queue(p, x_host, y_host, M, (M + 255) / 256 * 256, false);
 }
 
 int svdq_linear_plan_wait(svdq_linear_plan* p) {
@@ -607,10 +672,14 @@ int svdq_linear_plan_forward_host(svdq_linear_plan* p, const void* x_host, void*
   if (p == nullptr || x_host == nullptr || y_host == nullptr) return SVDQ_ERR_NULL;
   if (M <= 0 || M > p->max_M) return SVDQ_ERR_SHAPE;
   const size_t row = static_cast<size_t>(p->K > p->N ? p->K : p->N) * 2;
-  const int M_pad = (M + 255) / 256 * 256;
-  int chunk = static_cast<int>((kPlanChunkBytes + row * 256 - 1) / (row * 256)) * 256;
-  while ((M_pad + chunk - 1) / chunk > kPlanChunks) chunk += 256;
-  const int rc = plan_queue(p, x_host, y_host, M, chunk);
+  const int units = (M + 255) / 256;                             // chunks are whole units of 256 rows, as equal as they go
+  const double best = std::sqrt(static_cast<double>(kPlanChunkCost) * M * row);
+  const double want = best < kPlanChunkBytes ? best : kPlanChunkBytes;
+  const int each = static_cast<int>(want / (row * 256.0) + 0.5);
+  int n = each < 1 ? units : (units + each - 1) / each;
+  if (n > kPlanChunks) n = kPlanChunks;
+  const int chunk = (units + n - 1) / n * 256;
+  const int rc = plan_queue(p, x_host, y_host, M, chunk, true);
   return rc != SVDQ_OK ? rc : svdq_linear_plan_wait(p);
 }
 

@@ -520,8 +520,11 @@ class LinearPlan:
         M = x_host.shape[0]
         assert x_host.shape == (M, self.K) and y_host.shape == (M, self.N)
         assert x_host.dtype == self.dtype and y_host.dtype == self.dtype
-        with torch.cuda.device(self.device):
+        if torch.cuda.current_device() == self.device:           # the guard costs a small call 2 us
             rc = self._lib.svdq_linear_plan_forward_host(self._handle, _ptr(x_host), _ptr(y_host), M)
+        else:
+            with torch.cuda.device(self.device):
+                rc = self._lib.svdq_linear_plan_forward_host(self._handle, _ptr(x_host), _ptr(y_host), M)
         _lib.check(rc, "linear_plan_forward_host")
         return y_host
 
