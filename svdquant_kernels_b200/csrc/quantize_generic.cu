@@ -23,8 +23,10 @@ namespace svdq {
 // and more.  That matrix takes 48 us, 5.6 TB/s (a thread per group, whose loads lie 64 bytes apart and whose scale
 // bytes each touch a sector of their own: 75 us).  Small blocks, ten per SM (48 registers), because a block loads
 // nothing while it turns its scales: 3072 x 3840 fp32 takes 12.5 us (8 groups, 256 threads, six blocks per SM: 14.4;
-// nine of the small blocks: 15.6, a second wave; twelve: 14.7).  A 16-byte piece of a 16-bit type is twice the
-// arithmetic of one of fp32 and needs half as many loads ahead: 15360 x 3840 bf16 takes 38 us with two, 44 with four.
+// nine of the small blocks: 15.6, a second wave; twelve: 14.7).
+// A 16-byte piece of a 16-bit type holds eight elements, and their arithmetic is the bound: 16-bit values take the
+// near quotients of quantize_math.cuh, one multiplication an element instead of a multiplication, a truncation and
+// another, and their maximum two elements at a time.  15360 x 3840 bf16 37.8 -> 33.5 us, 4526 x 10304 30.0 -> 27.3.
 constexpr int kPackRows = 128, kPackGroups = 4, kPackThreads = 128;
 
 template <typename T>
@@ -34,11 +36,15 @@ quantize_rows_kernel(const T* __restrict__ x, const T* __restrict__ smooth, uint
   constexpr int EPL = 16 / sizeof(T);                     // elements per lane
   constexpr int LPG = 16 / EPL;                           // lanes per group
   constexpr int ITEMS = kPackRows * kPackGroups * LPG;    // 16-byte pieces of a tile
-  constexpr int BATCH = sizeof(T) == 4 ? 4 : 2;
+  constexpr int BATCH = 4;
   using Code = typename std::conditional<EPL == 4, uint16_t, uint32_t>::type;
   __shared__ __align__(16) uint8_t sc[kPackGroups][kPackRows];
-  __shared__ float2 lut[qmath::kScaleLutEntries];
-  qmath::fill_scale_lut(lut, threadIdx.x, kPackThreads);
+  constexpr bool k16 = sizeof(T) == 2;
+  using Pair = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
+  __shared__ float2 lut[k16 ? 1 : qmath::kScaleLutEntries];
+  __shared__ float near_lut[k16 ? qmath::kScaleLutEntries : 1];
+  if constexpr (k16) qmath::fill_near_lut(near_lut, threadIdx.x, kPackThreads);
+  else qmath::fill_scale_lut(lut, threadIdx.x, kPackThreads);
   __syncthreads();
   // launched with programmatic serialization: nothing below may run before the kernel ahead has finished
   pdl_trigger();
@@ -71,32 +77,57 @@ quantize_rows_kernel(const T* __restrict__ x, const T* __restrict__ smooth, uint
       const int r = r0 + (step + b) * ROWS_PER_STEP, m = m0 + r;
       // amax as the reference has it (a NaN does not count), and whether there is a NaN
       float f[EPL], amax = 0.0f;
-      bool odd = false;
+      bool odd = false, packed = false;
 #pragma unroll
       for (int i = 0; i < EPL; ++i) {
         f[i] = to_f32(reinterpret_cast<const T*>(&raw[b])[i]);
         if (smooth != nullptr) f[i] = __fdiv_rn(f[i], sm[i]);
-        amax = fmaxf(amax, fabsf(f[i]));
-        odd |= f[i] != f[i];
+        if constexpr (!k16) {
+          amax = fmaxf(amax, fabsf(f[i]));
+          odd |= f[i] != f[i];
+        }
+      }
+      if constexpr (k16) {
+        if (smooth == nullptr) {                          // two elements an instruction; a NaN comes through
+          const Pair* h = reinterpret_cast<const Pair*>(&raw[b]);
+          const Pair top = __hmax2_nan(__hmax2_nan(__habs2(h[0]), __habs2(h[1])), __hmax2_nan(__habs2(h[2]), __habs2(h[3])));
+          amax = to_f32(__hmax_nan(top.x, top.y));
+          packed = amax == amax;
+        }
+        if (!packed) {
+          amax = 0.0f;
+#pragma unroll
+          for (int i = 0; i < EPL; ++i) {
+            amax = fmaxf(amax, fabsf(f[i]));
+            odd |= f[i] != f[i];
+          }
+        }
       }
 #pragma unroll
       for (int d = 1; d < LPG; d *= 2) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
       uint32_t code = 0, sbyte = 0;
       if (m < rows && g < groups) {                       // rows of the padding get zero codes and scales
-        sbyte = qmath::scale_byte(fminf(amax, 1e30f));    // the three-step divide wants a finite value; 448 is reached long before
-        const float2 c = lut[sbyte];
+        const float2 zero = make_float2(0.0f, 0.0f);      // the + 0 below makes a -0 a +0
+        float2 c;
+        if constexpr (k16) {
+          sbyte = qmath::scale_byte_near(amax);
+          c = make_float2(near_lut[sbyte], 0.0f);
+        } else {
+          sbyte = qmath::scale_byte(fminf(amax, 1e30f));  // the three-step divide wants a finite value; 448 is reached long before
+          c = lut[sbyte];
+        }
         if (c.x != 0.0f && !odd) {
-          // the conversion instruction's path of quantize_math.cuh; the + 0 makes a -0 input a +0
-          const float2 zero = make_float2(0.0f, 0.0f), mult = make_float2(c.x, c.x), rj = make_float2(c.y, c.y);
+          // the conversion instruction's paths of quantize_math.cuh: near quotients for 16-bit values, exact floors for fp32
+          const float2 mult = make_float2(c.x, c.x), rj = make_float2(c.y, c.y);
           float w[EPL];
 #pragma unroll
           for (int i = 0; i < EPL; i += 2) {
-            const float2 t = __ffma2_rn(make_float2(f[i], f[i + 1]), mult, zero);
-            const float2 q = __fmul2_rn(make_float2(truncf(t.x), truncf(t.y)), rj);
+            float2 q = __ffma2_rn(make_float2(f[i], f[i + 1]), mult, zero);
+            if constexpr (!k16) q = __fmul2_rn(make_float2(truncf(q.x), truncf(q.y)), rj);
             w[i] = q.x; w[i + 1] = q.y;
           }
           code = qmath::cvt_e2m1<EPL>(w);
-        } else {
+        } else if (!k16 || amax != 0.0f) {                // a group of zeros (and NaN) has zero codes
           const GroupBounds gb = bounds_for_scale(e4m3_to_f32(static_cast<uint8_t>(sbyte)));
 #pragma unroll
           for (int i = 0; i < EPL; ++i) code |= e2m1_code(f[i], gb) << (4 * i);

@@ -228,6 +228,16 @@ __device__ __forceinline__ float rcp_approx(float v) {
   return r;
 }
 
+// Multiplier of the codes of a group with scale byte sb, 1 <= sb < 0x7E
+__device__ __forceinline__ float near_multiplier(uint32_t sb) {
+  const __half_raw h = __nv_cvt_fp8_to_halfraw(static_cast<__nv_fp8_storage_t>(sb), __NV_E4M3);
+  return rcp_approx(__half2float(__half(h))) * 1.000000476837158203125f;     // 1 + 2^-21
+}
+// The same for every scale byte; 0 for the two that take the compare path
+__device__ __forceinline__ void fill_near_lut(float* lut, int tid, int nthreads) {
+  for (int i = tid; i < kScaleLutEntries; i += nthreads) lut[i] = static_cast<uint32_t>(i) - 1u < 0x7Du ? near_multiplier(i) : 0.0f;
+}
+
 // One 16-element group of near quotients: scale byte and eight code bytes
 __device__ __forceinline__ void quantize_group_near(const float2 (&f)[8], uint32_t& code_lo, uint32_t& code_hi, uint32_t& sbyte) {
   const float amax = group_amax(f);
@@ -235,8 +245,7 @@ __device__ __forceinline__ void quantize_group_near(const float2 (&f)[8], uint32
   sbyte = sb;
   code_lo = code_hi = 0u;
   if (sb - 1u < 0x7Du) {
-    const __half_raw h = __nv_cvt_fp8_to_halfraw(static_cast<__nv_fp8_storage_t>(sb), __NV_E4M3);
-    const float c = rcp_approx(__half2float(__half(h))) * 1.000000476837158203125f;     // 1 + 2^-21
+    const float c = near_multiplier(sb);
     const float2 cc = make_float2(c, c);
     float2 w[8];
 #pragma unroll
