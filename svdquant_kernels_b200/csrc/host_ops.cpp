@@ -15,6 +15,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
@@ -59,7 +60,7 @@ struct Ref {                            // owned reference
   ~Ref() { Py_XDECREF(p); }
 };
 
-// A twin as the launches need it; `hold` keeps a twin with a storage of its own alive.
+// A twin as the launches need it; `hold` or `hold_storage` keeps it alive.
 struct Twin {
   void* ptr = nullptr;
   ScalarType type = at::kByte;
@@ -70,38 +71,31 @@ struct Twin {
   void* data() const { return numel > 0 ? ptr : nullptr; }
 };
 
-// Twins that live in their owner's own storage (see `allocate_together`): storage -> where they are and for
-// which version of which tensor of that storage they hold.  A weak reference keeps the StorageImpl's address from
-// being used again while an entry exists, not its memory; entries of storages that are gone are swept out every
-// kSweep insertions.  All access with the GIL held.
-struct InnerTwin {
-  int64_t offset, numel;                // the owner: storage offset in its own elements, element count
-  uint32_t version;
-  int64_t byte_offset, twin_numel;      // the twin
-  ScalarType type;
+// The storage of an output that has a twin: the twin hangs on it directly and goes when it goes, with no Python object
+// in between (a record on a storage's Python object costs a call some 1.5 us).  It stands for the whole output,
+// (offset 0, numel); twins of other views of it are recorded on the Python object like everything else's.  All access
+// with the GIL held.
+struct OutputStorage final : c10::StorageImpl {
+  OutputStorage(size_t nbytes, c10::Allocator* allocator, int64_t numel)
+      : c10::StorageImpl(use_byte_size_t(), nbytes, allocator, /*resizable=*/true), numel(numel) {}
+  void release_resources() override {
+    c10::StorageImpl::release_resources();
+    twin = Tensor();
+  }
+  const int64_t numel;
+  Tensor twin;
+  uint32_t version = 0;                 // of the owner that the twin was made from
 };
-struct InnerTwins {
-  c10::weak_intrusive_ptr<c10::StorageImpl> storage;
-  InnerTwin rec[2];
-};
-constexpr size_t kSweep = 256;
-std::unordered_map<const c10::StorageImpl*, InnerTwins>& inner_twins() {
-  static auto* table = new std::unordered_map<const c10::StorageImpl*, InnerTwins>();     // outlives every tensor
-  return *table;
-}
-InnerTwin* inner_twin(const Tensor& owner) {
-  auto& table = inner_twins();
-  if (table.empty()) return nullptr;
-  const auto it = table.find(owner.storage().unsafeGetStorageImpl());
-  if (it == table.end()) return nullptr;
-  for (InnerTwin& r : it->second.rec)
-    if (r.offset == owner.storage_offset() && r.numel == owner.numel()) return &r;
-  return nullptr;
+OutputStorage* output_storage(const Tensor& owner) {
+  auto* const st = dynamic_cast<OutputStorage*>(owner.storage().unsafeGetStorageImpl());
+  return st != nullptr && owner.storage_offset() == 0 && owner.numel() == st->numel ? st : nullptr;
 }
 
 // What `attached` last found on the storage objects of weights and smoothing factors, which a layer looks up on every
 // call: a hash lookup instead of half a dozen Python calls (0.25 us each, three a layer).  An entry holds nothing alive,
-// is good for one version of one tensor, and is swept like those above.
+// is good for one version of one tensor; its weak references keep the StorageImpls' addresses from being used again, not
+// their memory.  Entries of storages that are gone are swept out every kSweep insertions.
+constexpr size_t kSweep = 256;
 struct KnownTwin {
   c10::weak_intrusive_ptr<c10::StorageImpl> owner, twin;
   int64_t offset, numel;
@@ -119,13 +113,13 @@ c10::weak_intrusive_ptr<c10::StorageImpl> weak(const Tensor& t) {
       c10::intrusive_ptr<c10::StorageImpl>::unsafe_reclaim_from_nonowning(t.storage().unsafeGetStorageImpl()));
 }
 
-// The twin recorded for `owner`: in its own storage, or on its storage object (the records ops._attach keeps:
+Twin with(const Tensor& t) { return Twin{t.numel() > 0 ? t.data_ptr() : nullptr, t.scalar_type(), t.numel(), t, {}}; }
+
+// The twin recorded for `owner`: on its storage, or on the storage's Python object (the records ops._attach keeps:
 // {(offset, numel): (twin, version)}); not found if there is none or it is out of date.  GIL held.
 Twin attached(const Tensor& owner, bool any_version = false) {
-  if (const InnerTwin* r = inner_twin(owner)) {
-    if (any_version || r->version == owner._version())
-      return Twin{static_cast<char*>(owner.storage().mutable_data()) + r->byte_offset, r->type, r->twin_numel, Tensor(), {}};
-  }
+  if (const OutputStorage* st = output_storage(owner))
+    return st->twin.defined() && (any_version || st->version == owner._version()) ? with(st->twin) : Twin();
   auto& known = known_twins();
   const c10::StorageImpl* const impl = owner.storage().unsafeGetStorageImpl();
   if (!any_version) {
@@ -161,6 +155,11 @@ Twin attached(const Tensor& owner, bool any_version = false) {
 
 // Record `twin` as the derived form of `owner`'s current contents.  GIL held; false with a Python error set.
 bool attach(const Tensor& owner, const Tensor& twin) {
+  if (OutputStorage* st = output_storage(owner)) {
+    st->twin = twin;
+    st->version = static_cast<uint32_t>(owner._version());
+    return true;
+  }
   Ref st(THPStorage_Wrap(owner.storage()));
   if (st.p == nullptr) return false;
   PyObject* recs = PyObject_GetAttr(st.p, g_twins_name);
@@ -177,13 +176,6 @@ bool attach(const Tensor& owner, const Tensor& twin) {
   return rec.p != nullptr && PyDict_SetItem(recs, key.p, rec.p) == 0;
 }
 
-// Record a twin found or made by this file: an inner one only needs its version brought up to date.
-bool record(const Tensor& owner, const Twin& twin) {
-  if (twin.hold.defined()) return attach(owner, twin.hold);
-  if (InnerTwin* r = inner_twin(owner)) r->version = owner._version();
-  return true;
-}
-
 // A tensor the kernels can take as it is: on the current device, contiguous, no subclass behaviour, and
 // with a version counter (inference tensors have none, so no twin can be tied to their contents).
 bool plain(const Tensor& t, c10::DeviceIndex dev) {
@@ -195,11 +187,14 @@ Tensor empty(at::IntArrayRef sizes, ScalarType t, c10::DeviceIndex dev) {
   return Tensor(at::detail::empty_cuda(sizes, t, c10::Device(c10::kCUDA, dev), std::nullopt));
 }
 
-// A tensor on part of `base`'s storage, with a version counter of its own (no view of anything).
-Tensor on_storage(const Tensor& base, int64_t byte_offset, at::IntArrayRef sizes, ScalarType t) {
-  Tensor r = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(base.storage()), base.key_set(), c10::scalarTypeToTypeMeta(t));
-  r.unsafeGetTensorImpl()->set_storage_offset(byte_offset / static_cast<int64_t>(c10::elementSize(t)));
-  r.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+// An output that gets a twin, on a storage that the twin can hang on
+Tensor empty_output(int64_t rows, int64_t cols, ScalarType t, c10::DeviceIndex dev) {
+  const int64_t numel = rows * cols;
+  if (numel == 0) return empty({rows, cols}, t, dev);
+  auto st = c10::make_intrusive<OutputStorage>(static_cast<size_t>(numel) * c10::elementSize(t), c10::cuda::CUDACachingAllocator::get(), numel);
+  Tensor r = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(std::move(st)), c10::DispatchKeySet(c10::DispatchKey::CUDA),
+                                                      c10::scalarTypeToTypeMeta(t));
+  r.unsafeGetTensorImpl()->set_sizes_contiguous({rows, cols});
   return r;
 }
 
@@ -212,41 +207,6 @@ bool int_sized(int64_t v) { return v >= 0 && v <= INT32_MAX; }
 struct Quantized {
   Tensor act, ascales, lora_act;
 };
-
-// The quantizer's three outputs and their twins on one storage.  Calls of a few hundred rows are bound by the host, and
-// there five allocations, two records on storage objects and five releases were half of a call's 8.4 us.  They
-// live and die together in practice; above kTogetherBytes, where the GPU sets the pace, each gets a storage of its own.
-constexpr int64_t kTogetherBytes = 4 << 20;
-bool allocate_together(int64_t Mp, int64_t K, int64_t R, ScalarType t, bool want_swz, c10::DeviceIndex dev, Quantized& out,
-                       Twin& swz, Twin& la16) {
-  auto up = [](int64_t n) { return (n + 511) & ~int64_t{511}; };
-  const int64_t n_act = Mp * (K / 2), n_sc = Mp * (K / 16), n_la = Mp * R * 4;
-  const int64_t n_16 = R > 0 ? svdq_lora_act16_elems(static_cast<int>(Mp), static_cast<int>(R), dtype_code(t)) : 0;
-  const int64_t o_sc = up(n_act), o_swz = o_sc + up(n_sc), o_la = o_swz + (want_swz ? up(n_sc) : 0), o_16 = o_la + up(n_la);
-  const int64_t total = o_16 + n_16 * 2;
-  if (total > kTogetherBytes) return false;
-  const Tensor base = empty({total}, at::kByte, dev);
-  out.act = on_storage(base, 0, {Mp, K / 2}, at::kByte);
-  out.ascales = on_storage(base, o_sc, {K / 16, Mp}, at::kFloat8_e4m3fn);
-  out.lora_act = on_storage(base, o_la, {Mp, R}, at::kFloat);
-  char* const p = static_cast<char*>(base.storage().mutable_data());
-  auto& table = inner_twins();
-  static size_t inserted = 0;
-  if (++inserted % kSweep == 0)
-    for (auto it = table.begin(); it != table.end();) it = it->second.storage.expired() ? table.erase(it) : std::next(it);
-  InnerTwins e{weak(base),
-               {{-1, -1, 0, 0, 0, at::kByte}, {-1, -1, 0, 0, 0, at::kByte}}};
-  if (want_swz) {
-    swz = Twin{p + o_swz, at::kByte, n_sc, Tensor(), {}};
-    e.rec[0] = InnerTwin{o_sc, n_sc, out.ascales._version(), o_swz, n_sc, at::kByte};
-  }
-  if (R > 0) {
-    la16 = Twin{p + o_16, t, n_16, Tensor(), {}};
-    e.rec[1] = InnerTwin{o_la / 4, Mp * R, out.lora_act._version(), o_16, n_16, t};
-  }
-  if (want_swz || R > 0) table.insert_or_assign(base.storage().unsafeGetStorageImpl(), std::move(e));
-  return true;
-}
 
 // GIL held.  False: not taken.
 bool quantize(const Tensor& x, const Tensor& ld, const Tensor& smooth, int64_t pad, const Quantized* into, Quantized& out) {
@@ -267,7 +227,6 @@ bool quantize(const Tensor& x, const Tensor& ld, const Tensor& smooth, int64_t p
   }
   const bool want_swz = Mp % 128 == 0 && K % 64 == 0;
   Twin swz, la16;
-  bool recorded = false;
   if (into != nullptr) {
     out = *into;
     if (!plain(out.act, dev) || !plain(out.ascales, dev) || !plain(out.lora_act, dev)) return false;
@@ -281,20 +240,13 @@ bool quantize(const Tensor& x, const Tensor& ld, const Tensor& smooth, int64_t p
     la16 = attached(out.lora_act, true);
     if (la16.found() && la16.type != t) la16 = Twin();
   } else {
-    recorded = allocate_together(Mp, K, R, t, want_swz, dev, out, swz, la16);
-    if (!recorded) {
-      out.act = empty({Mp, K / 2}, at::kByte, dev);
-      out.ascales = empty({K / 16, Mp}, at::kFloat8_e4m3fn, dev);
-      out.lora_act = empty({Mp, R}, at::kFloat, dev);
-    }
+    out.act = empty({Mp, K / 2}, at::kByte, dev);
+    out.ascales = empty_output(K / 16, Mp, at::kFloat8_e4m3fn, dev);
+    out.lora_act = empty_output(Mp, R, at::kFloat, dev);
   }
-  auto fresh = [&](int64_t n, ScalarType type) {
-    Tensor h = empty({n}, type, dev);
-    void* const ptr = h.data_ptr();
-    return Twin{ptr, type, n, std::move(h), {}};
-  };
-  if (want_swz && !swz.found()) swz = fresh(Mp * (K / 16), at::kByte);
-  if (R > 0 && !la16.found()) la16 = fresh(svdq_lora_act16_elems(static_cast<int>(Mp), static_cast<int>(R), dtype_code(t)), t);
+  if (want_swz && !swz.found()) swz = with(empty({Mp * (K / 16)}, at::kByte, dev));
+  if (R > 0 && !la16.found())
+    la16 = with(empty({svdq_lora_act16_elems(static_cast<int>(Mp), static_cast<int>(R), dtype_code(t))}, t, dev));
   void* const stream = c10::cuda::getCurrentCUDAStream(dev).stream();
   auto ptr = [](const Tensor& v) -> void* { return v.defined() && v.numel() > 0 ? v.data_ptr() : nullptr; };
   int rc;
@@ -305,10 +257,8 @@ bool quantize(const Tensor& x, const Tensor& ld, const Tensor& smooth, int64_t p
                                           static_cast<int>(K), static_cast<int>(R), static_cast<int>(Mp), dtype_code(t), 0, stream);
   }
   if (rc != SVDQ_OK) throw_status("quantize_w4a4_act_fuse_lora", rc);
-  if (!recorded) {
-    if (swz.found() && !record(out.ascales, swz)) throw python_error();
-    if (la16.found() && !record(out.lora_act, la16)) throw python_error();
-  }
+  if (swz.found() && !attach(out.ascales, swz.hold)) throw python_error();
+  if (la16.found() && !attach(out.lora_act, la16.hold)) throw python_error();
   return true;
 }
 
@@ -490,14 +440,29 @@ PyObject* py_pack(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// inner_twin(owner, any_version): the twin in owner's own storage as a tensor, or None
-PyObject* py_inner_twin(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+// output_twin(owner, any_version): what `attached` finds on the owner's storage itself, or None
+PyObject* py_output_twin(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  if (nargs != 2 || !THPVariable_Check(args[0])) { PyErr_SetString(PyExc_TypeError, "inner_twin(owner, any_version)"); return nullptr; }
+  if (nargs != 2 || !THPVariable_Check(args[0])) { PyErr_SetString(PyExc_TypeError, "output_twin(owner, any_version)"); return nullptr; }
   const Tensor& owner = THPVariable_Unpack(args[0]);
-  const InnerTwin* r = inner_twin(owner);
-  if (r == nullptr || (r->version != owner._version() && PyObject_IsTrue(args[1]) != 1)) Py_RETURN_NONE;
-  return THPVariable_Wrap(on_storage(owner, r->byte_offset, {r->twin_numel}, r->type));
+  if (output_storage(owner) == nullptr) Py_RETURN_NONE;
+  const Twin twin = attached(owner, PyObject_IsTrue(args[1]) == 1);
+  if (!twin.found()) Py_RETURN_NONE;
+  return THPVariable_Wrap(twin.hold);
+  END_HANDLE_TH_ERRORS
+}
+
+// attach_output(owner, twin): record the twin if it belongs on the owner's storage itself; whether it does
+PyObject* py_attach_output(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 2 || !THPVariable_Check(args[0]) || !THPVariable_Check(args[1])) {
+    PyErr_SetString(PyExc_TypeError, "attach_output(owner, twin)");
+    return nullptr;
+  }
+  const Tensor& owner = THPVariable_Unpack(args[0]);
+  if (output_storage(owner) == nullptr) Py_RETURN_FALSE;
+  attach(owner, THPVariable_Unpack(args[1]));
+  Py_RETURN_TRUE;
   END_HANDLE_TH_ERRORS
 }
 
@@ -609,7 +574,8 @@ PyMethodDef g_methods[] = {
     {"quantize", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_quantize)), METH_FASTCALL, nullptr},
     {"gemm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_gemm)), METH_FASTCALL, nullptr},
     {"pack", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_pack)), METH_FASTCALL, nullptr},
-    {"inner_twin", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_inner_twin)), METH_FASTCALL, nullptr},
+    {"output_twin", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_output_twin)), METH_FASTCALL, nullptr},
+    {"attach_output", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_attach_output)), METH_FASTCALL, nullptr},
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_bind)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_host", "Native host path of the operators.", -1, g_methods, nullptr, nullptr, nullptr, nullptr};

@@ -58,7 +58,9 @@ def _attach(owner: torch.Tensor, twin: torch.Tensor) -> None:
     storage, and the storage object lives exactly as long as the memory does, so a record can
     neither be lost on the way nor outlive its data and be found by a later tensor at the same
     address.  The owner's version counter (bumped by every in-place torch op) guards against
-    edits after the fact."""
+    edits after the fact.  Outputs of the native host path carry their record on the storage itself."""
+    if _lib._host is not None and _lib._host.attach_output(owner, twin):
+        return
     st = owner.untyped_storage()
     recs = getattr(st, _TWIN, None)
     if recs is None:
@@ -68,13 +70,16 @@ def _attach(owner: torch.Tensor, twin: torch.Tensor) -> None:
 
 
 def _attached(owner: torch.Tensor, any_version: bool = False) -> Optional[torch.Tensor]:
-    """The recorded twin of `owner`, or None.  Outputs of a small quantizer call share one storage with their
-    twins, and the native host path keeps the record."""
+    """The recorded twin of `owner`, or None."""
+    if _lib._host is not None:
+        twin = _lib._host.output_twin(owner, any_version)
+        if twin is not None:
+            return twin
     recs = getattr(owner.untyped_storage(), _TWIN, None)
     rec = None if recs is None else recs.get((owner.storage_offset(), owner.numel()))
-    if rec is not None and (rec[1] == owner._version or any_version):
-        return rec[0]
-    return None if _lib._host is None else _lib._host.inner_twin(owner, any_version)
+    if rec is None or (rec[1] != owner._version and not any_version):
+        return None
+    return rec[0]
 
 
 class _on_device:

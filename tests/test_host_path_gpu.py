@@ -65,3 +65,44 @@ def test_registered_ops_have_no_backward():
     assert la.requires_grad and not act.requires_grad
     with pytest.raises(RuntimeError):
         la.sum().backward()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,K", [(64, 128), (300, 512), (4352, 512)])
+def test_outputs_have_storages_of_their_own(M, K, dtype):
+    """None of a call's outputs shares memory with another or holds more than its own bytes: what is saved, shared or
+    kept of one does not bring the others along, and dropping the others gives their memory back."""
+    from svdquant_kernels_b200 import ops, torch_ops  # noqa: F401
+    x, sm, ld, *_ = _layer(dtype, M=M, K=K)
+    for call in (ops.quantize_w4a4_act_fuse_lora, torch.ops.svdq_b200.quantize_w4a4_act_fuse_lora):
+        call(x, ld, sm)                                        # makes the smooth table
+        held = lambda: torch.cuda.memory_stats()["requested_bytes.all.current"]
+        before = held()
+        out = call(x, ld, sm)
+        stores = [t.untyped_storage() for t in out]
+        assert len({s.data_ptr() for s in stores}) == 3
+        assert [s.nbytes() for s in stores] == [t.numel() * t.element_size() for t in out]
+        act = out[0]
+        del out, stores
+        assert held() - before == act.numel()                  # the twins went with their owners
+        del act
+
+
+def test_out_tensors_that_change_type_keep_their_twins_right():
+    """The outputs' own types do not depend on the input's, so a call may write into those of a call of the other type:
+    the 16-bit form of lora_act that the GEMM reads is then the last call's, in either order."""
+    from svdquant_kernels_b200 import ops
+    g = torch.Generator().manual_seed(9)
+    M, K, N, R = 256, 512, 256, 32
+    wgt, wsc = ops.quantize_nvfp4_rows((torch.randn(N, K, generator=g) * 0.02).cuda())
+    x, ld, lu = (torch.randn(M, K, generator=g), torch.randn(K, R, generator=g) / K ** 0.5, torch.randn(N, R, generator=g) * 0.01)
+    at = {t: (x.to(t).cuda(), ld.to(t).cuda(), lu.to(t).cuda()) for t in (torch.float16, torch.bfloat16)}
+    out = ops.quantize_w4a4_act_fuse_lora(*at[torch.float16][:2], None)
+    for i, t in enumerate((torch.bfloat16, torch.float16, torch.bfloat16)):
+        xt, ldt, lut = at[t]
+        xt = xt * (i + 1)
+        want = ops.quantize_w4a4_act_fuse_lora(xt, ldt, None)
+        got = ops.quantize_w4a4_act_fuse_lora(xt, ldt, None, out=out)
+        for u in (torch.float16, torch.bfloat16):
+            y0, y1 = (ops.gemm_w4a4(q[0], wgt, q[1], wsc, q[2], at[u][2], None, None, u) for q in (want, got))
+            assert torch.equal(y0, y1), (i, t, u)

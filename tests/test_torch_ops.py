@@ -93,3 +93,30 @@ def test_cuda_graph_through_the_dispatcher_matches_the_oracle(dtype):
     y2 = ops.gemm_w4a4(a2, wgt, s2, wsc, l2, lu_d, c_d, b_d, dtype)
     torch.cuda.synchronize()
     assert torch.equal(y, y2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M", [100, 2304])
+def test_registered_ops_keep_what_their_schemas_say(M, dtype):
+    """torch.library.opcheck on calls whose twins are not made yet, whose twins are there, and without options: outputs
+    alias neither each other nor an input, the fake kernels agree with the real ones, autograd and tracing see the ops."""
+    from svdquant_kernels_b200 import ops, torch_ops  # noqa: F401
+    g = torch.Generator().manual_seed(4)
+    K, N, R = 512, 384, 32
+    x = torch.randn(M, K, generator=g).to(dtype).cuda()
+    sm = (torch.rand(K, generator=g) + 0.5).to(dtype).cuda()
+    ld = (torch.randn(K, R, generator=g) / K ** 0.5).to(dtype).cuda()
+    lu = (torch.randn(N, R, generator=g) * 0.01).to(dtype).cuda()
+    c = (torch.rand(N, generator=g) + 0.5).to(dtype).cuda()
+    wgt, wsc = ops.quantize_nvfp4_rows((torch.randn(N, K, generator=g) * 0.02).cuda())
+    quantize, gemm = torch.ops.svdq_b200.quantize_w4a4_act_fuse_lora.default, torch.ops.svdq_b200.gemm_w4a4.default
+    for args in ((x, ld, sm), (x, ld, sm, 64), (x, ld)):
+        for _ in range(2):
+            torch.library.opcheck(quantize, args)
+    act, asc, la = quantize(x, ld, sm)
+    # (the schema check compares inputs with torch.allclose, which has no e4m3 form)
+    tests = ("test_autograd_registration", "test_faketensor", "test_aot_dispatch_dynamic")
+    for args in ((act, wgt, asc, wsc, la, lu, c, c, dtype), (act, wgt, asc, wsc)):
+        for _ in range(2):
+            torch.library.opcheck(gemm, args, test_utils=tests)
