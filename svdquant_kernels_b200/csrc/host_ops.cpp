@@ -27,6 +27,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/library.h>
 
+#include <functional>
 #include <unordered_map>
 
 #include "../../include/svdq_b200.h"
@@ -91,21 +92,32 @@ OutputStorage* output_storage(const Tensor& owner) {
   return st != nullptr && owner.storage_offset() == 0 && owner.numel() == st->numel ? st : nullptr;
 }
 
-// What `attached` last found on the storage objects of weights and smoothing factors, which a layer looks up on every
-// call: a hash lookup instead of half a dozen Python calls (0.25 us each, three a layer).  An entry holds nothing alive,
-// is good for one version of one tensor; its weak references keep the StorageImpls' addresses from being used again, not
-// their memory.  Entries of storages that are gone are swept out every kSweep insertions.
+// What `attached` found on the storage objects of weights and smoothing factors, which a layer looks up on every call: a
+// hash lookup instead of half a dozen Python calls (0.25 us each, three a layer).  One entry per owner - the views of a
+// flat buffer are owners each - good for one version of it.  It holds nothing alive: its weak references keep the
+// StorageImpls' addresses from being used again, not their memory.  Entries of storages that are gone are swept out every
+// kSweep insertions.
 constexpr size_t kSweep = 256;
+struct Owner {
+  const c10::StorageImpl* storage;
+  int64_t offset, numel;
+  explicit Owner(const Tensor& t) : storage(t.storage().unsafeGetStorageImpl()), offset(t.storage_offset()), numel(t.numel()) {}
+  bool operator==(const Owner& o) const { return storage == o.storage && offset == o.offset && numel == o.numel; }
+};
+struct OwnerHash {
+  size_t operator()(const Owner& o) const {
+    return std::hash<const void*>()(o.storage) ^ (static_cast<size_t>(o.offset) * 0x9E3779B97F4A7C15ull + static_cast<size_t>(o.numel));
+  }
+};
 struct KnownTwin {
   c10::weak_intrusive_ptr<c10::StorageImpl> owner, twin;
-  int64_t offset, numel;
   uint32_t version;
   void* ptr;
   ScalarType type;
   int64_t twin_numel;
 };
-std::unordered_map<const c10::StorageImpl*, KnownTwin>& known_twins() {
-  static auto* table = new std::unordered_map<const c10::StorageImpl*, KnownTwin>();
+std::unordered_map<Owner, KnownTwin, OwnerHash>& known_twins() {
+  static auto* table = new std::unordered_map<Owner, KnownTwin, OwnerHash>();             // outlives every tensor
   return *table;
 }
 c10::weak_intrusive_ptr<c10::StorageImpl> weak(const Tensor& t) {
@@ -121,11 +133,10 @@ Twin attached(const Tensor& owner, bool any_version = false) {
   if (const OutputStorage* st = output_storage(owner))
     return st->twin.defined() && (any_version || st->version == owner._version()) ? with(st->twin) : Twin();
   auto& known = known_twins();
-  const c10::StorageImpl* const impl = owner.storage().unsafeGetStorageImpl();
+  const Owner me(owner);
   if (!any_version) {
-    const auto it = known.find(impl);
-    if (it != known.end() && it->second.offset == owner.storage_offset() && it->second.numel == owner.numel() &&
-        it->second.version == owner._version()) {
+    const auto it = known.find(me);
+    if (it != known.end() && it->second.version == owner._version()) {
       auto alive = it->second.twin.lock();
       if (alive) return Twin{it->second.ptr, it->second.type, it->second.twin_numel, Tensor(), std::move(alive)};
     }
@@ -146,9 +157,9 @@ Twin attached(const Tensor& owner, bool any_version = false) {
   if (!any_version && ptr != nullptr) {
     static size_t inserted = 0;
     if (++inserted % kSweep == 0)
-      for (auto it = known.begin(); it != known.end();) it = it->second.owner.expired() ? known.erase(it) : std::next(it);
-    known.insert_or_assign(impl, KnownTwin{weak(owner), weak(t), owner.storage_offset(), owner.numel(), static_cast<uint32_t>(owner._version()),
-                                           ptr, t.scalar_type(), t.numel()});
+      for (auto it = known.begin(); it != known.end();)
+        it = it->second.owner.expired() || it->second.twin.expired() ? known.erase(it) : std::next(it);
+    known.insert_or_assign(me, KnownTwin{weak(owner), weak(t), static_cast<uint32_t>(owner._version()), ptr, t.scalar_type(), t.numel()});
   }
   return Twin{ptr, t.scalar_type(), t.numel(), t, {}};
 }

@@ -106,3 +106,47 @@ def test_out_tensors_that_change_type_keep_their_twins_right():
         for u in (torch.float16, torch.bfloat16):
             y0, y1 = (ops.gemm_w4a4(q[0], wgt, q[1], wsc, q[2], at[u][2], None, None, u) for q in (want, got))
             assert torch.equal(y0, y1), (i, t, u)
+
+
+def test_views_of_one_buffer_are_known_side_by_side():
+    """Smoothing factors (or weights) kept as views of one flat buffer: the native table has an entry for each.  With the
+    records on the buffer's storage object taken away it is the table alone that answers."""
+    from svdquant_kernels_b200 import _lib, ops
+    x, _, ld, *_ = _layer(torch.float16)
+    host = _lib.host()
+    flat = torch.rand(4 * 512, generator=torch.Generator().manual_seed(3)).add_(0.5).half().cuda()
+    views = flat.chunk(4)
+    want = [ops.quantize_w4a4_act_fuse_lora(x, ld, v.clone()) for v in views]
+    for v in views:
+        ops.quantize_w4a4_act_fuse_lora(x, ld, v)              # makes the record
+        assert host.quantize(x, ld, v, 256, None) is not None  # finds it
+    twins = [ops._attached(v) for v in views]
+    del flat.untyped_storage()._svdq_twins
+    for v, w in zip(views, want):
+        got = host.quantize(x, ld, v, 256, None)
+        assert got is not None
+        assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(got, w))
+    flat.mul_(1.0)                                             # a new version: no entry is good any more
+    assert all(host.quantize(x, ld, v, 256, None) is None for v in views)
+    del twins
+
+
+def test_replaced_weights_are_told_apart():
+    """More short-lived owners than the native table sweeps at a time, most of them at an address an earlier one had:
+    every call uses the factors it is given."""
+    from svdquant_kernels_b200 import _lib, ops
+    g = torch.Generator().manual_seed(8)
+    x, ld = torch.randn(64, 128, generator=g).half().cuda(), torch.randn(128, 16, generator=g).half().cuda()
+    kept, seen = [], set()
+    for i in range(600):
+        sm = (torch.rand(128, generator=g) + 0.5).half().cuda()
+        seen.add(sm.data_ptr())
+        want = ops.quantize_w4a4_act_fuse_lora(x, ld, sm, _force=_lib.QUANT_FORCE_GENERIC)
+        for _ in range(2):                                     # with the table made by this call, and with a known one
+            got = ops.quantize_w4a4_act_fuse_lora(x, ld, sm)
+            assert torch.equal(got[0], want[0]) and torch.equal(got[1].view(torch.uint8), want[1].view(torch.uint8)), i
+        if i % 3 == 0:
+            kept.append((sm, want[0]))
+    assert len(seen) < 600
+    for sm, want in kept:
+        assert torch.equal(ops.quantize_w4a4_act_fuse_lora(x, ld, sm)[0], want)
