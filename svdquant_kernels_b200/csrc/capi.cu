@@ -324,11 +324,13 @@ int svdq_gemm_w4a4_static_ws(const void* act, const void* wgt, const void* ascal
                              const void* wcscales, const void* bias, void* y, int M, int N, int K, int R, int dtype,
                              int variant, void* stream) {
   if (!gemm_supported(M, N, K, R)) return SVDQ_ERR_SHAPE;
-  // what this call would park in the workspace: the library's own plan, or the forced split count
+  // what this call would park in the workspace: the library's own plan, or the forced split count.  Everything else
+  // (whole 256-row tiles, which split within clusters; plain tiles) uses none of it.
+  const int form = variant & ~(SVDQ_GEMM_LORA_INTERLEAVE | SVDQ_GEMM_LORA_AT_END | SVDQ_GEMM_NO_SPLIT);
   size_t need = 0;
-  if (variant == 0) need = gemm_split_workspace_bytes(M, N, K, R);
-  else if (variant >= 10000)
-    need = kSplitTicketBytes + static_cast<size_t>(M / 128) * (N / 128) * (variant / 10000) * (128 * 128 * 4);
+  if (form == 0 && (variant & SVDQ_GEMM_NO_SPLIT) == 0 && M % 256 != 0) need = gemm_split_workspace_bytes(M, N, K, R);
+  else if (form >= 10000 && form % 10000 == 128)
+    need = kSplitTicketBytes + static_cast<size_t>(M / 128) * (N / 128) * (form / 10000) * (128 * 128 * 4);
   if (need > kStaticWsBytes) return SVDQ_ERR_UNSUPPORTED;
   // the array's address on the current device, looked up once per device and kept
   void* ws = nullptr;

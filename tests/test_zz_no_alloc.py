@@ -21,7 +21,7 @@ def _inputs(M, K, N, R, dtype, seed):
     lu = (torch.randn(N, R, generator=g) * 0.01).to(dtype).cuda()
     c = (torch.rand(N, generator=g) + 0.5).to(dtype).cuda()
     b = (torch.randn(N, generator=g) * 0.01).to(dtype).cuda()
-    act, asc, la = ops.quantize_w4a4_act_fuse_lora(x, ld, sm)
+    act, asc, la = ops.quantize_w4a4_act_fuse_lora(x, ld, sm, pad_size=128)
     wgt, wsc = ops.quantize_nvfp4_rows(w, pad_size=1)
     return act, wgt, asc, wsc, la, lu, c, b
 
@@ -43,13 +43,19 @@ def _static_call(args, dtype, variant=0):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-def test_static_workspace_matches_caller_owned_workspace(dtype):
+@pytest.mark.parametrize("M", [128, 256, 384])
+def test_static_workspace_matches_caller_owned_workspace(M, dtype):
+    """Odd multiples of 128 rows split through the workspace (the caller's is seen to be written), whole 256-row tiles
+    within clusters, without it."""
     from svdquant_kernels_b200 import ops, _lib
-    M, K, N, R = 256, 10240, 3072, 32
-    assert int(_lib.load().svdq_gemm_w4a4_workspace_bytes(M, N, K, R)) > 0      # this shape takes the split-K form
+    K, N, R = 10240, 3072, 32
+    need = int(_lib.load().svdq_gemm_w4a4_workspace_bytes(M, N, K, R))
     args = _inputs(M, K, N, R, dtype, 21)
     act, wgt, asc, wsc, la, lu, c, b = args
+    ws = ops._split_workspace(act.device, need)
+    ws[1024:].fill_(0xFF)
     want = ops.gemm_w4a4(act, wgt, asc, wsc, la, lu, c, b, dtype)              # svdq_gemm_w4a4_ws
+    assert bool((ws[1024:need] != 0xFF).any()) == (M % 256 != 0)
     for call in range(2):
         rc, y = _static_call(args, dtype)
         torch.cuda.synchronize()
@@ -67,22 +73,32 @@ def test_static_workspace_matches_caller_owned_workspace(dtype):
 
 
 def test_static_workspace_refuses_what_does_not_fit():
-    from svdquant_kernels_b200 import _lib
+    from svdquant_kernels_b200 import _lib, ops
     args = _inputs(256, 10240, 3072, 32, torch.float16, 23)
     rc, _ = _static_call(args, torch.float16, variant=40128)      # 48 tiles x 4 splits = 192 partial tiles > 148
     assert rc == 7, _lib.status_string(rc)
+    # ... and nothing else: a call that uses none of the workspace is not held to its size
+    act, wgt, asc, wsc, la, lu, c, b = args
+    whole = ops.gemm_w4a4(act, wgt, asc, wsc, la, lu, c, b, torch.float16, _splits=1)
+    for variant in (_lib.GEMM_NO_SPLIT, _lib.GEMM_NO_SPLIT | _lib.GEMM_LORA_AT_END):
+        rc, y = _static_call(args, torch.float16, variant=variant)
+        assert rc == 0 and torch.equal(y, whole)
+    rc, y = _static_call(args, torch.float16, variant=_lib.GEMM_LORA_AT_END)
+    assert rc == 0 and torch.equal(y, ops.gemm_w4a4(act, wgt, asc, wsc, la, lu, c, b, torch.float16))
     torch.cuda.synchronize()
     assert_device_clean()
 
 
-def test_static_workspace_calls_allocate_nothing_and_chain_without_host_syncs():
+@pytest.mark.parametrize("M", [128, 256, 384])
+def test_static_workspace_calls_allocate_nothing_and_chain_without_host_syncs(M):
     """The point of the entry point: once it has been called on a device, further calls take no device
     memory from anywhere (free memory as the driver reports it does not move), and calls queued back to
     back on one stream with no host synchronisation in between - each starts its set-up while the one
-    before it is still running - all return the result of the caller-workspace form."""
+    before it is still running, and all park their partial tiles in the one array - all return the result
+    of the caller-workspace form."""
     from svdquant_kernels_b200 import ops
     dtype = torch.float16
-    args = _inputs(256, 10240, 3072, 32, dtype, 24)
+    args = _inputs(M, 10240, 3072, 32, dtype, 24)
     act, wgt, asc, wsc, la, lu, c, b = args
     want = ops.gemm_w4a4(act, wgt, asc, wsc, la, lu, c, b, dtype)
     rc, y = _static_call(args, dtype)                 # first call on this device may look the array's address up
