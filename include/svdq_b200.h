@@ -122,8 +122,9 @@ int svdq_quantize_w4a4_act_fuse_lora_ws(const void* x, const void* lora_down, co
                                         void* stream);
 
 /*
- * How many clusters of `k_split` CTAs (1, 2, 4 or 8) of the fused quantizer the current device can
- * keep resident at once for LoRA rank R; -1 on error.  Introspection for tuning; the reference
+ * How many clusters of `k_split` CTAs of the fused quantizer the current device can keep resident at
+ * once for LoRA rank R; -1 on error.  It answers for 1, 2, 4 and 8; the quantizer also launches other
+ * sizes (up to 16) and asks the runtime about those by itself.  Introspection for tuning; the reference
  * has no counterpart (its Triton launch picks k_splits from a table,
  * triton_kernels/quantize_w4a4_act_fuse_lora/kernel.py:344-378).
  */
@@ -212,14 +213,18 @@ int svdq_gemm_w4a4_next(const void* act, const void* wgt, const void* ascales_sw
  * svdq_gemm_w4a4 with a caller-owned workspace in device memory, for problems with few output tiles
  * (a few hundred rows: the small-M shapes of GEMM_SHAPES in
  * cute_kernels/gemm_w4a4/harness.py:17-24, where the reference's kernels leave most SMs idle).
- * With variant 0, M an odd multiple of 128 and a workspace of at least
- * svdq_gemm_w4a4_workspace_bytes(M, N, K, R) bytes (room for forced splits otherwise) the library shares each 128 x 128 tile's K loop among several CTAs (split-K): each adds its part in
- * fp32, parks it in the workspace, and the CTA that arrives last sums the parts in a fixed order
- * and writes y, so results do not depend on timing.  variant 10000 * S + 128 forces S CTAs per tile.
- * M a multiple of 256: svdq_gemm_w4a4 itself, with or without a workspace, shares 256 x 128 tiles among
- * the CTA pairs of a cluster, equally deterministic; variant 10000 * S + 2128 forces S pairs per tile.
- * svdq_gemm_w4a4_workspace_bytes returns 0 where splitting does not apply; then (or with a NULL or
- * smaller workspace) the call is svdq_gemm_w4a4.
+ * M an odd multiple of 128: with variant 0 and a workspace of at least
+ * svdq_gemm_w4a4_workspace_bytes(M, N, K, R) bytes the library shares each 128 x 128 tile's K loop
+ * among several CTAs (split-K): each adds its part in fp32, parks it in the workspace, and the CTA
+ * that arrives last sums the parts in a fixed order and writes y, so results do not depend on
+ * timing.  Where the function returns 0, or with a NULL or smaller workspace, the call is
+ * svdq_gemm_w4a4.
+ * M a multiple of 256: with variant 0 the workspace is never used (pass NULL and 0).  svdq_gemm_w4a4
+ * itself shares 256 x 128 tiles among the CTA pairs of a cluster, equally deterministic; variant
+ * 10000 * S + 2128 forces S pairs per tile, which needs no workspace either.
+ * variant 10000 * S + 128 forces S CTAs per 128 x 128 tile for either kind of M and needs
+ * 1024 + (M / 128) * (N / 128) * S * 65536 bytes.  svdq_gemm_w4a4_workspace_bytes returns that size for
+ * the S it would plan, or 0; for M a multiple of 256 it is of use to such a forced call only.
  * The first 1024 bytes of the workspace are ticket counters: zero them once before the first call;
  * every call leaves them zero.  Calls that share a workspace must not overlap in time (same stream,
  * or ordered by events); after a call whose bounded wait expired (svdq_device_status != 0) zero it again.
@@ -238,8 +243,8 @@ int svdq_gemm_w4a4_ws(const void* act, const void* wgt, const void* ascales_swz,
  * call; a latency-bound loop that cannot afford the device-wide synchronisation an allocation or
  * a release may bring.  The function itself allocates and frees nothing, on the host or the device.
  * The workspace is a static array in device memory of 1024 + 148 * 65536 bytes (9.25 MiB, taken on
- * every device that loads the library); a call whose split plan (or forced split count, variant
- * 10000 * S + 128) needs more returns SVDQ_ERR_UNSUPPORTED and launches nothing.  Otherwise the
+ * every device that loads the library); a call that uses the workspace (see svdq_gemm_w4a4_ws) and
+ * whose plan or forced split count needs more returns SVDQ_ERR_UNSUPPORTED and launches nothing.  Otherwise the
  * result is that of svdq_gemm_w4a4_ws with a large enough workspace, bit for bit.
  * The first call on each device looks the array's address up through the runtime, which may load
  * the module: make that call before any stream capture is begun on that device.

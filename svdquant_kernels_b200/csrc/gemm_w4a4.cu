@@ -948,7 +948,8 @@ int gemm_cluster_split(int M, int N, int K, int R) {
   return 1;
 }
 
-// Workspace form, for row counts that are an odd multiple of 128.
+// Workspace form.  The library runs this plan for row counts that are an odd multiple of 128; for whole 256-row tiles
+// (split within clusters above) it only tells a caller who forces the form how much room that takes.
 // Split-K plan for a problem with few tiles: 128 x 128 tiles, each tile's slabs shared by S CTAs that
 // all run at once (tiles * S <= SMs).  One CTA streams a tile's slabs at about 0.3 us each however
 // few tiles there are (32 KB per slab through one SM's load path), so with a few dozen tiles most

@@ -71,7 +71,10 @@ def test_argument_validation_needs_no_device(lib_path):
     assert dst.tolist() == [1.0, -0.0078125, 0.0, 2.0]
     big = np.array([0x4800], dtype=np.uint16)                                   # 131072 as bf16
     assert lib.svdq_lora_up_to_f16(big.ctypes.data, dst.ctypes.data, 1) == 7
-    # split-K workspace: only for few tiles and a long K; ticket block + tiles x splits partial tiles of 64 KB
+    # split-K workspace: only for few tiles and a long K; ticket block + tiles x splits partial tiles of 64 KB.  Variant 0
+    # uses it for odd multiples of 128 rows; for whole 256-row tiles it is the room a forced split of that count takes
+    assert lib.svdq_gemm_w4a4_workspace_bytes(128, 3072, 10240, 32) == 1024 + 24 * 4 * 65536
+    assert lib.svdq_gemm_w4a4_workspace_bytes(384, 3072, 10240, 32) == 1024 + 72 * 2 * 65536
     assert lib.svdq_gemm_w4a4_workspace_bytes(256, 3072, 10240, 32) == 1024 + 48 * 3 * 65536
     assert lib.svdq_gemm_w4a4_workspace_bytes(256, 3840, 15360, 128) == 1024 + 60 * 2 * 65536
     assert lib.svdq_gemm_w4a4_workspace_bytes(256, 3072, 3840, 128) == 0          # K too short to repay the split

@@ -19,7 +19,7 @@ def _ops():
     return ops
 
 
-def _case(M, K, N, R, dtype, seed, wc=True, bias=True, tiler=None, act="gauss", splits=None, repeat=1):
+def _case(M, K, N, R, dtype, seed, wc=True, bias=True, tiler=None, act="gauss", splits=None, repeat=1, pad=256):
     ops = _ops()
     g = torch.Generator().manual_seed(seed)
     x = torch.randn(M, K, generator=g)
@@ -34,7 +34,7 @@ def _case(M, K, N, R, dtype, seed, wc=True, bias=True, tiler=None, act="gauss", 
     b = (torch.randn(N, generator=g) * 0.01).to(dtype) if bias else None
     c = (torch.rand(N, generator=g) + 0.5).to(dtype) if wc else None
     dev = "cuda"
-    act_t, asc, la = ops.quantize_w4a4_act_fuse_lora(x.to(dev), ld.to(dev), sm.to(dev))
+    act_t, asc, la = ops.quantize_w4a4_act_fuse_lora(x.to(dev), ld.to(dev), sm.to(dev), pad_size=pad)
     wgt, wsc = ops.quantize_nvfp4_rows(w.to(dev), pad_size=1)
     has_lora = R > 0
     for _ in range(repeat):
@@ -218,17 +218,24 @@ def test_back_to_back_steps_keep_their_results():
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("M,K,N,R,splits", [(256, 7680, 3072, 128, None), (256, 3840, 3072, 128, 2), (256, 3840, 3072, 128, 3),
                                             (128, 1024, 256, 0, 4), (128, 2560, 512, 32, 6), (384, 704, 1280, 256, 3),
-                                            (128, 10240, 3072, 32, None), (512, 15360, 1024, 64, None)])
+                                            (128, 10240, 3072, 32, None), (512, 15360, 1024, 64, None),
+                                            (384, 7680, 3072, 128, None), (640, 15360, 1024, 64, None)])
 def test_split_k(M, K, N, R, splits, dtype):
     """Few output tiles: a tile's K loop is shared by several CTAs whose fp32 partial tiles are summed
-    in a fixed order by the last one to arrive.  Chosen by the library (None) or forced; twice in a
-    row and with changing split counts on the same workspace (the ticket counters return to zero)."""
+    in a fixed order by the last one to arrive.  Chosen by the library (None: through the workspace for
+    an odd multiple of 128 rows, within clusters otherwise) or forced; twice in a row and with changing
+    split counts on the same workspace (the ticket counters return to zero)."""
     ops = _ops()
     if splits is None:
-        assert int(ops._lib.load().svdq_gemm_w4a4_workspace_bytes(M, N, K, R)) > 0, "this shape should split"
-    assert _case(M, K, N, R, dtype, seed=M + K, splits=splits, repeat=2) <= TOL
-    assert _case(M, K, N, R, dtype, seed=M + K + 1, splits=2, repeat=1) <= TOL
-    assert _case(M, K, N, R, dtype, seed=M + K + 2, splits=1) <= TOL
+        need = int(ops._lib.load().svdq_gemm_w4a4_workspace_bytes(M, N, K, R))
+        assert need > 0, "this shape should split"
+        ws = ops._split_workspace(torch.device("cuda"), need)
+        ws[1024:].fill_(0xFF)
+    assert _case(M, K, N, R, dtype, seed=M + K, splits=splits, repeat=2, pad=128) <= TOL
+    if splits is None:
+        assert bool((ws[1024:need] != 0xFF).any()) == (M % 256 != 0)
+    assert _case(M, K, N, R, dtype, seed=M + K + 1, splits=2, repeat=1, pad=128) <= TOL
+    assert _case(M, K, N, R, dtype, seed=M + K + 2, splits=1, pad=128) <= TOL
 
 
 def test_split_k_is_deterministic():

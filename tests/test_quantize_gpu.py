@@ -316,8 +316,8 @@ def test_out_argument_reuses_buffers_and_twins():
 
 
 def test_cluster_capacity_query():
-    """How many clusters of 1, 2, 4 and 8 CTAs of the fused kernel the device holds at once: the query
-    answers for every split the kernel can be launched with."""
+    """How many clusters of 1, 2, 4 and 8 CTAs of the fused kernel the device holds at once: the sizes the query answers
+    for (the launch asks the runtime about the others it uses)."""
     from svdquant_kernels_b200 import _lib
     lib = _lib.load()
     caps = {ks: lib.svdq_quantizer_max_active_clusters(128, ks, _lib.DTYPE_F16) for ks in (1, 2, 4, 8)}
