@@ -26,13 +26,6 @@ __device__ __forceinline__ float to_f32(__half v) { return __half2float(v); }
 __device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
 __device__ __forceinline__ float to_f32(float v) { return v; }
 
-// e4m3 byte of clamp(amax/6, 1e-12, 448); round-to-nearest-even incl. subnormals.
-__device__ __forceinline__ uint8_t scale_byte_from_amax(float amax) {
-  float s = __fdiv_rn(amax, 6.0f);
-  s = fminf(fmaxf(s, 1e-12f), 448.0f);
-  return static_cast<uint8_t>(__nv_cvt_float_to_fp8(s, __NV_SATFINITE, __NV_E4M3));
-}
-
 // exact value of a non-negative e4m3 byte
 __device__ __forceinline__ float e4m3_to_f32(uint8_t b) {
   uint32_t e = (b >> 3) & 0xF, m = b & 7;

@@ -152,10 +152,9 @@ quantize_rows_kernel(const T* __restrict__ x, const T* __restrict__ smooth, uint
   // the tensor-core order exists only for whole tiles of 128 rows and 4 groups: word w of an atom is row
   // 32 (w % 4) + w / 4, its bytes the row's four groups
   if (scales_swz != nullptr) {
-    const int a = threadIdx.x >> 7, w = threadIdx.x & 127, r = 32 * (w & 3) + (w >> 2);
-    if (g0 + 4 * a < groups)
-      *reinterpret_cast<uint32_t*>(scales_swz + sf_swizzled_offset(m0 + r, g0 + 4 * a, groups)) =
-          sc[4 * a][r] | (sc[4 * a + 1][r] << 8) | (sc[4 * a + 2][r] << 16) | (static_cast<uint32_t>(sc[4 * a + 3][r]) << 24);
+    const int w = threadIdx.x, r = 32 * (w & 3) + (w >> 2);
+    *reinterpret_cast<uint32_t*>(scales_swz + sf_swizzled_offset(m0 + r, g0, groups)) =
+        sc[0][r] | (sc[1][r] << 8) | (sc[2][r] << 16) | (static_cast<uint32_t>(sc[3][r]) << 24);
   }
 }
 

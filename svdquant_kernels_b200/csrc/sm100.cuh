@@ -203,15 +203,6 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
-// Same, issued from either CTA of a pair; `bar_cluster_addr` is a shared::cluster
-// address, so the bytes can be counted on the partner CTA's barrier.
-__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* m, int x, int y,
-                                                 uint32_t bar_cluster_addr) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr), "r"(x), "r"(y)
-      : "memory");
-}
 // Tiled load whose completion bytes are counted on the barrier at the shared::cluster address
 // `bar`.  CG = 1: a barrier of this CTA.  CG = 2: the .cta_group::2 form, which lets either CTA
 // of a pair count its bytes on the partner's barrier.
@@ -234,13 +225,6 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gmem_sr
   asm volatile(
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(gmem_src)), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ void bulk_load_1d_cluster_bar(void* smem_dst, const void* gmem_src, uint32_t bytes,
-                                                         uint32_t bar_cluster_addr) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(gmem_src)), "r"(bytes), "r"(bar_cluster_addr)
       : "memory");
 }
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* smem_src, int x, int y) {
@@ -458,10 +442,6 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t cta_
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(cta_rank));
   return r;
 }
-__device__ __forceinline__ void st_cluster_f4(uint32_t cluster_addr, float4 v) {
-  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
-               ::"r"(cluster_addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
-}
 // Copy engine, this CTA's shared memory -> another CTA of the cluster; the bytes are counted on a barrier
 // of the receiving CTA (both destination addresses are cluster addresses from map_to_cta).  The source
 // must stay in place until the receiver has seen its barrier complete and said so.
@@ -469,11 +449,6 @@ __device__ __forceinline__ void bulk_copy_smem_to_cluster(uint32_t dst_cluster_a
                                                           uint32_t bytes, uint32_t bar_cluster_addr) {
   asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(dst_cluster_addr), "r"(src_cta_addr), "r"(bytes), "r"(bar_cluster_addr) : "memory");
-}
-__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t cluster_addr) {
-  uint32_t v;
-  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");
-  return v;
 }
 // volatile: in order with the barriers around it; no memory clobber, so that the use of one load need not precede the next
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
