@@ -1,4 +1,4 @@
-"""The row packer at the edges of its 128-row x 8-group tiles, all input types, against the oracle."""
+"""The row packer at the edges of its 128-row x 4-group tiles, all input types, against the oracle."""
 import numpy as np
 import pytest
 import torch

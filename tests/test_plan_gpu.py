@@ -103,8 +103,8 @@ def test_few_rows_long_k():
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("M,K,N,R", [(1100, 4096, 256, 32), (1300, 256, 4096, 48), (600, 15360, 512, 32)])
 def test_chunked_call_matches_device_ops(M, K, N, R, dtype):
-    """Calls of more than 6 MB a side walk their rows in chunks (the last one ragged here); the result is
-    that of the device operators on all rows at once, bit for bit, split-K shapes included."""
+    """Tall calls walk their rows in chunks whose size goes with the square root of the call's bytes (the last one ragged
+    here); the result is that of the device operators on all rows at once, bit for bit, split-K shapes included."""
     plan, device_path, g = _setup(M, K, N, R, dtype, 13)
     try:
         for pinned in (True, False, True):
