@@ -14,7 +14,6 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
-#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
@@ -81,10 +80,10 @@ struct OutputStorage final : c10::StorageImpl {
       : c10::StorageImpl(use_byte_size_t(), nbytes, allocator, /*resizable=*/true), numel(numel) {}
   void release_resources() override {
     c10::StorageImpl::release_resources();
-    twin = Tensor();
+    twin = Twin();
   }
   const int64_t numel;
-  Tensor twin;
+  Twin twin;
   uint32_t version = 0;                 // of the owner that the twin was made from
 };
 OutputStorage* output_storage(const Tensor& owner) {
@@ -125,13 +124,11 @@ c10::weak_intrusive_ptr<c10::StorageImpl> weak(const Tensor& t) {
       c10::intrusive_ptr<c10::StorageImpl>::unsafe_reclaim_from_nonowning(t.storage().unsafeGetStorageImpl()));
 }
 
-Twin with(const Tensor& t) { return Twin{t.numel() > 0 ? t.data_ptr() : nullptr, t.scalar_type(), t.numel(), t, {}}; }
-
 // The twin recorded for `owner`: on its storage, or on the storage's Python object (the records ops._attach keeps:
 // {(offset, numel): (twin, version)}); not found if there is none or it is out of date.  GIL held.
 Twin attached(const Tensor& owner, bool any_version = false) {
   if (const OutputStorage* st = output_storage(owner))
-    return st->twin.defined() && (any_version || st->version == owner._version()) ? with(st->twin) : Twin();
+    return any_version || st->version == owner._version() ? st->twin : Twin();
   auto& known = known_twins();
   const Owner me(owner);
   if (!any_version) {
@@ -164,8 +161,34 @@ Twin attached(const Tensor& owner, bool any_version = false) {
   return Twin{ptr, t.scalar_type(), t.numel(), t, {}};
 }
 
+// A tensor on a storage of its own, without the checks and guards of at::empty: every caller has seen a tensor on the
+// current device `dev` already.  Five of these are most of a small quantizer call's host time.
+Tensor on_storage(c10::intrusive_ptr<c10::StorageImpl> st, at::IntArrayRef sizes, ScalarType t) {
+  Tensor r = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(std::move(st)), c10::DispatchKeySet(c10::DispatchKey::CUDA),
+                                                      c10::scalarTypeToTypeMeta(t));
+  r.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+  return r;
+}
+c10::intrusive_ptr<c10::StorageImpl> new_storage(int64_t numel, ScalarType t) {
+  return c10::make_intrusive<c10::StorageImpl>(c10::StorageImpl::use_byte_size_t(), static_cast<size_t>(numel) * c10::elementSize(t),
+                                               c10::cuda::CUDACachingAllocator::get(), /*resizable=*/true);
+}
+Tensor empty(at::IntArrayRef sizes, ScalarType t) { return on_storage(new_storage(c10::multiply_integers(sizes), t), sizes, t); }
+// An output that gets a twin, on a storage that the twin can hang on
+Tensor empty_output(int64_t rows, int64_t cols, ScalarType t) {
+  const int64_t numel = rows * cols;
+  return on_storage(c10::make_intrusive<OutputStorage>(static_cast<size_t>(numel) * c10::elementSize(t), c10::cuda::CUDACachingAllocator::get(), numel),
+                    {rows, cols}, t);
+}
+Twin empty_twin(int64_t numel, ScalarType t) {
+  auto st = new_storage(numel, t);
+  void* const ptr = st->mutable_data();
+  return Twin{ptr, t, numel, Tensor(), std::move(st)};
+}
+Tensor tensor_of(const Twin& twin) { return twin.hold.defined() ? twin.hold : on_storage(twin.hold_storage, {twin.numel}, twin.type); }
+
 // Record `twin` as the derived form of `owner`'s current contents.  GIL held; false with a Python error set.
-bool attach(const Tensor& owner, const Tensor& twin) {
+bool attach(const Tensor& owner, const Twin& twin) {
   if (OutputStorage* st = output_storage(owner)) {
     st->twin = twin;
     st->version = static_cast<uint32_t>(owner._version());
@@ -181,7 +204,7 @@ bool attach(const Tensor& owner, const Tensor& twin) {
   }
   Ref hold(recs);
   Ref key(Py_BuildValue("(LL)", static_cast<long long>(owner.storage_offset()), static_cast<long long>(owner.numel())));
-  Ref wrapped(THPVariable_Wrap(twin));
+  Ref wrapped(THPVariable_Wrap(tensor_of(twin)));
   if (key.p == nullptr || wrapped.p == nullptr) return false;
   Ref rec(Py_BuildValue("(Ol)", wrapped.p, static_cast<long>(owner._version())));
   return rec.p != nullptr && PyDict_SetItem(recs, key.p, rec.p) == 0;
@@ -192,21 +215,6 @@ bool attach(const Tensor& owner, const Tensor& twin) {
 bool plain(const Tensor& t, c10::DeviceIndex dev) {
   return t.defined() && t.is_cuda() && t.device().index() == dev && t.is_contiguous() && !t.is_inference() &&
          t.layout() == at::kStrided && !t.is_conj() && !t.is_neg();
-}
-
-Tensor empty(at::IntArrayRef sizes, ScalarType t, c10::DeviceIndex dev) {
-  return Tensor(at::detail::empty_cuda(sizes, t, c10::Device(c10::kCUDA, dev), std::nullopt));
-}
-
-// An output that gets a twin, on a storage that the twin can hang on
-Tensor empty_output(int64_t rows, int64_t cols, ScalarType t, c10::DeviceIndex dev) {
-  const int64_t numel = rows * cols;
-  if (numel == 0) return empty({rows, cols}, t, dev);
-  auto st = c10::make_intrusive<OutputStorage>(static_cast<size_t>(numel) * c10::elementSize(t), c10::cuda::CUDACachingAllocator::get(), numel);
-  Tensor r = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(std::move(st)), c10::DispatchKeySet(c10::DispatchKey::CUDA),
-                                                      c10::scalarTypeToTypeMeta(t));
-  r.unsafeGetTensorImpl()->set_sizes_contiguous({rows, cols});
-  return r;
 }
 
 void throw_status(const char* what, int rc) {
@@ -251,13 +259,12 @@ bool quantize(const Tensor& x, const Tensor& ld, const Tensor& smooth, int64_t p
     la16 = attached(out.lora_act, true);
     if (la16.found() && la16.type != t) la16 = Twin();
   } else {
-    out.act = empty({Mp, K / 2}, at::kByte, dev);
-    out.ascales = empty_output(K / 16, Mp, at::kFloat8_e4m3fn, dev);
-    out.lora_act = empty_output(Mp, R, at::kFloat, dev);
+    out.act = empty({Mp, K / 2}, at::kByte);
+    out.ascales = empty_output(K / 16, Mp, at::kFloat8_e4m3fn);
+    out.lora_act = R > 0 ? empty_output(Mp, R, at::kFloat) : empty({Mp, R}, at::kFloat);
   }
-  if (want_swz && !swz.found()) swz = with(empty({Mp * (K / 16)}, at::kByte, dev));
-  if (R > 0 && !la16.found())
-    la16 = with(empty({svdq_lora_act16_elems(static_cast<int>(Mp), static_cast<int>(R), dtype_code(t))}, t, dev));
+  if (want_swz && !swz.found()) swz = empty_twin(Mp * (K / 16), at::kByte);
+  if (R > 0 && !la16.found()) la16 = empty_twin(svdq_lora_act16_elems(static_cast<int>(Mp), static_cast<int>(R), dtype_code(t)), t);
   void* const stream = c10::cuda::getCurrentCUDAStream(dev).stream();
   auto ptr = [](const Tensor& v) -> void* { return v.defined() && v.numel() > 0 ? v.data_ptr() : nullptr; };
   int rc;
@@ -268,8 +275,8 @@ bool quantize(const Tensor& x, const Tensor& ld, const Tensor& smooth, int64_t p
                                           static_cast<int>(K), static_cast<int>(R), static_cast<int>(Mp), dtype_code(t), 0, stream);
   }
   if (rc != SVDQ_OK) throw_status("quantize_w4a4_act_fuse_lora", rc);
-  if (swz.found() && !attach(out.ascales, swz.hold)) throw python_error();
-  if (la16.found() && !attach(out.lora_act, la16.hold)) throw python_error();
+  if (swz.found() && !attach(out.ascales, swz)) throw python_error();
+  if (la16.found() && !attach(out.lora_act, la16)) throw python_error();
   return true;
 }
 
@@ -324,15 +331,15 @@ bool gemm(const GemmArgs& a, ScalarType out_t, GemmResult& r) {
   const int m = static_cast<int>(M), n = static_cast<int>(N), k = static_cast<int>(K), rr = static_cast<int>(R), dt = dtype_code(out_t);
   auto ptr = [](const Tensor& v) -> void* { return v.defined() && v.numel() > 0 ? v.data_ptr() : nullptr; };
   if (a.smooth_next.defined()) {
-    if (!r.y.defined()) r.y = empty({M, N}, out_t, dev);
-    r.qout = empty({M, N / 2}, at::kByte, dev);
-    r.oscales = empty({N / 16, M}, at::kFloat8_e4m3fn, dev);
-    const Tensor oswz = empty({M * (N / 16)}, at::kByte, dev);
+    if (!r.y.defined()) r.y = empty({M, N}, out_t);
+    r.qout = empty({M, N / 2}, at::kByte);
+    r.oscales = empty_output(N / 16, M, at::kFloat8_e4m3fn);
+    const Twin oswz = empty_twin(M * (N / 16), at::kByte);
     int rc;
     {
       GilRelease nogil;
       rc = svdq_gemm_w4a4_next(ptr(a.act), ptr(a.wgt), sa.data(), sw.data(), la.data(), ptr(lu), lu16.data(), ptr(a.wcscales), ptr(a.bias),
-                               ptr(r.y), ptr(a.smooth_next), ptr(r.qout), ptr(r.oscales), ptr(oswz), m, n, k, rr, dt, 0, stream);
+                               ptr(r.y), ptr(a.smooth_next), ptr(r.qout), ptr(r.oscales), oswz.data(), m, n, k, rr, dt, 0, stream);
     }
     if (rc != SVDQ_OK) throw_status("gemm_w4a4_next", rc);
     if (!attach(r.oscales, oswz)) throw python_error();
@@ -347,7 +354,7 @@ bool gemm(const GemmArgs& a, ScalarType out_t, GemmResult& r) {
     ws = THPVariable_Unpack(w);
     if (static_cast<unsigned long long>(ws.numel()) < need) return false;
   }
-  if (!r.y.defined()) r.y = empty({M, N}, out_t, dev);
+  if (!r.y.defined()) r.y = empty({M, N}, out_t);
   int rc;
   {
     GilRelease nogil;
@@ -434,17 +441,18 @@ PyObject* py_pack(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (rows == 0 || K == 0 || K % 16 != 0) Py_RETURN_NONE;
   const int64_t rp = (rows + pad - 1) / pad * pad;
   if (!int_sized(rp) || !int_sized(K)) Py_RETURN_NONE;
-  Tensor packed = empty({rp, K / 2}, at::kByte, dev), scales = empty({K / 16, rp}, at::kFloat8_e4m3fn, dev), swz;
-  if (rp % 128 == 0 && K % 64 == 0) swz = empty({rp * (K / 16)}, at::kByte, dev);
+  Tensor packed = empty({rp, K / 2}, at::kByte), scales = empty({K / 16, rp}, at::kFloat8_e4m3fn);
+  Twin swz;
+  if (rp % 128 == 0 && K % 64 == 0) swz = empty_twin(rp * (K / 16), at::kByte);
   void* const stream = c10::cuda::getCurrentCUDAStream(dev).stream();
   int rc;
   {
     GilRelease nogil;
-    rc = svdq_quantize_nvfp4_rows(x.data_ptr(), packed.data_ptr(), scales.data_ptr(), swz.defined() ? swz.data_ptr() : nullptr,
+    rc = svdq_quantize_nvfp4_rows(x.data_ptr(), packed.data_ptr(), scales.data_ptr(), swz.data(),
                                   static_cast<int>(rows), static_cast<int>(rp), static_cast<int>(K), dtype_code(x.scalar_type()), stream);
   }
   if (rc != SVDQ_OK) throw_status("quantize_nvfp4_rows", rc);
-  if (swz.defined() && !attach(scales, swz)) throw python_error();
+  if (swz.found() && !attach(scales, swz)) throw python_error();
   Ref p(THPVariable_Wrap(std::move(packed))), s(THPVariable_Wrap(std::move(scales)));
   if (p.p == nullptr || s.p == nullptr) return nullptr;
   return PyTuple_Pack(2, p.p, s.p);
@@ -459,7 +467,7 @@ PyObject* py_output_twin(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (output_storage(owner) == nullptr) Py_RETURN_NONE;
   const Twin twin = attached(owner, PyObject_IsTrue(args[1]) == 1);
   if (!twin.found()) Py_RETURN_NONE;
-  return THPVariable_Wrap(twin.hold);
+  return THPVariable_Wrap(tensor_of(twin));
   END_HANDLE_TH_ERRORS
 }
 
@@ -472,7 +480,8 @@ PyObject* py_attach_output(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   }
   const Tensor& owner = THPVariable_Unpack(args[0]);
   if (output_storage(owner) == nullptr) Py_RETURN_FALSE;
-  attach(owner, THPVariable_Unpack(args[1]));
+  const Tensor& t = THPVariable_Unpack(args[1]);
+  attach(owner, Twin{t.numel() > 0 ? t.data_ptr() : nullptr, t.scalar_type(), t.numel(), t, {}});
   Py_RETURN_TRUE;
   END_HANDLE_TH_ERRORS
 }

@@ -85,8 +85,8 @@ def test_plan_rejects_bad_calls():
 
 
 def test_few_rows_long_k():
-    """A plan whose calls have few rows and a long K: its GEMM takes the split-K form with the plan's own
-    workspace, and the result is still the device operators' result bit for bit."""
+    """A plan whose calls have few rows and a long K: its GEMM shares each tile's K loop within a cluster, and the result
+    is still the device operators' result bit for bit."""
     M, K, N, R, dtype = 200, 6144, 512, 32, torch.float16
     plan, device_path, g = _setup(M, K, N, R, dtype, 11)
     try:
