@@ -1039,22 +1039,27 @@ int launch_gemm_w4a4(const void* act, const void* wgt, const void* ascales_swz, 
     }
   }
   if (variant == 0) {
-    // Pick the tile shape with the least estimated time: waves of tiles over the SMs (or SM pairs)
-    // times the measured relative time of one tile (a 128-column tile takes 0.72 of a 256-column
-    // one, not half: it moves more operand bytes per flop; a single CTA per tile takes 1.12 of a
-    // pair's time for loading all of B itself).  Large problems end on 256 x 256 pair tiles, a few
-    // hundred rows on narrower tiles that put more SMs to work.
-    const int sms = sm_count();
+    // Pairs wherever the rows allow them: single CTAs, which load all of B themselves, are slower at every size that
+    // both take (256 x 3840 x 3072 6.3 / 7.5 us, 1536 x 3840 x 3840 13.1 / 16.1, 4352 x 3840 x 3072 21.3 / 24.1).
+    // The tile's width by the least estimated time, rounds of tiles over the pairs (or SMs) times the relative time of
+    // a tile.  A 128-column tile takes more than half of a 256-column one, for it moves more operand bytes per flop:
+    // 0.65 of it for a pair (one round at 256 x 15360 x 3840 16.3 / 24.8 us, at 256 x 3840 x 3072 6.3 / 9.2), 0.84 for a
+    // single CTA (21.3 / 25.5).  So narrow tiles where both widths take one round, and with pairs where three narrow
+    // rounds replace two wide ones that the second leaves half empty: 1024 x 3840 x 5888 13.1 / 14.5 us, 1536 x 3840 x
+    // 3840 13.1 / 14.6, 1536 x 1280 x 3840 9.1 / 9.5, with the next layer's codes 18.8 / 21.5 and 15.7 / 17.5.  Further up
+    // the line is flat: two rounds against one 9.73 / 9.83 (1024 x 3840 x 3072), five against three 21.2 / 20.2 (3072 x
+    // 3840 x 3840).  The column-sharded form stores through shared memory, which narrow tiles do more often: three rounds
+    // against two 14.9 / 14.4 (1536 x 3840 x 3840), 31.6 / 29.4 (4352 x 10240 x 1536).
+    cg = M % 256 == 0 ? 2 : 1;
+    const long long units = sm_count() / cg;
     double best = 1e30;
-    cg = 1; bn = 128;
-    for (int c : {2, 1})
-      for (int b : {256, 128}) {
-        if (M % (128 * c) != 0 || N % b != 0) continue;
-        const long long tiles = static_cast<long long>(M / (128 * c)) * (N / b);
-        const long long units = sms / c;
-        const double cost = static_cast<double>((tiles + units - 1) / units) * (b == 256 ? 1.0 : 0.72) * (c == 2 ? 1.0 : 1.12);
-        if (cost < best) { best = cost; cg = c; bn = b; }
-      }
+    bn = 128;
+    for (int b : {256, 128}) {
+      if (N % b != 0) continue;
+      const long long tiles = static_cast<long long>(M / (128 * cg)) * (N / b);
+      const double cost = static_cast<double>((tiles + units - 1) / units) * (b == 256 ? 1.0 : tp.y_ld > 0 ? 0.72 : cg == 2 ? 0.65 : 0.84);
+      if (cost < best) { best = cost; bn = b; }
+    }
   } else if (variant == 128 || variant == 256) {
     cg = 1; bn = variant;
   } else {

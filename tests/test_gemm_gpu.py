@@ -94,6 +94,32 @@ def test_every_tile_shape(tiler):
     assert _case(256, 320, 256, 16, torch.float16, seed=3, tiler=tiler) <= TOL
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,N", [(1024, 5888), (1536, 3840), (2560, 3072), (2304, 1280), (384, 512), (640, 15360)])
+def test_picked_tiles_equal_the_forced_ones(M, N, dtype):
+    """On either side of the lines between tile shapes (three narrow rounds against two wide ones, one against one, pairs
+    against single CTAs): an element's products are added in the same order in every tile shape, so y and the next
+    layer's codes and scales are the same bit for bit."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(M + N)
+    K, R = 320, 16
+    x = torch.randn(M, K, generator=g).to(dtype).cuda()
+    ld = (torch.randn(K, R, generator=g) / K ** 0.5).to(dtype).cuda()
+    lu = (torch.randn(N, R, generator=g) * 0.01).to(dtype).cuda()
+    sn = (torch.rand(N, generator=g) + 0.5).to(dtype).cuda()
+    act, asc, la = ops.quantize_w4a4_act_fuse_lora(x, ld, None, pad_size=128)
+    wgt, wsc = ops.quantize_nvfp4_rows((torch.randn(N, K, generator=g) * 0.02).cuda())
+    args = (act, wgt, asc, wsc, la, lu, sn, None, dtype)
+    y = ops.gemm_w4a4(*args)
+    y_next, codes, scales = ops.gemm_w4a4(*args, smooth_next=sn)
+    assert torch.equal(y, y_next)
+    for tiler in [(m, n) for m in (128, 256) for n in (128, 256) if M % m == 0]:
+        f_y, f_codes, f_scales = ops.gemm_w4a4(*args, tiler_mn=tiler, smooth_next=sn)
+        assert torch.equal(f_y, y) and torch.equal(ops.gemm_w4a4(*args, tiler_mn=tiler), y)
+        assert torch.equal(f_codes, codes) and torch.equal(f_scales.view(torch.uint8), scales.view(torch.uint8))
+    assert_device_clean()
+
+
 def test_main_product_is_exact_without_lora():
     """fp4 x fp4 products with e4m3 scales accumulate exactly in fp32 at this size, so the
     kernel equals the oracle bit for bit (the reference recorded rel = 0 for its no-LoRA
