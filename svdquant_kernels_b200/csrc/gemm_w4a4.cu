@@ -951,22 +951,27 @@ int gemm_cluster_split(int M, int N, int K, int R) {
 // Workspace form.  The library runs this plan for row counts that are an odd multiple of 128; for whole 256-row tiles
 // (split within clusters above) it only tells a caller who forces the form how much room that takes.
 // Split-K plan for a problem with few tiles: 128 x 128 tiles, each tile's slabs shared by S CTAs that
-// all run at once (tiles * S <= SMs).  One CTA streams a tile's slabs at about 0.3 us each however
+// all run at once (tiles * S <= SMs).  One CTA streams a tile's slabs at about 0.235 us each however
 // few tiles there are (32 KB per slab through one SM's load path), so with a few dozen tiles most
-// SMs idle and the run time is one tile's K loop.  Splitting costs about 3.3 us (partials to L2, a
-// fence, the ticket, one read per partial), which the shorter loops repay from about 24 slabs on
-// (measured, 256 rows x 3072 columns: K = 3840 9.1 -> 10.0 us, K = 10240 16.1 -> 12.7 us,
-// K = 15360 22.6 -> 17.7 us).  Returns S (1 = no split).
+// SMs idle and the run time is one tile's K loop.  Splitting costs about 2.8 + 0.5 S us (partials to
+// L2, a fence, the ticket, one read per partial), 12 + 2 S slabs, against the n (1 - 1 / S) slabs that
+// it saves.  Plain / S = 2 / 3 / 4 in us, 128 rows x 3072 columns, K = 3840 7.5 / 9.4 / 9.5 / 9.8,
+// K = 6144 9.4 / 10.4 / 10.0 / 10.4, K = 7680 10.9 / 11.2 / 10.6 / 10.7, K = 10240 13.2 / 12.4 / 11.5 / 11.6,
+// K = 15360 18.0 / 15.0 / 13.2 / 12.6; 384 rows, which fit two CTAs a tile, K = 7680 11.2 / 11.8, K = 10240
+// 13.6 / 13.0.  Returns S (1 = no split).
 int gemm_split_plan(int M, int N, int K, int R) {
   if (!gemm_supported(M, N, K, R)) return 1;
   const long long tiles = static_cast<long long>(M / 128) * (N / 128);
-  const int slabs = (K + gemm::BK - 1) / gemm::BK;
+  const int slabs = (K + gemm::BK - 1) / gemm::BK, n = slabs + (R + 63) / 64;
   const int sms = sm_count();
-  if (tiles * 2 > sms || tiles > kSplitMaxTiles || slabs < 24) return 1;
-  int s = static_cast<int>(sms / tiles);
-  if (s > 4) s = 4;
-  if (s > slabs / 6) s = slabs / 6;               // at least six slabs per split
-  return s < 2 ? 1 : s;
+  if (tiles * 2 > sms || tiles > kSplitMaxTiles) return 1;
+  int best = 1;
+  double best_cost = 0.0;                         // of a split, in slabs, over not splitting
+  for (int s = 2; s <= 4 && tiles * s <= sms && s <= slabs / 6; ++s) {      // at least six slabs per split
+    const double cost = 12.0 + 2.0 * s - n * (1.0 - 1.0 / s);
+    if (cost < best_cost) { best_cost = cost; best = s; }
+  }
+  return best;
 }
 
 size_t gemm_split_workspace_bytes(int M, int N, int K, int R) {

@@ -78,6 +78,9 @@ def test_argument_validation_needs_no_device(lib_path):
     assert lib.svdq_gemm_w4a4_workspace_bytes(256, 3072, 10240, 32) == 1024 + 48 * 3 * 65536
     assert lib.svdq_gemm_w4a4_workspace_bytes(256, 3840, 15360, 128) == 1024 + 60 * 2 * 65536
     assert lib.svdq_gemm_w4a4_workspace_bytes(256, 3072, 3840, 128) == 0          # K too short to repay the split
+    assert lib.svdq_gemm_w4a4_workspace_bytes(128, 3072, 6144, 64) == 0           # ... by a little
+    assert lib.svdq_gemm_w4a4_workspace_bytes(128, 3072, 7680, 64) == 1024 + 24 * 4 * 65536
+    assert lib.svdq_gemm_w4a4_workspace_bytes(384, 3072, 7680, 64) == 0           # room for two CTAs a tile only
     assert lib.svdq_gemm_w4a4_workspace_bytes(4352, 3072, 10240, 32) == 0         # plenty of tiles
     assert lib.svdq_gemm_w4a4_workspace_bytes(100, 3072, 10240, 32) == 0          # not a supported shape
     # the workspace forms check their arguments like the plain call, before anything is launched

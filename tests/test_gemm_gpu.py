@@ -245,7 +245,8 @@ def test_back_to_back_steps_keep_their_results():
 @pytest.mark.parametrize("M,K,N,R,splits", [(256, 7680, 3072, 128, None), (256, 3840, 3072, 128, 2), (256, 3840, 3072, 128, 3),
                                             (128, 1024, 256, 0, 4), (128, 2560, 512, 32, 6), (384, 704, 1280, 256, 3),
                                             (128, 10240, 3072, 32, None), (512, 15360, 1024, 64, None),
-                                            (384, 7680, 3072, 128, None), (640, 15360, 1024, 64, None)])
+                                            (384, 10240, 3072, 128, None), (640, 15360, 1024, 64, None),
+                                            (128, 7168, 1024, 64, None)])
 def test_split_k(M, K, N, R, splits, dtype):
     """Few output tiles: a tile's K loop is shared by several CTAs whose fp32 partial tiles are summed
     in a fixed order by the last one to arrive.  Chosen by the library (None: through the workspace for
