@@ -441,8 +441,6 @@ struct svdq_linear_plan {
   PlanSlot slot[kPlanSlots];
   unsigned long long submitted;
   void *wgt, *wscales_swz, *lora_down, *lora_up, *lora_up_f16, *smooth, *smooth_table, *wc, *bias;  // resident weights
-  void* quant_ws;                                                // workspace of the quantizer's streaming form, or null
-  size_t quant_ws_bytes;
 };
 
 // Whether `ptr` is page-locked host memory, and the address under which kernels reach it (null: they cannot).
@@ -536,12 +534,6 @@ int svdq_linear_plan_create(svdq_linear_plan** out, int max_M, int K, int N, int
   }
   if (rc == SVDQ_OK) rc = dev_upload(&p->wc, wcscales_host, static_cast<size_t>(N) * 2, st);
   if (rc == SVDQ_OK) rc = dev_upload(&p->bias, bias_host, static_cast<size_t>(N) * 2, st);
-  if (rc == SVDQ_OK && R > 0) {
-    // calls of any height up to max_M: room for eight K ranks of the tallest one
-    p->quant_ws_bytes = 2048 + static_cast<size_t>(8) * max_M_pad * 128 * 4;
-    if (cudaMalloc(&p->quant_ws, p->quant_ws_bytes) != cudaSuccess ||
-        cudaMemsetAsync(p->quant_ws, 0, 2048, st) != cudaSuccess) rc = SVDQ_ERR_CUDA;
-  }
   if (rc == SVDQ_OK && cudaStreamSynchronize(st) != cudaSuccess) rc = SVDQ_ERR_CUDA;
   if (wscales_dev != nullptr) cudaFree(wscales_dev);
   if (rc != SVDQ_OK) {
@@ -629,7 +621,7 @@ static int plan_queue(svdq_linear_plan* p, const void* x_host, void* y_host, int
     }
     if (bad) break;
     rc = quantize_entry(x, p->lora_down, p->smooth, p->smooth_table, act, sc, la, swz, la16, rows, K, R, rows_pad, p->dtype,
-                        SVDQ_QUANT_AUTO, p->quant_ws, p->quant_ws_bytes, p->s_run, M_pad);
+                        SVDQ_QUANT_AUTO, nullptr, 0, p->s_run, M_pad);
     if (rc != SVDQ_OK) return plan_give_up(p, rc);
     rc = svdq_gemm_w4a4(act, p->wgt, swz, p->wscales_swz, R > 0 ? la16 : nullptr, R > 0 ? p->lora_up : nullptr,
                            R > 0 ? p->lora_up_f16 : nullptr, p->wc, p->bias, y, rows_pad, N, K, R, p->dtype, variant, p->s_run);
@@ -702,7 +694,7 @@ void svdq_linear_plan_destroy(svdq_linear_plan* p) {
     for (cudaEvent_t e : q.y_part)
       if (e != nullptr) cudaEventDestroy(e);
   }
-  void* dev[] = {p->wgt, p->wscales_swz, p->lora_down, p->lora_up, p->lora_up_f16, p->smooth, p->smooth_table, p->wc, p->bias, p->quant_ws};
+  void* dev[] = {p->wgt, p->wscales_swz, p->lora_down, p->lora_up, p->lora_up_f16, p->smooth, p->smooth_table, p->wc, p->bias};
   for (void* d : dev)
     if (d != nullptr) cudaFree(d);
   if (p->s_in != nullptr) cudaStreamDestroy(p->s_in);

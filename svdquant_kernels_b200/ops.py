@@ -454,7 +454,6 @@ def _gemm_checked(act, wgt, ascales, wscales, lora_act_in=None, lora_up=None, wc
 
 _SPLIT_WS: dict = {}     # GEMM split-K workspaces
 _QUANT_WS: dict = {}     # quantizer (streaming form) workspaces
-_QUANT_WS_BYTES: dict = {}
 _QUANT_WS_FORCED = 2048 + 8 * 8192 * 512     # room for any forced split of up to 8192 padded rows
 
 
@@ -473,14 +472,6 @@ def _workspace(table: dict, dev: torch.device, nbytes: int, head: int) -> torch.
 
 def _split_workspace(dev: torch.device, nbytes: int) -> torch.Tensor:
     return _workspace(_SPLIT_WS, dev, nbytes, 1024)
-
-
-def _quant_ws_bytes(M: int, K: int, R: int, M_pad: int) -> int:
-    key = (M, K, R, M_pad)
-    n = _QUANT_WS_BYTES.get(key)
-    if n is None:
-        n = _QUANT_WS_BYTES[key] = int(_lib.load().svdq_quantize_workspace_bytes(M, K, R, M_pad))
-    return n
 
 
 def reset_workspaces() -> None:
