@@ -48,8 +48,10 @@ NSETS = 6  # rotating input/output sets: 6 x ~70 MB is > 3 x the 126 MB L2
 # L2 when a captured launch ends, so the write-back of y / act shows up in later launches, not here.
 # Configurations without a capture report null.
 NCU_DRAM_BYTES = {
-    "c1": {"gemm_w4a4_kernel": 17_990_400 + 27_904, "quantize_fused_kernel": 34_496_256 + 7_168},
-    "c2": {"gemm_w4a4_kernel": 47_763_456 + 84_982_272},
+    "c1": {"gemm_w4a4_kernel": 17_976_064 + 18_688, "quantize_fused_kernel": 34_477_568 + 25_856},
+    "c2": {"gemm_w4a4_kernel": 47_781_120 + 86_947_328},
+    "c3": {"gemm_w4a4_kernel": 86_103_296 + 19_201_280, "quantize_fused_kernel": 137_756_928 + 22_604_288},
+    "c4": {"gemm_w4a4_kernel": 43_434_496 + 6_994_432, "quantize_fused_kernel": 89_886_720 + 10_120_704},
 }
 
 
