@@ -314,7 +314,6 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   tc_fence_after_sync();
   // Everything above touched only this CTA's shared and tensor memory, so it may overlap the tail of
   // the kernel before this one in the stream; from here on its outputs are read.
-  pdl_trigger();
   pdl_wait();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);   // warp-uniform, for the same reason as the warp index
   const uint32_t tmem_sf = tmem_base + C::ACC_COLS;              // SF_BUFS buffers of [SFA 16 | SFB] columns
@@ -386,6 +385,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       for (int pos = kt_lo; pos < kt_hi; ++pos, ++it) {
         const int kt = walk.at(pos);
         if (!uwait(&empty[s], ph, ctx, kDevWaitEmpty, it)) { ok = false; break; }
+        if (it == C::STAGES) pdl_trigger();       // the first stage has been consumed: see pdl_trigger
         uint8_t* st = smem + s * C::STAGE_BYTES;
         // Codes past K are zero-filled by TMA.  The scale atoms of a (128-row block, slab) are four
         // consecutive 512-byte rows of the swizzled scale buffer seen as a [blocks * K/64, 512 B] matrix;
@@ -421,6 +421,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (++s == C::STAGES) { s = 0; ph ^= 1; }
       }
     }
+    if (it <= C::STAGES) pdl_trigger();
   } else if (warp == EPI_WARPS + 1) {
     // ------------------------------ MMA issuer (leader CTA only) ------------------------------
     if (rank == 0) {

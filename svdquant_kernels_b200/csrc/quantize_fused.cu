@@ -185,7 +185,6 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   tc_fence_after_sync();
   const uint32_t tmem_acc = __shfl_sync(0xffffffffu, *tmem_slot, 0);   // warp-uniform, like the warp index
   // set-up done; what follows reads and writes global memory
-  pdl_trigger();
   pdl_wait();
   // out-of-range smooth anywhere in K (flag word behind the table) selects the IEEE divide
   const bool use_fdiv = has_table && reinterpret_cast<const uint32_t*>(p.table + 2 * p.K)[0] != 0u;
@@ -236,6 +235,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     uint32_t s = issuer, ph = 0, sw = issuer, phw = 0;
     for (int i = issuer; i < my_slabs; i += C::ISSUERS) {
       if (!uwait(&full[s], ph, kDevWaitFull, i)) break;
+      if (i == 0) pdl_trigger();                 // the first loads have landed: see pdl_trigger
       if (has_lora && !uwait(&wfull[sw], phw, kDevWaitFull, 0x50000 + i)) break;
       tc_fence_after_sync();
       const uint64_t da = kDescA + (x16 + s * (X_BYTES / 16)), db = kDescB + (w16 + sw * (C::W_BYTES / 16));
