@@ -172,18 +172,22 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     tma_prefetch_desc(&tmX);
     if (has_lora) tma_prefetch_desc(&tmW);
   }
-  if (warp == 1) {
-    tmem_alloc(tmem_slot, C::TMEM_COLS);
-    tmem_relinquish();
-  }
-  tc_fence_before_sync();
   __syncthreads();
   // Two K ranks hand their partial sums to each other through the copy engine, counted on the partner's
-  // barrier, so that barrier must exist (and be armed) before either touches it.  (The CTAs of a cluster
-  // start together; this costs a fraction of a microsecond, before the wait for the kernel ahead.)
-  if (kDirectExchange && ks == 2 && has_lora) cluster_sync_all();
-  tc_fence_after_sync();
-  const uint32_t tmem_acc = __shfl_sync(0xffffffffu, *tmem_slot, 0);   // warp-uniform, like the warp index
+  // barrier, so that barrier must exist (and be armed) before either touches it: whoever touches it waits for this.
+  const bool direct = kDirectExchange && ks == 2 && has_lora;
+  if (direct) cluster_arrive();
+  // Tensor memory: the issuers wait for it (loads are under way by then), the epilogue reads the address once the sums are complete.
+  if (has_lora && (warp == 1 || warp == 3)) {
+    if (warp == 1) {
+      tmem_alloc(tmem_slot, C::TMEM_COLS);
+      tmem_relinquish();
+    }
+    tc_fence_before_sync();
+    asm volatile("bar.sync 4, 64;" ::: "memory");
+    tc_fence_after_sync();
+  }
+  auto tmem_base = [&]() -> uint32_t { return __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_slot), 0); };   // warp-uniform, like the warp index
   // set-up done; what follows reads and writes global memory
   pdl_wait();
   // out-of-range smooth anywhere in K (flag word behind the table) selects the IEEE divide
@@ -229,7 +233,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     constexpr uint64_t kDescB = smem_desc_base(SLAB_K * 128, 1024, kSwizzle128B);    // lora_down slab, R-major (its own ring)
     constexpr uint32_t kIdesc = idesc_f16(kBf16, kBf16, TILE_M, RP, false, true);
     const int issuer = warp >> 1;                                  // 0 or 1
-    const uint32_t acc = tmem_acc + issuer * RP;
+    const uint32_t acc = (has_lora ? tmem_base() : 0u) + issuer * RP;
     const int last = C::ISSUERS == 1 ? my_slabs - 1 : ((my_slabs - 1 - issuer) & ~1) + issuer;   // this issuer's last slab (negative: none)
     const uint32_t x16 = smem_desc_addr(smem), w16 = smem_desc_addr(wring);
     uint32_t s = issuer, ph = 0, sw = issuer, phw = 0;
@@ -315,6 +319,12 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     asm volatile("bar.sync 2, %0;" ::"n"(QUANT_WARPS * 32) : "memory");
   }
 
+  bool tmem_held = has_lora && warp == 1;
+  auto free_tmem = [&]() {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base(), C::TMEM_COLS);
+    tmem_held = false;
+  };
   // 32 accumulator columns of this warp's lanes: the even slabs' accumulator plus, if there is more than one
   // slab, the odd slabs' (always in this order)
   auto acc_ld = [&](uint32_t taddr, uint32_t (&v)[32]) {
@@ -343,6 +353,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     // wanted); own rows wait there for the partner's.  Then all four warps add the two partial sums (two
     // terms: the order does not matter) and write the finished rows out, consecutive lanes taking
     // consecutive 16 bytes of a row.
+    cluster_wait();
     if (warp < AUX_WARPS) {
       constexpr uint32_t RP4 = RP / 4;
       constexpr uint32_t HALF_BYTES = 16u * RP * 4u;                 // one warp's 16 rows
@@ -350,7 +361,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       tc_fence_after_sync();
       const bool mine = static_cast<uint32_t>(warp >> 1) == krank;
       const uint32_t row_local = 16u * (warp & 1) + (lane & 15);     // row within the owner's 32
-      const uint32_t taddr = tmem_acc + (static_cast<uint32_t>(warp * 32) << 16);
+      const uint32_t taddr = tmem_base() + (static_cast<uint32_t>(warp * 32) << 16);
       float4* send = reinterpret_cast<float4*>(wring);                // [32 rows][RP / 4], slots as partial_slot
       float4* own = reinterpret_cast<float4*>(wring + C::RECV_BYTES);
       float4* dst = mine ? own : send;
@@ -401,6 +412,8 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
         asm volatile("bar.sync 3, %0;" ::"n"(AUX_WARPS * 32) : "memory");
         if (threadIdx.x == 0) lora16_flags(p.lora16, static_cast<size_t>(p.M_pad) * p.R)[m0 / 32 + krank] = *lora_unfit;
       }
+      // tensor memory goes back while the quantize warps are still busy
+      if (warp == 1 && *abort_flag == 0) free_tmem();
       // the partner has everything this CTA sent: only then may the memory it was copied from go away
       if (warp == 0) (void)__all_sync(0xffffffffu, mbar_wait_cluster(ack_bar, 0, ctx, kDevWaitMisc, 0x41000));
     }
@@ -418,7 +431,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
 #pragma unroll 1
         for (int c0 = cpart * C::EPI_COLS; c0 < (cpart + 1) * C::EPI_COLS; c0 += 32) {
           uint32_t v[32];
-          acc_ld(tmem_acc + (static_cast<uint32_t>(quarter * 32) << 16) + c0, v);
+          acc_ld(tmem_base() + (static_cast<uint32_t>(quarter * 32) << 16) + c0, v);
           if (lane < 16) {
             if (ks > 1) {
 #pragma unroll
@@ -450,10 +463,11 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       tc_fence_before_sync();
       __syncwarp();
       cluster_sync_all();                                     // every CTA's partial is in its shared memory
+      if (warp == 1 && *abort_flag == 0) free_tmem();         // (the sums below start with the last warps)
       // CTA k sums float4s [k T / KS, (k + 1) T / KS) of the tile's T over the cluster
       const uint32_t item_lo = krank * (TILE_M * RP4) / ks, item_hi = (krank + 1) * (TILE_M * RP4) / ks;
       const uint32_t base_addr = smem_u32(partial);
-      for (uint32_t it = item_lo + threadIdx.x; it < item_hi; it += NUM_THREADS) {
+      for (uint32_t it = item_lo + (NUM_THREADS - 1 - threadIdx.x); it < item_hi; it += NUM_THREADS) {
         const uint32_t row = it / RP4, c4 = it % RP4;
         const uint32_t off = base_addr + partial_slot(row, c4, RP4) * 16u;
         // Its own part first, then the next ranks in turn (a fixed order for every element): with all CTAs asking rank 0
@@ -494,23 +508,22 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     }
   }
 
-  tc_fence_before_sync();
-  __syncthreads();
-  if (kBf16 && has_lora && p.lora16 != nullptr && threadIdx.x == 0 && ks == 1) {
-    // one word per 32 rows: this CTA wrote rows [m0, m0 + 64) alone
-    uint32_t* flags = lora16_flags(p.lora16, static_cast<size_t>(p.M_pad) * p.R);
-    const uint32_t unfit = *lora_unfit;
-    flags[m0 / 32] = unfit & 1u; flags[m0 / 32 + 1] = (unfit >> 1) & 1u;
+  if (ks == 1) {
+    tc_fence_before_sync();
+    __syncthreads();
+    if (kBf16 && has_lora && p.lora16 != nullptr && threadIdx.x == 0) {
+      // one word per 32 rows: this CTA wrote rows [m0, m0 + 64) alone
+      uint32_t* flags = lora16_flags(p.lora16, static_cast<size_t>(p.M_pad) * p.R);
+      const uint32_t unfit = *lora_unfit;
+      flags[m0 / 32] = unfit & 1u; flags[m0 / 32 + 1] = (unfit >> 1) & 1u;
+    }
   }
   if (*abort_flag) {
+    // give copies that were already in flight time to land before the CTA's memory is released
     const unsigned long long t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 50000ull) { __nanosleep(1000); }
-    __syncthreads();
   }
-  if (warp == 1) {
-    tc_fence_after_sync();
-    tmem_dealloc(tmem_acc, C::TMEM_COLS);
-  }
+  if (tmem_held) free_tmem();
 }
 
 // The smoothing table: K reciprocals, K factors, one flag word: 1 if any smooth value lies outside [2^-60, 2^60]
