@@ -16,9 +16,8 @@
 // slabs) accumulate x_tile @ lora_down_slab into [64 x R] fp32 accumulators in
 // tensor memory, one each, and sixteen quantize warps turn the tile into codes
 // and scales.  x is read from HBM exactly once.  With KS > 1 the partial
-// accumulators are summed in a fixed order (two ranks: through the copy engine
-// into the partner's shared memory; more: through distributed shared memory
-// loads): no atomics, no zero-fill, no scratch in global
+// accumulators are summed in a fixed order, brought together by the copy engine (two ranks: halves, into the partner's
+// shared memory; more: every rank's share of the tile): no atomics, no zero-fill, no scratch in global
 // memory.  Large inputs run with KS = 2; larger clusters are for inputs of
 // a few hundred to two thousand rows, where pairs would leave most SMs idle (256 x 10240:
 // 36.0 -> 6.3 us), and are taken only if all of them are resident at once.
@@ -54,15 +53,13 @@ constexpr int X_BYTES = TILE_M * 128;      // 8 KB
 #endif
 constexpr int QUANT_GROUPS = SVDQ_QUANT_GROUPS;   // groups of 4 warps take slabs round-robin
 constexpr int QUANT_WARPS = 4 * QUANT_GROUPS;
-#ifndef SVDQ_DIRECT_EXCHANGE
-#define SVDQ_DIRECT_EXCHANGE 1
-#endif
-constexpr bool kDirectExchange = SVDQ_DIRECT_EXCHANGE != 0;
 constexpr int AUX_WARPS = 4;                // x producer, MMA issuer (even slabs), lora_down producer, MMA issuer (odd slabs); with two K ranks they exchange the LoRA sums
 constexpr int NUM_THREADS = (AUX_WARPS + QUANT_WARPS) * 32;
 constexpr int TB_BYTES = SLAB_K * 4;       // smoothing-table entries of a slab's columns
+constexpr int kMaxKSplit = 16;             // CTAs of a cluster
 
-template <int RP>
+// PUSH: clusters of more than two CTAs (see the exchange of LoRA sums below)
+template <int RP, bool PUSH>
 struct Cfg {
   // Two rings.  An x stage holds a 64 x 64 tile of x (8 KB) and, in an area of their own, the slab's 64 table
   // entries; it is read by the MMA and by one quantize group and released by both.  A lora_down slab (64 x RP, 16 KB at
@@ -72,14 +69,16 @@ struct Cfg {
   static constexpr int W_BYTES = SLAB_K * RP * 2;                 // lora_down slab
   // Six lora_down stages: a slab comes out of L2 in about 1.7 us while x streams in beside it, and slabs pass at
   // 0.3 us (2 / 4 / 6 / 8 stages, 4352 rows: K = 3840 22.0 / 16.2 / 14.9 / 15.6 us, K = 10240 42.5 / 30.3 / 29.0 / 29.5);
-  // at rank 256 three are what fits.
-  static constexpr int W_STAGES = RP > 128 ? 3 : 6;
+  // at rank 256 three are what fits, two beside the larger receive buffer of PUSH.
+  static constexpr int W_STAGES = RP > 128 ? (PUSH ? 2 : 3) : 6;
   // MMA-issuing warps.  Two take the slabs by turns; then both rings must be even, so that an issuer meets only slabs
   // of its own in a stage: one that went on to slab i could otherwise look at the stage while slab i - W_STAGES,
   // the other issuer's, is still on its way into it, and a one-bit parity would tell it that slab i is there.
   static constexpr int ISSUERS = W_STAGES % 2 == 0 ? 2 : 1;
   static constexpr int W_RING_BYTES = W_STAGES * W_BYTES;
-  static constexpr int RECV_BYTES = (TILE_M / 2) * RP * 4;        // two K ranks: the peer's partial sums of this CTA's 32 rows
+  // Receive buffer for partial sums: of the peer for this CTA's 32 rows (two K ranks), of all ranks for this CTA's share
+  // of the tile (PUSH; shares are rounded up to whole float4s)
+  static constexpr int RECV_BYTES = PUSH ? TILE_M * RP * 4 + kMaxKSplit * 16 : (TILE_M / 2) * RP * 4;
   static constexpr int STAGES_RAW = (232448 - 1024 - 512 - RECV_BYTES - W_RING_BYTES) / (X_BYTES + TB_BYTES);
   // A multiple of the group count: a group then always meets the same stages, and the slab it waits
   // for is the direct successor (in that stage) of one it consumed itself.  A one-bit phase parity
@@ -91,10 +90,10 @@ struct Cfg {
   static constexpr int SMEM_BYTES = 1024 + BARS_OFF + 512 + RECV_BYTES;          // rings, table entries, barriers, receive buffer
   static constexpr int TMEM_COLS = ISSUERS * RP;                  // an accumulator per issuer; a power of two >= 64
   static constexpr int EPI_COLS = RP / 4 < 32 ? 32 : RP / 4;      // accumulator columns per epilogue warp
-  static_assert(TILE_M * RP * 4 <= RING_BYTES, "partial accumulator must fit in the x ring");
+  static_assert(!PUSH || TILE_M * RP * 4 <= RING_BYTES, "the sums must fit in the x ring");
   static_assert(STAGES >= QUANT_GROUPS && STAGES % QUANT_GROUPS == 0 && (ISSUERS == 1 || STAGES % 2 == 0), "ring depth");
   static_assert((2 * STAGES + 2 * W_STAGES + 3) * 8 + 64 <= 512, "barrier block");
-  static_assert(2 * RECV_BYTES <= W_RING_BYTES, "the exchange stages both halves of the accumulator in the lora_down ring");
+  static_assert(PUSH || 2 * RECV_BYTES <= W_RING_BYTES, "the exchange stages both halves of the accumulator in the lora_down ring");
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 };
 
@@ -116,10 +115,10 @@ __device__ __forceinline__ uint32_t partial_slot(uint32_t row, uint32_t c4, uint
 
 using qmath::unpack_group;
 
-template <typename T, int RP>
+template <typename T, int RP, bool PUSH>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const Params p) {
-  using C = Cfg<RP>;
+  using C = Cfg<RP, PUSH>;
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
 
   extern __shared__ uint8_t smem_raw[];
@@ -133,12 +132,12 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   uint64_t* wfull = bars + 2 * C::STAGES;      // [W_STAGES]  lora_down slab landed
   uint64_t* wempty = wfull + C::W_STAGES;      // [W_STAGES]  lora_down slab consumed (MMA)
   uint64_t* acc_done = wempty + C::W_STAGES;   // MMA -> epilogue
-  uint64_t* recv_bar = acc_done + 1;           // two K ranks: the peer's partial sums have landed in `recv`
+  uint64_t* recv_bar = acc_done + 1;           // the other ranks' partial sums have landed in `recv`
   uint64_t* ack_bar = recv_bar + 1;            // two K ranks: the peer has received what this CTA sent
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ack_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint32_t* lora_unfit = tmem_slot + 2;        // bf16 form: some LoRA value this CTA wrote does not fit fp16 (other than two K ranks: a bit per 32 rows)
-  float4* recv = reinterpret_cast<float4*>(smem + C::BARS_OFF + 512);        // [32 rows][RP / 4], slots as partial_slot
+  uint32_t* lora_unfit = tmem_slot + 2;        // bf16 form: some LoRA value this CTA wrote does not fit fp16 (one rank: a bit per 32 rows)
+  float4* recv = reinterpret_cast<float4*>(smem + C::BARS_OFF + 512);        // [32 rows][RP / 4], slots as partial_slot; PUSH: [rank][share]
   const WaitCtx ctx{abort_flag};
 
   // warp index through a shuffle: provably warp-uniform, so the role branches are convergent code
@@ -159,15 +158,22 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   const int my_slabs = base + (static_cast<int>(krank) < rem ? 1 : 0);
   const int k_begin = slab_begin * SLAB_K;
 
+  // PUSH: the tile's sums as float4s, row by row, the ranks' columns rounded up to whole chunks of 32 and, inside a chunk of
+  // eight float4s, XORed by the row (for the banks).  Rank k sums numbers [k T / KS, (k + 1) T / KS) of the T.
+  const uint32_t row4 = (static_cast<uint32_t>(p.R) + 31u) / 32u * 8u, tile4 = TILE_M * row4;
+  auto share_begin = [&](uint32_t rank) -> uint32_t { return rank * tile4 / ks; };
+  const uint32_t item_lo = share_begin(krank), item_hi = share_begin(krank + 1), share = (tile4 + ks - 1) / ks;
+
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     *lora_unfit = 0u;
     for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1 + QUANT_WARPS / QUANT_GROUPS); }
     for (int s = 0; s < C::W_STAGES; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], 1); }
     mbar_init(acc_done, C::ISSUERS == 2 && my_slabs > 1 ? 2 : 1);     // one arrival per MMA issuer that has slabs
-    mbar_init(recv_bar, 1);                    // armed below with the bytes of the peer's two copies
+    mbar_init(recv_bar, 1);                    // armed here with all the bytes that will come
     mbar_init(ack_bar, 1);
-    if (kDirectExchange && ks == 2 && has_lora) mbar_arrive_expect_tx(recv_bar, C::RECV_BYTES);
+    if (PUSH && has_lora) mbar_arrive_expect_tx(recv_bar, (ks - 1) * 16u * (item_hi - item_lo));
+    else if (!PUSH && ks == 2 && has_lora) mbar_arrive_expect_tx(recv_bar, C::RECV_BYTES);
     fence_barrier_init();
     tma_prefetch_desc(&tmX);
     if (has_lora) tma_prefetch_desc(&tmW);
@@ -175,8 +181,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   __syncthreads();
   // Two K ranks hand their partial sums to each other through the copy engine, counted on the partner's
   // barrier, so that barrier must exist (and be armed) before either touches it: whoever touches it waits for this.
-  const bool direct = kDirectExchange && ks == 2 && has_lora;
-  if (direct) cluster_arrive();
+  if (!PUSH && ks == 2 && has_lora) cluster_arrive();
   // Tensor memory: the issuers wait for it (loads are under way by then), the epilogue reads the address once the sums are complete.
   if (has_lora && (warp == 1 || warp == 3)) {
     if (warp == 1) {
@@ -190,6 +195,12 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   auto tmem_base = [&]() -> uint32_t { return __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_slot), 0); };   // warp-uniform, like the warp index
   // set-up done; what follows reads and writes global memory
   pdl_wait();
+  if constexpr (PUSH) {
+    // bf16: no value of the tile is known not to fit fp16; ranks that meet one say so after the cluster barrier begun here
+    if (kBf16 && has_lora && p.lora16 != nullptr && krank == 0 && threadIdx.x < 2) lora16_flags(p.lora16, static_cast<size_t>(p.M_pad) * p.R)[m0 / 32 + threadIdx.x] = 0u;
+    __syncwarp();
+    if (has_lora) cluster_arrive();
+  }
   // out-of-range smooth anywhere in K (flag word behind the table) selects the IEEE divide
   const bool use_fdiv = has_table && reinterpret_cast<const uint32_t*>(p.table + 2 * p.K)[0] != 0u;
 
@@ -287,8 +298,9 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       if (has_table) {
         unpack_group<T, false>(raw[0][0], raw[0][1], f[0]);
         unpack_group<T, false>(raw[1][0], raw[1][1], f[1]);
-        // this lane's 16 columns' entries landed with the slab
-        qmath::smooth_divide2(f[0], f[1], reinterpret_cast<const float4*>(smem + C::TB_OFF + s * TB_BYTES) + g, use_fdiv);
+        // this lane's 16 columns' reciprocals landed with the slab; a flagged launch reads the factors where they are
+        if (!use_fdiv) qmath::smooth_multiply2(f[0], f[1], reinterpret_cast<const float4*>(smem + C::TB_OFF + s * TB_BYTES) + g);
+        else qmath::smooth_divide2(f[0], f[1], reinterpret_cast<const float4*>(smem + C::TB_OFF + s * TB_BYTES) + g);
       } else {
         unpack_group<T, true>(raw[0][0], raw[0][1], f[0]);
         unpack_group<T, true>(raw[1][0], raw[1][1], f[1]);
@@ -315,8 +327,8 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
         if (p.scales_swz != nullptr) p.scales_swz[sf_swizzled_offset(m0 + row, gi, groups)] = static_cast<uint8_t>(s_b);
       }
     }
-    // every quantize warp is done reading the ring before it is reused below
-    asm volatile("bar.sync 2, %0;" ::"n"(QUANT_WARPS * 32) : "memory");
+    // PUSH: every quantize warp is done reading the x ring before it is used again below
+    if constexpr (PUSH) asm volatile("bar.sync 2, %0;" ::"n"(QUANT_WARPS * 32) : "memory");
   }
 
   bool tmem_held = has_lora && warp == 1;
@@ -343,7 +355,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   // ------------------------------ LoRA epilogue ------------------------------
   // The 64 accumulator rows live in lanes 0-15 of each 32-lane quarter of tensor memory:
   // row r is lane (r % 16) + 32 * (r / 16).
-  if (kDirectExchange && has_lora && ks == 2) {
+  if (!PUSH && has_lora && ks == 2) {
     // Two K ranks (the form for tall activations): CTA k owns rows [32 k, 32 k + 32) of the tile.  The four
     // auxiliary warps do the whole exchange while the quantize warps are still busy with the last slabs:
     // warp w reads rows 16 w .. 16 w + 15 of the accumulator (lanes 0-15 of its quarter of tensor
@@ -353,6 +365,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     // wanted); own rows wait there for the partner's.  Then all four warps add the two partial sums (two
     // terms: the order does not matter) and write the finished rows out, consecutive lanes taking
     // consecutive 16 bytes of a row.
+    __syncwarp();
     cluster_wait();
     if (warp < AUX_WARPS) {
       constexpr uint32_t RP4 = RP / 4;
@@ -418,25 +431,45 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       if (warp == 0) (void)__all_sync(0xffffffffu, mbar_wait_cluster(ack_bar, 0, ctx, kDevWaitMisc, 0x41000));
     }
   } else if (has_lora) {
-    constexpr uint32_t RP4 = RP / 4;
-    float4* partial = reinterpret_cast<float4*>(smem);       // reuses the ring
+    // One rank writes its sums out.  More than two (PUSH) lay them out in the x ring, which nobody needs any more, and the
+    // copy engine brings every rank its share of them, counted on that rank's barrier: one trip.  (Ranks that fetched their
+    // shares themselves, behind a cluster barrier, took 0.8 us for the barrier and three trips of 0.4 us.  Now the
+    // transfer is the bound, 30 KB into every CTA at some 16 bytes a cycle at rank 128; 16-byte st.async from the registers
+    // need no staging but arrive one by one: 5.8 instead of 6.0 us at rank 32, 6.5 instead of 5.8 at rank 128.  256 x 15360
+    // 9.6 -> 9.3 us, 256 x 10240 6.5 -> 6.1, 256 x 3840 5.9 -> 5.8.)
+    float4* const stage = reinterpret_cast<float4*>(smem);
+    if constexpr (PUSH) { __syncwarp(); cluster_wait(); }     // all ranks' barriers exist
     if (warp >= AUX_WARPS) {
       const int qw = warp - AUX_WARPS;
       const int quarter = warp & 3;                           // TMEM lanes this warp may read
       const int cpart = qw >> 2;                              // column part
+      // PUSH, worked out before the sums are there: the copy that this warp issues (one each: fifteen lanes of one warp took
+      // 0.7 us to issue theirs; each rank starts with its neighbour) and the first float4 that this thread sums
+      [[maybe_unused]] const uint32_t to = krank + 1 + qw < ks ? krank + 1 + qw : krank + 1 + qw - ks;
+      [[maybe_unused]] uint32_t copy_lo = 0, copy_bytes = 0, copy_to = 0, copy_bar = 0, row_first = 0;
+      [[maybe_unused]] const uint32_t first = item_lo + (NUM_THREADS - 1 - threadIdx.x);
+      if constexpr (PUSH) {
+        if (static_cast<uint32_t>(qw) + 1 < ks) {
+          copy_lo = share_begin(to);
+          copy_bytes = (share_begin(to + 1) - copy_lo) * 16u;
+          copy_to = map_to_cta(smem_u32(recv + krank * share), to);
+          copy_bar = map_to_cta(smem_u32(recv_bar), to);
+        }
+        row_first = first / row4;
+      }
       if (cpart * C::EPI_COLS < RP) {
         const bool ok = mbar_wait(acc_done, 0, ctx, kDevWaitAcc, 0);
         tc_fence_after_sync();
         const uint32_t row = quarter * 16 + (lane & 15);
 #pragma unroll 1
-        for (int c0 = cpart * C::EPI_COLS; c0 < (cpart + 1) * C::EPI_COLS; c0 += 32) {
+        for (int c0 = cpart * C::EPI_COLS; c0 < (cpart + 1) * C::EPI_COLS && c0 < p.R; c0 += 32) {
           uint32_t v[32];
           acc_ld(tmem_base() + (static_cast<uint32_t>(quarter * 32) << 16) + c0, v);
           if (lane < 16) {
-            if (ks > 1) {
+            if constexpr (PUSH) {
 #pragma unroll
               for (int j = 0; j < 8; ++j)
-                partial[partial_slot(row, (c0 >> 2) + j, RP4)] =
+                stage[partial_slot(row, (c0 >> 2) + j, row4)] =
                     make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
             } else if (ok) {
               const size_t gm = static_cast<size_t>(m0 + row);
@@ -444,11 +477,10 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
               for (int j = 0; j < 8; ++j) {
                 const int c = c0 + 4 * j;
                 if (c < p.R) {
-                  *reinterpret_cast<float4*>(p.lora + gm * p.R + c) =
-                      make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+                  const float4 o = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                               __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+                  *reinterpret_cast<float4*>(p.lora + gm * p.R + c) = o;
                   if (p.lora16 != nullptr) {
-                    const float4 o = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
-                                                 __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
                     store_lora16x4<T>(p.lora16, gm * p.R + c, static_cast<size_t>(p.M_pad) * p.R, o);
                     if (kBf16 && !fits_f16(o)) atomicOr(lora_unfit, 1u << (row / 32));
                   }
@@ -458,53 +490,44 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
           }
         }
       }
-    }
-    if (ks > 1) {
-      tc_fence_before_sync();
-      __syncwarp();
-      cluster_sync_all();                                     // every CTA's partial is in its shared memory
-      if (warp == 1 && *abort_flag == 0) free_tmem();         // (the sums below start with the last warps)
-      // CTA k sums float4s [k T / KS, (k + 1) T / KS) of the tile's T over the cluster
-      const uint32_t item_lo = krank * (TILE_M * RP4) / ks, item_hi = (krank + 1) * (TILE_M * RP4) / ks;
-      const uint32_t base_addr = smem_u32(partial);
-      for (uint32_t it = item_lo + (NUM_THREADS - 1 - threadIdx.x); it < item_hi; it += NUM_THREADS) {
-        const uint32_t row = it / RP4, c4 = it % RP4;
-        const uint32_t off = base_addr + partial_slot(row, c4, RP4) * 16u;
-        // Its own part first, then the next ranks in turn (a fixed order for every element): with all CTAs asking rank 0
-        // first, then rank 1, one SM at a time would serve them all.  In batches, so that remote loads travel together.
-        float4 acc = partial[partial_slot(row, c4, RP4)];
-#pragma unroll 1
-        for (uint32_t j0 = 1; j0 < ks; j0 += 5) {
-          float4 t[5];
-#pragma unroll
-          for (uint32_t i = 0; i < 5; ++i) {
-            const uint32_t r = krank + j0 + i;
-            if (j0 + i < ks) t[i] = ld_cluster_f4(map_to_cta(off, r < ks ? r : r - ks));
-          }
-#pragma unroll
-          for (uint32_t i = 0; i < 5; ++i)
-            if (j0 + i < ks) { acc.x += t[i].x; acc.y += t[i].y; acc.z += t[i].z; acc.w += t[i].w; }
-        }
-        const int c = c4 * 4;
-        if (c < p.R) {
-          const size_t gm = static_cast<size_t>(m0 + row);
-          *reinterpret_cast<float4*>(p.lora + gm * p.R + c) = acc;
-          if (p.lora16 != nullptr) {
-            store_lora16x4<T>(p.lora16, gm * p.R + c, static_cast<size_t>(p.M_pad) * p.R, acc);
-            // one "does not fit fp16" word per 32 rows, kept as bits of the first CTA's word until all have had their say
-            if (kBf16 && !fits_f16(acc)) {
-              red_or_cluster(map_to_cta(smem_u32(lora_unfit), 0), 1u << (row / 32));
-              fence_acq_rel_cluster();
+      if constexpr (PUSH) {
+        tc_fence_before_sync();
+        fence_proxy_async_smem();                             // the copy engine reads what the lanes wrote
+        asm volatile("bar.sync 2, %0;" ::"n"(QUANT_WARPS * 32) : "memory");
+        if (copy_bytes != 0 && elect_one()) bulk_copy_smem_to_cluster(copy_to, smem_u32(stage + copy_lo), copy_bytes, copy_bar);
+        __syncwarp();
+        const bool got = first < item_hi && mbar_wait_cluster(recv_bar, 0, ctx, kDevWaitMisc, 0x40000);
+        __syncwarp();
+        cluster_arrive_relaxed();                             // this rank's share has come: nobody need keep it for it
+        if (got) {
+          for (uint32_t item = first; item < item_hi; item += QUANT_WARPS * 32) {
+            const uint32_t row = item == first ? row_first : item / row4, c = 4 * ((item - row * row4) ^ (row & 7u));
+            if (c >= static_cast<uint32_t>(p.R)) continue;
+            // this rank's part first, then the following ranks' in turn: a fixed order for every element
+            float4 acc = stage[item];
+            auto add_ranks = [&](uint32_t r, uint32_t r_end) {
+              const float4* part = recv + r * share + (item - item_lo);
+#pragma unroll 4
+              for (; r < r_end; ++r, part += share) { const float4 t = *part; acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w; }
+            };
+            add_ranks(krank + 1, ks);
+            add_ranks(0, krank);
+            const size_t idx = static_cast<size_t>(m0 + row) * p.R + c;
+            *reinterpret_cast<float4*>(p.lora + idx) = acc;
+            if (p.lora16 != nullptr) {
+              store_lora16x4<T>(p.lora16, idx, static_cast<size_t>(p.M_pad) * p.R, acc);
+              if (kBf16 && !fits_f16(acc)) lora16_flags(p.lora16, static_cast<size_t>(p.M_pad) * p.R)[(m0 + row) / 32] = 1u;
             }
           }
         }
+        __syncwarp();
       }
-      // Nobody leaves while its memory is being read.  What was read is in use above, and the rare verdict is fenced: the
-      // arrival itself has nothing to wait for (as a releasing one it waited for all the stores above).
+    } else if constexpr (PUSH) {
       cluster_arrive_relaxed();
-      cluster_wait();
-      if (kBf16 && p.lora16 != nullptr && krank == 0 && threadIdx.x < 2)
-        lora16_flags(p.lora16, static_cast<size_t>(p.M_pad) * p.R)[m0 / 32 + threadIdx.x] = (*lora_unfit >> threadIdx.x) & 1u;
+    }
+    if constexpr (PUSH) {
+      cluster_wait();                                         // no CTA leaves before its copies have been read
+      if (warp == 1 && *abort_flag == 0) free_tmem();
     }
   }
 
@@ -575,9 +598,8 @@ static int pick_k_split(int M_pad, int K, MaxClusters max_clusters) {
   }
   return best;
 }
-constexpr int kMaxKSplit = 16;
 
-template <typename T, int RP> static int max_clusters_t(int ks);
+template <typename T, int RP, bool PUSH> static int max_clusters_t(int ks);
 
 bool quantize_fused_supported(int M, int K, int R, int M_pad) {
   if (M <= 0 || K <= 0 || M_pad < M) return false;
@@ -596,9 +618,9 @@ int launch_smooth_table(const void* smooth, void* table, int K, int dtype, cudaS
   return cudaGetLastError() == cudaSuccess ? SVDQ_OK : SVDQ_ERR_LAUNCH;
 }
 
-template <typename T, int RP>
-static int launch_qf(const void* x, const void* w, const qf::Params& p, cudaStream_t stream, int split_rows) {
-  using C = qf::Cfg<RP>;
+template <typename T, int RP, bool PUSH>
+static int launch_qf_form(const void* x, const void* w, const qf::Params& p, int ks, int dev, cudaStream_t stream) {
+  using C = qf::Cfg<RP, PUSH>;
   CUtensorMap tmX, tmW;
   int rc;
   if ((rc = make_tmap_2d(&tmX, x, 2, p.M, p.K, static_cast<uint64_t>(p.K) * 2, qf::TILE_M, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
@@ -607,25 +629,15 @@ static int launch_qf(const void* x, const void* w, const qf::Params& p, cudaStre
   } else {
     tmW = tmX;
   }
-  auto kern = qf::quantize_fused_kernel<T, RP>;
+  auto kern = qf::quantize_fused_kernel<T, RP, PUSH>;
   // the attribute is per device: remember which devices of this process have it
   static bool configured[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return SVDQ_ERR_CUDA;
   if (dev < 0 || dev >= 64 || !configured[dev]) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) != cudaSuccess) return SVDQ_ERR_LAUNCH;
     // clusters of more than eight
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return SVDQ_ERR_LAUNCH;
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  // clusters the device can hold, by size and device, asked for when first needed (value + 2; 0: not asked yet)
-  static int caps[64][kMaxKSplit + 1];
-  auto max_clusters = [&](int k) -> int {
-    if (dev < 0 || dev >= 64) return 0;
-    if (caps[dev][k] == 0) caps[dev][k] = max_clusters_t<T, RP>(k) + 2;
-    return caps[dev][k] - 2;
-  };
-  const int ks = pick_k_split(split_rows > p.M_pad ? split_rows : p.M_pad, p.K, max_clusters);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(p.M_pad / qf::TILE_M, ks, 1);
   cfg.blockDim = dim3(qf::NUM_THREADS, 1, 1);
@@ -645,9 +657,24 @@ static int launch_qf(const void* x, const void* w, const qf::Params& p, cudaStre
 }
 
 template <typename T, int RP>
+static int launch_qf(const void* x, const void* w, const qf::Params& p, cudaStream_t stream, int split_rows) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return SVDQ_ERR_CUDA;
+  // clusters the device can hold, by size and device, asked for when first needed (value + 2; 0: not asked yet)
+  static int caps[64][qf::kMaxKSplit + 1];
+  auto max_clusters = [&](int k) -> int {
+    if (dev < 0 || dev >= 64) return 0;
+    if (caps[dev][k] == 0) caps[dev][k] = max_clusters_t<T, RP, true>(k) + 2;
+    return caps[dev][k] - 2;
+  };
+  const int ks = pick_k_split(split_rows > p.M_pad ? split_rows : p.M_pad, p.K, max_clusters);
+  return ks > 2 ? launch_qf_form<T, RP, true>(x, w, p, ks, dev, stream) : launch_qf_form<T, RP, false>(x, w, p, ks, dev, stream);
+}
+
+template <typename T, int RP, bool PUSH>
 static int max_clusters_t(int ks) {
-  using C = qf::Cfg<RP>;
-  auto kern = qf::quantize_fused_kernel<T, RP>;
+  using C = qf::Cfg<RP, PUSH>;
+  auto kern = qf::quantize_fused_kernel<T, RP, PUSH>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) != cudaSuccess ||
       cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
     return -1;
@@ -664,10 +691,16 @@ static int max_clusters_t(int ks) {
   return n;
 }
 
+template <typename T>
+static int max_clusters_r(int R, int ks) {
+  auto form = [&](auto push) {
+    constexpr bool P = decltype(push)::value;
+    return R <= 64 ? max_clusters_t<T, 64, P>(ks) : R <= 128 ? max_clusters_t<T, 128, P>(ks) : max_clusters_t<T, 256, P>(ks);
+  };
+  return ks > 2 ? form(std::true_type{}) : form(std::false_type{});
+}
 int quantize_fused_max_clusters(int R, int ks, int dtype) {
-  const int rp = R <= 64 ? 64 : (R <= 128 ? 128 : 256);
-  if (dtype == SVDQ_DTYPE_F16) return rp == 64 ? max_clusters_t<__half, 64>(ks) : rp == 128 ? max_clusters_t<__half, 128>(ks) : max_clusters_t<__half, 256>(ks);
-  return rp == 64 ? max_clusters_t<__nv_bfloat16, 64>(ks) : rp == 128 ? max_clusters_t<__nv_bfloat16, 128>(ks) : max_clusters_t<__nv_bfloat16, 256>(ks);
+  return dtype == SVDQ_DTYPE_F16 ? max_clusters_r<__half>(R, ks) : max_clusters_r<__nv_bfloat16>(R, ks);
 }
 
 int launch_quantize_fused(const void* x, const void* lora_down, const void* smooth_table, void* act, void* ascales,

@@ -79,25 +79,29 @@ __device__ __forceinline__ float smooth_reciprocal(float s) {
 }
 
 // Near quotients of two rows of the same 16 columns; tb points at the group's chunk 0 of the slab's 64 entries in
-// shared memory (the smoothing factors themselves when the launch divides with __fdiv_rn).  Every entry is loaded
-// once for both rows: a 16-byte shared-memory load costs its wavefronts however many lanes share its address,
-// and the load/store unit is what the fused quantizer keeps busiest.
-__device__ __forceinline__ void smooth_divide2(float2 (&f0)[8], float2 (&f1)[8], const float4* tb, bool use_fdiv) {
+// shared memory.  Every entry is loaded once for both rows: a 16-byte shared-memory load costs its wavefronts however
+// many lanes share its address, and the load/store unit is what the fused quantizer keeps busiest.
+__device__ __forceinline__ void smooth_multiply2(float2 (&f0)[8], float2 (&f1)[8], const float4* tb) {
   const float2 zero = make_float2(0.0f, 0.0f);
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const float4 t = tb[4 * j];
     const float2 a = make_float2(t.x, t.y), b = make_float2(t.z, t.w);
-    if (!use_fdiv) {
-      f0[2 * j] = __ffma2_rn(f0[2 * j], a, zero); f0[2 * j + 1] = __ffma2_rn(f0[2 * j + 1], b, zero);
-      f1[2 * j] = __ffma2_rn(f1[2 * j], a, zero); f1[2 * j + 1] = __ffma2_rn(f1[2 * j + 1], b, zero);
-    } else {
-      auto div = [](float2 v, float2 d) {                          // an underflow to -0 counts as +0
-        return make_float2(__fadd_rn(__fdiv_rn(v.x, d.x), 0.0f), __fadd_rn(__fdiv_rn(v.y, d.y), 0.0f));
-      };
-      f0[2 * j] = div(f0[2 * j], a); f0[2 * j + 1] = div(f0[2 * j + 1], b);
-      f1[2 * j] = div(f1[2 * j], a); f1[2 * j + 1] = div(f1[2 * j + 1], b);
-    }
+    f0[2 * j] = __ffma2_rn(f0[2 * j], a, zero); f0[2 * j + 1] = __ffma2_rn(f0[2 * j + 1], b, zero);
+    f1[2 * j] = __ffma2_rn(f1[2 * j], a, zero); f1[2 * j + 1] = __ffma2_rn(f1[2 * j + 1], b, zero);
+  }
+}
+// The exact quotients for a launch whose table is flagged: tb points at the smoothing factors themselves.
+__device__ __forceinline__ void smooth_divide2(float2 (&f0)[8], float2 (&f1)[8], const float4* tb) {
+  auto div = [](float2 v, float2 d) {                              // an underflow to -0 counts as +0
+    return make_float2(__fadd_rn(__fdiv_rn(v.x, d.x), 0.0f), __fadd_rn(__fdiv_rn(v.y, d.y), 0.0f));
+  };
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float4 t = tb[4 * j];
+    const float2 a = make_float2(t.x, t.y), b = make_float2(t.z, t.w);
+    f0[2 * j] = div(f0[2 * j], a); f0[2 * j + 1] = div(f0[2 * j + 1], b);
+    f1[2 * j] = div(f1[2 * j], a); f1[2 * j + 1] = div(f1[2 * j + 1], b);
   }
 }
 

@@ -254,7 +254,8 @@ quantize_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
       if (has_table) {
         qmath::unpack_group<T, false>(raw[0][0], raw[0][1], f[0]);
         qmath::unpack_group<T, false>(raw[1][0], raw[1][1], f[1]);
-        qmath::smooth_divide2(f[0], f[1], reinterpret_cast<const float4*>(st + C::X_BYTES + W_BYTES) + g, use_fdiv);
+        const float4* tb = reinterpret_cast<const float4*>(st + C::X_BYTES + W_BYTES) + g;
+        if (use_fdiv) qmath::smooth_divide2(f[0], f[1], tb); else qmath::smooth_multiply2(f[0], f[1], tb);
       } else {
         qmath::unpack_group<T, true>(raw[0][0], raw[0][1], f[0]);
         qmath::unpack_group<T, true>(raw[1][0], raw[1][1], f[1]);
