@@ -201,8 +201,6 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     __syncwarp();
     if (has_lora) cluster_arrive();
   }
-  // out-of-range smooth anywhere in K (flag word behind the table) selects the IEEE divide
-  const bool use_fdiv = has_table && reinterpret_cast<const uint32_t*>(p.table + 2 * p.K)[0] != 0u;
 
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
@@ -214,7 +212,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       if (elect_one()) {
         mbar_arrive_expect_tx(&full[s], stage_bytes);
         tma_load_2d(smem + s * X_BYTES, &tmX, k0, m0, &full[s]);
-        if (has_table) bulk_load_1d(smem + C::TB_OFF + s * TB_BYTES, p.table + (use_fdiv ? p.K : 0) + k0, TB_BYTES, &full[s]);
+        if (has_table) bulk_load_1d(smem + C::TB_OFF + s * TB_BYTES, p.table + k0, TB_BYTES, &full[s]);
       }
       __syncwarp();
     }
@@ -282,6 +280,9 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     const int row_base = 16 * wq + (lane >> 2);
     const int groups = p.K >> 4;
     uint8_t* const act_base = p.act + static_cast<size_t>(m0) * (p.K >> 1);
+    // Out-of-range smooth anywhere in K (flag word behind the table) selects the IEEE divide.  Only these warps look at it,
+    // while their first slab is on its way: as a condition of the table's loads it stood, 0.7 us, in front of everything.
+    const bool use_fdiv = has_table && *reinterpret_cast<const volatile uint32_t*>(p.table + 2 * p.K) != 0u;
     for (int i = grp; i < my_slabs; i += QUANT_GROUPS) {
       const uint32_t s = i % C::STAGES, ph = (i / C::STAGES) & 1;
       if (!mbar_wait(&full[s], ph, ctx, kDevWaitFull, 0x10000 + i)) break;
@@ -300,7 +301,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
         unpack_group<T, false>(raw[1][0], raw[1][1], f[1]);
         // this lane's 16 columns' reciprocals landed with the slab; a flagged launch reads the factors where they are
         if (!use_fdiv) qmath::smooth_multiply2(f[0], f[1], reinterpret_cast<const float4*>(smem + C::TB_OFF + s * TB_BYTES) + g);
-        else qmath::smooth_divide2(f[0], f[1], reinterpret_cast<const float4*>(smem + C::TB_OFF + s * TB_BYTES) + g);
+        else qmath::smooth_divide2(f[0], f[1], reinterpret_cast<const float4*>(p.table + p.K + k_begin + i * SLAB_K) + g);
       } else {
         unpack_group<T, true>(raw[0][0], raw[0][1], f[0]);
         unpack_group<T, true>(raw[1][0], raw[1][1], f[1]);
