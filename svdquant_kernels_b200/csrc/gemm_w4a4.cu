@@ -307,7 +307,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
   if constexpr (NEXT) qmath::fill_scale_lut(scale_lut, threadIdx.x, NUM_THREADS);
   __syncthreads();
-  if constexpr (CG == 2) cluster_arrive();
+  if constexpr (CG == 2) cluster_arrive_relaxed();       // (fence_barrier_init is what releases the barriers)
   // Tensor memory: only the issuer waits for it (its loads are under way by then), the epilogue reads the address once an
   // accumulator is complete.
   if (warp == EPI_WARPS + 1) {

@@ -242,9 +242,8 @@ __device__ __forceinline__ void fill_near_lut(float* lut, int tid, int nthreads)
   for (int i = tid; i < kScaleLutEntries; i += nthreads) lut[i] = static_cast<uint32_t>(i) - 1u < 0x7Du ? near_multiplier(i) : 0.0f;
 }
 
-// One 16-element group of near quotients: scale byte and eight code bytes
-__device__ __forceinline__ void quantize_group_near(const float2 (&f)[8], uint32_t& code_lo, uint32_t& code_hi, uint32_t& sbyte) {
-  const float amax = group_amax(f);
+// One 16-element group of near quotients and its group_amax: scale byte and eight code bytes
+__device__ __forceinline__ void quantize_group_near(const float2 (&f)[8], float amax, uint32_t& code_lo, uint32_t& code_hi, uint32_t& sbyte) {
   const uint32_t sb = scale_byte_near(amax);
   sbyte = sb;
   code_lo = code_hi = 0u;

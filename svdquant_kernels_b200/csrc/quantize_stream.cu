@@ -275,7 +275,7 @@ quantize_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
         // one group after the other, each stored as soon as it is done: running both groups' scale chains
         // side by side and keeping their results in registers until the end measured 5-8 % slower
         uint32_t c_lo, c_hi, s_b;
-        qmath::quantize_group_near(f[rr], c_lo, c_hi, s_b);
+        qmath::quantize_group_near(f[rr], qmath::group_amax(f[rr]), c_lo, c_hi, s_b);
         *reinterpret_cast<uint2*>(act_base + static_cast<size_t>(row) * (p.K >> 1) + (k0 >> 1)) = make_uint2(c_lo, c_hi);
         p.scales[static_cast<size_t>(gi) * p.M_pad + m0 + row] = static_cast<uint8_t>(s_b);
         if (p.scales_swz != nullptr) p.scales_swz[sf_swizzled_offset(m0 + row, gi, groups)] = static_cast<uint8_t>(s_b);

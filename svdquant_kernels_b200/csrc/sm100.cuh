@@ -86,6 +86,19 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// Arrival that cannot be performed before `a` and `b` are known, whatever they are (no float has the bits it tests for:
+// fmax returns the canonical NaN).  For handing a stage that was read with ordinary loads to the copy engine: the arrival
+// is done by a unit of its own, which does not wait for loads that nothing has used yet, but once a value made from
+// all of them exists they have been performed, for the whole warp.  (A fence does the same, but also waits for the
+// warp's stores on their way.)
+__device__ __forceinline__ void mbar_arrive_after(uint64_t* bar, float a, float b) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %1, 0xffffffff;\n\t"
+      "setp.ne.and.b32 q, %2, 0xffffffff, p;\n\t"
+      "@q mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}"
+      ::"r"(smem_u32(bar)), "r"(__float_as_uint(a)), "r"(__float_as_uint(b)) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
