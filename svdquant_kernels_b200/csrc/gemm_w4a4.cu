@@ -320,10 +320,10 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     __syncwarp();
     if (lane == 0) { if constexpr (CG == 2) mbar_arrive_cluster(tmem_ready, leader); else mbar_arrive(tmem_ready); }
   }
-  // Everything above touched only this CTA's shared and tensor memory, so it may overlap the tail of
-  // the kernel before this one in the stream; from here on its outputs are read.
-  pdl_wait();
-
+  // Everything above touched only this CTA's shared and tensor memory, so it may overlap the tail of the kernel before this
+  // one in the stream.  Each role waits for that kernel (pdl_wait) before it reads what may be its outputs; the producer
+  // has its first tile and addresses worked out by then.  (With the wait here they took it another 0.25 us, and bf16
+  // tiles' words 0.8 us more, before the first load: 256 x 3840 -> 3072 6.4 -> 6.2 us, 1003 x 3840 -> 3072 bf16 10.1 -> 9.7.)
   const int kt_main = (p.K + BK - 1) / BK;   // the last slab may hold fewer than four 64-element k-blocks
   const int lora_slabs = (p.R + 63) / 64;
   // bf16 output: lora_act comes as hi and lo bf16 planes (two passes over the same lora_up slab) and
@@ -341,13 +341,16 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int total_tiles = p.tiles_m * p.tiles_n;
   const int k_groups4 = p.K / 64;            // scale atoms along K
   // Work items: tiles, or (tile, split) pairs numbered tile-major so that the CTAs sharing a tile run
-  // at the same time.  Split i of a tile with n slabs (LoRA slabs included, at the end) takes slabs
-  // [i n / S, (i + 1) n / S).
+  // at the same time.  Split i of a tile with n slabs (LoRA slabs of one pass included, at the end) takes slabs
+  // [i n / S, (i + 1) n / S); a second LoRA pass is the last split's.  So where a range begins, and all of it before the
+  // LoRA slabs, does not depend on the number of passes, and no role waits for the words before its first slab.
   const int S = SK ? p.splits : 1;
   const int total_work = total_tiles * S;
-  auto slab_range = [&](int split, int kt_all, int& lo, int& hi) {
-    if (SK) { lo = split * kt_all / S; hi = (split + 1) * kt_all / S; } else { lo = 0; hi = kt_all; }
+  auto slab_range = [&](int split, int& lo, int& hi) {
+    const int n = kt_main + lora_slabs;
+    if (SK) { lo = split * n / S; hi = (split + 1) * n / S; } else { lo = 0; hi = n; }
   };
+  auto slabs_end = [&](int split, int hi, bool fp16_pass) -> int { return split == S - 1 ? kt_main + lora_parts(fp16_pass) * lora_slabs : hi; };
   // Which slab runs at position pos of a tile's kt_all = kt_main + n_lora slabs.  Slab numbers below
   // kt_main are main slabs, the others LoRA slabs.  End-grouped: position = number.  Interleaved (the
   // reference's schedule, cute_kernels/gemm_w4a4/kernel_v2_fa4.py:299-303): LoRA slab j sits at position
@@ -386,57 +389,74 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // ------------------------------ producer (both CTAs) ------------------------------
     uint32_t s = 0, ph = 1, it = 0;
     bool ok = true;
-    uint32_t words = lora_words(pair);
+    uint32_t words = 1u;
+    bool waited = false;
+    auto wait_ahead = [&]() {
+      if (!waited) { pdl_wait(); words = lora_words(pair); waited = true; }
+    };
     for (int w = pair; w < total_work && ok; w += num_pairs) {
       const int tile = SK ? w / S : w, split = SK ? w - tile * S : 0;
       const int mb = tile % p.tiles_m, nb = tile / p.tiles_m;
       const int m0 = (mb * CG + rank) * BM;
       const int nrow0 = nb * BN + static_cast<int>(rank) * C::B_ROWS;
-      const bool la_fp16 = lora_fp16(words);
-      words = lora_words(w + num_pairs);
-      const int kt_all = kt_main + lora_parts(la_fp16) * lora_slabs;
       int kt_lo, kt_hi;
-      slab_range(split, kt_all, kt_lo, kt_hi);
+      slab_range(split, kt_lo, kt_hi);
+      // The number of LoRA passes: of the first tile only when its first LoRA slab is due (unless they are interleaved).
+      bool la_fp16 = false, la_known = !kBf16;
       SlabWalk walk;
-      walk.start(kt_main, kt_all, p.interleave, lora_stride(la_fp16), kt_lo);
-      for (int pos = kt_lo; pos < kt_hi; ++pos, ++it) {
-        const int kt = walk.at(pos);
-        if (!uwait(&empty[s], ph, ctx, kDevWaitEmpty, it)) { ok = false; break; }
-        if (it == C::STAGES) pdl_trigger();       // the first stage has been consumed: see pdl_trigger
-        uint8_t* st = smem + s * C::STAGE_BYTES;
-        // Codes past K are zero-filled by TMA.  The scale atoms of a (128-row block, slab) are four
-        // consecutive 512-byte rows of the swizzled scale buffer seen as a [blocks * K/64, 512 B] matrix;
-        // a short last slab just fetches (and never uses) the rows that follow.  Every byte of a box
-        // counts toward the barrier whether it was in bounds or not.
-        constexpr uint32_t kSfBytes = SFA_BYTES + C::SFB_BYTES, kAbBytes = A_BYTES + C::B_BYTES;
-        // the barrier that counts this CTA's bytes: its own for CG = 1, the leader's for a pair
-        const uint32_t bar = (CG == 2) ? map_to_cta(smem_u32(&full[s]), leader) : smem_u32(&full[s]);
-        if (elect_one()) {
-          if (kt < kt_main) {
-            if (rank == 0) mbar_arrive_expect_tx(&full[s], (kSfBytes + kAbBytes) * CG);
-            tma_load_2d_bar<CG>(st + A_BYTES + C::B_BYTES, &tmSFA, 0, (mb * CG + rank) * k_groups4 + kt * 4, bar);
+      auto lora_verdict = [&]() {
+        wait_ahead();
+        la_fp16 = lora_fp16(words);
+        words = lora_words(w + num_pairs);
+        kt_hi = slabs_end(split, kt_hi, la_fp16);
+        la_known = true;
+      };
+      if (it > 0 || p.interleave) lora_verdict();
+      walk.start(kt_main, kt_main + lora_parts(la_fp16) * lora_slabs, p.interleave, lora_stride(la_fp16), kt_lo);
+      for (int pos = kt_lo; pos < kt_hi && ok;) {
+        if (!la_known && pos >= kt_main) lora_verdict();
+        const int stop = la_known || kt_hi < kt_main ? kt_hi : kt_main;
+        for (; pos < stop; ++pos, ++it) {
+          const int kt = walk.at(pos);
+          if (!uwait(&empty[s], ph, ctx, kDevWaitEmpty, it)) { ok = false; break; }
+          if (it == C::STAGES) pdl_trigger();       // the first stage has been consumed: see pdl_trigger
+          uint8_t* st = smem + s * C::STAGE_BYTES;
+          // Codes past K are zero-filled by TMA.  The scale atoms of a (128-row block, slab) are four
+          // consecutive 512-byte rows of the swizzled scale buffer seen as a [blocks * K/64, 512 B] matrix;
+          // a short last slab just fetches (and never uses) the rows that follow.  Every byte of a box
+          // counts toward the barrier whether it was in bounds or not.
+          constexpr uint32_t kSfBytes = SFA_BYTES + C::SFB_BYTES, kAbBytes = A_BYTES + C::B_BYTES;
+          // the barrier that counts this CTA's bytes: its own for CG = 1, the leader's for a pair
+          const uint32_t bar = (CG == 2) ? map_to_cta(smem_u32(&full[s]), leader) : smem_u32(&full[s]);
+          wait_ahead();
+          if (elect_one()) {
+            if (kt < kt_main) {
+              if (rank == 0) mbar_arrive_expect_tx(&full[s], (kSfBytes + kAbBytes) * CG);
+              tma_load_2d_bar<CG>(st + A_BYTES + C::B_BYTES, &tmSFA, 0, (mb * CG + rank) * k_groups4 + kt * 4, bar);
 #pragma unroll
-            for (int h = 0; h < BN / 128; ++h)
-              tma_load_2d_bar<CG>(st + A_BYTES + C::B_BYTES + SFA_BYTES + h * 2048, &tmSFB, 0,
-                                  (nb * (BN / 128) + h) * k_groups4 + kt * 4, bar);
-            tma_load_2d_bar<CG>(st, &tmA, kt * 128, m0, bar);
-            tma_load_2d_bar<CG>(st + A_BYTES, &tmB, kt * 128, nrow0, bar);
-          } else {
-            if (rank == 0) mbar_arrive_expect_tx(&full[s], kAbBytes * CG);
-            const int lt = kt - kt_main;
-            const int part = lt / lora_slabs, r0 = (lt % lora_slabs) * 64;
-            if (la_fp16) {
-              tma_load_2d_bar<CG>(st, &tmLAf, r0, m0, bar);
-              tma_load_2d_bar<CG>(st + A_BYTES, &tmLUf, r0, nrow0, bar);
+              for (int h = 0; h < BN / 128; ++h)
+                tma_load_2d_bar<CG>(st + A_BYTES + C::B_BYTES + SFA_BYTES + h * 2048, &tmSFB, 0,
+                                    (nb * (BN / 128) + h) * k_groups4 + kt * 4, bar);
+              tma_load_2d_bar<CG>(st, &tmA, kt * 128, m0, bar);
+              tma_load_2d_bar<CG>(st + A_BYTES, &tmB, kt * 128, nrow0, bar);
             } else {
-              tma_load_2d_bar<CG>(st, &tmLA, r0, part * p.M + m0, bar);    // lora_act parts are stacked along rows
-              tma_load_2d_bar<CG>(st + A_BYTES, &tmLU, r0, nrow0, bar);
+              if (rank == 0) mbar_arrive_expect_tx(&full[s], kAbBytes * CG);
+              const int lt = kt - kt_main;
+              const int part = lt / lora_slabs, r0 = (lt % lora_slabs) * 64;
+              if (la_fp16) {
+                tma_load_2d_bar<CG>(st, &tmLAf, r0, m0, bar);
+                tma_load_2d_bar<CG>(st + A_BYTES, &tmLUf, r0, nrow0, bar);
+              } else {
+                tma_load_2d_bar<CG>(st, &tmLA, r0, part * p.M + m0, bar);    // lora_act parts are stacked along rows
+                tma_load_2d_bar<CG>(st + A_BYTES, &tmLU, r0, nrow0, bar);
+              }
             }
           }
+          __syncwarp();
+          if (++s == C::STAGES) { s = 0; ph ^= 1; }
         }
-        __syncwarp();
-        if (++s == C::STAGES) { s = 0; ph ^= 1; }
       }
+      if (!la_known) words = lora_words(w + num_pairs);
     }
     if (it <= C::STAGES) pdl_trigger();
   } else if (warp == EPI_WARPS + 1) {
@@ -454,17 +474,23 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       tc_fence_after_sync();
       const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_slot), 0);   // warp-uniform, for the same reason as the warp index
       const uint32_t tmem_sf = tmem_base + C::ACC_COLS;              // SF_BUFS buffers of [SFA 16 | SFB] columns
+      pdl_wait();
       uint32_t words = lora_words(pair);
       for (int w = pair; w < total_work && ok; w += num_pairs, ++tcount) {
         const int tile = SK ? w / S : w, split = SK ? w - tile * S : 0;
         const uint32_t as = tcount & 1;
-        const bool la_fp16 = lora_fp16(words);
-        words = lora_words(w + num_pairs);
-        const int kt_all = kt_main + lora_parts(la_fp16) * lora_slabs;
         int kt_lo, kt_hi;
-        slab_range(split, kt_all, kt_lo, kt_hi);
+        slab_range(split, kt_lo, kt_hi);
+        bool la_fp16 = false, la_known = !kBf16;
         SlabWalk walk;
-        walk.start(kt_main, kt_all, p.interleave, lora_stride(la_fp16), kt_lo);
+        auto lora_verdict = [&]() {
+          la_fp16 = lora_fp16(words);
+          words = lora_words(w + num_pairs);
+          kt_hi = slabs_end(split, kt_hi, la_fp16);
+          la_known = true;
+        };
+        if (tcount > 0 || p.interleave) lora_verdict();
+        walk.start(kt_main, kt_main + lora_parts(la_fp16) * lora_slabs, p.interleave, lora_stride(la_fp16), kt_lo);
         if (!uwait(&acc_empty[as], ((tcount >> 1) & 1) ^ 1, ctx, kDevWaitAccFree, tcount)) break;
         tc_fence_after_sync();
         const uint32_t acc = tmem_base + as * 128;
@@ -473,47 +499,53 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (!uwait(acc_shared, (tcount - 1) & 1, ctx, kDevWaitAccFree, 0x20000 + tcount)) break;
           tc_fence_after_sync();
         }
-        for (int pos = kt_lo; pos < kt_hi; ++pos, ++it) {
-          const int kt = walk.at(pos);
-          if (!uwait(&full[s], ph, ctx, kDevWaitFull, it)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t stage16 = smem16 + s * (C::STAGE_BYTES / 16);
-          const uint64_t da = kDescAB + stage16, db = da + A_BYTES / 16;
-          const uint32_t accumulate = pos == kt_lo ? 0u : 1u;
-          if (elect_one()) {
-            if (kt < kt_main) {
-              const uint64_t dsa = kDescSF + stage16 + (A_BYTES + C::B_BYTES) / 16, dsb = dsa + SFA_BYTES / 16;
-              const uint32_t tsfa = tmem_sf + sb * C::SF_COLS, tsfb = tsfa + C::SFA_COLS;
-              // the slab's k-blocks: all their scales, then their MMAs
-              auto k_blocks = [&](int nkb) {
+        for (int pos = kt_lo; pos < kt_hi && ok;) {
+          if (!la_known && pos >= kt_main) lora_verdict();
+          const int stop = la_known || kt_hi < kt_main ? kt_hi : kt_main;
+          const int last = stop == kt_hi ? kt_hi - 1 : -1;          // the tile's last position, if it is in this stretch
+          for (; pos < stop; ++pos, ++it) {
+            const int kt = walk.at(pos);
+            if (!uwait(&full[s], ph, ctx, kDevWaitFull, it)) { ok = false; break; }
+            tc_fence_after_sync();
+            const uint32_t stage16 = smem16 + s * (C::STAGE_BYTES / 16);
+            const uint64_t da = kDescAB + stage16, db = da + A_BYTES / 16;
+            const uint32_t accumulate = pos == kt_lo ? 0u : 1u;
+            if (elect_one()) {
+              if (kt < kt_main) {
+                const uint64_t dsa = kDescSF + stage16 + (A_BYTES + C::B_BYTES) / 16, dsb = dsa + SFA_BYTES / 16;
+                const uint32_t tsfa = tmem_sf + sb * C::SF_COLS, tsfb = tsfa + C::SFA_COLS;
+                // the slab's k-blocks: all their scales, then their MMAs
+                auto k_blocks = [&](int nkb) {
+#pragma unroll
+                  for (int j = 0; j < 4; ++j)
+                    if (j < nkb) {
+                      tmem_cp_scales<CG>(tsfa + j * 4, dsa + j * 32);
+#pragma unroll
+                      for (int h = 0; h < BN / 128; ++h) tmem_cp_scales<CG>(tsfb + j * (BN / 32) + h * 4, dsb + h * 128 + j * 32);
+                    }
+#pragma unroll
+                  for (int j = 0; j < 4; ++j)
+                    if (j < nkb)
+                      mma_nvfp4<CG>(acc, da + j * 2, db + j * 2, kIdescMain, tsfa + j * 4, tsfb + j * (BN / 32), j != 0 ? 1u : accumulate);
+                };
+                const int nkb = k_groups4 - kt * 4;
+                if (nkb >= 4) k_blocks(4); else k_blocks(nkb);      // the last slab may be short
+              } else {
+                const uint32_t idesc = la_fp16 ? kIdescLoraF16 : kIdescLora;
+                const int nkb = (p.R - ((kt - kt_main) % lora_slabs) * 64) / 16;
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                  if (j < nkb) {
-                    tmem_cp_scales<CG>(tsfa + j * 4, dsa + j * 32);
-#pragma unroll
-                    for (int h = 0; h < BN / 128; ++h) tmem_cp_scales<CG>(tsfb + j * (BN / 32) + h * 4, dsb + h * 128 + j * 32);
-                  }
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                  if (j < nkb)
-                    mma_nvfp4<CG>(acc, da + j * 2, db + j * 2, kIdescMain, tsfa + j * 4, tsfb + j * (BN / 32), j != 0 ? 1u : accumulate);
-              };
-              const int nkb = k_groups4 - kt * 4;
-              if (nkb >= 4) k_blocks(4); else k_blocks(nkb);      // the last slab may be short
-            } else {
-              const uint32_t idesc = la_fp16 ? kIdescLoraF16 : kIdescLora;
-              const int nkb = (p.R - ((kt - kt_main) % lora_slabs) * 64) / 16;
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                if (j < nkb) mma_f16<CG>(acc, da + j * 2, db + j * 2, idesc, j != 0 ? 1u : accumulate);
+                  if (j < nkb) mma_f16<CG>(acc, da + j * 2, db + j * 2, idesc, j != 0 ? 1u : accumulate);
+              }
+              tc_commit_mask<CG>(&empty[s], mask);          // stage reusable (in both CTAs) once these MMAs have read it
+              if (pos == last) tc_commit_mask<CG>(&acc_full[as], mask);    // accumulator complete
             }
-            tc_commit_mask<CG>(&empty[s], mask);          // stage reusable (in both CTAs) once these MMAs have read it
-            if (pos == kt_hi - 1) tc_commit_mask<CG>(&acc_full[as], mask);    // accumulator complete
+            __syncwarp();
+            if (++sb == C::SF_BUFS) sb = 0;
+            if (++s == C::STAGES) { s = 0; ph ^= 1; }
           }
-          __syncwarp();
-          if (++sb == C::SF_BUFS) sb = 0;
-          if (++s == C::STAGES) { s = 0; ph ^= 1; }
         }
+        if (!la_known) words = lora_words(w + num_pairs);
       }
     }
   } else {
@@ -524,6 +556,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int quarter = warp & 3, chalf = warp >> 2;
     uint32_t tcount = 0;
     bool ok = true, drained = false;
+    pdl_wait();
     for (int w = pair; w < total_work && ok; w += num_pairs, ++tcount) {
       const int tile = SK ? w / S : w, split = SK ? w - tile * S : 0;
       const int mb = tile % p.tiles_m, nb = tile / p.tiles_m;
