@@ -126,7 +126,7 @@ struct Cfg {
   static constexpr int TMEM_COLS = 512;
   static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + STORE_BYTES + TAIL_BYTES;
   static_assert(ACC_COLS + SF_BUFS * SF_COLS <= TMEM_COLS && SF_BUFS >= 2, "tensor memory budget");
-  static_assert(STAGES >= 3, "ring too shallow");
+  static_assert(STAGES >= 3 && STAGES * STAGE_BYTES >= BN / 128 * EPI_WARPS * STORE_BUF_BYTES, "ring too shallow");
   static_assert((2 * STAGES + 6) * 8 + 16 <= 512, "barrier block");
 };
 
@@ -587,8 +587,9 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
       }
       // One strip: 64 columns from column cbase of the tile, the 64 accumulator values of this lane's row in v.
-      auto strip = [&](uint32_t (&v)[64], int cbase) {
-        [[maybe_unused]] uint8_t* buf = store_bufs + warp * STORE_BUF_BYTES;     // TP: this warp's staging strip
+      // STAGED: y through shared memory (the TP form's strips; the last tile's, see below).
+      auto strip = [&](uint32_t (&v)[64], int cbase, [[maybe_unused]] uint8_t* buf, auto staged) {
+        constexpr bool STAGED = decltype(staged)::value;
         if constexpr (TP) {
           // the TMA store that last read this warp's buffer must be done with it
           if (lane == 0) tma_store_wait_read<0>();
@@ -647,7 +648,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               }
             }
           }
-          if constexpr (TP) {
+          if constexpr (STAGED) {
             // row `lane` of the strip: 16-byte chunks hc*4 .. hc*4+3, XOR-swizzled like the TMA box
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -668,6 +669,20 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 *reinterpret_cast<uint4*>(dst + 16 * i + 8) = make_uint4(o[8 * i + 4], o[8 * i + 5], o[8 * i + 6], o[8 * i + 7]);
               }
             }
+          }
+        }
+        if constexpr (STAGED && !TP) {
+          // The CTA's last tile, whose stores nothing hides: out of the ring, which is free by now, eight lanes a row, so that an
+          // instruction touches 4 lines instead of 32 (an SM takes a line in some two cycles: the last stores of a
+          // 256-column tile ended 1.4 us earlier).  256 x 3840 -> 3072 6.2 -> 6.0 us, 1003 x 3840 -> 3072 9.8 -> 9.4,
+          // 4352 x 3840 -> 3072 28.7 -> 28.2, 4352 x 3840 -> 15360 126.3 -> 125.6.
+          __syncwarp();
+          OutT* dst = static_cast<OutT*>(p.y) + static_cast<size_t>(m0 + quarter * 32 + (lane >> 3)) * p.N + n0 + cbase + (lane & 7) * 8;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int row = 4 * i + (lane >> 3);
+            const uint4 t = *reinterpret_cast<const uint4*>(buf + row * 128 + (((lane & 7) ^ (row & 7)) << 4));
+            *reinterpret_cast<uint4*>(dst + static_cast<size_t>(4 * i) * p.N) = t;
           }
         }
         if constexpr (TP) {
@@ -774,7 +789,12 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                                                                      __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
         finish = false;
       }
-      if (finish) strip(v, cbase);
+      if constexpr (TP) {
+        if (finish) strip(v, cbase, store_bufs + warp * STORE_BUF_BYTES, std::true_type{});      // this warp's staging strip
+      } else if (finish) {
+        if (w + num_pairs < total_work) strip(v, cbase, nullptr, std::false_type{});
+        else strip(v, cbase, smem + (q * EPI_WARPS + warp) * STORE_BUF_BYTES, std::true_type{});
+      }
       }
       // affine[] may be overwritten after this barrier; it also makes the eight warps agree on whether to go on
       uint32_t any_failed;
