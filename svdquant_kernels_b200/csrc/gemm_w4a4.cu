@@ -112,7 +112,7 @@ struct Cfg {
   // per-column rows of the current tile: wcscales, bias and, for the next layer's quantisation, -smooth_next and
   // 1 / smooth_next
   static constexpr int AFFINE_BYTES = (NEXT ? 4 : 2) * BN * 4;
-  static constexpr int LUT_BYTES = NEXT ? qmath::kScaleLutEntries * 8 : 0;    // the constants of each scale byte
+  static constexpr int LUT_BYTES = NEXT ? qmath::kScaleLutEntries * 4 : 0;    // the multiplier of each scale byte
   static constexpr int TAIL_BYTES = AFFINE_BYTES + LUT_BYTES + 512 /*barriers*/;
   static constexpr int STAGES_RAW = (232448 - 1024 - STORE_BYTES - TAIL_BYTES) / STAGE_BYTES;
   static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
@@ -198,7 +198,7 @@ template <> __device__ __forceinline__ float as_f32<__nv_bfloat16>(__nv_bfloat16
 // division, the scale and both code paths made the epilogue too large for the instruction cache (the top
 // stall reason was "no instruction", at 17 % issue utilisation).
 __device__ __noinline__ uint4 next_group_codes(float2 a0, float2 a1, float2 a2, float2 a3, float2 a4, float2 a5,
-                                               float2 a6, float2 a7, const float4* ns4, const float4* r4, const float2* lut,
+                                               float2 a6, float2 a7, const float4* ns4, const float4* r4, const float* lut,
                                                int tile_fdiv) {
   const float2 a[8] = {a0, a1, a2, a3, a4, a5, a6, a7};
   float2 q[8];
@@ -234,8 +234,8 @@ __device__ __noinline__ uint4 next_group_codes(float2 a0, float2 a1, float2 a2, 
     sb = qmath::group_scale_byte(q);
   }
   uint32_t lo, hi;
-  const float2 k = lut[sb];
-  if (k.x != 0.0f) qmath::group_codes_fast(q, k, lo, hi);
+  const float c = lut[sb];
+  if (c != 0.0f) qmath::group_codes_cut(q, c, lo, hi);
   else qmath::group_codes_compare(q, sb, lo, hi);
   return make_uint4(lo, hi, sb, 0u);
 }
@@ -260,7 +260,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   [[maybe_unused]] uint8_t* store_bufs = smem + C::STAGES * C::STAGE_BYTES;   // TP; 1024-aligned: every stage is a multiple of 1 KB
   uint8_t* tail = smem + C::STAGES * C::STAGE_BYTES + C::STORE_BYTES;
   float* affine = reinterpret_cast<float*>(tail);                 // [2 or 4][BN] : wcscales, bias, -smooth_next, 1/smooth_next of the current tile
-  [[maybe_unused]] float2* scale_lut = reinterpret_cast<float2*>(tail + C::AFFINE_BYTES);
+  [[maybe_unused]] float* scale_lut = reinterpret_cast<float*>(tail + C::AFFINE_BYTES);
   uint64_t* bars = reinterpret_cast<uint64_t*>(tail + C::AFFINE_BYTES + C::LUT_BYTES);
   uint64_t* full = bars;                                          // [STAGES] operands and scales landed (leader CTA's copy is used)
   uint64_t* empty = bars + C::STAGES;                             // [STAGES] stage consumed by the MMAs (per CTA)
@@ -305,7 +305,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (p.R > 0) { tma_prefetch_desc(&tmLA); tma_prefetch_desc(&tmLU); }
     if (p.R > 0 && p.la_flags != nullptr) { tma_prefetch_desc(&tmLAf); tma_prefetch_desc(&tmLUf); }
   }
-  if constexpr (NEXT) qmath::fill_scale_lut(scale_lut, threadIdx.x, NUM_THREADS);
+  if constexpr (NEXT) qmath::fill_near_lut(scale_lut, threadIdx.x, NUM_THREADS);
   __syncthreads();
   if constexpr (CG == 2) cluster_arrive_relaxed();       // (fence_barrier_init is what releases the barriers)
   // Tensor memory: only the issuer waits for it (its loads are under way by then), the epilogue reads the address once an

@@ -41,10 +41,8 @@ quantize_rows_kernel(const T* __restrict__ x, const T* __restrict__ smooth, uint
   __shared__ __align__(16) uint8_t sc[kPackGroups][kPackRows];
   constexpr bool k16 = sizeof(T) == 2;
   using Pair = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
-  __shared__ float2 lut[k16 ? 1 : qmath::kScaleLutEntries];
-  __shared__ float near_lut[k16 ? qmath::kScaleLutEntries : 1];
-  if constexpr (k16) qmath::fill_near_lut(near_lut, threadIdx.x, kPackThreads);
-  else qmath::fill_scale_lut(lut, threadIdx.x, kPackThreads);
+  __shared__ float near_lut[qmath::kScaleLutEntries];
+  qmath::fill_near_lut(near_lut, threadIdx.x, kPackThreads);
   __syncthreads();
   // launched with programmatic serialization: nothing below may run before the kernel ahead has finished
   pdl_trigger();
@@ -108,22 +106,23 @@ quantize_rows_kernel(const T* __restrict__ x, const T* __restrict__ smooth, uint
       uint32_t code = 0, sbyte = 0;
       if (m < rows && g < groups) {                       // rows of the padding get zero codes and scales
         const float2 zero = make_float2(0.0f, 0.0f);      // the + 0 below makes a -0 a +0
-        float2 c;
-        if constexpr (k16) {
-          sbyte = qmath::scale_byte_near(amax);
-          c = make_float2(near_lut[sbyte], 0.0f);
-        } else {
-          sbyte = qmath::scale_byte(fminf(amax, 1e30f));  // the three-step divide wants a finite value; 448 is reached long before
-          c = lut[sbyte];
-        }
-        if (c.x != 0.0f && !odd) {
-          // the conversion instruction's paths of quantize_math.cuh: near quotients for 16-bit values, exact floors for fp32
-          const float2 mult = make_float2(c.x, c.x), rj = make_float2(c.y, c.y);
+        if constexpr (k16) sbyte = qmath::scale_byte_near(amax);
+        else sbyte = qmath::scale_byte(fminf(amax, 1e30f));   // the three-step divide wants a finite value; 448 is reached long before
+        const float c = near_lut[sbyte];
+        if (c != 0.0f && !odd) {
+          // the conversion instruction's paths of quantize_math.cuh: near quotients for 16-bit values, cut values for fp32
+          const float2 mult = make_float2(c, c);
           float w[EPL];
 #pragma unroll
           for (int i = 0; i < EPL; i += 2) {
-            float2 q = __ffma2_rn(make_float2(f[i], f[i + 1]), mult, zero);
-            if constexpr (!k16) q = __fmul2_rn(make_float2(truncf(q.x), truncf(q.y)), rj);
+            float2 q;
+            if constexpr (k16) {
+              q = __ffma2_rn(make_float2(f[i], f[i + 1]), mult, zero);
+            } else {
+              // + 0 before the cut, which leaves a value below all bounds its sign
+              q = __fadd2_rn(make_float2(f[i], f[i + 1]), zero);
+              q = __fmul2_rn(make_float2(qmath::cut12(q.x), qmath::cut12(q.y)), mult);
+            }
             w[i] = q.x; w[i + 1] = q.y;
           }
           code = qmath::cvt_e2m1<EPL>(w);

@@ -25,14 +25,13 @@
 // Groups whose scale byte is 0 (everything non-zero saturates) or the 448 clamp (ratios are unbounded)
 // compare against the seven exact products instead.
 //
-// fp32 values (weights, the next layer's activations in the GEMM's epilogue) have 24 significant bits, so
-// their quotient by the scale needs an exact floor.  The scale byte is J * 2^E (J = 1..15), so
-// m = trunc(4 v / 2^E) is an integer with v's sign and the E2M1 code is the number of n in
-// {1,3,5,7,10,14,20} with n J <= |m|.  m / (4 J) lies on a rounding bound of E2M1 exactly when |m| = n J and at
-// least 1/(4 J) away from every bound otherwise, so RN(m * RN(1/(4 J)) * (1 + 2^-20))
-// is strictly above the bound in the first case and on the right side of it in the
-// second, and the hardware conversion cvt.rn.satfinite.e2m1x2.f32 of it returns the
-// reference's code, sign included (checked exhaustively over J and m on the CPU).
+// fp32 values (weights, the next layer's activations in the GEMM's epilogue) have 24 significant bits.  Scales have 4 and
+// bounds of codes 3, so every product scale * bound is among the numbers of 12 significant bits, and cutting a value
+// down to those (one AND, towards zero, the sign stays) leaves it on its side of all of them.  What is left and not on a
+// bound is off it by 2^-12 of it, far more than one multiplication by rcp(scale)(1 + 2^-21) errs, and a value on a bound
+// comes out above it: the conversion instruction of the product returns the reference's code.  (Exact floors of 4 v / 2^E,
+// rescaled by a second multiplication, take a slow conversion and a multiplication an element more: 15360 x 3840 fp32 52.3 -> 51.6 us, the next layer's codes of
+// 4352 x 1024 -> 3072 bf16, both kernels, 32.8 -> 30.0.)
 #pragma once
 
 #include "nvfp4_math.cuh"
@@ -105,19 +104,7 @@ __device__ __forceinline__ void smooth_divide2(float2 (&f0)[8], float2 (&f1)[8],
   }
 }
 
-// {2^(2-E), RN(1/(4 J)) (1 + 2^-20)} of scale byte sb = J 2^E; {0, 0} for the two bytes that take the compare path
-__device__ __forceinline__ float2 scale_constants(uint32_t sb) {
-  if (sb == 0u || sb >= 0x7Eu) return make_float2(0.0f, 0.0f);
-  const uint32_t e = sb >> 3, m3 = sb & 7u;
-  const uint32_t J = e ? 8u + m3 : m3;
-  const float mult = __uint_as_float((e ? 139u - e : 138u) << 23);
-  const float rj = __fmul_rn(__frcp_rn(static_cast<float>(4u * J)), 1.00000095367431640625f);
-  return make_float2(mult, rj);
-}
 constexpr int kScaleLutEntries = 128;
-__device__ __forceinline__ void fill_scale_lut(float2* lut, int tid, int nthreads) {
-  for (int i = tid; i < kScaleLutEntries; i += nthreads) lut[i] = scale_constants(static_cast<uint32_t>(i));
-}
 
 __device__ __forceinline__ float max3abs(float a, float b, float c) {
   float r;
@@ -176,22 +163,6 @@ __device__ __forceinline__ float group_amax(const float2 (&f)[8]) {
 // amax of a 16-element group -> scale byte
 __device__ __forceinline__ uint32_t group_scale_byte(const float2 (&f)[8]) { return scale_byte(group_amax(f)); }
 
-// Main path of the codes: k = {2^(2-E), ~1/(4J)} of the group's scale byte.
-// m = trunc(4 v / 2^E) keeps the sign of v (also as -0 for a small negative v, whose code is
-// "negative zero" in the reference too; v itself is never -0 here: inputs were made +0 and
-// quotients cannot underflow in this path)
-__device__ __forceinline__ void group_codes_fast(const float2 (&f)[8], float2 k, uint32_t& code_lo, uint32_t& code_hi) {
-  const float2 mult = make_float2(k.x, k.x), rj = make_float2(k.y, k.y);
-  float2 w[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float2 t = __fmul2_rn(f[j], mult);
-    w[j] = __fmul2_rn(make_float2(truncf(t.x), truncf(t.y)), rj);
-  }
-  code_lo = cvt_e2m1x8(w[0], w[1], w[2], w[3]);
-  code_hi = cvt_e2m1x8(w[4], w[5], w[6], w[7]);
-}
-
 // Zero scale (everything non-zero saturates) or the 448 clamp (ratios are unbounded): compare path
 __device__ __forceinline__ void group_codes_compare(const float2 (&f)[8], uint32_t sb, uint32_t& code_lo, uint32_t& code_hi) {
   float sf = e4m3_to_f32(static_cast<uint8_t>(sb));
@@ -240,6 +211,18 @@ __device__ __forceinline__ float near_multiplier(uint32_t sb) {
 // The same for every scale byte; 0 for the two that take the compare path
 __device__ __forceinline__ void fill_near_lut(float* lut, int tid, int nthreads) {
   for (int i = tid; i < kScaleLutEntries; i += nthreads) lut[i] = static_cast<uint32_t>(i) - 1u < 0x7Du ? near_multiplier(i) : 0.0f;
+}
+
+// An fp32 value cut to 12 significant bits (see the head of this file)
+__device__ __forceinline__ float cut12(float v) { return __uint_as_float(__float_as_uint(v) & 0xFFFFF000u); }
+// Codes of a group of fp32 values, c = near_multiplier of its scale byte (1 <= byte < 0x7E)
+__device__ __forceinline__ void group_codes_cut(const float2 (&f)[8], float c, uint32_t& code_lo, uint32_t& code_hi) {
+  const float2 cc = make_float2(c, c);
+  float2 w[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) w[j] = __fmul2_rn(make_float2(cut12(f[j].x), cut12(f[j].y)), cc);
+  code_lo = cvt_e2m1x8(w[0], w[1], w[2], w[3]);
+  code_hi = cvt_e2m1x8(w[4], w[5], w[6], w[7]);
 }
 
 // One 16-element group of near quotients and its group_amax: scale byte and eight code bytes

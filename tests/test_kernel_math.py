@@ -139,3 +139,32 @@ def test_division_through_the_rounded_reciprocal_equals_ieee_division_on_samples
             bad += int(q != want)
             checked += 1
     assert checked > 3000 and bad == 0
+
+
+def test_values_cut_to_twelve_bits_convert_to_the_reference_codes():
+    """Codes of fp32 values: RN(cut(v) * c) with v cut to 12 significant bits and c at either end of rcp(scale)(1 + 2^-21)'s
+    error (the reciprocal's is 1 ulp) falls on v's side of every bound, ties and the fp32 neighbours of each bound
+    included, for every scale that takes this path; a value below all bounds keeps its sign."""
+    def cut(v):
+        return (v.view(np.uint32) & np.uint32(0xFFFFF000)).view(np.float32)
+    bounds = np.array([0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0])
+    rng = np.random.default_rng(3)
+    for s in O._E4M3_POS[1:-1]:
+        p = (np.float64(s) * bounds).astype(np.float32)           # exact
+        near = [p]
+        for to in (np.float32(0), np.float32(1e30)):
+            q = p
+            for _ in range(3):
+                q = np.nextafter(q, to)
+                near.append(q)
+        near += [cut(np.nextafter(p, np.float32(0))), (rng.random(400) * 8 * float(s)).astype(np.float32)]
+        v = np.concatenate(near).astype(np.float32)
+        want = (v[:, None].astype(np.float64) >= np.float64(s) * bounds).sum(1)
+        rcp = f32(1.0) / f32(s)
+        for r in (np.nextafter(rcp, f32(0)), rcp, np.nextafter(rcp, f32(1e30))):
+            c = f32(r * (f32(1.0) + f32(2.0 ** -21)))
+            w = (cut(v) * c).astype(np.float32)
+            assert ((w[:, None].astype(np.float64) > bounds).sum(1) == want).all(), s
+            assert not np.isin(w.astype(np.float64), bounds).any(), s
+    tiny = -np.array([2.0 ** -149, 2.0 ** -140, 2.0 ** -126, 1e-30], dtype=np.float32)
+    assert np.signbit(cut(tiny)).all()
