@@ -191,53 +191,62 @@ template <> __device__ __forceinline__ float as_f32<__half>(__half v) { return _
 template <> __device__ __forceinline__ float as_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
 // Next layer's quantisation of one 16-column group of one row: the 16 fp32 results (already scaled and
-// biased) are divided by smooth_next and packed as NVFP4.  ns4 / r4: the group's four entries of the
-// -smooth_next and 1 / smooth_next rows.  Returns {codes 0-7, codes 8-15, scale byte, -}.
-// Not inlined on purpose: the epilogue calls it eight times per tile from fully unrolled code (the
-// accumulator lives in registers, which only constant indices can address), and eight copies of the
-// division, the scale and both code paths made the epilogue too large for the instruction cache (the top
-// stall reason was "no instruction", at 17 % issue utilisation).
-__device__ __noinline__ uint4 next_group_codes(float2 a0, float2 a1, float2 a2, float2 a3, float2 a4, float2 a5,
-                                               float2 a6, float2 a7, const float4* ns4, const float4* r4, const float* lut,
-                                               int tile_fdiv) {
+// biased) are divided by smooth_next and packed as NVFP4.  ns4: the group's four entries of the -smooth_next row.
+// Returns {codes 0-7, codes 8-15, scale byte, -}.  This form takes every case, by IEEE division of the uncast fp32
+// values, as the reference does; + 0 turns a -0 quotient into +0 (the reference gives a zero the sign bit only when the
+// value tests < 0).  Not inlined: it is for the rare ones (next_two_groups).
+__device__ __noinline__ uint4 next_group_any(float2 a0, float2 a1, float2 a2, float2 a3, float2 a4, float2 a5, float2 a6, float2 a7,
+                                             const float4* ns4, const float* lut) {
   const float2 a[8] = {a0, a1, a2, a3, a4, a5, a6, a7};
+  uint32_t bits = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) bits |= __float_as_uint(a[j].x) | __float_as_uint(a[j].y);
+  if ((bits & 0x7FFFFFFFu) == 0u) return make_uint4(0u, 0u, 0u, 0u);        // a group of zeros, as rows of the padding can be
   float2 q[8];
-  // IEEE divide of the uncast fp32 values, as the reference does; + 0 turns a -0 quotient into +0 (the
-  // reference gives a zero the sign bit only when the value tests < 0)
-  auto divide_ieee = [&]() {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float4 ns = ns4[j];
-      q[2 * j] = make_float2(__fadd_rn(__fdiv_rn(a[2 * j].x, -ns.x), 0.0f), __fadd_rn(__fdiv_rn(a[2 * j].y, -ns.y), 0.0f));
-      q[2 * j + 1] = make_float2(__fadd_rn(__fdiv_rn(a[2 * j + 1].x, -ns.z), 0.0f), __fadd_rn(__fdiv_rn(a[2 * j + 1].y, -ns.w), 0.0f));
-    }
-  };
-  if (!tile_fdiv) {
-    // the same quotients in three packed instructions per pair (qmath::divide_by_constant2)
-    const float2 zero = make_float2(0.0f, 0.0f);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float4 ns = ns4[j], r = r4[j];
-      q[2 * j] = __fadd2_rn(qmath::divide_by_constant2(a[2 * j], make_float2(ns.x, ns.y), make_float2(r.x, r.y)), zero);
-      q[2 * j + 1] = __fadd2_rn(qmath::divide_by_constant2(a[2 * j + 1], make_float2(ns.z, ns.w), make_float2(r.z, r.w)), zero);
-    }
-  } else {
-    divide_ieee();
+  for (int j = 0; j < 4; ++j) {
+    const float4 ns = ns4[j];
+    q[2 * j] = make_float2(__fadd_rn(__fdiv_rn(a[2 * j].x, -ns.x), 0.0f), __fadd_rn(__fdiv_rn(a[2 * j].y, -ns.y), 0.0f));
+    q[2 * j + 1] = make_float2(__fadd_rn(__fdiv_rn(a[2 * j + 1].x, -ns.z), 0.0f), __fadd_rn(__fdiv_rn(a[2 * j + 1].y, -ns.w), 0.0f));
   }
-  uint32_t sb = qmath::group_scale_byte(q);
-  if (!tile_fdiv && (sb == 0u || sb >= 0x7Eu)) {
-    // Scale byte 0 or 448: a group of tiny or of huge values, where the three-step quotient may have under-
-    // or overflowed on the way.  (With a byte in between, the group's largest quotient lies in [2^-10, 2700):
-    // every operand that can reach a rounding bound of a code is far from both ends of the range, and the
-    // quotients that matter are exact.)
-    divide_ieee();
-    sb = qmath::group_scale_byte(q);
-  }
+  const uint32_t sb = qmath::group_scale_byte(q);
   uint32_t lo, hi;
   const float c = lut[sb];
   if (c != 0.0f) qmath::group_codes_cut(q, c, lo, hi);
   else qmath::group_codes_compare(q, sb, lo, hi);
   return make_uint4(lo, hi, sb, 0u);
+}
+// Two neighbouring groups of one row, the same quotients in three packed instructions per pair
+// (qmath::divide_by_constant2).  Side by side and inline, so that one's chain of dependent steps fills the other's gaps: an
+// epilogue warp has only one other on its scheduler (a call per group: 4352 x 1024 -> 3072 bf16, both kernels, 30.0 -> 27.8 us,
+// 4352 x 3840 -> 3072 fp16 47.4 -> 46.5).  Groups that the three steps do not settle go to next_group_any: tile_fdiv, and a
+// scale byte of 0 or 448, a group of tiny or of huge values, where a quotient may have under- or overflowed on the way.
+// (With a byte in between, the group's largest quotient lies in [2^-10, 2700): every operand that can reach a rounding bound
+// of a code is far from both ends of the range, and the quotients that matter are exact.)
+__device__ __forceinline__ void next_two_groups(const float2 (&a)[16], const float4* ns4, const float4* r4, const float* lut, bool tile_fdiv,
+                                                uint32_t (&codes)[4], uint32_t (&sb)[2]) {
+  const float2 zero = make_float2(0.0f, 0.0f);
+  float2 q[2][8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float4 ns = ns4[j], r = r4[j];
+    q[j >> 2][2 * (j & 3)] = __fadd2_rn(qmath::divide_by_constant2(a[2 * j], make_float2(ns.x, ns.y), make_float2(r.x, r.y)), zero);
+    q[j >> 2][2 * (j & 3) + 1] = __fadd2_rn(qmath::divide_by_constant2(a[2 * j + 1], make_float2(ns.z, ns.w), make_float2(r.z, r.w)), zero);
+  }
+  sb[0] = qmath::group_scale_byte(q[0]);
+  sb[1] = qmath::group_scale_byte(q[1]);
+  const float c0 = lut[sb[0]], c1 = lut[sb[1]];
+  if (!tile_fdiv && c0 != 0.0f && c1 != 0.0f) {
+    qmath::group_codes_cut(q[0], c0, codes[0], codes[1]);
+    qmath::group_codes_cut(q[1], c1, codes[2], codes[3]);
+  } else {
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      const uint4 t = next_group_any(a[8 * g], a[8 * g + 1], a[8 * g + 2], a[8 * g + 3], a[8 * g + 4], a[8 * g + 5], a[8 * g + 6], a[8 * g + 7],
+                                     ns4 + 4 * g, lut);
+      codes[2 * g] = t.x; codes[2 * g + 1] = t.y; sb[g] = t.z;
+    }
+  }
 }
 
 // How a tile's K loop is split over CTAs (see the header comment): not at all, through a workspace, within a cluster
@@ -600,7 +609,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           const float4* wc4 = reinterpret_cast<const float4*>(affine + cbase + hc * 32);
           const float4* bs4 = reinterpret_cast<const float4*>(affine + BN + cbase + hc * 32);
           uint32_t o[16];
-          [[maybe_unused]] float2 qf[8];      // NEXT: the 16 values of the current column group
+          [[maybe_unused]] float2 qf[16];     // NEXT: the 32 values of this half strip
           [[maybe_unused]] uint32_t qcodes[4], qscales[2];
           // the four fp32 results of columns 4 i .. 4 i + 3 of this half strip
           auto affine_at = [&](int i, float& a0, float& a1, float& a2, float& a3) {
@@ -622,16 +631,14 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             o[2 * i] = pack2f<OutT>(a0, a1);
             o[2 * i + 1] = pack2f<OutT>(a2, a3);
             if constexpr (NEXT) {
-              qf[2 * (i & 3)] = make_float2(a0, a1);
-              qf[2 * (i & 3) + 1] = make_float2(a2, a3);
-              if ((i & 3) == 3) {
-                const int e4 = (cbase + hc * 32) / 4 + (i - 3);      // float4 index of the group's first column
-                const uint4 r = next_group_codes(qf[0], qf[1], qf[2], qf[3], qf[4], qf[5], qf[6], qf[7],
-                                                 reinterpret_cast<const float4*>(affine + 2 * BN) + e4,
-                                                 reinterpret_cast<const float4*>(affine + 3 * BN) + e4, scale_lut, tile_fdiv ? 1 : 0);
-                qcodes[2 * (i >> 2)] = r.x; qcodes[2 * (i >> 2) + 1] = r.y; qscales[i >> 2] = r.z;
-              }
+              qf[2 * i] = make_float2(a0, a1);
+              qf[2 * i + 1] = make_float2(a2, a3);
             }
+          }
+          if constexpr (NEXT) {
+            const int e4 = (cbase + hc * 32) / 4;
+            next_two_groups(qf, reinterpret_cast<const float4*>(affine + 2 * BN) + e4, reinterpret_cast<const float4*>(affine + 3 * BN) + e4, scale_lut,
+                            tile_fdiv, qcodes, qscales);
           }
           if constexpr (NEXT) {
             if (ok) {
