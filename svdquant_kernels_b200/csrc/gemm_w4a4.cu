@@ -144,6 +144,7 @@ struct Params {
   const uint32_t* la_flags;   // bf16 only: per 32 rows of lora_act, non-zero = does not fit fp16; null = always two-pass
   int M, N, K, R;
   int tiles_m, tiles_n; // in units of (CG*128) x BN
+  int whole_tiles;      // tiles from this one on are worked on as two halves of BN / 2 columns (see launch_gemm_t)
   // Column-sharded (tensor-parallel) form: this launch computes columns [col0, col0 + N) of a
   // [M, y_ld] result that every rank holds in full.  The local copy is written through a tensor map (built over
   // the local full matrix); each finished strip is also stored, by TMA from the same staging buffer,
@@ -252,7 +253,9 @@ __device__ __forceinline__ void next_two_groups(const float2 (&a)[16], const flo
 // How a tile's K loop is split over CTAs (see the header comment): not at all, through a workspace, within a cluster
 enum SplitForm : int { kNoSplit = 0, kWorkspaceSplit = 1, kClusterSplit = 2 };
 
-template <int CG, int BN, typename OutT, int SK = kNoSplit, bool NEXT = false, bool TP = false>
+// HALVES: the last round's tiles are worked on as two halves of BN / 2 columns each (see gemm_halved_tiles).  A form of its
+// own: with the choice in the issuing loop of every launch, those without halves took 1 % longer.
+template <int CG, int BN, typename OutT, int SK = kNoSplit, bool NEXT = false, bool TP = false, bool HALVES = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmLA, const __grid_constant__ CUtensorMap tmLU,
@@ -340,21 +343,24 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   // the fp16 plane and the fp16 copy of lora_up in a single pass.  Every role of both CTAs
   // evaluates this per tile from the same words, so they agree on the number of slabs.
   // The words come from L2, so a role asks for the next tile's while it works on this one's.
+  // Work items: tiles, tile halves after the first `whole_tiles` of them, or (tile, split) pairs.
+  static_assert(!HALVES || (CG == 2 && BN == 256 && SK == kNoSplit && !TP), "halved tiles");
+  const int total_tiles = p.tiles_m * p.tiles_n;
+  const int S = SK ? p.splits : 1;
+  const int total_work = HALVES ? 2 * total_tiles - p.whole_tiles : total_tiles * S;
+  auto is_half = [&](int work) -> bool { return HALVES && work >= p.whole_tiles; };
+  auto tile_of = [&](int work) -> int { return SK ? work / S : is_half(work) ? (work + p.whole_tiles) >> 1 : work; };
   auto lora_words = [&](int work) -> uint32_t {
-    if (!kBf16 || p.R == 0 || p.la_flags == nullptr || work >= p.tiles_m * p.tiles_n * (SK ? p.splits : 1)) return 1u;
+    if (!kBf16 || p.R == 0 || p.la_flags == nullptr || work >= total_work) return 1u;
     constexpr int kWords = CG * BM / 32;
-    return lane < kWords ? __ldg(p.la_flags + (SK ? work / p.splits : work) % p.tiles_m * kWords + lane) : 0u;
+    return lane < kWords ? __ldg(p.la_flags + tile_of(work) % p.tiles_m * kWords + lane) : 0u;
   };
   auto lora_fp16 = [&](uint32_t words) -> bool { return kBf16 && __all_sync(0xffffffffu, words == 0u) != 0; };
   auto lora_parts = [&](bool fp16_pass) -> int { return (kBf16 && !fp16_pass) ? 2 : 1; };
-  const int total_tiles = p.tiles_m * p.tiles_n;
   const int k_groups4 = p.K / 64;            // scale atoms along K
-  // Work items: tiles, or (tile, split) pairs numbered tile-major so that the CTAs sharing a tile run
-  // at the same time.  Split i of a tile with n slabs (LoRA slabs of one pass included, at the end) takes slabs
+  // (tile, split) pairs are numbered tile-major so that the CTAs sharing a tile run at the same time.  Split i of a tile with n slabs (LoRA slabs of one pass included, at the end) takes slabs
   // [i n / S, (i + 1) n / S); a second LoRA pass is the last split's.  So where a range begins, and all of it before the
   // LoRA slabs, does not depend on the number of passes, and no role waits for the words before its first slab.
-  const int S = SK ? p.splits : 1;
-  const int total_work = total_tiles * S;
   auto slab_range = [&](int split, int& lo, int& hi) {
     const int n = kt_main + lora_slabs;
     if (SK) { lo = split * n / S; hi = (split + 1) * n / S; } else { lo = 0; hi = n; }
@@ -404,10 +410,13 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (!waited) { pdl_wait(); words = lora_words(pair); waited = true; }
     };
     for (int w = pair; w < total_work && ok; w += num_pairs) {
-      const int tile = SK ? w / S : w, split = SK ? w - tile * S : 0;
+      const int tile = tile_of(w), split = SK ? w - tile * S : 0;
       const int mb = tile % p.tiles_m, nb = tile / p.tiles_m;
       const int m0 = (mb * CG + rank) * BM;
-      const int nrow0 = nb * BN + static_cast<int>(rank) * C::B_ROWS;
+      // a half: 128 columns, half of them this CTA's rows of B
+      const bool half = is_half(w);
+      const int hsel = half ? (w - p.whole_tiles) & 1 : 0;
+      const int nrow0 = nb * BN + hsel * (BN / 2) + static_cast<int>(rank) * (half ? C::B_ROWS / 2 : C::B_ROWS);
       int kt_lo, kt_hi;
       slab_range(split, kt_lo, kt_hi);
       // The number of LoRA passes: of the first tile only when its first LoRA slab is due (unless they are interleaved).
@@ -430,13 +439,18 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (!uwait(&empty[s], ph, ctx, kDevWaitEmpty, it)) { ok = false; break; }
           if (it == C::STAGES) pdl_trigger();       // the first stage has been consumed: see pdl_trigger
           uint8_t* st = smem + s * C::STAGE_BYTES;
+          // the barrier that counts this CTA's bytes: its own for CG = 1, the leader's for a pair
+          const uint32_t bar = (CG == 2) ? map_to_cta(smem_u32(&full[s]), leader) : smem_u32(&full[s]);
           // Codes past K are zero-filled by TMA.  The scale atoms of a (128-row block, slab) are four
           // consecutive 512-byte rows of the swizzled scale buffer seen as a [blocks * K/64, 512 B] matrix;
           // a short last slab just fetches (and never uses) the rows that follow.  Every byte of a box
           // counts toward the barrier whether it was in bounds or not.
-          constexpr uint32_t kSfBytes = SFA_BYTES + C::SFB_BYTES, kAbBytes = A_BYTES + C::B_BYTES;
-          // the barrier that counts this CTA's bytes: its own for CG = 1, the leader's for a pair
-          const uint32_t bar = (CG == 2) ? map_to_cta(smem_u32(&full[s]), leader) : smem_u32(&full[s]);
+          const uint32_t kSfBytes = SFA_BYTES + (half ? C::SFB_BYTES / 2 : C::SFB_BYTES), kAbBytes = A_BYTES + (half ? C::B_BYTES / 2 : C::B_BYTES);
+          // B rows: one box, or with HALVES two, of which a half takes one
+          auto load_b = [&](const CUtensorMap* m, int x) {
+            tma_load_2d_bar<CG>(st + A_BYTES, m, x, nrow0, bar);
+            if (HALVES && !half) tma_load_2d_bar<CG>(st + A_BYTES + C::B_BYTES / 2, m, x, nrow0 + C::B_ROWS / 2, bar);
+          };
           wait_ahead();
           if (elect_one()) {
             if (kt < kt_main) {
@@ -444,20 +458,21 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               tma_load_2d_bar<CG>(st + A_BYTES + C::B_BYTES, &tmSFA, 0, (mb * CG + rank) * k_groups4 + kt * 4, bar);
 #pragma unroll
               for (int h = 0; h < BN / 128; ++h)
-                tma_load_2d_bar<CG>(st + A_BYTES + C::B_BYTES + SFA_BYTES + h * 2048, &tmSFB, 0,
-                                    (nb * (BN / 128) + h) * k_groups4 + kt * 4, bar);
+                if (h == 0 || !half)
+                  tma_load_2d_bar<CG>(st + A_BYTES + C::B_BYTES + SFA_BYTES + h * 2048, &tmSFB, 0,
+                                      (nb * (BN / 128) + hsel + h) * k_groups4 + kt * 4, bar);
               tma_load_2d_bar<CG>(st, &tmA, kt * 128, m0, bar);
-              tma_load_2d_bar<CG>(st + A_BYTES, &tmB, kt * 128, nrow0, bar);
+              load_b(&tmB, kt * 128);
             } else {
               if (rank == 0) mbar_arrive_expect_tx(&full[s], kAbBytes * CG);
               const int lt = kt - kt_main;
               const int part = lt / lora_slabs, r0 = (lt % lora_slabs) * 64;
               if (la_fp16) {
                 tma_load_2d_bar<CG>(st, &tmLAf, r0, m0, bar);
-                tma_load_2d_bar<CG>(st + A_BYTES, &tmLUf, r0, nrow0, bar);
+                load_b(&tmLUf, r0);
               } else {
                 tma_load_2d_bar<CG>(st, &tmLA, r0, part * p.M + m0, bar);    // lora_act parts are stacked along rows
-                tma_load_2d_bar<CG>(st + A_BYTES, &tmLU, r0, nrow0, bar);
+                load_b(&tmLU, r0);
               }
             }
           }
@@ -473,7 +488,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (rank == 0) {
       constexpr uint64_t kDescAB = smem_desc_base(0, 1024, kSwizzle128B);   // K-major, 8-row groups 1024 B apart
       constexpr uint64_t kDescSF = smem_desc_base(0, 128, kSwizzleNone);    // 8 x 16 B core matrices, 128 B apart
-      constexpr uint32_t kIdescMain = idesc_nvfp4(BM * CG, BN);
+      constexpr uint32_t kIdescHalf = (BN / 2 >> 3) << 17;      // off a descriptor's columns for a half tile
       constexpr uint32_t kIdescLora = idesc_f16(kBf16, kBf16, BM * CG, BN, false, false);
       constexpr uint32_t kIdescLoraF16 = idesc_f16(false, false, BM * CG, BN, false, false);
       const uint16_t mask = static_cast<uint16_t>((CG == 2 ? 3u : 1u) << leader);     // both CTAs of the pair
@@ -486,7 +501,8 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       pdl_wait();
       uint32_t words = lora_words(pair);
       for (int w = pair; w < total_work && ok; w += num_pairs, ++tcount) {
-        const int tile = SK ? w / S : w, split = SK ? w - tile * S : 0;
+        const int split = SK ? w - tile_of(w) * S : 0;
+        const bool half = is_half(w);
         const uint32_t as = tcount & 1;
         int kt_lo, kt_hi;
         slab_range(split, kt_lo, kt_hi);
@@ -523,24 +539,29 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               if (kt < kt_main) {
                 const uint64_t dsa = kDescSF + stage16 + (A_BYTES + C::B_BYTES) / 16, dsb = dsa + SFA_BYTES / 16;
                 const uint32_t tsfa = tmem_sf + sb * C::SF_COLS, tsfb = tsfa + C::SFA_COLS;
-                // the slab's k-blocks: all their scales, then their MMAs
-                auto k_blocks = [&](int nkb) {
+                // the slab's k-blocks: all their scales, then their MMAs (a tile's columns, or a half's)
+                auto k_blocks = [&](int nkb, auto cols) {
+                  constexpr int COLS = decltype(cols)::value;
 #pragma unroll
                   for (int j = 0; j < 4; ++j)
                     if (j < nkb) {
                       tmem_cp_scales<CG>(tsfa + j * 4, dsa + j * 32);
 #pragma unroll
-                      for (int h = 0; h < BN / 128; ++h) tmem_cp_scales<CG>(tsfb + j * (BN / 32) + h * 4, dsb + h * 128 + j * 32);
+                      for (int h = 0; h < COLS / 128; ++h) tmem_cp_scales<CG>(tsfb + j * (BN / 32) + h * 4, dsb + h * 128 + j * 32);
                     }
 #pragma unroll
                   for (int j = 0; j < 4; ++j)
                     if (j < nkb)
-                      mma_nvfp4<CG>(acc, da + j * 2, db + j * 2, kIdescMain, tsfa + j * 4, tsfb + j * (BN / 32), j != 0 ? 1u : accumulate);
+                      mma_nvfp4<CG>(acc, da + j * 2, db + j * 2, idesc_nvfp4(BM * CG, COLS), tsfa + j * 4, tsfb + j * (BN / 32), j != 0 ? 1u : accumulate);
                 };
                 const int nkb = k_groups4 - kt * 4;
-                if (nkb >= 4) k_blocks(4); else k_blocks(nkb);      // the last slab may be short
+                const std::integral_constant<int, BN> all_cols;
+                const std::integral_constant<int, HALVES ? BN / 2 : BN> half_cols;
+                if (HALVES && half) k_blocks(nkb >= 4 ? 4 : nkb, half_cols);
+                else if (nkb >= 4) k_blocks(4, all_cols);
+                else k_blocks(nkb, all_cols);                       // the last slab may be short
               } else {
-                const uint32_t idesc = la_fp16 ? kIdescLoraF16 : kIdescLora;
+                const uint32_t idesc = (la_fp16 ? kIdescLoraF16 : kIdescLora) - (half ? kIdescHalf : 0u);
                 const int nkb = (p.R - ((kt - kt_main) % lora_slabs) * 64) / 16;
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
@@ -567,13 +588,15 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     bool ok = true, drained = false;
     pdl_wait();
     for (int w = pair; w < total_work && ok; w += num_pairs, ++tcount) {
-      const int tile = SK ? w / S : w, split = SK ? w - tile * S : 0;
+      const int tile = tile_of(w), split = SK ? w - tile * S : 0;
       const int mb = tile % p.tiles_m, nb = tile / p.tiles_m;
-      const int m0 = (mb * CG + rank) * BM, n0 = nb * BN;
+      const bool half_tile = is_half(w);
+      const int cols = half_tile ? BN / 2 : BN;
+      const int m0 = (mb * CG + rank) * BM, n0 = nb * BN + (half_tile ? ((w - p.whole_tiles) & 1) * (BN / 2) : 0);
       const uint32_t as = tcount & 1, aph = (tcount >> 1) & 1;
       // stage this tile's per-column affine terms (the previous tile's readers are past the barrier below)
       [[maybe_unused]] bool odd_smooth = false;     // NEXT: some smooth_next of this tile is outside [2^-20, 2^20]
-      for (int c = threadIdx.x; c < BN; c += EPI_WARPS * 32) {
+      for (int c = threadIdx.x; c < cols; c += EPI_WARPS * 32) {
         affine[c] = wc != nullptr ? as_f32<OutT>(wc[n0 + c]) : 1.0f;
         affine[BN + c] = bias != nullptr ? as_f32<OutT>(bias[n0 + c]) : 0.0f;
         if constexpr (NEXT) {
@@ -707,9 +730,9 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       tc_fence_after_sync();
       const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
 #pragma unroll 1
-      for (int q = 0; q < BN / 128; ++q) {
+      for (int q = 0; q < cols / 128; ++q) {
       // A 256-column tile's shared half first: the next tile is waiting for those columns.
-      const int half = C::SHARED_ACC ? (q == 0 ? 1 - static_cast<int>(as) : static_cast<int>(as)) : 0;
+      const int half = C::SHARED_ACC && !half_tile ? (q == 0 ? 1 - static_cast<int>(as) : static_cast<int>(as)) : 0;
       const int cbase = half * 128 + chalf * 64;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + as * 128 + cbase;
       // Drain: the strip goes to registers in one burst, its columns are handed back at once, and only then do the
@@ -724,7 +747,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           uint64_t* bar = (C::SHARED_ACC && q == 0) ? acc_shared : &acc_empty[as];
           if constexpr (CG == 2) mbar_arrive_cluster_relaxed(bar, leader); else mbar_arrive(bar);
         }
-      } else if (q == BN / 128 - 1 && SK != kClusterSplit) {
+      } else if (q == cols / 128 - 1 && SK != kClusterSplit) {
         // the last accumulator is in registers: nothing is left to hand back, and the tensor memory may go
         leave();
         drained = true;
@@ -900,23 +923,34 @@ bool gemm_supported(int M, int N, int K, int R) {
   return M > 0 && N > 0 && K > 0 && M % 128 == 0 && N % 128 == 0 && K % 64 == 0 && R >= 0 && R % 16 == 0;
 }
 
-template <int CG, int BN, typename OutT, int SK = gemm::kNoSplit, bool NEXT = false, bool TP = false>
+// 256-column pair tiles of a last round that leaves at least half of the pairs without one: they are worked on as two halves,
+// and the round takes 0.65 of a tile's time, the same sums in the same order.  Sustained, bf16, rank 64, 74 pairs:
+// 1536 x 3840 -> 3840 (16 tiles in the second round) 15.2 -> 14.2 us, 1024 x 3840 -> 5888 (18; 128-column tiles before) 16.2 ->
+// 15.0, 1280 x 6144 -> 5120 (26) 24.2 -> 22.7, 2048 x 512 -> 3072 (22) 7.9 -> 7.6, 4352 x 15360 -> 3840 (33 in the fourth)
+// 95.3 -> 93.6 in short runs, 109.8 -> 108.0 at the power cap.
+static int gemm_halved_tiles(long long tiles, long long pairs) {
+  const long long left = tiles % pairs;
+  return tiles > pairs && 2 * left <= pairs ? static_cast<int>(left) : 0;
+}
+
+template <int CG, int BN, typename OutT, int SK = gemm::kNoSplit, bool NEXT = false, bool TP = false, bool HALVES = false>
 static int launch_gemm_t(const void* act, const void* wgt, const void* sfa, const void* sfb, const void* la,
                          const void* lu, const void* lu_f16, const void* wc, const void* bias, void* y, int M, int N,
                          int K, int R, const GemmTp& tp, cudaStream_t stream, int splits = 1) {
   using C = gemm::Cfg<CG, BN, NEXT, TP>;
   constexpr bool kBf16 = std::is_same<OutT, __nv_bfloat16>::value;
+  constexpr int kBoxRows = HALVES ? C::B_ROWS / 2 : C::B_ROWS;
   CUtensorMap tmA, tmB, tmLA, tmLU, tmSFA, tmSFB, tmLAf, tmLUf;
   int rc;
   const uint64_t atoms_k = K / 64;
   if ((rc = make_tmap_2d(&tmSFA, sfa, 4, (M / 128) * atoms_k, 128, 512, 4, 128, kTmapSwizzleNone)) != SVDQ_OK) return rc;
   if ((rc = make_tmap_2d(&tmSFB, sfb, 4, (N / 128) * atoms_k, 128, 512, 4, 128, kTmapSwizzleNone)) != SVDQ_OK) return rc;
   if ((rc = make_tmap_2d(&tmA, act, 1, M, K / 2, K / 2, gemm::BM, 128, kTmapSwizzle128)) != SVDQ_OK) return rc;
-  if ((rc = make_tmap_2d(&tmB, wgt, 1, N, K / 2, K / 2, C::B_ROWS, 128, kTmapSwizzle128)) != SVDQ_OK) return rc;
+  if ((rc = make_tmap_2d(&tmB, wgt, 1, N, K / 2, K / 2, kBoxRows, 128, kTmapSwizzle128)) != SVDQ_OK) return rc;
   if (R > 0) {
     const uint64_t la_rows = static_cast<uint64_t>(M) * (std::is_same<OutT, __nv_bfloat16>::value ? 2 : 1);
     if ((rc = make_tmap_2d(&tmLA, la, 2, la_rows, R, static_cast<uint64_t>(R) * 2, gemm::BM, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
-    if ((rc = make_tmap_2d(&tmLU, lu, 2, N, R, static_cast<uint64_t>(R) * 2, C::B_ROWS, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
+    if ((rc = make_tmap_2d(&tmLU, lu, 2, N, R, static_cast<uint64_t>(R) * 2, kBoxRows, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
   } else {
     tmLA = tmA; tmLU = tmB;
   }
@@ -928,7 +962,7 @@ static int launch_gemm_t(const void* act, const void* wgt, const void* sfa, cons
     const size_t plane = static_cast<size_t>(M) * R;
     const void* la_f16 = static_cast<const uint16_t*>(la) + 2 * plane;
     if ((rc = make_tmap_2d(&tmLAf, la_f16, 2, M, R, static_cast<uint64_t>(R) * 2, gemm::BM, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
-    if ((rc = make_tmap_2d(&tmLUf, lu_f16, 2, N, R, static_cast<uint64_t>(R) * 2, C::B_ROWS, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
+    if ((rc = make_tmap_2d(&tmLUf, lu_f16, 2, N, R, static_cast<uint64_t>(R) * 2, kBoxRows, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
     p.la_flags = lora16_flags(la, plane);
   }
   p.wc = wc; p.bias = bias;
@@ -959,7 +993,7 @@ static int launch_gemm_t(const void* act, const void* wgt, const void* sfa, cons
   p.qout = static_cast<uint8_t*>(tp.qout);
   p.oscales = static_cast<uint8_t*>(tp.oscales);
   p.oscales_swz = static_cast<uint8_t*>(tp.oscales_swz);
-  auto kern = gemm::gemm_w4a4_kernel<CG, BN, OutT, SK, NEXT, TP>;
+  auto kern = gemm::gemm_w4a4_kernel<CG, BN, OutT, SK, NEXT, TP, HALVES>;
   // the attribute is per device: remember which devices of this process have it
   static bool configured[64] = {};
   int dev = 0;
@@ -969,8 +1003,10 @@ static int launch_gemm_t(const void* act, const void* wgt, const void* sfa, cons
     if (SK == gemm::kClusterSplit && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return SVDQ_ERR_LAUNCH;
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  const int tiles = p.tiles_m * p.tiles_n * p.splits;
   const int max_pairs = sm_count() / CG;
+  p.whole_tiles = p.tiles_m * p.tiles_n;
+  if (HALVES) p.whole_tiles -= gemm_halved_tiles(p.whole_tiles, max_pairs);
+  const int tiles = p.tiles_m * p.tiles_n * p.splits;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(pairs * CG, 1, 1);
@@ -992,6 +1028,10 @@ template <typename OutT, bool NEXT, bool TP>
 static int launch_gemm_dt(int cg, int bn, const void* act, const void* wgt, const void* sfa, const void* sfb,
                           const void* la, const void* lu, const void* lu_f16, const void* wc, const void* bias, void* y,
                           int M, int N, int K, int R, const GemmTp& tp, cudaStream_t stream) {
+  if constexpr (!TP) {
+    if (cg == 2 && bn == 256 && gemm_halved_tiles(static_cast<long long>(M / 256) * (N / 256), sm_count() / 2) > 0)
+      return launch_gemm_t<2, 256, OutT, gemm::kNoSplit, NEXT, TP, true>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
+  }
   if (cg == 2 && bn == 256) return launch_gemm_t<2, 256, OutT, gemm::kNoSplit, NEXT, TP>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
   if (cg == 2 && bn == 128) return launch_gemm_t<2, 128, OutT, gemm::kNoSplit, NEXT, TP>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
   if (cg == 1 && bn == 256) return launch_gemm_t<1, 256, OutT, gemm::kNoSplit, NEXT, TP>(act, wgt, sfa, sfb, la, lu, lu_f16, wc, bias, y, M, N, K, R, tp, stream);
@@ -1143,10 +1183,9 @@ int launch_gemm_w4a4(const void* act, const void* wgt, const void* ascales_swz, 
     // a tile.  A 128-column tile takes more than half of a 256-column one, for it moves more operand bytes per flop:
     // 0.65 of it for a pair (one round at 256 x 15360 x 3840 16.3 / 24.8 us, at 256 x 3840 x 3072 6.3 / 9.2), 0.84 for a
     // single CTA (21.3 / 25.5).  So narrow tiles where both widths take one round, and with pairs where three narrow
-    // rounds replace two wide ones that the second leaves half empty: 1024 x 3840 x 5888 13.1 / 14.5 us, 1536 x 3840 x
-    // 3840 13.1 / 14.6, 1536 x 1280 x 3840 9.1 / 9.5, with the next layer's codes 18.8 / 21.5 and 15.7 / 17.5.  Further up
-    // the line is flat: two rounds against one 9.73 / 9.83 (1024 x 3840 x 3072), five against three 21.2 / 20.2 (3072 x
-    // 3840 x 3840).  The column-sharded form stores through shared memory, which narrow tiles do more often: three rounds
+    // rounds replace two wide ones of which the second is more than half empty, but not a round that can be halved
+    // (gemm_halved_tiles; it counts as a narrow one).  Further up the line is flat: two rounds against one 9.73 / 9.83
+    // (1024 x 3840 x 3072), five against three 21.2 / 20.2 (3072 x 3840 x 3840).  The column-sharded form stores through shared memory, which narrow tiles do more often: three rounds
     // against two 14.9 / 14.4 (1536 x 3840 x 3840), 31.6 / 29.4 (4352 x 10240 x 1536).
     cg = M % 256 == 0 ? 2 : 1;
     const long long units = sm_count() / cg;
@@ -1155,7 +1194,8 @@ int launch_gemm_w4a4(const void* act, const void* wgt, const void* ascales_swz, 
     for (int b : {256, 128}) {
       if (N % b != 0) continue;
       const long long tiles = static_cast<long long>(M / (128 * cg)) * (N / b);
-      const double cost = static_cast<double>((tiles + units - 1) / units) * (b == 256 ? 1.0 : tp.y_ld > 0 ? 0.72 : cg == 2 ? 0.65 : 0.84);
+      double cost = static_cast<double>((tiles + units - 1) / units) * (b == 256 ? 1.0 : tp.y_ld > 0 ? 0.72 : cg == 2 ? 0.65 : 0.84);
+      if (b == 256 && cg == 2 && tp.y_ld <= 0 && gemm_halved_tiles(tiles, units) > 0) cost -= 0.35;
       if (cost < best) { best = cost; bn = b; }
     }
   } else if (variant == 128 || variant == 256) {
