@@ -135,6 +135,11 @@ struct PeerMaps {
   CUtensorMap y, m[7];
 };
 struct NoMaps {};
+// bf16: tensor maps of lora_act's fp16 plane and of lora_up's fp16 copy.  (fp16 kernels do without: a launch costs the host
+// 0.6 us per KB of parameters.)
+struct LoraF16Maps {
+  CUtensorMap la, lu;
+};
 
 struct Params {
   void* y;              // [M, N] (column-sharded form: through the tensor maps instead)
@@ -260,7 +265,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmLA, const __grid_constant__ CUtensorMap tmLU,
                  const __grid_constant__ CUtensorMap tmSFA, const __grid_constant__ CUtensorMap tmSFB,
-                 const __grid_constant__ CUtensorMap tmLAf, const __grid_constant__ CUtensorMap tmLUf,
+                 const __grid_constant__ typename std::conditional<std::is_same<OutT, __nv_bfloat16>::value, LoraF16Maps, NoMaps>::type lora_f16,
                  const __grid_constant__ typename std::conditional<TP, PeerMaps, NoMaps>::type maps, const Params p) {
   using C = Cfg<CG, BN, NEXT, TP>;
   constexpr bool kBf16 = std::is_same<OutT, __nv_bfloat16>::value;
@@ -315,7 +320,9 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if constexpr (TP) tma_prefetch_desc(&maps.y);
     tma_prefetch_desc(&tmSFA); tma_prefetch_desc(&tmSFB);
     if (p.R > 0) { tma_prefetch_desc(&tmLA); tma_prefetch_desc(&tmLU); }
-    if (p.R > 0 && p.la_flags != nullptr) { tma_prefetch_desc(&tmLAf); tma_prefetch_desc(&tmLUf); }
+    if constexpr (kBf16) {
+      if (p.R > 0 && p.la_flags != nullptr) { tma_prefetch_desc(&lora_f16.la); tma_prefetch_desc(&lora_f16.lu); }
+    }
   }
   if constexpr (NEXT) qmath::fill_near_lut(scale_lut, threadIdx.x, NUM_THREADS);
   __syncthreads();
@@ -467,13 +474,13 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               if (rank == 0) mbar_arrive_expect_tx(&full[s], kAbBytes * CG);
               const int lt = kt - kt_main;
               const int part = lt / lora_slabs, r0 = (lt % lora_slabs) * 64;
-              if (la_fp16) {
-                tma_load_2d_bar<CG>(st, &tmLAf, r0, m0, bar);
-                load_b(&tmLUf, r0);
-              } else {
-                tma_load_2d_bar<CG>(st, &tmLA, r0, part * p.M + m0, bar);    // lora_act parts are stacked along rows
-                load_b(&tmLU, r0);
+              const CUtensorMap *la_map = &tmLA, *lu_map = &tmLU;
+              int la_row = part * p.M + m0;                                  // lora_act parts are stacked along rows
+              if constexpr (kBf16) {
+                if (la_fp16) { la_map = &lora_f16.la; lu_map = &lora_f16.lu; la_row = m0; }
               }
+              tma_load_2d_bar<CG>(st, la_map, r0, la_row, bar);
+              load_b(lu_map, r0);
             }
           }
           __syncwarp();
@@ -940,7 +947,8 @@ static int launch_gemm_t(const void* act, const void* wgt, const void* sfa, cons
   using C = gemm::Cfg<CG, BN, NEXT, TP>;
   constexpr bool kBf16 = std::is_same<OutT, __nv_bfloat16>::value;
   constexpr int kBoxRows = HALVES ? C::B_ROWS / 2 : C::B_ROWS;
-  CUtensorMap tmA, tmB, tmLA, tmLU, tmSFA, tmSFB, tmLAf, tmLUf;
+  CUtensorMap tmA, tmB, tmLA, tmLU, tmSFA, tmSFB;
+  typename std::conditional<kBf16, gemm::LoraF16Maps, gemm::NoMaps>::type lora_f16;
   int rc;
   const uint64_t atoms_k = K / 64;
   if ((rc = make_tmap_2d(&tmSFA, sfa, 4, (M / 128) * atoms_k, 128, 512, 4, 128, kTmapSwizzleNone)) != SVDQ_OK) return rc;
@@ -956,14 +964,16 @@ static int launch_gemm_t(const void* act, const void* wgt, const void* sfa, cons
   }
   gemm::Params p;
   p.la_flags = nullptr;
-  tmLAf = tmLA; tmLUf = tmLU;
-  if (kBf16 && R > 0 && lu_f16 != nullptr) {
-    // bf16 form of lora_act: planes hi, lo, fp16, then the per-32-row flag words
-    const size_t plane = static_cast<size_t>(M) * R;
-    const void* la_f16 = static_cast<const uint16_t*>(la) + 2 * plane;
-    if ((rc = make_tmap_2d(&tmLAf, la_f16, 2, M, R, static_cast<uint64_t>(R) * 2, gemm::BM, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
-    if ((rc = make_tmap_2d(&tmLUf, lu_f16, 2, N, R, static_cast<uint64_t>(R) * 2, kBoxRows, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
-    p.la_flags = lora16_flags(la, plane);
+  if constexpr (kBf16) {
+    lora_f16.la = tmLA; lora_f16.lu = tmLU;
+    if (R > 0 && lu_f16 != nullptr) {
+      // bf16 form of lora_act: planes hi, lo, fp16, then the per-32-row flag words
+      const size_t plane = static_cast<size_t>(M) * R;
+      const void* la_f16 = static_cast<const uint16_t*>(la) + 2 * plane;
+      if ((rc = make_tmap_2d(&lora_f16.la, la_f16, 2, M, R, static_cast<uint64_t>(R) * 2, gemm::BM, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
+      if ((rc = make_tmap_2d(&lora_f16.lu, lu_f16, 2, N, R, static_cast<uint64_t>(R) * 2, kBoxRows, 64, kTmapSwizzle128)) != SVDQ_OK) return rc;
+      p.la_flags = lora16_flags(la, plane);
+    }
   }
   p.wc = wc; p.bias = bias;
   p.M = M; p.N = N; p.K = K; p.R = R;
@@ -1020,7 +1030,7 @@ static int launch_gemm_t(const void* act, const void* wgt, const void* sfa, cons
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  if (cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmLA, tmLU, tmSFA, tmSFB, tmLAf, tmLUf, maps, p) != cudaSuccess) return SVDQ_ERR_LAUNCH;
+  if (cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmLA, tmLU, tmSFA, tmSFB, lora_f16, maps, p) != cudaSuccess) return SVDQ_ERR_LAUNCH;
   return SVDQ_OK;
 }
 
