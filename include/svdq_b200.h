@@ -160,6 +160,11 @@ int svdq_cast_lora_act(const float* src, void* dst, int rows, int R, int dtype, 
  * multiplies bf16 lora_act by bf16 lora_up in one pass and accepts the 7e-3 error of that. */
 int svdq_lora_up_to_f16(const void* lora_up_bf16_host, void* out_f16_host, long long count);
 
+/* The same on the device, asynchronously on `stream`.  unfit: SVDQ_LORA_UP_WORDS words in device memory,
+ * all written; the output is unusable if any of them is non-zero afterwards. */
+enum { SVDQ_LORA_UP_WORDS = 148 };
+int svdq_lora_up_to_f16_device(const void* lora_up_bf16, void* out_f16, unsigned int* unfit, long long count, void* stream);
+
 /*
  * W4A4 GEMM + LoRA-up + per-column affine.
  * Stands in for launch_v2(act, wgt, ascales, wscales, lora_act_in, lora_up, wcscales, bias, out_dtype)

@@ -16,6 +16,7 @@ LIB_PATH = os.path.join(_PKG_DIR, "libsvdq_b200.so")
 DTYPE_F16, DTYPE_BF16, DTYPE_F32 = 0, 1, 2
 QUANT_AUTO, QUANT_FORCE_GENERIC, QUANT_FORCE_FUSED, QUANT_FORCE_STREAM = 0, 1, 2, 0x100000
 OK = 0
+LORA_UP_WORDS = 148
 GEMM_LORA_INTERLEAVE, GEMM_LORA_AT_END, GEMM_NO_SPLIT = 1 << 24, 1 << 25, 1 << 26
 
 # name -> (restype, argtypes); kept in the order of include/svdq_b200.h
@@ -35,6 +36,7 @@ SIGNATURES = {
     "svdq_lora_act16_elems": (c_longlong, [c_int, c_int, c_int]),
     "svdq_cast_lora_act": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "svdq_lora_up_to_f16": (c_int, [c_void_p, c_void_p, c_longlong]),
+    "svdq_lora_up_to_f16_device": (c_int, [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p]),
     "svdq_gemm_w4a4": (c_int, [c_void_p] * 10 + [c_int] * 6 + [c_void_p]),
     "svdq_gemm_w4a4_next": (c_int, [c_void_p] * 14 + [c_int] * 6 + [c_void_p]),
     "svdq_gemm_w4a4_workspace_bytes": (c_ulonglong, [c_int, c_int, c_int, c_int]),

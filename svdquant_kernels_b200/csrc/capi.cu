@@ -8,7 +8,6 @@
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
-#include <vector>
 
 #include "nvfp4_math.cuh"
 #include "sm100.cuh"
@@ -175,6 +174,12 @@ int svdq_lora_up_to_f16(const void* lora_up_bf16_host, void* out_f16_host, long 
     dst[i] = __float2half_rn(v);
   }
   return SVDQ_OK;
+}
+
+int svdq_lora_up_to_f16_device(const void* lora_up_bf16, void* out_f16, unsigned int* unfit, long long count, void* stream) {
+  if (count < 0) return SVDQ_ERR_SHAPE;
+  if (unfit == nullptr || (count > 0 && (lora_up_bf16 == nullptr || out_f16 == nullptr))) return SVDQ_ERR_NULL;
+  return launch_lora_up_f16(lora_up_bf16, out_f16, unfit, count, static_cast<cudaStream_t>(stream));
 }
 
 int svdq_quantizer_max_active_clusters(int R, int k_split, int dtype) {
@@ -520,12 +525,14 @@ int svdq_linear_plan_create(svdq_linear_plan** out, int max_M, int K, int N, int
   if (rc == SVDQ_OK) rc = launch_swizzle_scales(wscales_dev, p->wscales_swz, K / 16, N, st);
   if (rc == SVDQ_OK) rc = dev_upload(&p->lora_down, lora_down_host, static_cast<size_t>(K) * R * 2, st);
   if (rc == SVDQ_OK) rc = dev_upload(&p->lora_up, lora_up_host, static_cast<size_t>(N) * R * 2, st);
-  std::vector<uint16_t> lu16;                      // must outlive the asynchronous upload below
+  // fp16 copy of a bf16 lora_up for the single-pass LoRA route (dropped below if a value does not fit)
+  unsigned int* unfit = nullptr;
+  unsigned int unfit_host[SVDQ_LORA_UP_WORDS] = {};
   if (rc == SVDQ_OK && dtype == SVDQ_DTYPE_BF16 && R > 0) {
-    // fp16 copy of a bf16 lora_up for the single-pass LoRA route (skipped if a value does not fit)
-    lu16.resize(static_cast<size_t>(N) * R);
-    if (svdq_lora_up_to_f16(lora_up_host, lu16.data(), static_cast<long long>(lu16.size())) == SVDQ_OK)
-      rc = dev_upload(&p->lora_up_f16, lu16.data(), lu16.size() * 2, st);
+    const size_t n = static_cast<size_t>(N) * R;
+    if (cudaMalloc(&p->lora_up_f16, n * 2) != cudaSuccess || cudaMalloc(&unfit, sizeof(unfit_host)) != cudaSuccess) rc = SVDQ_ERR_CUDA;
+    if (rc == SVDQ_OK) rc = launch_lora_up_f16(p->lora_up, p->lora_up_f16, unfit, static_cast<long long>(n), st);
+    if (rc == SVDQ_OK && cudaMemcpyAsync(unfit_host, unfit, sizeof(unfit_host), cudaMemcpyDeviceToHost, st) != cudaSuccess) rc = SVDQ_ERR_CUDA;
   }
   if (rc == SVDQ_OK) rc = dev_upload(&p->smooth, smooth_host, static_cast<size_t>(K) * 2, st);
   if (rc == SVDQ_OK && p->smooth != nullptr) {
@@ -536,6 +543,12 @@ int svdq_linear_plan_create(svdq_linear_plan** out, int max_M, int K, int N, int
   if (rc == SVDQ_OK) rc = dev_upload(&p->bias, bias_host, static_cast<size_t>(N) * 2, st);
   if (rc == SVDQ_OK && cudaStreamSynchronize(st) != cudaSuccess) rc = SVDQ_ERR_CUDA;
   if (wscales_dev != nullptr) cudaFree(wscales_dev);
+  if (unfit != nullptr) cudaFree(unfit);
+  for (unsigned int word : unfit_host)
+    if (rc == SVDQ_OK && word != 0 && p->lora_up_f16 != nullptr) {
+      cudaFree(p->lora_up_f16);
+      p->lora_up_f16 = nullptr;
+    }
   if (rc != SVDQ_OK) {
     svdq_linear_plan_destroy(p);
     return rc;

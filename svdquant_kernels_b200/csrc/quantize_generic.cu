@@ -219,6 +219,30 @@ __global__ void cast_lora16_kernel(const float* __restrict__ src, void* __restri
     store_lora16<T>(dst, static_cast<size_t>(i), static_cast<size_t>(n), src[i]);
 }
 
+// bf16 -> fp16, eight values a thread where both sides are 16-byte aligned; unfit[block]: some value of the block's is NaN or
+// beyond fp16's range.  Launched with SVDQ_LORA_UP_WORDS blocks.
+__global__ void __launch_bounds__(256)
+lora_up_f16_kernel(const __nv_bfloat16* __restrict__ src, __half* __restrict__ dst, uint32_t* __restrict__ unfit, long long n, int vec) {
+  bool bad = false;
+  auto one = [&](__nv_bfloat16 b) -> __half {
+    const float v = __bfloat162float(b);
+    bad |= !(fabsf(v) <= 65504.0f);
+    return __float2half_rn(v);
+  };
+  const long long at = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x, step = static_cast<long long>(gridDim.x) * blockDim.x;
+  const long long whole = vec ? n / 8 : 0;
+  for (long long i = at; i < whole; i += step) {
+    const uint4 in = reinterpret_cast<const uint4*>(src)[i];
+    uint4 out;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) reinterpret_cast<__half*>(&out)[j] = one(reinterpret_cast<const __nv_bfloat16*>(&in)[j]);
+    reinterpret_cast<uint4*>(dst)[i] = out;
+  }
+  for (long long i = whole * 8 + at; i < n; i += step) dst[i] = one(src[i]);
+  const int any = __syncthreads_or(bad ? 1 : 0);
+  if (threadIdx.x == 0) unfit[blockIdx.x] = any != 0 ? 1u : 0u;
+}
+
 static int grid_for(long long items, int block) {
   long long g = (items + block - 1) / block;
   const long long cap = 148ll * 16;
@@ -280,6 +304,12 @@ int launch_swizzle_scales(const void* src, void* dst, int groups, int rows, cuda
   const long long n = static_cast<long long>(groups) * rows;
   if (n == 0) return SVDQ_OK;
   swizzle_scales_kernel<<<grid_for(n, 256), 256, 0, stream>>>(static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), groups, rows);
+  return cudaGetLastError() == cudaSuccess ? SVDQ_OK : SVDQ_ERR_LAUNCH;
+}
+
+int launch_lora_up_f16(const void* src, void* dst, uint32_t* unfit, long long n, cudaStream_t stream) {
+  const int vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0 ? 1 : 0;
+  lora_up_f16_kernel<<<SVDQ_LORA_UP_WORDS, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(src), static_cast<__half*>(dst), unfit, n, vec);
   return cudaGetLastError() == cudaSuccess ? SVDQ_OK : SVDQ_ERR_LAUNCH;
 }
 

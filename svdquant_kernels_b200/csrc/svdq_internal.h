@@ -15,6 +15,7 @@ int launch_quantize_rows(const void* x, const void* smooth, void* codes, void* s
 int launch_lora_down(const void* x, const void* w, float* out, void* out16, int M, int M_pad, int K, int R, int dtype,
                      cudaStream_t stream);
 int launch_swizzle_scales(const void* src, void* dst, int groups, int rows, cudaStream_t stream);
+int launch_lora_up_f16(const void* src, void* dst, uint32_t* unfit, long long n, cudaStream_t stream);
 int launch_cast_f32(const float* src, void* dst, int rows, int R, int dtype, cudaStream_t stream);
 
 // quantize_fused.cu

@@ -286,12 +286,16 @@ def _lora_up_f16(lora_up: torch.Tensor) -> Optional[torch.Tensor]:
     twin = _attached(lora_up)
     if twin is not None:
         return twin if twin.numel() else None
-    host = lora_up.detach().cpu().contiguous()
-    out = torch.empty(host.shape, dtype=torch.float16)
-    rc = _lib.load().svdq_lora_up_to_f16(_ptr(host), _ptr(out), host.numel())
-    dev_copy = out.to(lora_up.device) if rc == _lib.OK else torch.empty(0, dtype=torch.float16, device=lora_up.device)
-    _attach(lora_up, dev_copy)
-    return dev_copy if dev_copy.numel() else None
+    src = lora_up.detach().contiguous()
+    copy = torch.empty(src.shape, dtype=torch.float16, device=src.device)
+    unfit = torch.empty(_lib.LORA_UP_WORDS, dtype=torch.int32, device=src.device)
+    with _on_device(src.device):
+        rc = _lib.load().svdq_lora_up_to_f16_device(_ptr(src), _ptr(copy), _ptr(unfit), src.numel(), _stream(src.device))
+    _lib.check(rc, "lora_up_to_f16_device")
+    if unfit.cpu().any():
+        copy = torch.empty(0, dtype=torch.float16, device=src.device)
+    _attach(lora_up, copy)
+    return copy if copy.numel() else None
 
 
 def gemm_w4a4(
