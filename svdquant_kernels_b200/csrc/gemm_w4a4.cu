@@ -287,7 +287,8 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint64_t* tmem_ready = acc_shared + 1;                          // tensor memory allocated (leader's copy: in both CTAs)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_ready + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile uint32_t* sk_ticket = tmem_slot + 2;                   // split-K: the ticket this CTA drew for its tile
+  volatile uint32_t* sk_ticket = tmem_slot + 2;                   // split-K through a workspace: the ticket this CTA drew for its tile
+  [[maybe_unused]] volatile uint32_t* ahead_done = tmem_slot + 3; // split-K within clusters: the kernel ahead has finished
   const WaitCtx ctx{abort_flag};
   // bounded wait whose verdict is the same in all lanes of the calling (converged) warp
   auto uwait = [&](uint64_t* bar, uint32_t parity, const WaitCtx& c, unsigned int code, unsigned int tag) -> bool {
@@ -309,6 +310,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
+    *ahead_done = 0;
     for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], EPI_WARPS * CG); }
     mbar_init(acc_shared, EPI_WARPS * CG);
@@ -414,7 +416,12 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     uint32_t words = 1u;
     bool waited = false;
     auto wait_ahead = [&]() {
-      if (!waited) { pdl_wait(); words = lora_words(pair); waited = true; }
+      if (!waited) {
+        pdl_wait();
+        if (SK == kClusterSplit) *ahead_done = 1;
+        words = lora_words(pair);
+        waited = true;
+      }
     };
     for (int w = pair; w < total_work && ok; w += num_pairs) {
       const int tile = tile_of(w), split = SK ? w - tile * S : 0;
@@ -593,6 +600,25 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int quarter = warp & 3, chalf = warp >> 2;
     uint32_t tcount = 0;
     bool ok = true, drained = false;
+    if (SK == kClusterSplit && warp == 0) {
+      // Long K loops over weights that come from DRAM: a CTA that is here while the kernel ahead is still at work (the quantizer
+      // leaves half of the SMs to half of these CTAs) asks for its slabs of them, into L2, until that has ended.  Not before a
+      // moment has passed, and at a pace, or the hints stand in the copy engine in front of the loads: without either, and in
+      // every form, 256 x 15360 -> 3840 took 25.3 us instead of 23.8 for both kernels; this way 22.4 instead of 22.8, 256 x
+      // 10240 -> 3072 16.1 instead of 16.2, while forms with a short K loop gain nothing (256 x 3840 -> 3072 11.7 -> 11.8).
+      __nanosleep(300);
+      const int tile = tile_of(pair), nb = tile / p.tiles_m;
+      int lo, hi;
+      slab_range(pair - tile * S, lo, hi);
+      for (int kt = lo; kt < hi && kt < kt_main && *ahead_done == 0; ++kt) {
+        if (elect_one()) {
+          tma_prefetch_2d(&tmB, kt * 128, nb * BN + static_cast<int>(rank) * C::B_ROWS);
+          if (rank == 0) tma_prefetch_2d(&tmSFB, 0, nb * (BN / 128) * k_groups4 + kt * 4);
+        }
+        __syncwarp();
+        __nanosleep(40);
+      }
+    }
     pdl_wait();
     for (int w = pair; w < total_work && ok; w += num_pairs, ++tcount) {
       const int tile = tile_of(w), split = SK ? w - tile * S : 0;
