@@ -165,7 +165,7 @@ Twin attached(const Tensor& owner, bool any_version = false) {
 }
 
 // A tensor on a storage of its own, without the checks and guards of at::empty: every caller has seen a tensor on the
-// current device `dev` already.  Five of these are most of a small quantizer call's host time.
+// current device `dev` already.  Four of these are most of a small quantizer call's host time.
 Tensor on_storage(c10::intrusive_ptr<c10::StorageImpl> st, at::IntArrayRef sizes, ScalarType t) {
   Tensor r = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(std::move(st)), c10::DispatchKeySet(c10::DispatchKey::CUDA),
                                                       c10::scalarTypeToTypeMeta(t));

@@ -20,7 +20,7 @@
 // shared memory; more: every rank's share of the tile): no atomics, no zero-fill, no scratch in global
 // memory.  Large inputs run with KS = 2; larger clusters are for inputs of
 // a few hundred to two thousand rows, where pairs would leave most SMs idle (256 x 10240:
-// 36.0 -> 6.3 us), and are taken only if all of them are resident at once.
+// 36.0 -> 5.8 us), and are taken only if all of them are resident at once.
 // (64-row tiles with pairs, not 128-row tiles with quads: a B200 keeps
 // at most 33 four-CTA clusters of this size resident, one short of the 34 row
 // tiles of a 4352-row activation, while 68 pairs fit in one wave.  128-row tiles
@@ -585,8 +585,8 @@ __global__ void smooth_table_kernel(const T* __restrict__ smooth, float* __restr
 // tile would leave most SMs idle; they are taken only if all of them can be resident at once (max_clusters(ks):
 // clusters of that size the device can hold; 33 of four CTAs, 22 of six, 15 of eight, 11 of ten, 7 of sixteen).
 // Cost in slabs (0.24 us); the constants are the ways of bringing the LoRA partial sums together, which hardly depend
-// on the cluster size (256 x 3840: 4 / 6 / 8 / 10 / 16 CTAs 8.3 / 7.2 / 6.5 / 6.3 / 5.9 us; 256 x 15360: 8 / 16 CTAs
-// 13.0 / 9.5 us; 1003 x 3840: 2 / 4 / 6 CTAs 10.0 / 7.3 / 6.5 us).
+// on the cluster size (256 x 3840: 4 / 6 / 8 / 10 / 16 CTAs 7.4 / 6.3 / 5.7 / 5.4 / 5.4 us; 256 x 15360: 8 / 16 CTAs
+// 11.2 / 8.6 us; 1003 x 3840: 2 / 4 / 6 CTAs 9.6 / 6.9 / 6.3 us, seven, which are not all resident, 10.9).
 template <typename MaxClusters>
 static int pick_k_split(int M_pad, int K, MaxClusters max_clusters) {
   const int tiles = M_pad / qf::TILE_M;
