@@ -367,9 +367,10 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   auto lora_fp16 = [&](uint32_t words) -> bool { return kBf16 && __all_sync(0xffffffffu, words == 0u) != 0; };
   auto lora_parts = [&](bool fp16_pass) -> int { return (kBf16 && !fp16_pass) ? 2 : 1; };
   const int k_groups4 = p.K / 64;            // scale atoms along K
-  // (tile, split) pairs are numbered tile-major so that the CTAs sharing a tile run at the same time.  Split i of a tile with n slabs (LoRA slabs of one pass included, at the end) takes slabs
-  // [i n / S, (i + 1) n / S); a second LoRA pass is the last split's.  So where a range begins, and all of it before the
-  // LoRA slabs, does not depend on the number of passes, and no role waits for the words before its first slab.
+  // (tile, split) pairs are numbered tile-major so that the CTAs sharing a tile run at the same time.  Split i of a
+  // tile with n slabs (LoRA slabs of one pass included, at the end) takes slabs [i n / S, (i + 1) n / S); a second LoRA
+  // pass is the last split's.  So where a range begins, and all of it before the LoRA slabs, does not depend on the
+  // number of passes, and no role waits for the words before its first slab.
   auto slab_range = [&](int split, int& lo, int& hi) {
     const int n = kt_main + lora_slabs;
     if (SK) { lo = split * n / S; hi = (split + 1) * n / S; } else { lo = 0; hi = n; }
@@ -1221,8 +1222,9 @@ int launch_gemm_w4a4(const void* act, const void* wgt, const void* ascales_swz, 
     // single CTA (21.3 / 25.5).  So narrow tiles where both widths take one round, and with pairs where three narrow
     // rounds replace two wide ones of which the second is more than half empty, but not a round that can be halved
     // (gemm_halved_tiles; it counts as a narrow one).  Further up the line is flat: two rounds against one 9.73 / 9.83
-    // (1024 x 3840 x 3072), five against three 21.2 / 20.2 (3072 x 3840 x 3840).  The column-sharded form stores through shared memory, which narrow tiles do more often: three rounds
-    // against two 14.9 / 14.4 (1536 x 3840 x 3840), 31.6 / 29.4 (4352 x 10240 x 1536).
+    // (1024 x 3840 x 3072), five against three 21.2 / 20.2 (3072 x 3840 x 3840).  The column-sharded form stores
+    // through shared memory, which narrow tiles do more often: three rounds against two 14.9 / 14.4 (1536 x 3840 x
+    // 3840), 31.6 / 29.4 (4352 x 10240 x 1536).
     cg = M % 256 == 0 ? 2 : 1;
     const long long units = sm_count() / cg;
     double best = 1e30;
