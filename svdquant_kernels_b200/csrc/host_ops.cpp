@@ -188,21 +188,7 @@ Twin empty_twin(int64_t numel, ScalarType t) {
   void* const ptr = st->mutable_data();
   return Twin{ptr, t, numel, Tensor(), std::move(st)};
 }
-// Both twins of a quantizer call in one storage, which goes with the later of their owners
-void empty_twins(Twin& a, int64_t a_numel, ScalarType a_type, Twin& b, int64_t b_numel, ScalarType b_type) {
-  const int64_t b_at = (a_numel * static_cast<int64_t>(c10::elementSize(a_type)) + 511) / 512 * 512;
-  auto st = new_storage(b_at + b_numel * static_cast<int64_t>(c10::elementSize(b_type)), at::kByte);
-  char* const ptr = static_cast<char*>(st->mutable_data());
-  a = Twin{ptr, a_type, a_numel, Tensor(), st};
-  b = Twin{ptr + b_at, b_type, b_numel, Tensor(), std::move(st)};
-}
-Tensor tensor_of(const Twin& twin) {
-  if (twin.hold.defined()) return twin.hold;
-  Tensor t = on_storage(twin.hold_storage, {twin.numel}, twin.type);
-  const auto at = static_cast<const char*>(twin.ptr) - static_cast<const char*>(twin.hold_storage->data());
-  t.unsafeGetTensorImpl()->set_storage_offset(at / static_cast<int64_t>(c10::elementSize(twin.type)));
-  return t;
-}
+Tensor tensor_of(const Twin& twin) { return twin.hold.defined() ? twin.hold : on_storage(twin.hold_storage, {twin.numel}, twin.type); }
 
 // Record `twin` as the derived form of `owner`'s current contents.  GIL held; false with a Python error set.
 bool attach(const Tensor& owner, const Twin& twin) {
@@ -280,11 +266,9 @@ bool quantize(const Tensor& x, const Tensor& ld, const Tensor& smooth, int64_t p
     out.ascales = empty_output(K / 16, Mp, at::kFloat8_e4m3fn);
     out.lora_act = R > 0 ? empty_output(Mp, R, at::kFloat) : empty({Mp, R}, at::kFloat);
   }
-  const bool new_swz = want_swz && !swz.found(), new_la16 = R > 0 && !la16.found();
-  const int64_t la16_elems = new_la16 ? svdq_lora_act16_elems(static_cast<int>(Mp), static_cast<int>(R), dtype_code(t)) : 0;
-  if (new_swz && new_la16) empty_twins(la16, la16_elems, t, swz, Mp * (K / 16), at::kByte);
-  else if (new_swz) swz = empty_twin(Mp * (K / 16), at::kByte);
-  else if (new_la16) la16 = empty_twin(la16_elems, t);
+  // (a storage each: one kept by the scales would keep lora_act's planes too)
+  if (want_swz && !swz.found()) swz = empty_twin(Mp * (K / 16), at::kByte);
+  if (R > 0 && !la16.found()) la16 = empty_twin(svdq_lora_act16_elems(static_cast<int>(Mp), static_cast<int>(R), dtype_code(t)), t);
   void* const stream = c10::cuda::getCurrentCUDAStream(dev).stream();
   auto ptr = [](const Tensor& v) -> void* { return v.defined() && v.numel() > 0 ? v.data_ptr() : nullptr; };
   int rc;

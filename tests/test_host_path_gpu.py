@@ -88,6 +88,26 @@ def test_outputs_have_storages_of_their_own(M, K, dtype):
         del act
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,K", [(64, 128), (300, 512)])
+def test_a_kept_output_keeps_its_own_twin_only(M, K, dtype):
+    """An output that outlives the others of its call holds its own bytes and those of its own twin: the scales do not keep
+    the planes of lora_act, nor lora_act the scales' second form, nor the codes either."""
+    from svdquant_kernels_b200 import ops, torch_ops  # noqa: F401
+    x, sm, ld, *_ = _layer(dtype, M=M, K=K)
+    nbytes = lambda t: 0 if t is None else t.numel() * t.element_size()
+    held = lambda: torch.cuda.memory_stats()["requested_bytes.all.current"]
+    for call in (ops.quantize_w4a4_act_fuse_lora, torch.ops.svdq_b200.quantize_w4a4_act_fuse_lora):
+        call(x, ld, sm)                                        # makes the smooth table
+        for kept in range(3):
+            before = held()
+            out = call(x, ld, sm)[kept]
+            twin = ops._attached(out)
+            assert (twin is None) == (kept == 0)
+            assert held() - before == nbytes(out) + nbytes(twin), kept
+            del out, twin
+
+
 def test_out_tensors_that_change_type_keep_their_twins_right():
     """The outputs' own types do not depend on the input's, so a call may write into those of a call of the other type:
     the 16-bit form of lora_act that the GEMM reads is then the last call's, in either order."""
