@@ -69,16 +69,18 @@ struct Cfg {
   static constexpr int W_BYTES = SLAB_K * RP * 2;                 // lora_down slab
   // Six lora_down stages: a slab comes out of L2 in about 1.7 us while x streams in beside it, and slabs pass at
   // 0.3 us (2 / 4 / 6 / 8 stages, 4352 rows: K = 3840 22.0 / 16.2 / 14.9 / 15.6 us, K = 10240 42.5 / 30.3 / 29.0 / 29.5);
-  // at rank 256 three are what fits, two beside the larger receive buffer of PUSH.
-  static constexpr int W_STAGES = RP > 128 ? (PUSH ? 2 : 3) : 6;
+  // at rank 256 three are what fits.
+  static constexpr int W_STAGES = RP > 128 ? 3 : 6;
   // MMA-issuing warps.  Two take the slabs by turns; then both rings must be even, so that an issuer meets only slabs
   // of its own in a stage: one that went on to slab i could otherwise look at the stage while slab i - W_STAGES,
   // the other issuer's, is still on its way into it, and a one-bit parity would tell it that slab i is there.
   static constexpr int ISSUERS = W_STAGES % 2 == 0 ? 2 : 1;
   static constexpr int W_RING_BYTES = W_STAGES * W_BYTES;
-  // Receive buffer for partial sums: of the peer for this CTA's 32 rows (two K ranks), of all ranks for this CTA's share
-  // of the tile (PUSH; shares are rounded up to whole float4s)
-  static constexpr int RECV_BYTES = PUSH ? TILE_M * RP * 4 + kMaxKSplit * 16 : (TILE_M / 2) * RP * 4;
+  // Receive buffer for partial sums: of the peer for this CTA's 32 rows (two K ranks), of the other ranks for this CTA's
+  // share of the tile (PUSH; shares are rounded up to whole float4s).  With room for this rank's own part too the x ring lost a
+  // third of its stages at rank 128 and the lora_down ring one of three above it: rank 256, fp16, 512 x 10240 14.2 us instead
+  // of 11.9, 1003 x 3840 10.4 / 9.6, 2000 x 15360 43.3 / 34.0; rank 128, 2000 x 10240 16.4 / 16.1, elsewhere the same.
+  static constexpr int RECV_BYTES = PUSH ? TILE_M * RP * 4 / kMaxKSplit * (kMaxKSplit - 1) + kMaxKSplit * 16 : (TILE_M / 2) * RP * 4;
   static constexpr int STAGES_RAW = (232448 - 1024 - 512 - RECV_BYTES - W_RING_BYTES) / (X_BYTES + TB_BYTES);
   // A multiple of the group count: a group then always meets the same stages, and the slab it waits
   // for is the direct successor (in that stage) of one it consumed itself.  A one-bit phase parity
@@ -96,6 +98,9 @@ struct Cfg {
   static_assert(PUSH || 2 * RECV_BYTES <= W_RING_BYTES, "the exchange stages both halves of the accumulator in the lora_down ring");
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 };
+template <int RP> constexpr bool kPushKeepsTheRings =
+    Cfg<RP, true>::STAGES >= Cfg<RP, false>::STAGES && Cfg<RP, true>::W_STAGES >= Cfg<RP, false>::W_STAGES;
+static_assert(kPushKeepsTheRings<64> && kPushKeepsTheRings<128> && kPushKeepsTheRings<256>, "the receive buffer takes stages from the rings");
 
 struct Params {
   const float* table;     // smoothing table (layout in quantize_math.cuh), or null (no smoothing)
@@ -137,7 +142,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ack_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   uint32_t* lora_unfit = tmem_slot + 2;        // bf16 form: some LoRA value this CTA wrote does not fit fp16 (one rank: a bit per 32 rows)
-  float4* recv = reinterpret_cast<float4*>(smem + C::BARS_OFF + 512);        // [32 rows][RP / 4], slots as partial_slot; PUSH: [rank][share]
+  float4* recv = reinterpret_cast<float4*>(smem + C::BARS_OFF + 512);        // [32 rows][RP / 4], slots as partial_slot; PUSH: [following rank][share]
   const WaitCtx ctx{abort_flag};
 
   // warp index through a shuffle: provably warp-uniform, so the role branches are convergent code
@@ -460,7 +465,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
         if (static_cast<uint32_t>(qw) + 1 < ks) {
           copy_lo = share_begin(to);
           copy_bytes = (share_begin(to + 1) - copy_lo) * 16u;
-          copy_to = map_to_cta(smem_u32(recv + krank * share), to);
+          copy_to = map_to_cta(smem_u32(recv + (ks - 2 - qw) * share), to);      // seen from there, this rank is number ks - 1 - qw after it
           copy_bar = map_to_cta(smem_u32(recv_bar), to);
         }
         row_first = first / row4;
@@ -513,13 +518,9 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
             if (c >= static_cast<uint32_t>(p.R)) continue;
             // this rank's part first, then the following ranks' in turn: a fixed order for every element
             float4 acc = stage[item];
-            auto add_ranks = [&](uint32_t r, uint32_t r_end) {
-              const float4* part = recv + r * share + (item - item_lo);
+            const float4* part = recv + (item - item_lo);
 #pragma unroll 4
-              for (; r < r_end; ++r, part += share) { const float4 t = *part; acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w; }
-            };
-            add_ranks(krank + 1, ks);
-            add_ranks(0, krank);
+            for (uint32_t r = 1; r < ks; ++r, part += share) { const float4 t = *part; acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w; }
             const size_t idx = static_cast<size_t>(m0 + row) * p.R + c;
             *reinterpret_cast<float4*>(p.lora + idx) = acc;
             if (p.lora16 != nullptr) {

@@ -18,6 +18,15 @@ def test_cluster_splits_match_oracle(M, slabs, R, dtype):
     _check(x, ld, sm, FUSED)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,slabs,R", [(256, 160, 256), (700, 100, 136), (1500, 44, 200), (300, 240, 128), (1003, 75, 64)])
+def test_cluster_splits_over_many_ring_revolutions(M, slabs, R, dtype):
+    """Every rank's share of K goes round both rings several times, at ranks of all three widths and with receive buffers
+    whose shares do and do not divide evenly."""
+    x, ld, sm = _inputs(M, 64 * slabs, R, dtype, M + slabs)
+    _check(x, ld, sm, FUSED)
+
+
 def test_cluster_split_is_deterministic():
     from svdquant_kernels_b200 import ops
     x, ld, sm = _inputs(256, 3840, 128, torch.float16, 3)
