@@ -172,14 +172,6 @@ struct Params {
   uint8_t* oscales_swz;
 };
 
-__device__ __forceinline__ uint32_t pack2(__half a, __half b) {
-  __half2 h = __halves2half2(a, b);
-  return *reinterpret_cast<uint32_t*>(&h);
-}
-__device__ __forceinline__ uint32_t pack2(__nv_bfloat16 a, __nv_bfloat16 b) {
-  __nv_bfloat162 h = __halves2bfloat162(a, b);
-  return *reinterpret_cast<uint32_t*>(&h);
-}
 template <typename T> __device__ __forceinline__ uint32_t pack2f(float a, float b);
 template <> __device__ __forceinline__ uint32_t pack2f<__half>(float a, float b) {
   __half2 h = __floats2half2_rn(a, b);
@@ -189,9 +181,6 @@ template <> __device__ __forceinline__ uint32_t pack2f<__nv_bfloat16>(float a, f
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
 }
-template <typename T> __device__ __forceinline__ T from_f32(float v);
-template <> __device__ __forceinline__ __half from_f32<__half>(float v) { return __float2half_rn(v); }
-template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 template <typename T> __device__ __forceinline__ float as_f32(T v);
 template <> __device__ __forceinline__ float as_f32<__half>(__half v) { return __half2float(v); }
 template <> __device__ __forceinline__ float as_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
