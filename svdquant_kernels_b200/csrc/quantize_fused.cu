@@ -213,17 +213,26 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     }
   }
 
+  // Out-of-range smooth anywhere in K (flag word behind the table) selects the IEEE divide by the factors.  Asked for where it is
+  // out of the way of the first loads: as a condition of those it stood, 0.7 us, in front of everything.  So the first round of
+  // the ring holds reciprocals in any case and a flagged launch reads that round's factors where they are, which makes it slower
+  // than with factors in the ring throughout (4352 rows, x 3840 22.2 us instead of 20.2, x 10240 48 / 44.6, x 15360 69 / 66; with
+  // every round's factors read from global memory 25.4 / 59 / 87).
+  auto table_flagged = [&]() -> bool { return has_table && *reinterpret_cast<const volatile uint32_t*>(p.table + 2 * p.K) != 0u; };
+
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
     const uint32_t stage_bytes = X_BYTES + (has_table ? TB_BYTES : 0);
+    const float* table = p.table;              // reciprocals; a flagged launch (below): factors, from the second round of the ring on
     for (int i = 0; i < my_slabs; ++i) {
       const uint32_t s = i % C::STAGES, ph = (i / C::STAGES) & 1;
       if (!uwait(&empty[s], ph ^ 1, kDevWaitEmpty, i)) break;
+      if (i == C::STAGES && table_flagged()) table += p.K;
       const int k0 = k_begin + i * SLAB_K;
       if (elect_one()) {
         mbar_arrive_expect_tx(&full[s], stage_bytes);
         tma_load_2d(smem + s * X_BYTES, &tmX, k0, m0, &full[s]);
-        if (has_table) bulk_load_1d(smem + C::TB_OFF + s * TB_BYTES, p.table + k0, TB_BYTES, &full[s]);
+        if (has_table) bulk_load_1d(smem + C::TB_OFF + s * TB_BYTES, table + k0, TB_BYTES, &full[s]);
       }
       __syncwarp();
     }
@@ -293,9 +302,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     const int row_base = 16 * wq + (lane >> 2);
     const int groups = p.K >> 4;
     uint8_t* const act_base = p.act + static_cast<size_t>(m0) * (p.K >> 1);
-    // Out-of-range smooth anywhere in K (flag word behind the table) selects the IEEE divide.  Only these warps look at it,
-    // while their first slab is on its way: as a condition of the table's loads it stood, 0.7 us, in front of everything.
-    const bool use_fdiv = has_table && *reinterpret_cast<const volatile uint32_t*>(p.table + 2 * p.K) != 0u;
+    const bool use_fdiv = table_flagged();     // while the first slab is on its way
     for (int i = grp; i < my_slabs; i += QUANT_GROUPS) {
       const uint32_t s = i % C::STAGES, ph = (i / C::STAGES) & 1;
       if (!mbar_wait(&full[s], ph, ctx, kDevWaitFull, 0x10000 + i)) break;
@@ -312,9 +319,9 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       if (has_table) {
         unpack_group<T, false>(raw[0][0], raw[0][1], f[0]);
         unpack_group<T, false>(raw[1][0], raw[1][1], f[1]);
-        // this lane's 16 columns' reciprocals landed with the slab; a flagged launch reads the factors where they are
+        // this lane's 16 columns' reciprocals, or factors, landed with the slab
         if (!use_fdiv) qmath::smooth_multiply2(f[0], f[1], reinterpret_cast<const float4*>(smem + C::TB_OFF + s * TB_BYTES) + g);
-        else qmath::smooth_divide2(f[0], f[1], reinterpret_cast<const float4*>(p.table + p.K + k_begin + i * SLAB_K) + g);
+        else qmath::smooth_divide2(f[0], f[1], (i < C::STAGES ? reinterpret_cast<const float4*>(p.table + p.K + k_begin + i * SLAB_K) : reinterpret_cast<const float4*>(smem + C::TB_OFF + s * TB_BYTES)) + g);
       } else {
         unpack_group<T, true>(raw[0][0], raw[0][1], f[0]);
         unpack_group<T, true>(raw[1][0], raw[1][1], f[1]);

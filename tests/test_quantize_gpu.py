@@ -263,6 +263,16 @@ def test_signed_zeros_and_negative_smooth(dtype, smooth_kind):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,slabs,R", [(2400, 40, 128), (2400, 28, 256), (1003, 110, 64), (300, 150, 256), (64, 5, 16)])
+def test_out_of_range_smooth_over_many_ring_rounds(M, slabs, R, dtype):
+    """Smoothing factors outside the multiplications' domain: the first round of the x ring carries reciprocals that a
+    flagged launch must not use, the later ones the factors; two and more K ranks, rings of eight to sixteen stages."""
+    x, ld, sm = _inputs(M, 64 * slabs, R, dtype, M + slabs)
+    sm[::37] *= -1.0
+    _check(x, ld, sm, FUSED)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_no_rows_and_strided_input(dtype):
     """An input without rows gives empty outputs of the right shapes and types and launches nothing
     that fails; a non-contiguous view of x is quantised like its contiguous copy."""
@@ -329,8 +339,8 @@ def test_cluster_capacity_query():
 @pytest.mark.parametrize("M,K", [(256, 3840), (1024, 2560), (2304, 1024)])
 def test_fits_fp16_words_are_exact_for_every_split(M, K):
     """bf16: the word per 32 rows that tells the GEMM whether lora_act fits fp16 there.  Few rows run with
-    four or eight CTAs per row tile, whose verdicts on a shared 32-row block are gathered through
-    distributed shared memory; many rows with two.  Rows 40-49 and the last 20 rows are blown up past
+    up to sixteen CTAs per row tile, the first of which clears a 32-row block's word before any of them may set
+    it; many rows with two.  Rows 40-49 and the last 20 rows are blown up past
     65504, everything else fits: exactly those blocks must be marked."""
     dtype, R = torch.bfloat16, 64
     g = torch.Generator().manual_seed(77 + M)
