@@ -594,8 +594,13 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       // Long K loops over weights that come from DRAM: a CTA that is here while the kernel ahead is still at work (the quantizer
       // leaves half of the SMs to half of these CTAs) asks for its slabs of them, into L2, until that has ended.  Not before a
       // moment has passed, and at a pace, or the hints stand in the copy engine in front of the loads: without either, and in
-      // every form, 256 x 15360 -> 3840 took 25.3 us instead of 23.8 for both kernels; this way 22.4 instead of 22.8, 256 x
-      // 10240 -> 3072 16.1 instead of 16.2, while forms with a short K loop gain nothing (256 x 3840 -> 3072 11.7 -> 11.8).
+      // every form, 256 x 15360 -> 3840 took 25.3 us instead of 23.8 for both kernels, and forms with a short K loop gain
+      // nothing this way either (256 x 3840 -> 3072 11.7 -> 11.8).  Both kernels without / with the hints, us, over eight to
+      // twelve sets of weights, more than L2 holds, as in a model whose layers run in turn: 256 x 15360 -> 3840 22.58 / 22.40,
+      // -> 3072 22.28 / 21.89, -> 1536 17.52 / 17.48, 256 x 12800 -> 4608 20.31 / 20.31, 256 x 10240 -> 3072 16.69 / 16.35, 256 x
+      // 7680 -> 2304 14.85 / 14.89, 512 x 12288 -> 1536 20.01 / 19.76, 768 x 6592 -> 512 14.58 / 14.48; none of the other splits
+      // lost either.  Weights that are in L2 already have nothing to gain, and pay for it: over two sets 22.26 / 22.27, 21.58 /
+      // 21.7, 16.39 / 16.48, 19.5 / 19.6, 15.72 / 15.82, 13.72 / 13.96, 19.24 / 19.4, 13.84 / 13.88.
       __nanosleep(300);
       const int tile = tile_of(pair), nb = tile / p.tiles_m;
       int lo, hi;

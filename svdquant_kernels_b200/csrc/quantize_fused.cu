@@ -20,7 +20,7 @@
 // shared memory; more: every rank's share of the tile): no atomics, no zero-fill, no scratch in global
 // memory.  Large inputs run with KS = 2; larger clusters are for inputs of
 // a few hundred to two thousand rows, where pairs would leave most SMs idle (256 x 10240:
-// 36.0 -> 5.8 us), and are taken only if all of them are resident at once.
+// 36.0 -> 5.8 us, rank 32), and are taken only if all of them are resident at once.
 // (64-row tiles with pairs, not 128-row tiles with quads: a B200 keeps
 // at most 33 four-CTA clusters of this size resident, one short of the 34 row
 // tiles of a 4352-row activation, while 68 pairs fit in one wave.  128-row tiles
@@ -261,7 +261,7 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     constexpr uint64_t kDescA = smem_desc_base(0, 1024, kSwizzle128B);               // x tile, K-major
     constexpr uint64_t kDescB = smem_desc_base(SLAB_K * 128, 1024, kSwizzle128B);    // lora_down slab, R-major (its own ring)
     // As many columns as the rank needs of the RP that a slab holds (what the accumulator's others hold is never used): at rank
-    // 32 half of the tensor core's time and of its reads of lora_down (256 x 10240 6.03 -> 5.92 us, 4352 x 10240 28.4 -> 28.2).
+    // 32 half of the tensor core's time and of its reads of lora_down (when it came, 256 x 10240 6.03 -> 5.92 us, 4352 x 10240 28.4 -> 28.2).
     const uint32_t idesc = idesc_f16(kBf16, kBf16, TILE_M, (static_cast<uint32_t>(p.R) + 15u) & ~15u, false, true);
     const int issuer = warp >> 1;                                  // 0 or 1
     const uint32_t acc = (has_lora ? tmem_base() : 0u) + issuer * RP;
@@ -320,8 +320,9 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
         unpack_group<T, false>(raw[0][0], raw[0][1], f[0]);
         unpack_group<T, false>(raw[1][0], raw[1][1], f[1]);
         // this lane's 16 columns' reciprocals, or factors, landed with the slab
-        if (!use_fdiv) qmath::smooth_multiply2(f[0], f[1], reinterpret_cast<const float4*>(smem + C::TB_OFF + s * TB_BYTES) + g);
-        else qmath::smooth_divide2(f[0], f[1], (i < C::STAGES ? reinterpret_cast<const float4*>(p.table + p.K + k_begin + i * SLAB_K) : reinterpret_cast<const float4*>(smem + C::TB_OFF + s * TB_BYTES)) + g);
+        const float4* landed = reinterpret_cast<const float4*>(smem + C::TB_OFF + s * TB_BYTES);
+        if (!use_fdiv) qmath::smooth_multiply2(f[0], f[1], landed + g);
+        else qmath::smooth_divide2(f[0], f[1], (i < C::STAGES ? reinterpret_cast<const float4*>(p.table + p.K + k_begin + i * SLAB_K) : landed) + g);
       } else {
         unpack_group<T, true>(raw[0][0], raw[0][1], f[0]);
         unpack_group<T, true>(raw[1][0], raw[1][1], f[1]);
@@ -455,8 +456,10 @@ quantize_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     // copy engine brings every rank its share of them, counted on that rank's barrier: one trip.  (Ranks that fetched their
     // shares themselves, behind a cluster barrier, took 0.8 us for the barrier and three trips of 0.4 us.  Now the
     // transfer is the bound, 30 KB into every CTA at some 16 bytes a cycle at rank 128; 16-byte st.async from the registers
-    // need no staging but arrive one by one: 5.8 instead of 6.0 us at rank 32, 6.5 instead of 5.8 at rank 128.  256 x 15360
-    // 9.6 -> 9.3 us, 256 x 10240 6.5 -> 6.1, 256 x 3840 5.9 -> 5.8.)
+    // need no staging but arrive one by one: 5.8 instead of 6.0 us at rank 32, 6.5 instead of 5.8 at rank 128.  When it came, 256 x
+    // 15360 9.6 -> 9.3 us, 256 x 10240 6.5 -> 6.1, 256 x 3840 5.9 -> 5.8; now 8.9, 5.8 and 5.6.)  A rank's share is cut out of the
+    // float4s as they lie here, so which rank adds an element, and with that the order of its sum, goes by R and the number of
+    // ranks; it is the same from call to call.
     float4* const stage = reinterpret_cast<float4*>(smem);
     if constexpr (PUSH) { __syncwarp(); cluster_wait(); }     // all ranks' barriers exist
     if (warp >= AUX_WARPS) {
@@ -595,8 +598,9 @@ __global__ void smooth_table_kernel(const T* __restrict__ smooth, float* __restr
 // tile would leave most SMs idle; they are taken only if all of them can be resident at once (max_clusters(ks):
 // clusters of that size the device can hold; 33 of four CTAs, 22 of six, 15 of eight, 11 of ten, 7 of sixteen).
 // Cost in slabs (0.24 us); the constants are the ways of bringing the LoRA partial sums together, which hardly depend
-// on the cluster size (256 x 3840: 4 / 6 / 8 / 10 / 16 CTAs 7.4 / 6.3 / 5.7 / 5.4 / 5.4 us; 256 x 15360: 8 / 16 CTAs
-// 11.2 / 8.6 us; 1003 x 3840: 2 / 4 / 6 CTAs 9.6 / 6.9 / 6.3 us, seven, which are not all resident, 10.9).
+// on the cluster size (256 x 3840: 4 / 6 / 8 / 10 / 16 CTAs 7.5 / 6.3 / 5.7 / 5.3 / 5.4 us; 256 x 15360: 8 / 12 / 16 CTAs
+// 11.4 / 9.4 / 8.7 us; 1003 x 3840, rank 64: 2 / 4 / 6 CTAs 10.5 / 6.5 / 6.1 us, seven, which are not all resident, 10.8; 2048 x
+// 3840: 2 / 3 / 4 CTAs 11.6 / 9.8 / 8.5).
 template <typename MaxClusters>
 static int pick_k_split(int M_pad, int K, MaxClusters max_clusters) {
   const int tiles = M_pad / qf::TILE_M;

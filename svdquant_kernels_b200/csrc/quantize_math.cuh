@@ -30,8 +30,8 @@
 // down to those (one AND, towards zero, the sign stays) leaves it on its side of all of them.  What is left and not on a
 // bound is off it by 2^-12 of it, far more than one multiplication by rcp(scale)(1 + 2^-21) errs, and a value on a bound
 // comes out above it: the conversion instruction of the product returns the reference's code.  (Exact floors of 4 v / 2^E,
-// rescaled by a second multiplication, took a slow conversion and a multiplication an element more: 15360 x 3840 fp32
-// 52.3 -> 51.6 us, the next layer's codes of 4352 x 1024 -> 3072 bf16, both kernels, 32.8 -> 30.0.)
+// rescaled by a second multiplication, took a slow conversion and a multiplication an element more: the next layer's codes of
+// 4352 x 1024 -> 3072 bf16, both kernels, 32.8 -> 30.0 us; packing, which memory bounds, takes the same time.)
 #pragma once
 
 #include "nvfp4_math.cuh"
